@@ -14,7 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libfrank_b200.so")
-SOURCES = ["api.cu", "ops.cu", "hodlr.cu"]
+SOURCES = ["api.cu", "ops.cu", "hodlr.cu", "recompress_f32.cu", "recompress_f64.cu", "recompress_batch_f32.cu",
+           "recompress_batch_f64.cu"]
 OBJDIR = os.path.join(LIBDIR, "obj")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -16,6 +16,18 @@
 #include <string>
 #include <vector>
 
+namespace frank {
+// The recompression kernels are compiled in translation units of their own
+// (recompress_*.cu), in parallel with this one.
+#define FRANK_RECOMP_EXTERN(T)                                                                                       \
+  extern template __global__ void k_recompress<T>(BlrView<T>, FactorWs<T>, int, int, int, double, int, int*, int,    \
+                                                  double*, int*, int, int, int);                                     \
+  extern template __global__ void k_recompress_b<T>(const SysDev<T>*, int);
+FRANK_RECOMP_EXTERN(double)
+FRANK_RECOMP_EXTERN(float)
+#undef FRANK_RECOMP_EXTERN
+}  // namespace frank
+
 using namespace frank;
 
 namespace {
@@ -167,7 +179,7 @@ template <typename T>
 FactorWs<T> factor_ws(frank_blr* p) {
   FactorWs<T> w;
   w.perm = p->perm; w.ipiv = p->ipiv;
-  w.Linv = static_cast<T*>(p->Linv); w.Uinv = static_cast<T*>(p->Uinv);
+  w.Linv = static_cast<T*>(p->Linv); w.Uinv = static_cast<T*>(p->Uinv); w.UinvT = nullptr;
   w.WL = static_cast<T*>(p->WL); w.WU = static_cast<T*>(p->WU);
   w.getrf_scratch = p->getrf_scratch;
   w.dscratch = p->dscratch; w.dscratch_stride = p->dstride;
@@ -276,37 +288,23 @@ int enqueue_factor(frank_blr* p, cudaStream_t s, bool timing = true) {
         H, W, ws, p->core_scale * p->eps, p->rscratch, p->rstride);
     ++launches;
   }
-  // explicit inverses of a step's diagonal factors, all column blocks in
-  // parallel; on the second stream right after the leaf getrf, except in a
+  // packed LU and explicit inverses of a step's diagonal factors, all column
+  // blocks in parallel; on the second stream right after the leaf getrf, except in a
   // replay with timing events (there on the main stream, serialised)
   auto trinv_on = [&](int step, cudaStream_t st) -> int {
-    const int cw = trinv_width(p->bmax);
-    const int nblk = (int)((p->off_h[step + 1] - p->off_h[step] + cw - 1) / cw);
+    const int w = leaf_width(p->bmax), np = (p->off_h[step + 1] - p->off_h[step] + w - 1) / w;
     if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, step, FLOP_TRINV, 0), st, cudaEventRecordExternal));
-    k_trinv<T><<<2 * nblk, TRINV_THREADS, (size_t)p->bmax * cw * sizeof(double), st>>>(W, ws, step, cw);
+    k_leaf_final<T><<<3 * np, leaf_threads(p->bmax), leaf_smem(p->bmax), st>>>(W, ws, step);
     if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, step, FLOP_TRINV, 1), st, cudaEventRecordExternal));
     ++launches;
     return FRANK_OK;
   };
   auto getrf_on_aux = [&](int step) -> int {
     if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, step, FLOP_GETRF, 0), s2, cudaEventRecordExternal));
-    {
-      // leaf LU as load / (panel, tiled trailing update) x panels / store
-      const int b = p->off_h[step + 1] - p->off_h[step];
-      k_getrf_load<T><<<64, GETRF_AUX_THREADS, 0, s2>>>(W, ws, step);
-      for (int jb = 0; jb < b; jb += 32) {
-        k_getrf_panel<T><<<1, GETRF_THREADS, 0, s2>>>(W, ws, step, jb);
-        const int m2 = b - jb - std::min(32, b - jb);
-        if (m2 > 0) {
-          const int nt = (m2 + 63) / 64;
-          k_getrf_trail<T><<<nt * nt, GETRF_AUX_THREADS, 0, s2>>>(W, ws, step, jb);
-          ++launches;
-        }
-        ++launches;
-      }
-      k_getrf_store<T><<<64, GETRF_AUX_THREADS, 0, s2>>>(W, ws, step);
-      launches += 1;
-    }
+    const int w = leaf_width(p->bmax), np = (p->off_h[step + 1] - p->off_h[step] + w - 1) / w;
+    for (int q = 0; q < np; ++q)
+      k_leaf_step<T><<<np, leaf_threads(p->bmax), leaf_smem(p->bmax), s2>>>(W, ws, step, q);
+    launches += np;
     if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, step, FLOP_GETRF, 1), s2, cudaEventRecordExternal));
     if (!timing) {
       const int rc2 = trinv_on(step, s2);
@@ -317,7 +315,6 @@ int enqueue_factor(frank_blr* p, cudaStream_t s, bool timing = true) {
   };
   int rc = getrf_on_aux(0);
   if (rc) return rc;
-  ++launches;   // the getrf load kernel
   for (int i = 0; i < p->nb; ++i) {
     CUDA_TRY(cudaStreamWaitEvent(s, p->getrf_done[i], 0));
     if (timing && (rc = trinv_on(i, s))) return rc;
@@ -358,7 +355,6 @@ int enqueue_factor(frank_blr* p, cudaStream_t s, bool timing = true) {
         CUDA_TRY(cudaStreamWaitEvent(s2, p->next_done[i], 0));
       }
       if ((rc = getrf_on_aux(i + 1))) return rc;
-      ++launches;   // the getrf load kernel
       if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, i, FLOP_DENSE, 0), sd, cudaEventRecordExternal));
       if (m > 1) {
         k_update_dense<T><<<(int)std::min<int64_t>((int64_t)mm * nbands, p->grid_dense), DUPD_THREADS, 0, sd>>>(
@@ -821,7 +817,7 @@ int create_impl(const frank_blr_desc* d, const double* points, int dim, frank_bl
   ALLOC(t, nb * bm * bm * ts); p->Uinv = t;
   ALLOC(t, nb * bm * bm * ts); p->WL = t;
   ALLOC(t, nb * bm * bm * ts); p->WU = t;
-  ALLOC(p->getrf_scratch, bm * bm + 32 * bm);
+  ALLOC(p->getrf_scratch, leaf_scratch((int)bm));
   // dscratch / rscratch are allocated at the first factorization (ensure_scratch),
   // so frank_blr_set_grid can size them for batched use first.
   ALLOC(t, p->n * 8 * ts); p->z = t;
@@ -876,14 +872,18 @@ int create_impl(const frank_blr_desc* d, const double* points, int dim, frank_bl
   cudaFuncSetAttribute(k_solve_scatter_cl<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, shs);
   cudaFuncSetAttribute(k_solve_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
   cudaFuncSetAttribute(k_solve_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-  cudaFuncSetAttribute(k_trinv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRINV_SMEM_MAX);
-  cudaFuncSetAttribute(k_trinv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRINV_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_step<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_final<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
   cudaFuncSetAttribute(k_recompress<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, RECOMP_SMEM_BYTES);
   cudaFuncSetAttribute(k_recompress<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, RECOMP_SMEM_BYTES);
   cudaFuncSetAttribute(k_recompress_b<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, RECOMP_SMEM_BYTES);
   cudaFuncSetAttribute(k_recompress_b<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, RECOMP_SMEM_BYTES);
-  cudaFuncSetAttribute(k_trinv_b<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRINV_SMEM_MAX);
-  cudaFuncSetAttribute(k_trinv_b<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRINV_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_step_b<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_step_b<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_final_b<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
+  cudaFuncSetAttribute(k_leaf_final_b<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
   cudaFuncSetAttribute(k_recompress_gram<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAM_SMEM_BYTES);
   cudaFuncSetAttribute(k_recompress_gram<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAM_SMEM_BYTES);
   *out = p;
@@ -1788,7 +1788,7 @@ int enqueue_factor_stepwise(frank_batch* B, cudaStream_t s) {
   };
   cudaStream_t s2 = B->aux;
   const int b = q->bmax;
-  const int cw = trinv_width(b);
+  const int np = (b + leaf_width(b) - 1) / leaf_width(b);
   const int rt = (b + PANEL_TILE - 1) / PANEL_TILE;
   const int band = std::min(q->dupd_band, b);
   const int nbands = (b + band - 1) / band;
@@ -1804,18 +1804,9 @@ int enqueue_factor_stepwise(frank_batch* B, cudaStream_t s) {
     k_truncate_lr_b<T><<<dim3(std::max(q->grid_recomp, q->grid_gram), 1, K), TRUNC_THREADS, 0, s>>>(S);
   auto getrf_step = [&](int step) -> int {
     const int Kz = active(step);
-    k_getrf_load_b<T><<<dim3(64, 1, Kz), GETRF_AUX_THREADS, 0, s2>>>(S, step);
-    for (int jb = 0; jb < b; jb += 32) {
-      k_getrf_panel_b<T><<<dim3(1, 1, Kz), GETRF_THREADS, 0, s2>>>(S, step, jb);
-      const int m2 = b - jb - std::min(32, b - jb);
-      if (m2 > 0) {
-        const int nt = (m2 + 63) / 64;
-        k_getrf_trail_b<T><<<dim3(nt * nt, 1, Kz), GETRF_AUX_THREADS, 0, s2>>>(S, step, jb);
-      }
-    }
-    k_getrf_store_b<T><<<dim3(64, 1, Kz), GETRF_AUX_THREADS, 0, s2>>>(S, step);
-    k_trinv_b<T><<<dim3(2 * ((b + cw - 1) / cw), 1, Kz), TRINV_THREADS, (size_t)b * cw * sizeof(double), s2>>>(
-        S, step, cw);
+    for (int p = 0; p < np; ++p)
+      k_leaf_step_b<T><<<dim3(np, 1, Kz), leaf_threads(b), leaf_smem(b), s2>>>(S, step, p);
+    k_leaf_final_b<T><<<dim3(3 * np, 1, Kz), leaf_threads(b), leaf_smem(b), s2>>>(S, step);
     CUDA_TRY(cudaEventRecord(B->ev_getrf[step], s2));
     return FRANK_OK;
   };
@@ -1970,41 +1961,6 @@ extern "C" int frank_batch_refine_device(frank_batch* B, const double* const* d_
   if (status) return fail(status, "a system of the batch reached maxit before the tolerance");
   return FRANK_OK;
 }
-
-#ifdef FRANK_PHASE_TIMING
-// Read and clear the recompression phase counters (timing builds only).
-extern "C" int frank_debug_getrf_cycles(unsigned long long* c8) {
-  CUDA_TRY(cudaMemcpyFromSymbol(c8, g_getrf_cycles, sizeof(unsigned long long) * 8));
-  unsigned long long z[8] = {0};
-  CUDA_TRY(cudaMemcpyToSymbol(g_getrf_cycles, z, sizeof(z)));
-  return FRANK_OK;
-}
-
-extern "C" int frank_debug_sub_cycles(unsigned long long* c16) {
-  CUDA_TRY(cudaMemcpyFromSymbol(c16, g_sub_cycles, sizeof(unsigned long long) * 16));
-  unsigned long long z[16] = {0};
-  CUDA_TRY(cudaMemcpyToSymbol(g_sub_cycles, z, sizeof(z)));
-  return FRANK_OK;
-}
-
-extern "C" int frank_debug_tlog(long long* out, unsigned long long* n) {
-  CUDA_TRY(cudaMemcpyFromSymbol(n, g_tlog_n, sizeof(unsigned long long)));
-  const unsigned long long k = *n < 200000 ? *n : 200000;
-  if (out) CUDA_TRY(cudaMemcpyFromSymbol(out, g_tlog, sizeof(long long) * 6 * k));
-  unsigned long long z = 0;
-  CUDA_TRY(cudaMemcpyToSymbol(g_tlog_n, &z, sizeof(z)));
-  return FRANK_OK;
-}
-
-extern "C" int frank_debug_phase_cycles(unsigned long long* cycles24, unsigned long long* count3) {
-  CUDA_TRY(cudaMemcpyFromSymbol(cycles24, g_phase_cycles, sizeof(unsigned long long) * 24));
-  CUDA_TRY(cudaMemcpyFromSymbol(count3, g_phase_count, sizeof(unsigned long long) * 3));
-  unsigned long long z[24] = {0};
-  CUDA_TRY(cudaMemcpyToSymbol(g_phase_cycles, z, sizeof(z)));
-  CUDA_TRY(cudaMemcpyToSymbol(g_phase_count, z, sizeof(unsigned long long) * 3));
-  return FRANK_OK;
-}
-#endif
 
 // ===========================================================================
 // Allocation-free dense getrf (frank_getrf_dense_noalloc).

@@ -13,6 +13,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 namespace frank {
 
 template <typename T>
@@ -34,46 +36,6 @@ struct BlrView {
   FRANK_D T* vt(int i, int j) const { return Vt + (int64_t)lslot[i * nb + j] * bmax * kcap; }
 };
 
-// Optional per-phase cycle counters of the recompression kernels (build with
-// -DFRANK_PHASE_TIMING; off by default).  Slots: [size class][phase], the
-// classes stacked sizes <= 64, <= 160 and larger.
-#ifdef FRANK_PHASE_TIMING
-__device__ unsigned long long g_getrf_cycles[8];
-#define GPHASE(k)                                                                           \
-  do {                                                                                      \
-    if (threadIdx.x == 0) {                                                                 \
-      const long long _t = clock64();                                                      \
-      atomicAdd(&g_getrf_cycles[(k)], (unsigned long long)(_t - _g_t0));                    \
-      _g_t0 = _t;                                                                           \
-    }                                                                                       \
-  } while (0)
-#define GPHASE_BEGIN() long long _g_t0 = clock64()
-#else
-#define GPHASE(k) do {} while (0)
-#define GPHASE_BEGIN() do {} while (0)
-#endif
-#ifdef FRANK_PHASE_TIMING
-__device__ unsigned long long g_phase_cycles[3][8];
-__device__ unsigned long long g_phase_count[3];
-#define PHASE_BEGIN() long long _ph_t0 = clock64(); int _ph_last = 0
-#define PHASE_MARK(cls, k)                                                                  \
-  do {                                                                                      \
-    if (threadIdx.x == 0) {                                                                 \
-      const long long _t = clock64();                                                      \
-      atomicAdd(&g_phase_cycles[(cls)][(k)], (unsigned long long)(_t - _ph_t0));            \
-      _ph_t0 = _t;                                                                          \
-    }                                                                                       \
-    (void)_ph_last;                                                                         \
-  } while (0)
-#else
-#define PHASE_BEGIN() do {} while (0)
-#define PHASE_MARK(cls, k) do {} while (0)
-#endif
-#ifdef FRANK_PHASE_TIMING
-__device__ unsigned long long g_tlog_n;
-__device__ long long g_tlog[200000][6];
-FRANK_D long long gtimer() { long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-#endif
 
 // Per-factorization workspace (device pointers).
 template <typename T>
@@ -82,9 +44,10 @@ struct FactorWs {
   int* ipiv;      // [nb][bmax]: LAPACK-style 0-based pivots per diagonal block
   T* Linv;        // [nb][bmax*bmax]: unit-lower inverse per diagonal block
   T* Uinv;        // [nb][bmax*bmax]: upper inverse per diagonal block
+  T* UinvT;       // its transpose, or null where the caller keeps none
   T* WL;          // [nb][bmax*bmax]: (S V)^T of column-panel blocks, by block row
   T* WU;          // [nb][bmax*bmax]: U S of row-panel blocks, by block column
-  double* getrf_scratch;  // bmax*bmax + 32*bmax
+  double* getrf_scratch;  // leaf_scratch(bmax) doubles (k_getrf: bmax*bmax + 32*bmax)
   double* dscratch;       // dense-update scratch, per CTA slot
   int64_t dscratch_stride;
   double* rscratch;       // recompression scratch, per CTA slot
@@ -187,7 +150,7 @@ constexpr int TRUNC_THREADS = 256;
 // assume (the on-device constructions produce them already).  One CTA per
 // block at a time; scratch per CTA: 2 (bmax + kcap) kcap + 3 kcap^2 doubles.
 constexpr int ORTH_THREADS = 256;
-__global__ void __launch_bounds__(ORTH_THREADS) k_orthonormalize_lr(BlrView<double> H, double* scratch,
+static __global__ void __launch_bounds__(ORTH_THREADS) k_orthonormalize_lr(BlrView<double> H, double* scratch,
                                                                    int64_t stride) {
   __shared__ double gsm[2 * 16 * 64];
   __shared__ double red[32];
@@ -482,13 +445,11 @@ __global__ void __launch_bounds__(GETRF_THREADS) k_getrf(BlrView<T> A, FactorWs<
   int* perm = ws.perm + (int64_t)i * A.bmax;
   T* Li = ws.Linv + (int64_t)i * A.bmax * A.bmax;
   T* Ui = ws.Uinv + (int64_t)i * A.bmax * A.bmax;
-  GPHASE_BEGIN();
   for (int64_t e = threadIdx.x; e < (int64_t)b * b; e += blockDim.x) {
     const int r = e % b, c = e / b;
     Wm[r + (int64_t)c * b] = double(Dp[r + (int64_t)c * ldA]);
   }
   __syncthreads();
-  GPHASE(0);
   int first_zero = -1;
   __shared__ double prow[32];          // pivot row of the panel, broadcast
   __shared__ double xrow[32];          // row exchanged with the pivot row
@@ -498,14 +459,12 @@ __global__ void __launch_bounds__(GETRF_THREADS) k_getrf(BlrView<T> A, FactorWs<
       const int z = getrf_panel_step(b, jb, Wm, Gp, piv, red, redi, gsm, tri, prow, xrow);
       if (z >= 0 && first_zero < 0) first_zero = z;
     }
-    GPHASE(1);
     const int m2 = b - jb - jn;
     if (m2 > 0)
       cta_gemm<double, GETRF_THREADS>(m2, m2, jn, -1.0, Wm + (jb + jn) + (int64_t)jb * b, b, false,
                                       Wm + jb + (int64_t)(jb + jn) * b, b, false, 1.0,
                                       Wm + (jb + jn) + (int64_t)(jb + jn) * b, b, gsm);
   }
-  GPHASE(3);
   if (threadIdx.x == 0) {
     atomicAdd(ws.flops + FLOP_GETRF, (unsigned long long)(2.0 / 3.0 * (double)b * b * b));
     if (first_zero >= 0) atomicCAS(ws.err + ERR_SINGULAR_STEP, 0, i + 1);
@@ -522,201 +481,415 @@ __global__ void __launch_bounds__(GETRF_THREADS) k_getrf(BlrView<T> A, FactorWs<
     Dp[r + (int64_t)c * ldA] = T(Wm[r + (int64_t)c * b]);
   }
   __syncthreads();
-  GPHASE(5);
 }
 
 // ---------------------------------------------------------------------------
-// K1 as separate launches (the factorization path): the same leaf LU, with
-// the trailing update of each 32-column panel spread over 64 x 64 tiles on
-// many CTAs instead of one.  Sequence for diagonal block i:
-//   k_getrf_load; for each panel: k_getrf_panel (one CTA: getrf_panel_step),
-//   k_getrf_trail (tiles); k_getrf_store.
-// Per element the same operations in the same order as k_getrf.
+// K1 as separate launches (the factorization path): the leaf LU of a b x b
+// diagonal block by column tiles of W, one CTA per tile and one launch per
+// panel.  Launch p: the CTA of tile p brings its tile up to date with panel
+// p - 1 (row interchanges by a gather, U12 by substitution, the trailing
+// product on the FP64 tensor pipe) and factors it as panel p, while the CTAs
+// of the later tiles do the same update; the CTA of tile p - 1 inverts that
+// panel's two W x W triangles for the explicit inverses below; earlier tiles
+// apply the interchanges if there were any.  The tile lives in shared memory,
+// the panel in registers (RPT rows of W entries per thread), rows are never
+// moved: each thread keeps the position its row has been exchanged to.  A
+// column step is two block barriers (the pivot search on integer halves of
+// |a|, then the pivot row by broadcast), ties broken toward the smallest
+// position as in idamax.  A chain of b column steps bounds the whole thing,
+// so what counts is the latency of a step: the previous scheme (one CTA with
+// six barriers per step, a serial triangle inverse and exchanges through L2,
+// and a second launch for the trailing tiles) took 96 us + 19 us per panel at
+// b = 256 and 118 us + 21 us at b = 512.
+// After the last panel, k_leaf_final stores the packed LU (tile CTAs) and
+// forms Linv and Uinv: one CTA per column block of W of each, the block of
+// the inverse in shared memory, right-looking over the row blocks -- multiply
+// by the inverted diagonal triangle, then one product updates every row
+// still to come -- so each of the b / W steps is two short products instead
+// of one long inner-product chain (320 us at b = 256, 870 us at b = 512
+// before).
 // ---------------------------------------------------------------------------
-constexpr int GETRF_AUX_THREADS = 256;
+constexpr int LEAF_THREADS = 512;
+constexpr int LEAF_W = 32;            // panel width (b <= LEAF_THREADS)
+constexpr int LEAF_W_WIDE = 16;       // panel width of larger blocks (two rows per thread)
+constexpr int LEAF_WIDE_MAX = 1024;   // largest block order
 
-template <typename T>
-FRANK_D void k_getrf_load_impl(BlrView<T> A, FactorWs<T> ws, int i) {
-  const int b = A.bs(i), ld = A.bmax;
-  const T* Dp = A.dense(i, i);
-  double* Wm = ws.getrf_scratch;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)b * b;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int r = e % b, c = e / b;
-    Wm[r + (int64_t)c * b] = double(Dp[r + (int64_t)c * ld]);
-  }
+FRANK_HD int leaf_width(int b) { return b <= LEAF_THREADS ? LEAF_W : LEAF_W_WIDE; }
+// leading dimension of a tile in shared memory: 4 mod 16, so that the mma
+// fragments (4 rows of 4 columns per phase) fall into distinct banks
+FRANK_HD int leaf_lds(int b) { return ((b + 15) & ~15) + 4; }
+inline int leaf_threads(int b) { return b <= LEAF_THREADS ? std::max(128, (b + 31) & ~31) : LEAF_THREADS; }
+inline size_t leaf_smem(int b) { return (size_t)leaf_lds(b) * leaf_width(b) * sizeof(double); }
+constexpr int LEAF_SMEM_MAX = (LEAF_THREADS + 4) * LEAF_W * (int)sizeof(double);
+static_assert((LEAF_WIDE_MAX + 4) * LEAF_W_WIDE <= (LEAF_THREADS + 4) * LEAF_W, "tile sizes");
+// doubles of FactorWs::getrf_scratch: the working matrix, the inverted
+// diagonal triangles, the row maps of two panels and the exchange flags
+inline int64_t leaf_scratch(int bmax) { return (int64_t)bmax * bmax + 66 * (int64_t)bmax + 4096; }
+
+struct LeafScratch {
+  double* Wm;     // b x b (ld b)
+  double* dinv;   // per panel: Linv (W x W, ld W), Uinv
+  int* src;       // [2][bmax]: row at position r before the panel's exchanges
+  int* moved;     // [panels]: whether the panel exchanged any rows
+};
+
+template <int W>
+FRANK_D LeafScratch leaf_view(double* base, int bmax) {
+  LeafScratch s;
+  const int npmax = (bmax + W - 1) / W;
+  s.Wm = base;
+  s.dinv = base + (int64_t)bmax * bmax;
+  s.src = reinterpret_cast<int*>(s.dinv + (int64_t)npmax * 2 * W * W);
+  s.moved = s.src + 2 * bmax;
+  return s;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_load(BlrView<T> A, FactorWs<T> ws, int i) {
-  k_getrf_load_impl<T>(A, ws, i);
+struct LeafShared {
+  double tri[LEAF_W * (LEAF_W + 1)];
+  double prow[LEAF_W];
+  uint4 cand[LEAF_THREADS / 32];
+};
+
+// Largest |a| among the lanes' candidates with ties toward the smallest
+// position, as (high word, low word, position) in every lane: the bits of
+// non-negative doubles are ordered like unsigned integers, so three integer
+// warp reductions replace ten 64-bit shuffles.  pos = ~0u: no candidate.
+FRANK_D uint4 warp_pivot(unsigned hi, unsigned lo, unsigned pos) {
+  const bool on = pos != ~0u;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, on ? hi : 0u);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, on && hi == mh ? lo : 0u);
+  const unsigned mp = __reduce_min_sync(0xffffffffu, on && hi == mh && lo == ml ? pos : ~0u);
+  return make_uint4(mh, ml, mp, 0u);
 }
 
-template <typename T>
-FRANK_D void k_getrf_panel_impl(BlrView<T> A, FactorWs<T> ws, int i, int jb) {
-  __shared__ double red[32];
-  __shared__ int redi[32];
-  __shared__ double gsm[2 * 16 * 64];
-  __shared__ double tri[32 * 33];
-  __shared__ double prow[32];
-  __shared__ double xrow[32];
-  const int b = A.bs(i);
-  if (jb >= b) return;
-  double* Wm = ws.getrf_scratch;
-  double* Gp = Wm + (int64_t)A.bmax * A.bmax;
-  int* piv = ws.ipiv + (int64_t)i * A.bmax;
-  const int z = getrf_panel_step(b, jb, Wm, Gp, piv, red, redi, gsm, tri, prow, xrow);
-  if (z >= 0 && threadIdx.x == 0) atomicCAS(ws.err + ERR_SINGULAR_STEP, 0, i + 1);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(GETRF_THREADS) k_getrf_panel(BlrView<T> A, FactorWs<T> ws, int i, int jb) {
-  k_getrf_panel_impl<T>(A, ws, i, jb);
-}
-
-template <typename T>
-FRANK_D void k_getrf_trail_impl(BlrView<T> A, FactorWs<T> ws, int i, int jb) {
-  __shared__ double gsm[2 * 16 * 64];
-  const int b = A.bs(i);
-  if (jb >= b) return;
-  const int jn = min(32, b - jb), m2 = b - jb - jn;
-  if (m2 <= 0) return;
-  double* Wm = ws.getrf_scratch;
-  const int nt = (m2 + 63) / 64;
-  for (int tile = blockIdx.x; tile < nt * nt; tile += gridDim.x) {
-    const int r0 = (tile / nt) * 64, c0 = (tile % nt) * 64;
-    const int rn = min(64, m2 - r0), cn = min(64, m2 - c0);
-    cta_gemm<double, GETRF_AUX_THREADS>(rn, cn, jn, -1.0, Wm + (jb + jn + r0) + (int64_t)jb * b, b, false,
-                                        Wm + jb + (int64_t)(jb + jn + c0) * b, b, false, 1.0,
-                                        Wm + (jb + jn + r0) + (int64_t)(jb + jn + c0) * b, b, gsm);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_trail(BlrView<T> A, FactorWs<T> ws, int i, int jb) {
-  k_getrf_trail_impl<T>(A, ws, i, jb);
-}
-
-template <typename T>
-FRANK_D void k_getrf_store_impl(BlrView<T> A, FactorWs<T> ws, int i) {
-  const int b = A.bs(i), ld = A.bmax;
-  T* Dp = A.dense(i, i);
-  const double* Wm = ws.getrf_scratch;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    atomicAdd(ws.flops + FLOP_GETRF, (unsigned long long)(2.0 / 3.0 * (double)b * b * b));
-    const int* piv = ws.ipiv + (int64_t)i * ld;
-    int* perm = ws.perm + (int64_t)i * ld;
-    // permutation from the interchanges: (P B)[r] = B[perm[r]]
-    for (int r = 0; r < b; ++r) perm[r] = r;
-    for (int r = 0; r < b; ++r) {
-      const int p = piv[r];
-      const int t = perm[r]; perm[r] = perm[p]; perm[p] = t;
-    }
-  }
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)b * b;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int r = e % b, c = e / b;
-    Dp[r + (int64_t)c * ld] = T(Wm[r + (int64_t)c * b]);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_store(BlrView<T> A, FactorWs<T> ws, int i) {
-  k_getrf_store_impl<T>(A, ws, i);
-}
-
-// ---------------------------------------------------------------------------
-// K1': explicit inverses of the factors of diagonal block i, Uinv = U^{-1} and
-// Linv = L^{-1} (L unit lower), in column blocks of width cw: CTA q < nblk
-// forms column block q of Uinv, CTA nblk + q column block q of Linv.  The
-// column blocks are independent, so all 2 * nblk CTAs run at once.  A CTA
-// keeps its b x cw block X of the inverse in shared memory (FP64) and sweeps
-// the 32-row blocks in substitution order (upper: from the diagonal up to
-// row 0; lower: from the diagonal down): acc = E - T(rb, solved) X(solved)
-// by a CTA GEMM, then X(rb) = T(rb, rb)^{-1} acc by warp substitution (one
-// warp per column, lane = row, the solved value broadcast by shuffle).  The
-// packed LU is read from the block (precision T).  (LAPACK dtrtri forms the
-// same inverse, by column blocks in sequence.)
-// ---------------------------------------------------------------------------
-constexpr int TRINV_THREADS = 256;
-
-// Column-block width for block order bmax: X (bmax x cw doubles) must fit in
-// shared memory beside the static arrays.
-inline int trinv_width(int bmax) { return bmax <= 640 ? 32 : 16; }
-constexpr int TRINV_SMEM_MAX = 640 * 32 * (int)sizeof(double);   // covers 1024 x 16 too
-
-template <typename T>
-FRANK_D void k_trinv_impl(BlrView<T> A, FactorWs<T> ws, int i, int cw) {
-  extern __shared__ double X[];        // b x cw (ld b), rows indexed absolutely
-  __shared__ double tri[32 * 33];
-  __shared__ double acc[32 * 32];
-  __shared__ double gsm[2 * 16 * 64];
-  const int b = A.bs(i), ld = A.bmax;
-  const T* LU = A.dense(i, i);
-  const int nblk = (b + cw - 1) / cw;
-  const bool upper = (int)blockIdx.x < nblk;
-  const int cb = upper ? blockIdx.x : blockIdx.x - nblk;
-  const int c0 = cb * cw, cn = min(cw, b - c0);
-  if (c0 >= b) return;
-  T* out = (upper ? ws.Uinv : ws.Linv) + (int64_t)i * ld * ld;
+// Column steps j0 .. j1-1 of a panel whose current column is a[.][0] and whose
+// NV first entries are live (the entries shift down by one per step).
+template <int W, int RPT, int NV>
+FRANK_D void leaf_columns(int m, int j0, int j1, int jn, double (&a)[RPT][W], unsigned (&pos)[RPT], unsigned& done,
+                          double* sm, int lds, int* piv, int jb, int& zero, LeafShared& sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int nrb = (b + 31) / 32;
-  // upper: rows at or above the last diagonal row c0+cn-1; lower: from c0 down
-  const int rb_first = upper ? (c0 + cn - 1) / 32 : c0 / 32;
-  const int rb_last = upper ? 0 : nrb - 1;
-  const int rb_step = upper ? -1 : 1;
-  for (int rb = rb_first;; rb += rb_step) {
-    const int r0 = rb * 32, rn = min(32, b - r0);
-    for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
-      const int r = e % 32, c = e / 32;
-      acc[e] = (r < rn && c < cn && r0 + r == c0 + c) ? 1.0 : 0.0;
-      tri[r + c * 33] = (r < rn && c < rn) ? double(LU[(r0 + r) + (int64_t)(r0 + c) * ld]) : 0.0;
-    }
-    __syncthreads();
-    if (upper) {
-      const int k0 = r0 + rn, kn = c0 + cn - k0;   // solved rows of X below this block
-      if (kn > 0)
-        cta_gemm<double, TRINV_THREADS>(rn, cn, kn, -1.0, LU + r0 + (int64_t)k0 * ld, ld, false, X + k0, b, false,
-                                        1.0, acc, 32, gsm);
-    } else {
-      const int k0 = c0, kn = r0 - c0;              // solved rows of X above this block
-      if (kn > 0)
-        cta_gemm<double, TRINV_THREADS>(rn, cn, kn, -1.0, LU + r0 + (int64_t)k0 * ld, ld, false, X + k0, b, false,
-                                        1.0, acc, 32, gsm);
-    }
-    __syncthreads();
-    for (int c = wid; c < cn; c += nw) {
-      double v = lane < rn ? acc[lane + c * 32] : 0.0;
-      if (upper) {
-        for (int t = rn - 1; t >= 0; --t) {
-          const double xt = __shfl_sync(0xffffffffu, v, t) / tri[t + t * 33];
-          if (lane == t) v = xt;
-          else if (lane < t) v -= tri[lane + t * 33] * xt;
-        }
-      } else {
-        for (int t = 0; t < rn; ++t) {
-          const double xt = __shfl_sync(0xffffffffu, v, t);
-          if (lane > t) v -= tri[lane + t * 33] * xt;
-        }
+  for (int jj = j0; jj < j1; ++jj) {
+    unsigned bh = 0u, bl = 0u, bp = ~0u;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int row = threadIdx.x + k * blockDim.x;
+      if (row < m && !((done >> k) & 1u)) {
+        const double v = fabs(a[k][0]);
+        const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+        if (bp == ~0u || h > bh || (h == bh && (l > bl || (l == bl && pos[k] < bp)))) { bh = h; bl = l; bp = pos[k]; }
       }
-      if (lane < rn) X[r0 + lane + (int64_t)c * b] = v;
+    }
+    const uint4 wc = warp_pivot(bh, bl, bp);
+    if (lane == 0) sh.cand[wid] = wc;
+    __syncthreads();
+    uint4 c = lane < nw ? sh.cand[lane] : make_uint4(0u, 0u, ~0u, 0u);
+    c = warp_pivot(c.x, c.y, c.z);
+    const unsigned p = c.z;
+    const bool nonzero = (c.x | c.y) != 0u;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int row = threadIdx.x + k * blockDim.x;
+      if (row >= m || ((done >> k) & 1u)) continue;
+      if (pos[k] == p) {
+        // the pivot row: broadcast, and final as row jj of U
+#pragma unroll
+        for (int x = 0; x < NV; ++x) {
+          sh.prow[x] = a[k][x];
+          if (jj + x < jn) sm[row + (jj + x) * lds] = a[k][x];
+        }
+        pos[k] = jj;
+        done |= 1u << k;
+      } else if (pos[k] == (unsigned)jj) {
+        pos[k] = p;
+      }
+    }
+    // 1 / |pivot| while the pivot row is on its way
+    const double ra = 1.0 / __hiloint2double((int)c.x, (int)c.y);
+    if (threadIdx.x == 0) {
+      piv[jj] = jb + (int)p;
+      if (!nonzero && zero < 0) zero = jb + jj;
     }
     __syncthreads();
-    if (rb == rb_last) break;
+    const double rcp = sh.prow[0] < 0.0 ? -ra : ra;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int row = threadIdx.x + k * blockDim.x;
+      const double l = nonzero ? a[k][0] * rcp : a[k][0];
+      if (row < m && !((done >> k) & 1u)) sm[row + jj * lds] = l;
+      const double lu = nonzero ? l : 0.0;
+#pragma unroll
+      for (int x = 1; x < NV; ++x) a[k][x - 1] = fma(-lu, sh.prow[x], a[k][x]);
+      a[k][NV - 1] = 0.0;
+    }
   }
-  // upper: rows below the last diagonal row are zero; lower: rows above c0
-  const int rlo = upper ? 0 : c0, rhi = upper ? c0 + cn : b;
-  for (int e = threadIdx.x; e < b * cn; e += blockDim.x) {
-    const int r = e % b, c = e / b;
-    out[r + (int64_t)(c0 + c) * ld] = (r >= rlo && r < rhi) ? T(X[r + (int64_t)c * b]) : T(0);
+}
+
+// Partial-pivoted LU of the panel in sm (m x jn, ld lds; rows jb .. b-1 of the
+// block, columns jb ..), written to Wm in pivoted order with its pivots, row
+// map, exchange flag and the running permutation perm.
+template <int W, int RPT>
+FRANK_D void leaf_panel(int b, int jb, double* sm, int lds, const LeafScratch& L, int par, int panel, int* piv,
+                        int* perm, int* err, int step, LeafShared& sh) {
+  const int m = b - jb, jn = min(W, m);
+  double a[RPT][W];
+  unsigned pos[RPT], done = 0u;
+  int zero = -1;
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int row = threadIdx.x + k * blockDim.x;
+    pos[k] = row;
+#pragma unroll
+    for (int c = 0; c < W; ++c) a[k][c] = (row < m && c < jn) ? sm[row + c * lds] : 0.0;
   }
-  if (threadIdx.x == 0 && blockIdx.x == 0)
-    atomicAdd(ws.flops + FLOP_GETRF, (unsigned long long)(2.0 / 3.0 * (double)b * b * b));
+  constexpr int Q = W / 4;
+  leaf_columns<W, RPT, W>(m, 0, min(jn, Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  leaf_columns<W, RPT, 3 * Q>(m, Q, min(jn, 2 * Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  leaf_columns<W, RPT, 2 * Q>(m, 2 * Q, min(jn, 3 * Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  leaf_columns<W, RPT, Q>(m, 3 * Q, min(jn, W), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  if (threadIdx.x == 0 && zero >= 0) atomicCAS(err + ERR_SINGULAR_STEP, 0, step + 1);
+  int mv = 0, pv[RPT];
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int row = threadIdx.x + k * blockDim.x;
+    pv[k] = 0;
+    if (row >= m) continue;
+    const int to = jb + (int)pos[k];
+    for (int c = 0; c < jn; ++c) L.Wm[to + (int64_t)(jb + c) * b] = sm[row + c * lds];
+    L.src[par * b + to] = jb + row;
+    pv[k] = jb == 0 ? row : perm[jb + row];
+    mv |= (int)pos[k] != row;
+  }
+  mv = __syncthreads_or(mv);
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int row = threadIdx.x + k * blockDim.x;
+    if (row < m) perm[jb + pos[k]] = pv[k];
+  }
+  if (threadIdx.x == 0) L.moved[panel] = mv;
+}
+
+// Inverses of the two W x W triangles of a factored panel (identity beyond
+// the block): a warp per column, lane = row, the solved value by shuffle.
+template <int W>
+FRANK_D void leaf_dinv(int b, int jb, const double* Wm, double* out, LeafShared& sh) {
+  const int jn = min(W, b - jb);
+  for (int e = threadIdx.x; e < W * W; e += blockDim.x) {
+    const int r = e % W, c = e / W;
+    sh.tri[r + c * (W + 1)] = (r < jn && c < jn) ? Wm[(jb + r) + (int64_t)(jb + c) * b] : (r == c ? 1.0 : 0.0);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int r = min(lane, W - 1);
+  const double rd = 1.0 / sh.tri[r + r * (W + 1)];
+  for (int c = wid; c < W; c += nw) {
+    double lo = r == c ? 1.0 : 0.0, up = lo;
+    for (int t = 0; t < W; ++t) {
+      const double xl = __shfl_sync(0xffffffffu, lo, t);
+      if (r > t) lo = fma(-sh.tri[r + t * (W + 1)], xl, lo);
+      const int s = W - 1 - t;
+      const double xu = __shfl_sync(0xffffffffu, up * rd, s);
+      if (r < s) up = fma(-sh.tri[r + s * (W + 1)], xu, up);
+      else if (r == s) up = xu;
+    }
+    if (lane < W) {
+      out[r + c * W] = lo;
+      out[W * W + r + c * W] = r <= c ? up : 0.0;
+    }
+  }
+  __syncthreads();
+}
+
+template <typename T, int W, int RPT>
+FRANK_D void leaf_step_body(const BlrView<T>& A, const FactorWs<T>& ws, int i, int p) {
+  extern __shared__ double lsm[];
+  __shared__ LeafShared sh;
+  const int b = A.bs(i), ld = A.bmax, np = (b + W - 1) / W, q = blockIdx.x;
+  if (p >= np || q >= np) return;
+  const LeafScratch L = leaf_view<W>(ws.getrf_scratch, A.bmax);
+  const int lds = leaf_lds(b);
+  const int c0 = q * W, cn = min(W, b - c0);
+  int* piv = ws.ipiv + (int64_t)i * ld;
+  int* perm = ws.perm + (int64_t)i * ld;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double* panel = lsm;
+  if (p == 0) {
+    const T* Dp = A.dense(i, i) + (int64_t)c0 * ld;
+    for (int c = wid; c < cn; c += nw) {
+#pragma unroll 4
+      for (int r = lane; r < b; r += 32) {
+        const double v = double(Dp[r + (int64_t)c * ld]);
+        if (q == 0) lsm[r + c * lds] = v;
+        else L.Wm[r + (int64_t)(c0 + c) * b] = v;
+      }
+    }
+    if (q != 0) return;
+    __syncthreads();
+  } else {
+    const int j0 = (p - 1) * W, m = b - j0, par = (p - 1) & 1;
+    const int* src = L.src + par * b;
+    if (q == p - 1) {
+      leaf_dinv<W>(b, j0, L.Wm, L.dinv + (int64_t)q * 2 * W * W, sh);
+      return;
+    }
+    const bool mv = L.moved[p - 1] != 0;
+    if (q < p - 1 && !mv) return;
+    // rows j0 .. b-1 of the tile, exchanged by panel p - 1
+    for (int r = threadIdx.x; r < m; r += blockDim.x) {
+      const double* w = L.Wm + (mv ? src[j0 + r] : j0 + r) + (int64_t)c0 * b;
+#pragma unroll 8
+      for (int c = 0; c < cn; ++c) lsm[r + c * lds] = w[(int64_t)c * b];
+    }
+    if (q < p - 1) {
+      __syncthreads();
+      for (int r = threadIdx.x; r < m; r += blockDim.x)
+        for (int c = 0; c < cn; ++c) L.Wm[(j0 + r) + (int64_t)(c0 + c) * b] = lsm[r + c * lds];
+      return;
+    }
+    for (int e = threadIdx.x; e < W * W; e += blockDim.x)
+      sh.tri[e % W + (e / W) * (W + 1)] = L.Wm[(j0 + e % W) + (int64_t)(j0 + e / W) * b];
+    __syncthreads();
+    // U12 = L11^{-1} A12 (panel p - 1 has W columns: only the last one can have fewer)
+    for (int c = wid; c < cn; c += nw) {
+      const int r = min(lane, W - 1);
+      double v = lsm[r + c * lds];
+      for (int t = 0; t < W - 1; ++t) {
+        const double x = __shfl_sync(0xffffffffu, v, t);
+        if (r > t) v = fma(-sh.tri[r + t * (W + 1)], x, v);
+      }
+      if (lane < W) {
+        lsm[r + c * lds] = v;
+        L.Wm[(j0 + r) + (int64_t)(c0 + c) * b] = v;
+      }
+    }
+    __syncthreads();
+    // trailing rows: -= L21 U12
+    warps_dgemm<4, 2>(wid, nw, m - W, cn, W, -1.0, L.Wm + (j0 + W) + (int64_t)j0 * b, 1, b, lsm, lds, 1, 1.0, lsm + W,
+                      lds);
+    __syncthreads();
+    if (q > p) {
+      for (int c = wid; c < cn; c += nw)
+        for (int r = W + lane; r < m; r += 32) L.Wm[(j0 + r) + (int64_t)(c0 + c) * b] = lsm[r + c * lds];
+      return;
+    }
+    panel = lsm + W;
+  }
+  leaf_panel<W, RPT>(b, p * W, panel, lds, L, p & 1, p, piv, perm, ws.err, i, sh);
+  if (p == np - 1) {
+    __syncthreads();
+    leaf_dinv<W>(b, p * W, L.Wm, L.dinv + (int64_t)p * 2 * W * W, sh);
+  }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(TRINV_THREADS) k_trinv(BlrView<T> A, FactorWs<T> ws, int i, int cw) {
-  k_trinv_impl<T>(A, ws, i, cw);
+FRANK_D void k_leaf_step_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i, int p) {
+  if (A.bmax <= LEAF_THREADS) leaf_step_body<T, LEAF_W, 1>(A, ws, i, p);
+  else leaf_step_body<T, LEAF_W_WIDE, 2>(A, ws, i, p);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(LEAF_THREADS) k_leaf_step(BlrView<T> A, FactorWs<T> ws, int i, int p) {
+  k_leaf_step_impl<T>(A, ws, i, p);
+}
+
+// CTA q < np: the packed LU of tile q back into the block.  CTA np + cb
+// (np <= blockIdx.x < 2 np): column block cb of Linv; 2 np + cb: of Uinv (and
+// of its transpose, where the caller keeps one).
+template <typename T, int W>
+FRANK_D void leaf_final_body(const BlrView<T>& A, const FactorWs<T>& ws, int i) {
+  extern __shared__ double X[];        // b x W (ld lds)
+  const int b = A.bs(i), ld = A.bmax, np = (b + W - 1) / W;
+  const LeafScratch L = leaf_view<W>(ws.getrf_scratch, A.bmax);
+  const int lds = leaf_lds(b);
+  const int which = blockIdx.x / np, cb = blockIdx.x % np;
+  if (which > 2) return;
+  const int c0 = cb * W, cn = min(W, b - c0);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int jl = (np - 1) * W;                         // first row of the last panel
+  const int* src = L.src + ((np - 1) & 1) * b;         // its exchanges, not yet applied to the earlier tiles
+  if (which == 0) {
+    T* Dp = A.dense(i, i) + (int64_t)c0 * ld;
+    for (int c = wid; c < cn; c += nw)
+#pragma unroll 4
+      for (int r = lane; r < b; r += 32)
+        Dp[r + (int64_t)c * ld] = T(L.Wm[(r >= jl && cb < np - 1 ? src[r] : r) + (int64_t)(c0 + c) * b]);
+    if (threadIdx.x == 0 && cb == 0)
+      atomicAdd(ws.flops + FLOP_GETRF, 2 * (unsigned long long)(2.0 / 3.0 * (double)b * b * b));
+    return;
+  }
+  const bool lower = which == 1;
+  const int rlo = lower ? c0 : 0, rhi = lower ? b : c0 + cn;   // rows that are not zero
+  for (int c = wid; c < W; c += nw)
+    for (int r = rlo + lane; r < rhi; r += 32) X[r + c * lds] = r == c0 + c ? 1.0 : 0.0;
+  __syncthreads();
+  const int g = lane >> 2, t = lane & 3;
+  for (int rb = cb; lower ? rb < np : rb >= 0; rb += lower ? 1 : -1) {
+    const int r0 = rb * W, rn = min(W, b - r0);
+    const double* D = L.dinv + (int64_t)rb * 2 * W * W + (lower ? 0 : W * W);
+    // X(rb) <- T(rb, rb)^{-1} X(rb): one 8 x 8 tile per warp and pass, all read before any is written
+    constexpr int TW = W / 8;
+    double acc[(TW * TW + 3) / 4][2];                   // at least four warps
+    int nt = 0;
+    for (int tile = wid; tile < TW * TW; tile += nw, ++nt) {
+      double c1[1][1][2];
+      warp_dgemm_acc<1, 1>(rn, cn, 0, rn, D, 1, W, X + r0, lds, 1, (tile % TW) * 8, (tile / TW) * 8, c1);
+#pragma unroll
+      for (int z = 0; z < (TW * TW + 3) / 4; ++z)
+        if (z == nt) { acc[z][0] = c1[0][0][0]; acc[z][1] = c1[0][0][1]; }
+    }
+    __syncthreads();
+    nt = 0;
+    for (int tile = wid; tile < TW * TW; tile += nw, ++nt) {
+      const int r = (tile % TW) * 8 + g, c = (tile / TW) * 8 + 2 * t;
+#pragma unroll
+      for (int z = 0; z < (TW * TW + 3) / 4; ++z)
+        if (z == nt && r < rn) {
+          if (c < cn) X[r0 + r + c * lds] = acc[z][0];
+          if (c + 1 < cn) X[r0 + r + (c + 1) * lds] = acc[z][1];
+        }
+    }
+    __syncthreads();
+    // every row still to come: X(r) -= T(r, rb) X(rb)
+    const int u0 = lower ? r0 + W : 0, um = lower ? b - u0 : r0;
+    const int tm = (um + 31) / 32, tn = (cn + 15) / 16;
+    for (int tile = wid; um > 0 && tile < tm * tn; tile += nw) {
+      const int i0 = (tile % tm) * 32, j0 = (tile / tm) * 16;
+      double ac[4][2][2];
+      warp_dgemm_acc<4, 2>(um, cn, 0, rn, L.Wm + (int64_t)r0 * b, 1, b, X + r0, lds, 1, i0, j0, ac, [&](int r) {
+        const int a = u0 + r;
+        return lower && a >= jl && rb < np - 1 ? src[a] : a;
+      });
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int r = i0 + 8 * x + g, c = j0 + 8 * y + 2 * t;
+          if (r < um && c < cn) X[u0 + r + c * lds] -= ac[x][y][0];
+          if (r < um && c + 1 < cn) X[u0 + r + (c + 1) * lds] -= ac[x][y][1];
+        }
+    }
+    __syncthreads();
+  }
+  T* out = (lower ? ws.Linv : ws.Uinv) + (int64_t)i * ld * ld + (int64_t)c0 * ld;
+  for (int c = wid; c < cn; c += nw)
+    for (int r = lane; r < b; r += 32) out[r + (int64_t)c * ld] = (r >= rlo && r < rhi) ? T(X[r + c * lds]) : T(0);
+  if (!lower && ws.UinvT) {
+    T* outt = ws.UinvT + (int64_t)i * ld * ld + c0;
+    for (int e = threadIdx.x; e < b * cn; e += blockDim.x) {
+      const int c = e % cn, r = e / cn;
+      outt[c + (int64_t)r * ld] = r < rhi ? T(X[r + c * lds]) : T(0);
+    }
+  }
+}
+
+template <typename T>
+FRANK_D void k_leaf_final_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i) {
+  if (A.bmax <= LEAF_THREADS) leaf_final_body<T, LEAF_W>(A, ws, i);
+  else leaf_final_body<T, LEAF_W_WIDE>(A, ws, i);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(LEAF_THREADS) k_leaf_final(BlrView<T> A, FactorWs<T> ws, int i) {
+  k_leaf_final_impl<T>(A, ws, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -1242,18 +1415,9 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
       if (threadIdx.x == 0) atomicAdd(ws.err + ERR_BOUNDS, 1);
       continue;
     }
-    const int cls = (su <= 64 && sv <= 64) ? 0 : (su <= 160 && sv <= 160 ? 1 : 2);
-    PHASE_BEGIN();
-#ifdef FRANK_PHASE_TIMING
-    const long long t_start = gtimer();
-#endif
-#ifdef FRANK_PHASE_TIMING
-    if (threadIdx.x == 0) atomicAdd(&g_phase_count[cls], 1ull);
-#endif
     T* Uc = A.u(ic, k);
     T* Sc = A.s(ic, k);
     T* Vc = A.vt(ic, k);
-    SUB_BEGIN();
     // stacked bases in FP64
     for (int64_t e = threadIdx.x; do_u && e < (int64_t)bc * su; e += blockDim.x) {
       const int r = e % bc, c = e / bc;
@@ -1270,10 +1434,7 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     // the stacked bases are read across threads below (the V side of a split
     // target forms no core, whose barrier would otherwise cover this)
     __syncthreads();
-    SUB_MARK(9);
     if (do_u) form_core<T, RECOMP_THREADS>(o, bi, ld, Tm, gsm);
-    SUB_MARK(10);
-    PHASE_MARK(cls, 0);
     // Bases.  Stacked (rounded_addition, addition.cpp:93-127): Householder QR
     // of [U_C | U_B] and of [V_C | V_B].  Projected (fast_rounded_addition,
     // addition.cpp:133-189, the default of fixed-rank plans, and on request
@@ -1290,7 +1451,6 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
                                         Xo, gsm);
         cta_qr_blocked<RECOMP_THREADS>(bc, o.p, Ash + (int64_t)kc * bc, bc, tau_u, Tfu, Wq, smP, smT, gsm, red);
       }
-      PHASE_MARK(cls, 1);
       if (do_v) {
         cta_project_out<RECOMP_THREADS>(bk, kc, o.q, Bsh, bk, Bsh + (int64_t)kc * bk, bk, Rv + (int64_t)kc * sv, sv,
                                         Yo, gsm);
@@ -1299,12 +1459,10 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
       }
     } else {
       if (do_u) cta_qr_blocked<RECOMP_THREADS>(bc, su, Ash, bc, tau_u, Tfu, Wq, smP, smT, gsm, red);
-      PHASE_MARK(cls, 1);
       // the V side of a split target works in Mtmp (free until the core), so
       // that the two sides never share the W scratch
       if (do_v) cta_qr_blocked<RECOMP_THREADS>(bk, sv, Bsh, bk, tau_v, Tfv, side == 1 ? Mtmp : Wq, smP, smT, gsm, red);
     }
-    PHASE_MARK(cls, 2);
     if (side >= 0) {
       // publish this side; the second of the two CTAs goes on with the target
       __threadfence();
@@ -1350,7 +1508,6 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     const bool in_smem = core_need <= RECOMP_REGION && (mu < 64 || core_need <= core_smem);
     double* Mm = in_smem ? region : Mg;
     cta_gemm<double, RECOMP_THREADS>(mu, mv, sv, 1.0, Mtmp, mu, false, Rv, mv, true, 0.0, Mm, mu, gsm);
-    PHASE_MARK(cls, 3);
     int r = 0;
     if (core_method == CORE_RRQR && ws.fixed_rank == 0) {
       double f = 0.0;
@@ -1455,7 +1612,6 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
       }
       __syncthreads();
     }
-    PHASE_MARK(cls, 4);
     if (threadIdx.x == 0)
       atomicAdd(ws.flops + FLOP_RECOMP,
                 (unsigned long long)(proj ? fast_rounded_addition_flops(bc, bk, bi, kc, o.p, o.q, r)
@@ -1499,16 +1655,6 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     }
     if (threadIdx.x == 0) A.rank[blk] = r;
     __syncthreads();
-    PHASE_MARK(cls, 5);
-#ifdef FRANK_PHASE_TIMING
-    if (threadIdx.x == 0) {
-      const unsigned long long q = atomicAdd(&g_tlog_n, 1ull);
-      if (q < 200000) {
-        g_tlog[q][0] = i; g_tlog[q][1] = su; g_tlog[q][2] = sv; g_tlog[q][3] = r;
-        g_tlog[q][4] = t_start; g_tlog[q][5] = gtimer();
-      }
-    }
-#endif
   }
 }
 
@@ -1629,11 +1775,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
     // small targets: warp-level factorizations in shared memory; large ones:
     // CTA-level factorizations
     const bool small = in_sm && su <= 64 && sv <= 64;
-    const int cls = small ? 0 : 1;
-    PHASE_BEGIN();
-#ifdef FRANK_PHASE_TIMING
-    if (threadIdx.x == 0) atomicAdd(&g_phase_count[cls], 1ull);
-#endif
     // T = -WL^T WU (p x q); Gram matrices of the stacked bases (upper blocks)
     // skinny products: warp dot products when small, tiled GEMM otherwise
     auto tn = [&](int mm_, int nn_, int kk_, double al, const T* Ap, const T* Bp, double* Cp, int ldc_) {
@@ -1656,7 +1797,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
       Gb[(kc + c) + (int64_t)r * sv] = Gb[r + (int64_t)(kc + c) * sv];
     }
     __syncthreads();
-    PHASE_MARK(cls, 0);
     // pivoted Cholesky of both Gram matrices (one warp each when small)
     if (small) {
       if (wid == 0) {
@@ -1672,7 +1812,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
       if (threadIdx.x == 0) { s_r[0] = r0; s_r[1] = r1; }
     }
     __syncthreads();
-    PHASE_MARK(cls, 1);
     const int ra = s_r[0], rb = s_r[1];
     // M1 = Pa^T blockdiag(S_C, T) Pb (su x sv); zero the lower parts of Ra, Rb
     for (int64_t e = threadIdx.x; e < (int64_t)su * sv; e += blockDim.x) {
@@ -1713,7 +1852,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
     f = block_sum(f, red);
     const double thr = ws.fixed_rank > 0 ? 0.0 : core_scale * ws.eps * sqrt(f);
     const int maxr = ws.fixed_rank > 0 ? min(ws.fixed_rank, A.kcap) : A.kcap;
-    PHASE_MARK(cls, 2);
     if (small) {
       if (wid == 0) {
         const int r_ = (ra > 0 && rb > 0) ? warp_truncated_geqp3(ra, rb, Core, ra, thr, maxr, tc, cn, pn, jp) : 0;
@@ -1725,7 +1863,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
       if (threadIdx.x == 0) s_r[2] = r_;
     }
     __syncthreads();
-    PHASE_MARK(cls, 3);
     const int r = s_r[2];
     if (r == 0) {
       T* Uw = A.u(ic, k); T* Vw = A.vt(ic, k); T* Sw = A.s(ic, k);
@@ -1812,7 +1949,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
       cta_upper_solve(ra, Ga, su, r, X1, ra);
       cta_upper_solve(rb, Gb, sv, r, Yk, rb);
     }
-    PHASE_MARK(cls, 4);
     // scatter to the stacked order: Xf (su x r) reuses M1, Yf (sv x r) M3
     double* Xf = M1;
     double* Yf = M3;
@@ -1852,7 +1988,6 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
       const int rr = e % bk, c = e / bk;
       Vw[rr + (int64_t)c * ld] = T(Tm[e]);
     }
-    PHASE_MARK(cls, 5);
     if (threadIdx.x == 0) A.rank[blk] = r;
     __syncthreads();
   }
@@ -2192,7 +2327,7 @@ FRANK_HD size_t matvec_smem(int bmax, int kcap, int nrhs) {
 
 // Each element of the block (U, S, V or the dense block) is read once and
 // applied to all nrhs columns of x_j, which is staged in shared memory.
-__global__ void __launch_bounds__(MV_THREADS) k_matvec_blocks(BlrView<double> H, const double* x, int64_t ldx,
+static __global__ void __launch_bounds__(MV_THREADS) k_matvec_blocks(BlrView<double> H, const double* x, int64_t ldx,
                                                               int nrhs, double* part, int transpose) {
   // part(i, j) = A(i, j) x_j, or A(j, i)^T x_j when transposing
   const int i = blockIdx.y, j = blockIdx.x;
@@ -2308,7 +2443,7 @@ __global__ void __launch_bounds__(MV_THREADS) k_matvec_blocks(BlrView<double> H,
 }
 
 // y_i = sum_j part(i,j) (fixed order).  If b != null: y = b - A x (residual).
-__global__ void k_matvec_reduce(BlrView<double> H, const double* part, int nrhs, const double* bvec, int64_t ldb,
+static __global__ void k_matvec_reduce(BlrView<double> H, const double* part, int nrhs, const double* bvec, int64_t ldb,
                                 double* y, int64_t ldy) {
   const int i = blockIdx.x;
   const int nb = H.nb, ld = H.bmax;
@@ -2324,7 +2459,7 @@ __global__ void k_matvec_reduce(BlrView<double> H, const double* part, int nrhs,
 }
 
 // column 2-norms squared of an n x nrhs matrix: per-CTA partials part[blk*nrhs + h]
-__global__ void k_colnorm2(const double* v, int64_t n, int64_t ldv, int nrhs, double* part) {
+static __global__ void k_colnorm2(const double* v, int64_t n, int64_t ldv, int nrhs, double* part) {
   __shared__ double red[32];
   for (int h = 0; h < nrhs; ++h) {
     double s = 0.0;
@@ -2347,7 +2482,7 @@ __global__ void k_cast_copy(const TS* src, int64_t lds, TD* dst, int64_t ldd, in
 
 // x += T(d)
 // y0 = alpha * y + beta * y0 over n x nrhs (both ld n)
-__global__ void k_axpby(double alpha, const double* y, double beta, double* y0, int64_t n, int nrhs) {
+static __global__ void k_axpby(double alpha, const double* y, double beta, double* y0, int64_t n, int nrhs) {
   const int64_t tot = n * nrhs;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x)
     y0[e] = alpha * y[e] + (beta == 0.0 ? 0.0 : beta * y0[e]);
@@ -2371,7 +2506,7 @@ __global__ void k_axpy_cast(const TS* d, int64_t ldd, double* x, int64_t ldx, in
 // ---------------------------------------------------------------------------
 constexpr int DT_TILE = 64;
 
-__global__ void __launch_bounds__(256) k_dtheta_contract(const double* x, int dim, int64_t n, double theta,
+static __global__ void __launch_bounds__(256) k_dtheta_contract(const double* x, int dim, int64_t n, double theta,
                                                           const double* lam, int64_t ldl, const double* xv,
                                                           int64_t ldx, int nrhs, double* partial) {
   __shared__ double pi[3][DT_TILE], pj[3][DT_TILE];
@@ -2433,7 +2568,7 @@ FRANK_D double kernel_eval(const KernelDesc& K, int64_t gi, int64_t gj) {
 }
 
 // Dense blocks of A_H: one CTA per dense block (listed in blocks[]).
-__global__ void k_build_dense(BlrView<double> H, KernelDesc K, const int* blocks, int nblocks) {
+static __global__ void k_build_dense(BlrView<double> H, KernelDesc K, const int* blocks, int nblocks) {
   for (int t = blockIdx.x; t < nblocks; t += gridDim.x) {
     const int blk = blocks[t];
     const int i = blk / H.nb, j = blk % H.nb;
@@ -2454,7 +2589,7 @@ __global__ void k_build_dense(BlrView<double> H, KernelDesc K, const int* blocks
 // scratch per CTA slot: A (b x b), Q (b x b), X (b x b), norms, pivots.
 constexpr int BUILD_THREADS = 512;
 
-__global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank(BlrView<double> H, KernelDesc K, const int* blocks,
+static __global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank(BlrView<double> H, KernelDesc K, const int* blocks,
                                                                  int nblocks, double eps, double* scratch,
                                                                  int64_t stride, int* err) {
   __shared__ double red[32];
@@ -2642,7 +2777,7 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank(BlrView<double>
 // on B^T with the rotations accumulated in p appended rows, U = Q Ub, then
 // truncation to `rank`.  One CTA per block, FP64 scratch slot per CTA:
 // A (b x b), Y / Q (b x p), Bt (b + p) x p, small vectors.
-__global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank_rsvd(BlrView<double> H, KernelDesc K,
+static __global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank_rsvd(BlrView<double> H, KernelDesc K,
                                                                       const int* blocks, int nblocks, int rank,
                                                                       int p, const double* omega_full,
                                                                       const double* omega_last, int64_t stride,
@@ -2764,42 +2899,17 @@ __global__ void __launch_bounds__(TRUNC_THREADS) k_truncate_lr_b(const SysDev<T>
 }
 
 template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_load_b(const SysDev<T>* S, int i) {
+__global__ void __launch_bounds__(LEAF_THREADS) k_leaf_step_b(const SysDev<T>* S, int i, int p) {
   const SysDev<T>& s = S[blockIdx.z];
   if (i >= s.W.nb) return;
-  k_getrf_load_impl<T>(s.W, s.ws, i);
+  k_leaf_step_impl<T>(s.W, s.ws, i, p);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(GETRF_THREADS) k_getrf_panel_b(const SysDev<T>* S, int i, int jb) {
-  const SysDev<T>& s = S[blockIdx.z];
-  if (i >= s.W.nb || jb >= s.W.bs(i)) return;
-  k_getrf_panel_impl<T>(s.W, s.ws, i, jb);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_trail_b(const SysDev<T>* S, int i, int jb) {
+__global__ void __launch_bounds__(LEAF_THREADS) k_leaf_final_b(const SysDev<T>* S, int i) {
   const SysDev<T>& s = S[blockIdx.z];
   if (i >= s.W.nb) return;
-  const int b = s.W.bs(i);
-  const int m2 = b - jb - min(32, b - jb);
-  const int nt = (m2 + 63) / 64;
-  if (m2 <= 0 || (int)blockIdx.x >= nt * nt) return;
-  k_getrf_trail_impl<T>(s.W, s.ws, i, jb);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(GETRF_AUX_THREADS) k_getrf_store_b(const SysDev<T>* S, int i) {
-  const SysDev<T>& s = S[blockIdx.z];
-  if (i >= s.W.nb) return;
-  k_getrf_store_impl<T>(s.W, s.ws, i);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(TRINV_THREADS) k_trinv_b(const SysDev<T>* S, int i, int cw) {
-  const SysDev<T>& s = S[blockIdx.z];
-  if (i >= s.W.nb || (int)blockIdx.x >= 2 * ((s.W.bs(i) + cw - 1) / cw)) return;
-  k_trinv_impl<T>(s.W, s.ws, i, cw);
+  k_leaf_final_impl<T>(s.W, s.ws, i);
 }
 
 template <typename T>

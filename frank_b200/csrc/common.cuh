@@ -133,17 +133,181 @@ FRANK_D int block_argmax_abs1(double v, int idx, double* redv, int* redi, double
 }
 
 // ---------------------------------------------------------------------------
+// FP64 products on the tensor pipe: mma.sync m8n8k4 (the FP64 matrix shape of
+// this chip; FP64 has no tcgen05 kind).  Its peak equals the FP64 FMA peak
+// (measured: one instruction per 16 cycles and scheduler, 26 cycles latency),
+// but one instruction does 8 FMAs per lane from one operand value each, so a
+// product needs neither shared-memory staging nor block barriers: each warp
+// reads its operand fragments where they lie (shared memory or L2, 8 rows of
+// 64 contiguous bytes or 32-byte runs per load) and keeps its tile in
+// registers, and four warps saturate an SM.
+// ---------------------------------------------------------------------------
+FRANK_D void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// acc (8 MI x 8 NI tile at (i0, j0)) = sum over kk in [k0, k1) of
+// A(i, kk) B(kk, j), A(i, kk) at A[row(i) sai + kk sak], B(kk, j) at B[j sbj + kk
+// sbk].  Rows / columns beyond m / n repeat the last one (never stored).
+// Lane l holds A(l / 4, l % 4), B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
+struct RowIdentity {
+  FRANK_D int operator()(int r) const { return r; }
+};
+
+template <int MI, int NI, typename TA, typename TB, typename RowMap = RowIdentity>
+FRANK_D void warp_dgemm_acc(int m, int n, int k0, int k1, const TA* A, int64_t sai, int64_t sak, const TB* B,
+                            int64_t sbj, int64_t sbk, int i0, int j0, double (&acc)[MI][NI][2],
+                            RowMap row = RowMap()) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const TA* pa[MI];
+  const TB* pb[NI];
+#pragma unroll
+  for (int i = 0; i < MI; ++i) pa[i] = A + (int64_t)row(min(i0 + 8 * i + g, m - 1)) * sai + (int64_t)(k0 + t) * sak;
+#pragma unroll
+  for (int j = 0; j < NI; ++j) pb[j] = B + (int64_t)min(j0 + 8 * j + g, n - 1) * sbj + (int64_t)(k0 + t) * sbk;
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  constexpr int U = MI * NI >= 8 ? 2 : 4;   // k-quads whose loads are in flight together
+  int kk = k0;
+  for (; kk + 4 * U <= k1; kk += 4 * U) {
+    double a[U][MI], b[U][NI];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int i = 0; i < MI; ++i) a[u][i] = double(pa[i][u * 4 * sak]);
+#pragma unroll
+      for (int j = 0; j < NI; ++j) b[u][j] = double(pb[j][u * 4 * sbk]);
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i) pa[i] += U * 4 * sak;
+#pragma unroll
+    for (int j = 0; j < NI; ++j) pb[j] += U * 4 * sbk;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[u][i], b[u][j]);
+  }
+  for (; kk < k1; kk += 4) {
+    const bool in = kk + t < k1;
+    double a[MI], b[NI];
+#pragma unroll
+    for (int i = 0; i < MI; ++i) { a[i] = in ? double(*pa[i]) : 0.0; pa[i] += 4 * sak; }
+#pragma unroll
+    for (int j = 0; j < NI; ++j) { b[j] = in ? double(*pb[j]) : 0.0; pb[j] += 4 * sbk; }
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[i], b[j]);
+  }
+}
+
+template <typename TC>
+FRANK_D void dgemm_store(TC* p, double v, double alpha, double beta) {
+  v *= alpha;
+  if (beta != 0.0) v += beta * double(*p);
+  *p = TC(v);
+}
+
+// One pass of the CTA's (or warp group's) warps over the 8 MI x 8 NI tiles.
+template <int MI, int NI, typename TA, typename TB, typename TC>
+FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, const TA* A, int64_t sai, int64_t sak,
+                         const TB* B, int64_t sbj, int64_t sbk, double beta, TC* C, int64_t ldc) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int tm = (m + 8 * MI - 1) / (8 * MI), tn = (n + 8 * NI - 1) / (8 * NI);
+  for (int tile = wid; tile < tm * tn; tile += nw) {
+    const int i0 = (tile % tm) * 8 * MI, j0 = (tile / tm) * 8 * NI;
+    double acc[MI][NI][2];
+    warp_dgemm_acc<MI, NI>(m, n, 0, k, A, sai, sak, B, sbj, sbk, i0, j0, acc);
+#pragma unroll
+    for (int i = 0; i < MI; ++i) {
+      const int r = i0 + 8 * i + g;
+      if (r >= m) continue;
+#pragma unroll
+      for (int j = 0; j < NI; ++j) {
+        const int c = j0 + 8 * j + 2 * t;
+        if (c < n) dgemm_store(C + r + (int64_t)c * ldc, acc[i][j][0], alpha, beta);
+        if (c + 1 < n) dgemm_store(C + r + (int64_t)(c + 1) * ldc, acc[i][j][1], alpha, beta);
+      }
+    }
+  }
+}
+
+// CTA-wide FP64 product (see cta_gemm).  The tile shape is the one that takes
+// the fewest tensor-pipe cycles of the busiest warp; an output of at most
+// nw / 2 8 x 8 tiles splits the inner dimension over the warps, with the
+// partial tiles (at most 32 of them) summed in warp order through smem.
+template <int NT, typename TA, typename TB, typename TC>
+__device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha, const TA* A, int64_t lda, bool ta,
+                                       const TB* B, int64_t ldb, bool tb, double beta, TC* C, int64_t ldc,
+                                       double* smem) {
+  constexpr int nw = NT / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (m <= 0 || n <= 0) { __syncthreads(); return; }
+  const int64_t sai = ta ? lda : 1, sak = ta ? 1 : lda, sbj = tb ? 1 : ldb, sbk = tb ? ldb : 1;
+  const int t8 = ((m + 7) / 8) * ((n + 7) / 8);
+  if (2 * t8 <= nw && k >= 64) {
+    const int split = nw / t8;
+    const int tm = (m + 7) / 8;
+    const int kc = ((k + split - 1) / split + 3) & ~3;
+    const int tile = wid / split, part = wid % split;
+    if (tile < t8) {
+      const int i0 = (tile % tm) * 8, j0 = (tile / tm) * 8;
+      double acc[1][1][2];
+      warp_dgemm_acc<1, 1>(m, n, min(k, part * kc), min(k, (part + 1) * kc), A, sai, sak, B, sbj, sbk, i0, j0, acc);
+      smem[wid * 64 + 2 * lane] = acc[0][0][0];
+      smem[wid * 64 + 2 * lane + 1] = acc[0][0][1];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < t8 * 64; e += NT) {
+      const int tl = e >> 6, x = e & 63;
+      const int r = (tl % tm) * 8 + (x >> 3), c = (tl / tm) * 8 + (x & 7);
+      if (r < m && c < n) {
+        double v = 0.0;
+        for (int q = 0; q < split; ++q) v += smem[(tl * split + q) * 64 + x];
+        dgemm_store(C + r + (int64_t)c * ldc, v, alpha, beta);
+      }
+    }
+    __syncthreads();
+    return;
+  }
+  auto cost = [&](int mi, int ni) {
+    const int tiles = ((m + 8 * mi - 1) / (8 * mi)) * ((n + 8 * ni - 1) / (8 * ni));
+    return ((tiles + nw - 1) / nw) * (2 * mi * ni + mi + ni);
+  };
+  const int c42 = cost(4, 2), c22 = cost(2, 2), c11 = cost(1, 1);
+  const int best = min(c42, min(c22, c11));
+  if (best == c42)
+    warps_dgemm<4, 2>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  else if (best == c22)
+    warps_dgemm<2, 2>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  else
+    warps_dgemm<1, 1>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
 // CTA-wide GEMM: C(m x n) = alpha * op(A) * op(B) + beta * C, column-major.
 // op(A) is m x k: A is (m x k, lda) when !ta, (k x m, lda) when ta.
 // op(B) is k x n: B is (k x n, ldb) when !tb, (n x k, ldb) when tb.
-// beta == 0 never reads C.  64x64 output tiles, k in steps of 16, operands
-// staged through shared memory in the accumulate type.  `smem` must hold
-// 2 * 16 * 64 TACC values.  Requires blockDim.x == NT (256 or 512).
+// beta == 0 never reads C.  FP64 accumulation takes the tensor pipe
+// (cta_dgemm); FP32 accumulation 64x64 output tiles, k in steps of 16,
+// operands staged through shared memory.  `smem` must hold 2 * 16 * 64 TACC
+// values.  Requires blockDim.x == NT (256 or 512).
 // ---------------------------------------------------------------------------
 template <typename TACC, int NT, typename TA, typename TB, typename TC>
-FRANK_D void cta_gemm(int m, int n, int k, TACC alpha, const TA* __restrict__ A, int64_t lda, bool ta,
-                      const TB* __restrict__ B, int64_t ldb, bool tb, TACC beta, TC* C, int64_t ldc,
+FRANK_D void cta_gemm(int m, int n, int k, TACC alpha, const TA* A, int64_t lda, bool ta,
+                      const TB* B, int64_t ldb, bool tb, TACC beta, TC* C, int64_t ldc,
                       TACC* smem) {
+  if constexpr (sizeof(TACC) == 8) {
+    cta_dgemm<NT>(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, smem);
+    return;
+  }
   constexpr int BM = 64, BN = 64, BK = 16;
   constexpr int TM = 4, TN = (NT == 256) ? 4 : 2;
   static_assert((BM / TM) * (BN / TN) == NT, "tile/threads mismatch");
@@ -511,29 +675,12 @@ FRANK_D void cta_load_v(int mr, int jn, const double* Ap, int64_t lda, double* s
   __syncthreads();
 }
 
-#ifdef FRANK_PHASE_TIMING
-__device__ unsigned long long g_sub_cycles[16];
-#define SUB_BEGIN() long long _sb_t0 = clock64()
-#define SUB_MARK(k)                                                                         \
-  do {                                                                                      \
-    __syncthreads();                                                                        \
-    if (threadIdx.x == 0) {                                                                 \
-      const long long _t = clock64();                                                      \
-      atomicAdd(&g_sub_cycles[(k)], (unsigned long long)(_t - _sb_t0));                     \
-      _sb_t0 = _t;                                                                          \
-    }                                                                                       \
-  } while (0)
-#else
-#define SUB_BEGIN() do {} while (0)
-#define SUB_MARK(k) do {} while (0)
-#endif
 
 template <int NT>
 FRANK_D void cta_qr_blocked(int m, int n, double* A, int64_t lda, double* tau, double* Tf, double* W,
                             double* smP, double* smT, double* gsm, double* red, int max_panels = 1 << 20,
                             int max_jn = QRB) {
   const int kmin = m < n ? m : n;
-  SUB_BEGIN();
   for (int j0 = 0; j0 < kmin && j0 / QRB < max_panels; j0 += QRB) {
     const int jn = min(min(QRB, max_jn), kmin - j0);
     const int mr = m - j0;
@@ -543,20 +690,16 @@ FRANK_D void cta_qr_blocked(int m, int n, double* A, int64_t lda, double* tau, d
       smP[e] = Ap[r + (int64_t)c * lda];
     }
     __syncthreads();
-    SUB_MARK(0);
     cta_householder_qr(mr, jn, smP, mr, tau + j0, red);
-    SUB_MARK(1);
     for (int e = threadIdx.x; e < mr * jn; e += blockDim.x) {
       const int r = e % mr, c = e / mr;
       Ap[r + (int64_t)c * lda] = smP[e];
       smP[e] = (r > c) ? smP[e] : (r == c ? 1.0 : 0.0);
     }
     __syncthreads();
-    SUB_MARK(2);
     cta_larft(mr, jn, smP, tau + j0, smT);
     double* Tp = Tf + (int64_t)(j0 / QRB) * QRB * QRB;
     for (int e = threadIdx.x; e < QRB * QRB; e += blockDim.x) Tp[e] = smT[e];
-    SUB_MARK(3);
     const int nc = n - j0 - jn;
     if (nc > 0) {
       double* At = A + j0 + (int64_t)(j0 + jn) * lda;
@@ -582,7 +725,6 @@ FRANK_D void cta_qr_blocked(int m, int n, double* A, int64_t lda, double* tau, d
       // At -= V W
       panel_x_minus_vw(mr, jn, smP, mr, W, nc, At, lda);
     }
-    SUB_MARK(4);
   }
   __syncthreads();
 }
@@ -605,14 +747,11 @@ FRANK_D void cta_apply_q_blocked(int m, int k, const double* A, int64_t lda, con
     const int kr = min(mr, max(0, nz - j0));   // rows of X that can be nonzero
     nz = m;                                    // after this panel X is full
     if (kr == 0) continue;                     // V^T X = 0: the panel is the identity on X
-    SUB_BEGIN();
     cta_load_v(mr, jn, A + j0 + (int64_t)j0 * lda, lda, smP);
     for (int e = threadIdx.x; e < QRB * QRB; e += blockDim.x) smT[e] = Tf[(int64_t)p * QRB * QRB + e];
     __syncthreads();
-    SUB_MARK(5);
     double* Xp = X + j0;
     panel_vtx(kr, jn, smP, mr, Xp, ldx, r, W);
-    SUB_MARK(6);
     for (int c = threadIdx.x; c < r; c += blockDim.x) {
       // unrolled over the panel width so that w stays in registers
       double w[QRB];
@@ -629,9 +768,7 @@ FRANK_D void cta_apply_q_blocked(int m, int k, const double* A, int64_t lda, con
       }
     }
     __syncthreads();
-    SUB_MARK(7);
     panel_x_minus_vw(mr, jn, smP, mr, W, r, Xp, ldx);
-    SUB_MARK(8);
   }
 }
 

@@ -38,6 +38,8 @@
 #include <math.h>
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 // The BLR engine's kernels (leaf LU, explicit inverses, kernel evaluation)
 // are compiled into this translation unit under a private name, so that none
 // of their symbols collides with the engine's own copy in api.cu.
@@ -364,15 +366,6 @@ __global__ void __launch_bounds__(WT) k_h_core(int64_t s, int k, const double* V
     Sp[e] = -v;
   }
   if (tid == 0) *counter = 0;
-}
-
-// Uinv^T of one leaf (b x b), for the transposed substitution.
-__global__ void k_h_transpose(int b, const double* A, double* At) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)b * b;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int i = e % b, j = e / b;
-    At[j + (int64_t)i * b] = A[e];
-  }
 }
 
 // Dense leaves of A_H: D[p] = K(rows of p, cols of p).
@@ -797,6 +790,7 @@ void leaf_view(const frank_hodlr* h, int p, blr::BlrView<double>& A, blr::Factor
   ws.ipiv = h->ipiv + (int64_t)p * h->b;
   ws.Linv = h->Linv + (int64_t)p * h->b * h->b;
   ws.Uinv = h->Uinv + (int64_t)p * h->b * h->b;
+  ws.UinvT = h->UinvT + (int64_t)p * h->b * h->b;
   ws.getrf_scratch = h->getrf_scratch;
   ws.err = h->err;
   ws.flops = h->flops;
@@ -807,24 +801,11 @@ void enqueue_leaf(frank_hodlr* h, int p, cudaStream_t s) {
   blr::FactorWs<double> ws;
   leaf_view(h, p, A, ws);
   const int b = h->b;
-  blr::k_getrf_load<double><<<64, blr::GETRF_AUX_THREADS, 0, s>>>(A, ws, 0);
-  ++h->launches;
-  for (int jb = 0; jb < b; jb += 32) {
-    blr::k_getrf_panel<double><<<1, blr::GETRF_THREADS, 0, s>>>(A, ws, 0, jb);
-    ++h->launches;
-    const int m2 = b - jb - std::min(32, b - jb);
-    if (m2 > 0) {
-      const int nt = (m2 + 63) / 64;
-      blr::k_getrf_trail<double><<<nt * nt, blr::GETRF_AUX_THREADS, 0, s>>>(A, ws, 0, jb);
-      ++h->launches;
-    }
-  }
-  blr::k_getrf_store<double><<<64, blr::GETRF_AUX_THREADS, 0, s>>>(A, ws, 0);
-  const int cw = blr::trinv_width(b);
-  const int nblk = (b + cw - 1) / cw;
-  blr::k_trinv<double><<<2 * nblk, blr::TRINV_THREADS, (size_t)b * cw * sizeof(double), s>>>(A, ws, 0, cw);
-  hk::k_h_transpose<<<64, 256, 0, s>>>(b, ws.Uinv, h->UinvT + (int64_t)p * b * b);
-  h->launches += 3;
+  const int np = (b + blr::leaf_width(b) - 1) / blr::leaf_width(b);
+  for (int q = 0; q < np; ++q)
+    blr::k_leaf_step<double><<<np, blr::leaf_threads(b), blr::leaf_smem(b), s>>>(A, ws, 0, q);
+  blr::k_leaf_final<double><<<3 * np, blr::leaf_threads(b), blr::leaf_smem(b), s>>>(A, ws, 0);
+  h->launches += np + 1;
 }
 
 // LowRank(U_x, S'_node, V_x) (n_node x n_node, U_x ld s(lr), V_x ld k) added
@@ -1087,7 +1068,7 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(dalloc(&h->S0, sk)); A(dalloc(&h->S, sk));
   A(dalloc(&h->Linv, dd)); A(dalloc(&h->Uinv, dd)); A(dalloc(&h->UinvT, dd));
   A(dalloc(&h->perm, P * leaf)); A(dalloc(&h->ipiv, P * leaf));
-  A(dalloc(&h->getrf_scratch, (size_t)leaf * leaf + 32 * leaf));
+  A(dalloc(&h->getrf_scratch, (size_t)blr::leaf_scratch(leaf)));
   A(dalloc(&h->geom, 4)); A(dalloc(&h->flops, blr::FLOP_SLOTS)); A(dalloc(&h->err, hk::HERR_SLOTS));
   A(dalloc(&h->kfill, (size_t)(L + 1) * P)); A(dalloc(&h->counter, 1));
   A(dalloc(&h->Sp, (size_t)P * rank * rank)); A(dalloc(&h->core_part, (size_t)CORE_GRID * rank * rank));
@@ -1136,7 +1117,8 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaMemset(h->U0, 0, sizeof(double) * nk));
   A(cudaMemset(h->V0, 0, sizeof(double) * nk));
   A(cudaMemset(h->S0, 0, sizeof(double) * sk));
-  A(cudaFuncSetAttribute(blr::k_trinv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::TRINV_SMEM_MAX));
+  A(cudaFuncSetAttribute(blr::k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
+  A(cudaFuncSetAttribute(blr::k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(hk::k_h_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::WALK_SMEM));
   if (e == cudaSuccess && h->lr_shm > 0 && ::frank::ops::lr_add_prepare(h->lr_shm) != FRANK_OK) h->lr_shm = 0;
   if (e != cudaSuccess) {
