@@ -1080,12 +1080,10 @@ FRANK_D UpdOps<T> update_operands(const BlrView<T>& A, const FactorWs<T>& ws, in
 }
 
 // core T (p x q) = -WL^T WU, FP64, into Tm (ld p).
-template <typename T, int NT>
-FRANK_D void form_core(const UpdOps<T>& o, int bi, int ld, double* Tm, double* gsm) {
+template <typename T>
+FRANK_D void form_core(const Grp& g, const UpdOps<T>& o, int bi, int ld, double* Tm, GrpShared& s, GrpScratch x) {
   if (!o.left_dense && !o.right_dense) {
-    // small cores: one warp per entry (lanes along the b-long inner dimension)
-    if (o.p * o.q <= 1024) cta_gemm_tn_dot(o.p, o.q, bi, -1.0, o.WL, ld, o.WU, ld, Tm, o.p);
-    else cta_gemm<double, NT>(o.p, o.q, bi, -1.0, o.WL, ld, true, o.WU, ld, false, 0.0, Tm, o.p, gsm);
+    g_gemm_tn(g, o.p, o.q, bi, -1.0, o.WL, ld, o.WU, ld, Tm, o.p, x.part, s.part);
   } else if (!o.left_dense && o.right_dense) {
     // -WL^T (p x bi)
     for (int64_t e = threadIdx.x; e < (int64_t)o.p * o.q; e += blockDim.x) {
@@ -1106,6 +1104,21 @@ FRANK_D void form_core(const UpdOps<T>& o, int bi, int ld, double* Tm, double* g
     }
     __syncthreads();
   }
+}
+
+template <typename T, int NT>
+FRANK_D void form_core_cta(const UpdOps<T>& o, int bi, int ld, double* Tm, double* gsm) {
+  if (!o.left_dense && !o.right_dense) {
+    if (o.p * o.q <= 1024) cta_gemm_tn_dot(o.p, o.q, bi, -1.0, o.WL, ld, o.WU, ld, Tm, o.p);
+    else cta_gemm<double, NT>(o.p, o.q, bi, -1.0, o.WL, ld, true, o.WU, ld, false, 0.0, Tm, o.p, gsm);
+    return;
+  }
+  for (int64_t e = threadIdx.x; e < (int64_t)o.p * o.q; e += blockDim.x) {
+    const int r = e % o.p, c = e / o.p;
+    if (!o.left_dense) Tm[e] = -double(o.WL[c + (int64_t)r * ld]);
+    else Tm[e] = -double(o.WU[r + (int64_t)c * ld]);
+  }
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
@@ -1157,7 +1170,7 @@ FRANK_D void k_update_dense_impl(BlrView<T> A, FactorWs<T> ws, int i, int band_r
       cta_gemm<T, DUPD_THREADS>(rn, bk, bi, T(-1), o.XL + r0, ld, false, o.YR, ld, false, T(1), C, ld, gsmt);
       continue;
     }
-    form_core<T, DUPD_THREADS>(o, bi, ld, Tm, gsm);
+    form_core_cta<T, DUPD_THREADS>(o, bi, ld, Tm, gsm);
     // X = XL(r0 : r0+rn, :) T  (rn x q), accumulate in the working precision
     cta_gemm<T, DUPD_THREADS>(rn, o.q, o.p, T(1), o.XL + r0, ld, false, Tm, o.p, false, T(0), X, ldx, gsmt);
     // C(band) += X * YR^T
@@ -1190,14 +1203,34 @@ __global__ void __launch_bounds__(DUPD_THREADS) k_update_dense(BlrView<T> A, Fac
 //           (misc.cpp:133-146, quirk included) or the fixed rank; S diagonal;
 //   new U = Qu [Q_core; 0], new V^T = Qv [V_core; 0].
 // Persistent grid, one target per CTA at a time, FP64 scratch slot per CTA.
-// The core lives in shared memory when it fits (RECOMP_SMEM_CORE doubles).
+// A target is a chain of dependent column steps and short products, so the
+// U side and the V side run beside each other on the two halves of the CTA
+// (bases, then Q_core beside the RQ of the kept rows, then the new bases);
+// the halves meet for the core and its truncation.  Panels and the core live
+// in shared memory when they fit.
 // ---------------------------------------------------------------------------
 constexpr int RECOMP_THREADS = 512;
 constexpr int SPLIT_P = 32;       // split band-1 targets whose operand rank exceeds this (default)
 constexpr int SPLIT_MAX = 128;    // band-1 tasks eligible for the split (scratch slots)
+constexpr int RECOMP_BMAX = 810;  // largest block order (a panel of each side in shared memory)
 constexpr int RECOMP_SMEM_BYTES = 227 * 1024 - 512;     // dynamic shared memory (all but the static part)
-constexpr int RECOMP_GSM = 2 * 16 * 64;                 // cta_gemm tiles (doubles)
-constexpr int RECOMP_REGION = RECOMP_SMEM_BYTES / 8 - RECOMP_GSM;  // doubles for panels / core
+
+struct RecompShared {
+  GrpShared gs[2];               // one per half of the CTA
+  unsigned long long mx[GQ + 2];
+  double red[32];
+  int redi[32];
+  int iscr[3 * GQ];
+  int flags[4];
+};
+constexpr int RECOMP_REGION = (RECOMP_SMEM_BYTES - (int)sizeof(RecompShared)) / 8;  // doubles for panels / core
+
+// Panel width of the bases' QR: both sides' panels fit side by side.
+FRANK_HD int recomp_panel(int bmax) {
+  const int w = RECOMP_REGION / 2 / panel_ld(bmax);
+  return w < GQ ? w : GQ;
+}
+
 // Core of the recompression: RRQR (truncated pivoted QR + RQ of the core),
 // SVD (one-sided Jacobi, find_svd_truncation_rank or the fixed rank), FAST
 // (fast_rounded_addition, addition.cpp:133-189: fixed-rank targets with
@@ -1205,53 +1238,84 @@ constexpr int RECOMP_REGION = RECOMP_SMEM_BYTES / 8 - RECOMP_GSM;  // doubles fo
 // only the remainders are QR-factored; SVD core as above).
 enum CoreMethod { CORE_RRQR = 0, CORE_SVD = 1, CORE_FAST = 2 };
 
-// SVD of the recompression core Mm (mu x mv, ld mu), preconditioned
-// one-sided Jacobi: column-pivoted QR M P = Q R (in place in Mm), then
-// one-sided Jacobi on the columns of A = R^T (mv x k) with the rotations
-// accumulated in Z (k x k, appended rows); the pivoting leaves A's columns
-// nearly orthogonal, so a few sweeps converge (Drmac & Veselic, "New fast and
-// accurate Jacobi SVD algorithm", SIAM J. Matrix Anal. Appl. 29, 2008).
-// With A Z = W S: M = (Q Z) S (P W)^T, so the left singular vectors are Q Z
-// (the QR's reflectors applied to Z) and the right ones P W (the normalised
-// columns of A Z, rows permuted back); both sets are orthonormal to working
-// accuracy whatever the singular value, which the next projected addition
-// into this target relies on.  Tolerance plans stop the QR once the
+// Scratch doubles of an svd_core whose Jacobi matrix is not in shared memory.
+FRANK_HD int64_t svd_core_scratch(int mu, int mv) {
+  const int64_t k = mu < mv ? mu : mv;
+  return (mv + k) * k + 32 * (int64_t)mv;
+}
+
+// SVD of the recompression core Mm (mu x mv, ld ldm), preconditioned
+// one-sided Jacobi: column-pivoted QR M P = Q R, then one-sided Jacobi on the
+// columns of A = P R^T (mv x k) with the rotations accumulated in Z (k x k,
+// appended rows); the pivoting leaves A's columns nearly orthogonal, so a few
+// sweeps converge (Drmac & Veselic, "New fast and accurate Jacobi SVD
+// algorithm", SIAM J. Matrix Anal. Appl. 29, 2008).
+// With A Z = W S: M = (Q Z) S W^T, so the left singular vectors are Q Z (the
+// QR's reflectors applied to Z) and the right ones W (the normalised columns
+// of A Z); both sets are orthonormal to working accuracy whatever the
+// singular value, which the next projected addition into this target relies
+// on.  Tolerance plans stop the QR once the
 // remaining columns are below thr = 0.01 eps ||M||_F / sqrt(mv min(mu, mv)),
 // so the dropped block R22 moves the truncation test below by at most 1 % of
 // its threshold.  Rank: the fixed rank of the plan, else
 // find_svd_truncation_rank (misc.cpp:133-146, quirk included: the tail error
 // is (min_dim - r) sigma_r^2) at ws.eps with ||M||_F as the reference norm;
-// capped at kcap (counted as a rank overflow).  Scratch: the Jacobi matrix
-// ((mv + k) x k) in smem (region, cap doubles, after the core if the core is
-// there) when it fits, else in Atmp (global, (mv + min(mu,mv)) x min(mu,mv));
-// tau / cnorm / partial / jpvt (mv each), sig / ord (min(mu, mv)).  On return
-// partial[c] is the c-th largest singular value (c < r), Xo (bc x r, ld bc) =
-// [U_m(:, :r); 0] and Yo (bk x r, ld bk) = [V_m(:, :r); 0].  Returns r (all
-// threads).
+// capped at kcap (counted as a rank overflow).  A core in shared memory (in_smem;
+// it starts region) takes g_rrqr, a core in L2 the blocked pivoted QR.  The Jacobi matrix
+// ((mv + k) x k) lies behind the core in region (cap doubles) when it
+// fits, else in Atmp (global, svd_core_scratch doubles).
+// tau / cnorm / partial / jpvt (mv each), sig / ord (min(mu, mv)): global.  On return
+// partial[c] is the c-th largest singular value (c < r), Xo (mu x r) = U_m(:, :r)
+// and Yo (mv x r) = V_m(:, :r).  Returns r (all threads).
 template <typename T, int NT>
-FRANK_D int svd_core(int mu, int mv, double* Mm, const FactorWs<T>& ws, int kcap, double* region, int64_t cap,
-                     double* Atmp, double* tau, double* cnorm, double* partial, int* jpvt, double* sig, int* ord,
-                     double* Xo, int bc, double* Yo, int bk, double* gsm, double* red, int* redi, int* flag,
-                     int* s_rank) {
+FRANK_D int svd_core(int mu, int mv, double* Mm, int ldm, bool in_smem, const FactorWs<T>& ws, int kcap,
+                     double* region, int64_t cap, double* Atmp, double* tau, double* cnorm, double* partial, int* jpvt,
+                     double* sig, int* ord, double* Xo, double* Yo, RecompShared& sh, int* s_rank) {
+  const Grp g = grp_all();
   const int nsv = min(mu, mv);
   double f = 0.0;
-  for (int64_t e = threadIdx.x; e < (int64_t)mu * mv; e += blockDim.x) f += Mm[e] * Mm[e];
-  const double fro = sqrt(block_sum(f, red));
+  for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) {
+    const double v = Mm[e % mu + (int64_t)(e / mu) * ldm];
+    f += v * v;
+  }
+  const double fro = sqrt(block_sum(f, sh.red));
   const double thr = ws.fixed_rank > 0 ? 0.0 : 0.01 * ws.eps * fro / sqrt((double)mv * (double)nsv);
-  // a core in L2 takes the blocked pivoted QR (F, mv x 32, in Atmp)
-  const int k = Mm != region ? cta_truncated_geqp3_blocked<NT>(mu, mv, Mm, mu, thr, nsv, tau, cnorm, partial, jpvt,
-                                                               red, redi, Atmp, gsm)
-                             : cta_truncated_geqp3(mu, mv, Mm, mu, thr, nsv, tau, cnorm, partial, jpvt, red, redi);
-  // [A; I] with A = R(0:k, :)^T (mv x k), ld mv + k
-  const int ldj = mv + k;
-  const int64_t off = (Mm == region) ? (int64_t)mu * mv : 0;
-  double* Aj = off + (int64_t)ldj * k <= cap ? region + off : Atmp;
-  for (int64_t e = threadIdx.x; e < (int64_t)ldj * k; e += blockDim.x) {
-    const int c = e % ldj, j = e / ldj;
-    Aj[e] = c < mv ? ((c >= j) ? Mm[j + (int64_t)c * mu] : 0.0) : (c - mv == j ? 1.0 : 0.0);
+  int k;
+  int64_t off = 0;
+  double* Qm = Mm;              // reflectors for the left vectors
+  const double* stau = tau;
+  int* sord = nullptr;
+  if (in_smem) {
+    double* st = region + (int64_t)ldm * mv;            // tau, beta / scal
+    double* cand = st + 3 * nsv;
+    sord = reinterpret_cast<int*>(cand + 4 * (NT / 32));
+    int* at = sord + nsv;
+    off = (int64_t)ldm * mv + 3 * nsv + 4 * (NT / 32) + (nsv + mv + 2) / 2;
+    k = g_rrqr(g, mu, mv, Mm, ldm, thr, nsv, st, sord, at, st + nsv, cand);
+    stau = st;
+    const int ldj = mv + k;
+    double* Aj = off + (int64_t)ldj * k <= cap ? region + off : Atmp;
+    for (int e = threadIdx.x; e < ldj * k; e += blockDim.x) {
+      const int c = e % ldj, j = e / ldj;
+      Aj[e] = c < mv ? rrqr_r(Mm, ldm, at, j, c) : (c - mv == j ? 1.0 : 0.0);
+    }
+  } else {
+    // a core in L2: the panel-blocked pivoted QR (F, mv x 32, in Atmp); its columns
+    // are moved, so A's rows go back through jpvt
+    k = cta_truncated_geqp3_blocked<NT>(mu, mv, Mm, ldm, thr, nsv, tau, cnorm, partial, jpvt, sh.red, sh.redi, Atmp,
+                                        region);
+    const int ldj = mv + k;
+    double* Aj = (int64_t)ldj * k <= cap ? region : Atmp;
+    for (int64_t e = threadIdx.x; e < (int64_t)ldj * k; e += blockDim.x) {
+      const int c = e % ldj, j = e / ldj;
+      if (c < mv) Aj[jpvt[c] + (int64_t)j * ldj] = c >= j ? Mm[j + (int64_t)c * ldm] : 0.0;
+      else Aj[e] = c - mv == j ? 1.0 : 0.0;
+    }
   }
   __syncthreads();
-  const int sweeps = cta_jacobi_columns(mv, k, Aj, ldj, 60, flag, ldj);
+  const int ldj = mv + k;
+  double* Aj = off + (int64_t)ldj * k <= cap ? region + off : Atmp;
+  const int sweeps = g_jacobi(g, mv, k, Aj, ldj, 60, sh.flags, ldj);
   if (sweeps < 0 && threadIdx.x == 0) atomicAdd(ws.err + ERR_JACOBI, 1);
   for (int c = threadIdx.x >> 5; c < k; c += blockDim.x >> 5) {
     double sacc = 0.0;
@@ -1296,22 +1360,26 @@ FRANK_D int svd_core(int mu, int mv, double* Mm, const FactorWs<T>& ws, int kcap
   }
   __syncthreads();
   const int r = *s_rank;
-  // Yo (bk x r): V_M = P W, row jpvt[i] of V_M = row i of W (columns of A Z
-  // normalised); Xo (bc x r) = [Z(:, ord); 0], then Q applied below
-  for (int64_t e = threadIdx.x; e < (int64_t)bk * r; e += blockDim.x) Yo[e] = 0.0;
-  for (int64_t e = threadIdx.x; e < (int64_t)bc * r; e += blockDim.x) {
-    const int i = e % bc, c = e / bc;
-    Xo[e] = (i < k && c < k) ? Aj[mv + i + (int64_t)ord[c] * ldj] : 0.0;
-  }
-  __syncthreads();
-  for (int64_t e = threadIdx.x; e < (int64_t)mv * r; e += blockDim.x) {
+  // Yo (mv x r): the columns of A Z normalised; columns beyond the computed k are zero
+  for (int e = threadIdx.x; e < mv * r; e += blockDim.x) {
     const int i = e % mv, c = e / mv;
     const int src = c < k ? ord[c] : -1;
     const double sv_ = src >= 0 ? sig[src] : 0.0;
-    Yo[jpvt[i] + (int64_t)c * bk] = sv_ > 0.0 ? Aj[i + (int64_t)src * ldj] / sv_ : 0.0;
+    Yo[e] = sv_ > 0.0 ? Aj[i + (int64_t)src * ldj] / sv_ : 0.0;
   }
-  __syncthreads();
-  cta_apply_q(mu, k, Mm, mu, tau, r, Xo, (int64_t)bc);
+  // Xo (mu x r) = Q [Z(:, ord); 0]
+  if (in_smem) {
+    const int rk = min(r, k);
+    g_apply_rrqr(g, mu, k, rk, Qm, ldm, stau, sord, false, Aj + mv, ldj, ord, Xo, mu);
+    for (int e = threadIdx.x; e < mu * (r - rk); e += blockDim.x) Xo[mu * rk + e] = 0.0;
+  } else {
+    for (int e = threadIdx.x; e < mu * r; e += blockDim.x) {
+      const int i = e % mu, c = e / mu;
+      Xo[e] = (i < k && c < k) ? Aj[mv + i + (int64_t)ord[c] * ldj] : 0.0;
+    }
+    __syncthreads();
+    cta_apply_q(mu, k, Mm, ldm, tau, r, Xo, (int64_t)mu);
+  }
   // the kept singular values in order, in partial (free after the QR)
   for (int c = threadIdx.x; c < r; c += blockDim.x) partial[c] = c < k ? sig[ord[c]] : 0.0;
   __syncthreads();
@@ -1319,7 +1387,7 @@ FRANK_D int svd_core(int mu, int mv, double* Mm, const FactorWs<T>& ws, int kcap
 }
 
 struct RecompLayout {
-  int64_t ash, bsh, tm, rc, rv, mtmp, mglob, m0, xo, yo, tfu, tfv, w, tau_u, tau_v, tau_c, tau2, cn, pn, jp, ji, total;
+  int64_t ash, bsh, t, gu, gv, mtmp, mglob, y1, tv, tfu, tfv, tfc, tfr, om, w, part, tau_c, sig, cn, pn, jp, ji, total;
 };
 
 FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
@@ -1327,24 +1395,26 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
   int64_t o = 0;
   auto take = [&](int64_t n) { int64_t r = o; o += (n + 31) & ~int64_t(31); return r; };
   const int mu = smax < bmax ? smax : bmax;
-  const int64_t np = (smax + QRB - 1) / QRB;
+  const int64_t np = bmax / recomp_panel(bmax) + 1;
   L.ash = take((int64_t)bmax * smax);
   L.bsh = take((int64_t)bmax * smax);
-  L.tm = take((int64_t)bmax * bmax);
-  L.rc = take((int64_t)mu * smax);
-  L.rv = take((int64_t)mu * smax);
+  L.t = take((int64_t)bmax * bmax);
+  L.gu = take((int64_t)mu * smax);
+  L.gv = take((int64_t)mu * smax);
   L.mtmp = take((int64_t)mu * smax);
-  L.mglob = take((int64_t)mu * mu);
-  L.m0 = take((int64_t)mu * mu);
-  L.xo = take((int64_t)bmax * mu);
-  L.yo = take((int64_t)bmax * mu);
-  L.tfu = take(np * QRB * QRB);
-  L.tfv = take(np * QRB * QRB);
-  L.w = take((int64_t)QRB * (smax > bmax ? smax : bmax));
-  L.tau_u = take(smax);
-  L.tau_v = take(smax);
+  const int64_t svd = svd_core_scratch(mu, mu), sq = (int64_t)mu * mu;
+  L.mglob = take(sq);
+  L.y1 = take(sq);
+  L.tv = take(svd > (int64_t)bmax * mu ? svd : (int64_t)bmax * mu);
+  L.tfu = take(np * GQ * GQ);
+  L.tfv = take(np * GQ * GQ);
+  L.tfc = take((mu / 8 + 2) * (int64_t)GQ * GQ);
+  L.tfr = take((mu / 8 + 2) * (int64_t)GQ * GQ);
+  L.om = take((GQ + 8) * (int64_t)mu);
+  L.w = take(4 * (int64_t)GQ * (smax > bmax ? smax : bmax));
+  L.part = take(2 * (int64_t)G_TN_PART);
   L.tau_c = take(mu);
-  L.tau2 = take(mu);
+  L.sig = take(mu);
   L.cn = take(mu);
   L.pn = take(mu);
   L.jp = take(mu);
@@ -1360,35 +1430,21 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
                                                                double* split_base, int* split_done, int proj_tol,
                                                                int split_p, int core_smem) {
   extern __shared__ double dsm[];
-  double* gsm = dsm;
-  double* region = dsm + RECOMP_GSM;
-  __shared__ double red[32];
-  __shared__ int redi[32];
-  __shared__ int flag;
-  __shared__ int s_rank;
+  RecompShared& sh = *reinterpret_cast<RecompShared*>(dsm);
+  double* region = dsm + sizeof(RecompShared) / 8;
+  __shared__ int s_rank, s_last, s_task;
   const int m = A.nb - i - 1;
   const int ld = A.bmax;
   const int bi = A.bs(i);
   const RecompLayout L = recomp_layout(A.bmax, smax);
-  double* const cta_base = ws.rscratch + (int64_t)blockIdx.x * ws.rscratch_stride;
-  double *Ash, *Bsh, *Tm, *Rc, *Rv, *Mtmp, *Mg, *M0, *Xo, *Yo, *Tfu, *Tfv, *Wq, *tau_u, *tau_v, *tau_c, *tau2, *cnorm,
-      *pnorm;
-  int *jpvt, *jinv;
-  auto set_base = [&](double* base) {
-    Ash = base + L.ash; Bsh = base + L.bsh; Tm = base + L.tm; Rc = base + L.rc; Rv = base + L.rv;
-    Mtmp = base + L.mtmp; Mg = base + L.mglob; M0 = base + L.m0; Xo = base + L.xo; Yo = base + L.yo;
-    Tfu = base + L.tfu; Tfv = base + L.tfv; Wq = base + L.w; tau_u = base + L.tau_u; tau_v = base + L.tau_v;
-    tau_c = base + L.tau_c; tau2 = base + L.tau2; cnorm = base + L.cn; pnorm = base + L.pn;
-    jpvt = reinterpret_cast<int*>(base + L.jp); jinv = reinterpret_cast<int*>(base + L.ji);
-  };
-  __shared__ int s_last;
-  double* smP = region;
-  double* smT = region + (int64_t)A.bmax * QRB;
-  __shared__ int s_task;
+  const int wp = recomp_panel(A.bmax);
+  const Grp all = grp_all();
+  const int hf = threadIdx.x >= RECOMP_THREADS / 2;
+  const Grp half = grp_half(hf);
   const int ntask = m * (m - 1);
   // Split targets: band-1 targets (the first 2(m-1) tasks, largest ranks)
   // whose operands have ranks above SPLIT_P get one task per side of the
-  // stacked-basis QR, run on two CTAs into the target's own scratch slot;
+  // bases' QR, run on two CTAs into the target's own scratch slot;
   // the CTA that finishes second does the rest (no waiting).  The test uses
   // only operand ranks, which no CTA changes during the launch.
   const int nspl = split_base ? min(nsplit, 2 * (m - 1)) : 0;
@@ -1404,8 +1460,15 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     const bool split_t = tsk < nspl && split_p > 0 && A.is_lr(ic, i) && A.is_lr(i, k) &&
                          max(A.rank[ic * A.nb + i], A.rank[i * A.nb + k]) > split_p;
     if ((side >= 0) != split_t) continue;
-    set_base(side >= 0 ? split_base + (int64_t)tsk * ws.rscratch_stride : cta_base);
-    const bool do_u = side != 1, do_v = side != 0;
+    double* const base = side >= 0 ? split_base + (int64_t)tsk * ws.rscratch_stride
+                                   : ws.rscratch + (int64_t)blockIdx.x * ws.rscratch_stride;
+    double *Ash = base + L.ash, *Bsh = base + L.bsh, *Tm = base + L.t, *Gu = base + L.gu, *Gv = base + L.gv,
+           *Mtmp = base + L.mtmp, *Mg = base + L.mglob, *Y1 = base + L.y1, *Tv = base + L.tv;
+    const int64_t wstep = (int64_t)GQ * max(smax, A.bmax);
+    auto scratch_of = [&](int sd) {
+      return GrpScratch{base + L.w + 2 * sd * wstep, base + L.w + (2 * sd + 1) * wstep, base + L.part + sd * (int64_t)G_TN_PART};
+    };
+    int* jpvt = reinterpret_cast<int*>(base + L.jp);
     const int blk = ic * A.nb + k;
     const int bc = A.bs(ic), bk = A.bs(k);
     const int kc = A.rank[blk];
@@ -1418,23 +1481,6 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     T* Uc = A.u(ic, k);
     T* Sc = A.s(ic, k);
     T* Vc = A.vt(ic, k);
-    // stacked bases in FP64
-    for (int64_t e = threadIdx.x; do_u && e < (int64_t)bc * su; e += blockDim.x) {
-      const int r = e % bc, c = e / bc;
-      Ash[r + (int64_t)c * bc] = (c < kc) ? double(Uc[r + (int64_t)c * ld]) : double(o.XL[r + (int64_t)(c - kc) * ld]);
-    }
-    for (int64_t e = threadIdx.x; do_v && e < (int64_t)bk * sv; e += blockDim.x) {
-      const int r = e % bk, c = e / bk;
-      double v;
-      if (c < kc) v = double(Vc[r + (int64_t)c * ld]);
-      else if (!o.right_dense) v = double(o.YR[r + (int64_t)(c - kc) * ld]);
-      else v = double(o.YR[(c - kc) + (int64_t)r * ld]);  // A(i,k)^T
-      Bsh[r + (int64_t)c * bk] = v;
-    }
-    // the stacked bases are read across threads below (the V side of a split
-    // target forms no core, whose barrier would otherwise cover this)
-    __syncthreads();
-    if (do_u) form_core<T, RECOMP_THREADS>(o, bi, ld, Tm, gsm);
     // Bases.  Stacked (rounded_addition, addition.cpp:93-127): Householder QR
     // of [U_C | U_B] and of [V_C | V_B].  Projected (fast_rounded_addition,
     // addition.cpp:133-189, the default of fixed-rank plans, and on request
@@ -1445,24 +1491,53 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     // V side.  Both give the same sum C + B = [U_C | Q] M [V_C | Q']^T.
     const bool proj = (core_method == CORE_FAST ? ws.fixed_rank > 0 : proj_tol != 0) && kc > 0 && o.p > 0 &&
                       o.q > 0 && !o.left_dense && !o.right_dense && su <= bc && sv <= bk;
-    if (proj) {
-      if (do_u) {
-        cta_project_out<RECOMP_THREADS>(bc, kc, o.p, Ash, bc, Ash + (int64_t)kc * bc, bc, Rc + (int64_t)kc * su, su,
-                                        Xo, gsm);
-        cta_qr_blocked<RECOMP_THREADS>(bc, o.p, Ash + (int64_t)kc * bc, bc, tau_u, Tfu, Wq, smP, smT, gsm, red);
+    const int mu = proj ? su : min(bc, su), mv = proj ? sv : min(bk, sv);
+    // one side's basis: projected, [Zu; Ru] (su x p) in Gu and the clean V of
+    // the remainder's QR in Ash; stacked, R (mu x su) in Gu and V in Ash
+    auto basis = [&](const Grp& g, int sd, double* smP) {
+      const int bb = sd ? bk : bc, pp = sd ? o.q : o.p, ss = kc + pp, mm = sd ? mv : mu;
+      const T* C = sd ? Vc : Uc;
+      const T* X = sd ? o.YR : o.XL;
+      const bool xt = sd && o.right_dense;     // A(i,k)^T
+      double* S = sd ? Bsh : Ash;
+      double* G = sd ? Gv : Gu;
+      double* Tf = base + (sd ? L.tfv : L.tfu);
+      const GrpScratch x = scratch_of(sd);
+      GrpShared& s = sh.gs[sd];
+      const int lane = threadIdx.x & 31;
+      if (proj) {
+        const bool one = pp <= wp;             // a single panel: kept in shared memory from the start
+        double* Y = one ? smP : S;
+        const int ldy = one ? panel_ld(bb) : bb;
+        for (int c = g.wid; c < pp; c += g.nw)
+#pragma unroll 4
+          for (int r = lane; r < bb; r += 32) Y[r + c * ldy] = double(X[r + (int64_t)c * ld]);
+        g.sync();
+        g_project_out(g, bb, kc, pp, C, ld, Y, ldy, G, ss, sd ? Mg : Mtmp, s, x);
+        if (one) {
+          g_panel_qr(g, bb, pp, Y, ldy, G + kc, ss, s);
+          for (int c = g.wid; c < pp; c += g.nw)
+#pragma unroll 4
+            for (int r = lane; r < bb; r += 32) S[r + (int64_t)c * bb] = Y[r + c * ldy];
+          for (int e = g.tid; e < GQ * GQ; e += g.nt) Tf[e] = s.T[e];
+          g.sync();
+        } else {
+          g_qr(g, bb, pp, S, bb, G + kc, ss, Tf, wp, smP, s, x);
+        }
+      } else {
+        for (int c = g.wid; c < ss; c += g.nw)
+#pragma unroll 4
+          for (int r = lane; r < bb; r += 32)
+            S[r + (int64_t)c * bb] = c < kc ? double(C[r + (int64_t)c * ld])
+                                            : double(xt ? X[(c - kc) + (int64_t)r * ld] : X[r + (int64_t)(c - kc) * ld]);
+        g.sync();
+        g_qr(g, bb, ss, S, bb, G, mm, Tf, wp, smP, s, x);
       }
-      if (do_v) {
-        cta_project_out<RECOMP_THREADS>(bk, kc, o.q, Bsh, bk, Bsh + (int64_t)kc * bk, bk, Rv + (int64_t)kc * sv, sv,
-                                        Yo, gsm);
-        cta_qr_blocked<RECOMP_THREADS>(bk, o.q, Bsh + (int64_t)kc * bk, bk, tau_v, Tfv, side == 1 ? Mtmp : Wq, smP,
-                                       smT, gsm, red);
-      }
-    } else {
-      if (do_u) cta_qr_blocked<RECOMP_THREADS>(bc, su, Ash, bc, tau_u, Tfu, Wq, smP, smT, gsm, red);
-      // the V side of a split target works in Mtmp (free until the core), so
-      // that the two sides never share the W scratch
-      if (do_v) cta_qr_blocked<RECOMP_THREADS>(bk, sv, Bsh, bk, tau_v, Tfv, side == 1 ? Mtmp : Wq, smP, smT, gsm, red);
-    }
+    };
+    if (side != 1) form_core(all, o, bi, ld, Tm, sh.gs[0], scratch_of(0));
+    if (side >= 0) basis(all, side, region);
+    else basis(half, hf, region + hf * (RECOMP_REGION / 2));
+    __syncthreads();
     if (side >= 0) {
       // publish this side; the second of the two CTAs goes on with the target
       __threadfence();
@@ -1472,58 +1547,58 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
       if (s_last == 0) continue;
       __threadfence();
     }
-    const int mu = proj ? su : min(bc, su), mv = proj ? sv : min(bk, sv);
-    if (!proj) {
-      // clean upper-trapezoidal R factors
-      for (int64_t e = threadIdx.x; e < (int64_t)mu * su; e += blockDim.x) {
-        const int r = e % mu, c = e / mu;
-        Rc[e] = (r <= c) ? Ash[r + (int64_t)c * bc] : 0.0;
-      }
-      for (int64_t e = threadIdx.x; e < (int64_t)mv * sv; e += blockDim.x) {
-        const int r = e % mv, c = e / mv;
-        Rv[e] = (r <= c) ? Bsh[r + (int64_t)c * bk] : 0.0;
-      }
-    } else {
-      // Rc = [I Zu; 0 Ru] (su x su), Rv = [I Zv; 0 Rv'] (sv x sv); Zu, Zv are in place
-      for (int64_t e = threadIdx.x; e < (int64_t)mu * su; e += blockDim.x) {
-        const int r = e % mu, c = e / mu;
-        if (c < kc) Rc[e] = (r == c) ? 1.0 : 0.0;
-        else if (r >= kc) Rc[e] = (r - kc <= c - kc) ? Ash[(r - kc) + (int64_t)c * bc] : 0.0;
-      }
-      for (int64_t e = threadIdx.x; e < (int64_t)mv * sv; e += blockDim.x) {
-        const int r = e % mv, c = e / mv;
-        if (c < kc) Rv[e] = (r == c) ? 1.0 : 0.0;
-        else if (r >= kc) Rv[e] = (r - kc <= c - kc) ? Bsh[(r - kc) + (int64_t)c * bk] : 0.0;
-      }
-    }
-    __syncthreads();
-    // Mtmp (mu x sv) = [Rc[:, :kc] S_C | Rc[:, kc:] T]
-    cta_gemm<double, RECOMP_THREADS>(mu, kc, kc, 1.0, Rc, mu, false, Sc, A.kcap, false, 0.0, Mtmp, mu, gsm);
-    cta_gemm<double, RECOMP_THREADS>(mu, o.q, o.p, 1.0, Rc + (int64_t)kc * mu, mu, false, Tm, o.p, false, 0.0,
-                                     Mtmp + (int64_t)kc * mu, mu, gsm);
-    // core M (mu x mv) = Mtmp Rv^T, in shared memory if it fits
-    // the core in shared memory when it fits and is not above the tuned size
-    // (small cores always: the L2 paths need mu >= 64 for their T scratch)
-    const int64_t core_need = (int64_t)mu * mv + 4 * (int64_t)mv + 2 * mu;
-    const bool in_smem = core_need <= RECOMP_REGION && (mu < 64 || core_need <= core_smem);
+    // Core M (mu x mv), in shared memory if it fits with the panel of its RQ and is not above the tuned size
+    // (small cores always: the L2 path works on panels of its own).
+    // Projected: M = [I Zu; 0 Ru] blockdiag(S_C, T) [I Zv; 0 Rv']^T = [Zu; Ru] T [Zv; Rv']^T + S_C;
+    // stacked: M = [Ru(:, :kc) S_C | Ru(:, kc:) T] Rv^T.
+    const int ldm_s = rrqr_ld(mu);
+    const int64_t vecs = 3 * (int64_t)min(mu, mv) + 4 * (RECOMP_THREADS / 32) + (min(mu, mv) + mv + 2) / 2;
+    const int64_t core_need = (int64_t)ldm_s * mv + vecs;
+    const bool in_smem = core_need + 8 * (int64_t)panel_ld(mv) <= RECOMP_REGION && mu <= G_COLS_MAX &&
+                         (mu < 64 || core_need <= core_smem);
     double* Mm = in_smem ? region : Mg;
-    cta_gemm<double, RECOMP_THREADS>(mu, mv, sv, 1.0, Mtmp, mu, false, Rv, mv, true, 0.0, Mm, mu, gsm);
+    const int ldm = in_smem ? ldm_s : mu;
+    GrpShared& s0 = sh.gs[0];
+    const GrpScratch x0 = scratch_of(0);
+    if (proj) {
+      g_gemm(all, mu, o.q, o.p, 1.0, Gu, mu, false, Tm, o.p, false, 0.0, Mtmp, mu, s0.part);
+      g_gemm(all, mu, mv, o.q, 1.0, Mtmp, mu, false, Gv, mv, true, 0.0, Mm, ldm, s0.part);
+      for (int e = threadIdx.x; e < kc * kc; e += blockDim.x) {
+        const int r = e % kc, c = e / kc;
+        Mm[r + (int64_t)c * ldm] += double(Sc[r + (int64_t)c * A.kcap]);
+      }
+      __syncthreads();
+    } else {
+      g_gemm(all, mu, kc, kc, 1.0, Gu, mu, false, Sc, A.kcap, false, 0.0, Mtmp, mu, s0.part);
+      g_gemm(all, mu, o.q, o.p, 1.0, Gu + (int64_t)kc * mu, mu, false, Tm, o.p, false, 0.0, Mtmp + (int64_t)kc * mu,
+             mu, s0.part);
+      g_gemm(all, mu, mv, sv, 1.0, Mtmp, mu, false, Gv, mv, true, 0.0, Mm, ldm, s0.part);
+    }
     int r = 0;
+    double* X1 = Gu;              // Q_core (mu x r); Gu is free once the core is formed
     if (core_method == CORE_RRQR && ws.fixed_rank == 0) {
       double f = 0.0;
-      for (int64_t e = threadIdx.x; e < (int64_t)mu * mv; e += blockDim.x) f += Mm[e] * Mm[e];
-      f = block_sum(f, red);
-      double* cn = in_smem ? region + (int64_t)mu * mv : cnorm;
-      double* pn = in_smem ? cn + mv : pnorm;
-      double* tc = in_smem ? pn + mv : tau_c;
-      // a core in L2 (too large for shared memory) takes the pivoted QR with
-      // randomized block pivoting (panel GEMMs instead of one pass over the
-      // core per column), its scratch in Mtmp (free until the RQ below)
+      for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) {
+        const double v = Mm[e % mu + (int64_t)(e / mu) * ldm];
+        f += v * v;
+      }
+      f = block_sum(f, sh.red);
       const double thr_c = core_scale * ws.eps * sqrt(f);
-      r = (!in_smem && rqrcp_scratch(mu, mv) <= L.mglob - L.mtmp)
-              ? cta_rand_qrcp<RECOMP_THREADS>(mu, mv, Mm, mu, thr_c, A.kcap, tc, jpvt, Mtmp, smP, smT, gsm, red,
-                                              redi)
-              : cta_truncated_geqp3(mu, mv, Mm, mu, thr_c, A.kcap, tc, cn, pn, jpvt, red, redi);
+      // shared-memory vectors of the pivoted QR, behind the core
+      double* tau = region + (int64_t)ldm_s * mv;
+      double* cand = tau + 3 * min(mu, mv);
+      int* ord = reinterpret_cast<int*>(cand + 4 * (RECOMP_THREADS / 32));
+      int* at = ord + min(mu, mv);
+      double* Rm = Gv;            // rows of R of a core in L2 (Gv is free too)
+      double* Tfc = base + L.tfc;
+      // panel width of the L2 path: its sketch and its panel fit shared memory
+      int wc = GQ;
+      while (wc > 8 && rand_qrcp_smem(mu, mv, wc) > RECOMP_REGION) wc -= 8;
+      if (in_smem)
+        r = g_rrqr(all, mu, mv, Mm, ldm, thr_c, A.kcap, tau, ord, at, tau + min(mu, mv), cand);
+      else
+        r = g_rand_qrcp(all, mu, mv, Mm, ldm, Rm, mu, thr_c, A.kcap, wc, jpvt, Tfc, base + L.om, base + L.cn, region,
+                        sh.iscr, sh.mx, s0, x0);
       if (r == 0) {
         // zero core: rank-1 zero block (geqp3.cpp:97-102)
         if (threadIdx.x == 0) { atomicMax(ws.err + ERR_MAX_RANK, 1); atomicAdd(ws.err + ERR_RECOMP, 1); }
@@ -1538,77 +1613,50 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
         atomicMax(ws.err + ERR_MAX_RANK, r);
         atomicAdd(ws.err + ERR_RECOMP, 1);
       }
-      // the small factors (Q_core, the RQ of its kept rows and its explicit Q)
-      // stay in shared memory after the core when they fit
-      const int64_t voff = (int64_t)mu * mv + 4 * (int64_t)mv + 2 * (int64_t)mu;
-      const bool t_sm = in_smem && voff + 2 * (int64_t)mv * r + (int64_t)mu * r <= RECOMP_REGION;
-      // Xo (bc x r) = [Q_core; 0]
-      if (t_sm) {
-        double* X1s = region + voff + 2 * (int64_t)mv * r;   // mu x r
-        for (int64_t e = threadIdx.x; e < (int64_t)mu * r; e += blockDim.x) X1s[e] = ((e % mu) == (e / mu)) ? 1.0 : 0.0;
-        __syncthreads();
-        cta_apply_q(mu, r, Mm, mu, tc, r, X1s, (int64_t)mu);
-        for (int64_t e = threadIdx.x; e < (int64_t)bc * r; e += blockDim.x) {
-          const int rr = e % bc, c = e / bc;
-          Xo[e] = rr < mu ? X1s[rr + (int64_t)c * mu] : 0.0;
+      if (hf == 0) {
+        // X1 = Q_core(:, :r)
+        if (in_smem) {
+          g_apply_rrqr(half, mu, r, r, Mm, ldm, tau, ord, true, nullptr, 0, nullptr, X1, mu);
+        } else {
+          for (int e = half.tid; e < mu * r; e += half.nt) X1[e] = (e % mu) == (e / mu) ? 1.0 : 0.0;
+          half.sync();
+          g_apply_q(half, mu, r, Mm, ldm, Tfc, wc, r, X1, mu, r, s0, x0);
         }
       } else {
-        for (int64_t e = threadIdx.x; e < (int64_t)bc * r; e += blockDim.x) {
-          const int rr = e % bc, c = e / bc;
-          Xo[e] = (rr == c) ? 1.0 : 0.0;
+        // RQ of the kept rows R P^T = S Q': QR of X2 (mv x r) = (R P^T)^T J, S = J Rt^T J
+        const GrpScratch x1 = scratch_of(1);
+        double* X2 = Mtmp;
+        for (int e = half.tid; e < mv * r; e += half.nt) {
+          const int c = e % mv, row = r - 1 - e / mv;
+          if (in_smem) X2[e] = rrqr_r(Mm, ldm, at, row, c);
+          else X2[jpvt[c] + (int64_t)(e / mv) * mv] = row <= c ? Rm[row + (int64_t)c * mu] : 0.0;
         }
-        __syncthreads();
-        if (!in_smem) {
-          // a core in L2: the reflectors in panels of QRB (T factors in M0,
-          // free in this branch), applied as blocked WY -- one reflector at a
-          // time would sweep the r x r block once per reflector
-          cta_form_t(mu, r, Mm, mu, tc, M0, smP, smT);
-          cta_apply_q_blocked<RECOMP_THREADS>(mu, r, Mm, mu, M0, r, Xo, (int64_t)bc, Wq, smP, smT, gsm, r);
-        } else {
-          cta_apply_q(mu, r, Mm, mu, tc, r, Xo, (int64_t)bc);
+        half.sync();
+        double* smP = in_smem ? region + core_need : region;
+        const int w2 = min((int)GQ, (int)((RECOMP_REGION - (in_smem ? core_need : 0)) / panel_ld(mv)));
+        double* Tfr = base + L.tfr;
+        double* Rt = Y1;                       // r x r
+        g_qr(half, mv, r, X2, mv, Rt, r, Tfr, w2, smP, sh.gs[1], x1);
+        for (int e = half.tid; e < r * r; e += half.nt) {
+          const int a = e % r, c = e / r;
+          const int ra = r - 1 - c, ca = r - 1 - a;
+          Sc[a + (int64_t)c * A.kcap] = T(ra <= ca ? Rt[ra + (int64_t)ca * r] : 0.0);
         }
-      }
-      // X2 (mv x r) = R_perm^T J, R_perm[:, jpvt[c']] = R[:, c']
-      for (int c = threadIdx.x; c < mv; c += blockDim.x) jinv[jpvt[c]] = c;
-      __syncthreads();
-      double* X2 = t_sm ? region + voff : Mtmp;
-      for (int64_t e = threadIdx.x; e < (int64_t)mv * r; e += blockDim.x) {
-        const int c = e % mv, a = e / mv;
-        const int row = r - 1 - a, src = jinv[c];
-        X2[e] = (row <= src) ? Mm[row + (int64_t)src * mu] : 0.0;
-      }
-      __syncthreads();
-      if (!in_smem) cta_qr_blocked<RECOMP_THREADS>(mv, r, X2, mv, tau2, M0, Wq, smP, smT, gsm, red);
-      else cta_householder_qr(mv, r, X2, mv, tau2, red);
-      // S = J Rt^T J (upper triangular)
-      for (int64_t e = threadIdx.x; e < (int64_t)r * r; e += blockDim.x) {
-        const int a = e % r, c = e / r;
-        const int ra = r - 1 - c, ca = r - 1 - a;
-        Sc[a + (int64_t)c * A.kcap] = T((ra <= ca) ? X2[ra + (int64_t)ca * mv] : 0.0);
-      }
-      // Qt (mv x r) explicit, then Yo[:, a] = [Qt[:, r-1-a]; 0]
-      double* Qt = t_sm ? X2 + (int64_t)mv * r : Rc;
-      for (int64_t e = threadIdx.x; e < (int64_t)mv * r; e += blockDim.x) {
-        const int rr = e % mv, c = e / mv;
-        Qt[e] = (rr == c) ? 1.0 : 0.0;
-      }
-      __syncthreads();
-      if (!in_smem)
-        cta_apply_q_blocked<RECOMP_THREADS>(mv, r, X2, mv, M0, r, Qt, (int64_t)mv, Wq, smP, smT, gsm, r);
-      else
-        cta_apply_q(mv, r, X2, mv, tau2, r, Qt, (int64_t)mv);
-      for (int64_t e = threadIdx.x; e < (int64_t)bk * r; e += blockDim.x) {
-        const int rr = e % bk, a = e / bk;
-        Yo[e] = (rr < mv) ? Qt[rr + (int64_t)(r - 1 - a) * mv] : 0.0;
+        double* Qt = Gv;                       // R has been read
+        for (int e = half.tid; e < mv * r; e += half.nt) Qt[e] = (e % mv) == (e / mv) ? 1.0 : 0.0;
+        half.sync();
+        g_apply_q(half, mv, r, X2, mv, Tfr, w2, r, Qt, mv, r, sh.gs[1], x1);
+        for (int e = half.tid; e < mv * r; e += half.nt) Y1[e] = Qt[e % mv + (int64_t)(r - 1 - e / mv) * mv];
       }
       __syncthreads();
     } else {
-      // SVD core (Rc / Rv are free once the core is formed: Jacobi scratch)
-      r = svd_core<T, RECOMP_THREADS>(mu, mv, Mm, ws, A.kcap, region, RECOMP_REGION, Rc, tau_c, cnorm, pnorm, jpvt,
-                                      tau2, jinv, Xo, bc, Yo, bk, gsm, red, redi, &flag, &s_rank);
-      for (int64_t e = threadIdx.x; e < (int64_t)r * r; e += blockDim.x) {
+      double* pn = base + L.pn;
+      r = svd_core<T, RECOMP_THREADS>(mu, mv, Mm, ldm, in_smem, ws, A.kcap, region, RECOMP_REGION, Tv,
+                                      base + L.tau_c, base + L.cn, pn, jpvt, base + L.sig,
+                                      reinterpret_cast<int*>(base + L.ji), X1, Y1, sh, &s_rank);
+      for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
         const int rr = e % r, c = e / r;
-        Sc[rr + (int64_t)c * A.kcap] = T(rr == c ? pnorm[c] : 0.0);
+        Sc[rr + (int64_t)c * A.kcap] = T(rr == c ? pn[c] : 0.0);
       }
       __syncthreads();
     }
@@ -1616,43 +1664,28 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
       atomicAdd(ws.flops + FLOP_RECOMP,
                 (unsigned long long)(proj ? fast_rounded_addition_flops(bc, bk, bi, kc, o.p, o.q, r)
                                           : rounded_addition_flops(bc, bk, bi, kc, o.p, o.q, r)));
-    if (!proj) {
-      // U = Qu Xo ; Vt = Qv Yo  (blocked WY application)
-      // Xo = [Q_core; 0], Yo = [V_core; 0]: rows at or below mu (mv) are zero
-      cta_apply_q_blocked<RECOMP_THREADS>(bc, mu, Ash, bc, Tfu, r, Xo, (int64_t)bc, Wq, smP, smT, gsm, mu);
-      cta_apply_q_blocked<RECOMP_THREADS>(bk, mv, Bsh, bk, Tfv, r, Yo, (int64_t)bk, Wq, smP, smT, gsm, mv);
-      for (int64_t e = threadIdx.x; e < (int64_t)bc * r; e += blockDim.x) {
-        const int rr = e % bc, c = e / bc;
-        Uc[rr + (int64_t)c * ld] = T(Xo[e]);
-      }
-      for (int64_t e = threadIdx.x; e < (int64_t)bk * r; e += blockDim.x) {
-        const int rr = e % bk, c = e / bk;
-        Vc[rr + (int64_t)c * ld] = T(Yo[e]);
-      }
-    } else {
-      // U = [U_C | Q_u] Xo = Q_u [Xo(kc:mu); 0] + U_C Xo(0:kc), through Tm
-      // (bc x r); U_C is read from its FP64 copy in Ash, so Uc is written last
-      for (int side2 = 0; side2 < 2; ++side2) {
-        const int bb = side2 ? bk : bc, pp = side2 ? o.q : o.p;
-        double* X = side2 ? Yo : Xo;
-        double* Bs = side2 ? Bsh : Ash;
-        T* out = side2 ? Vc : Uc;
-        for (int64_t e = threadIdx.x; e < (int64_t)bb * r; e += blockDim.x) {
-          const int rr = e % bb, c = e / bb;
-          Tm[e] = rr < pp ? X[kc + rr + (int64_t)c * bb] : 0.0;
-        }
-        __syncthreads();
-        cta_apply_q_blocked<RECOMP_THREADS>(bb, pp, Bs + (int64_t)kc * bb, bb, side2 ? Tfv : Tfu, r, Tm, (int64_t)bb,
-                                            Wq, smP, smT, gsm, pp);
-        if (r <= 16) cta_gemm_tall(bb, r, kc, Bs, bb, X, bb, Tm, bb, true);
-        else cta_gemm<double, RECOMP_THREADS>(bb, r, kc, 1.0, Bs, bb, false, X, bb, false, 1.0, Tm, bb, gsm);
-        for (int64_t e = threadIdx.x; e < (int64_t)bb * r; e += blockDim.x) {
-          const int rr = e % bb, c = e / bb;
-          out[rr + (int64_t)c * ld] = T(Tm[e]);
-        }
-        __syncthreads();
-      }
+    {
+      // new bases, a side per half.  Stacked: U = Qu [X1; 0]; projected:
+      // U = [U_C | Q_u] X1 = Q_u [X1(kc:); 0] + U_C X1(:kc), in FP64 scratch
+      // (U_C is an operand, so the block itself is written last)
+      const int bb = hf ? bk : bc, pp = hf ? o.q : o.p, mm = hf ? mv : mu;
+      const double* X = hf ? Y1 : X1;
+      double* Tn = hf ? Tv : Tm;
+      T* out = hf ? Vc : Uc;
+      const GrpScratch x = scratch_of(hf);
+      const int skip = proj ? kc : 0, refl = proj ? pp : mm;
+      for (int c = half.wid; c < r; c += half.nw)
+#pragma unroll 4
+        for (int e = threadIdx.x & 31; e < bb; e += 32)
+          Tn[e + (int64_t)c * bb] = e < refl ? X[skip + e + (int64_t)c * mm] : 0.0;
+      half.sync();
+      g_apply_q(half, bb, refl, hf ? Bsh : Ash, bb, base + (hf ? L.tfv : L.tfu), wp, r, Tn, bb, refl, sh.gs[hf], x);
+      if (proj) g_gemm(half, bb, r, kc, 1.0, (const T*)out, ld, false, X, mm, false, 1.0, Tn, bb, sh.gs[hf].part);
+      for (int c = half.wid; c < r; c += half.nw)
+#pragma unroll 4
+        for (int e = threadIdx.x & 31; e < bb; e += 32) out[e + (int64_t)c * ld] = T(Tn[e + (int64_t)c * bb]);
     }
+    __syncthreads();
     if (threadIdx.x == 0) A.rank[blk] = r;
     __syncthreads();
   }

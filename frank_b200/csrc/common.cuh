@@ -243,7 +243,7 @@ FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, con
 // nw / 2 8 x 8 tiles splits the inner dimension over the warps, with the
 // partial tiles (at most 32 of them) summed in warp order through smem.
 template <int NT, typename TA, typename TB, typename TC>
-__device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha, const TA* A, int64_t lda, bool ta,
+static __device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha, const TA* A, int64_t lda, bool ta,
                                        const TB* B, int64_t ldb, bool tb, double beta, TC* C, int64_t ldc,
                                        double* smem) {
   constexpr int nw = NT / 32;
@@ -518,276 +518,6 @@ FRANK_D int cta_jacobi_columns(int m, int n, double* G, int64_t ldg, int max_swe
 }  // namespace frank
 
 namespace frank {
-
-// ---------------------------------------------------------------------------
-// Blocked Householder QR in FP64 (LAPACK dgeqrf with dgeqr2 panels, dlarft
-// forward/columnwise T factors and dlarfb trailing updates), column-major A
-// (m x n, lda) in global memory.  Panels of QRB columns are factored in shared
-// memory; the trailing matrix is updated as A -= V (T^T (V^T A)) by two
-// CTA GEMMs.  On return A holds R and the reflectors, tau[min(m,n)], and the
-// T factor of panel p at Tf + p*QRB*QRB (column-major, ld QRB).
-// Shared memory: smP (m*QRB doubles), smT (QRB*QRB), gsm (cta_gemm tiles),
-// red (32).  Global scratch W (QRB x n doubles).
-// ---------------------------------------------------------------------------
-constexpr int QRB = 32;
-
-// After the call, p[0] of lane l holds the sum over the warp of p[l] (the 32
-// sums of a warp's 32-vectors, one per lane, by recursive halving: 31
-// exchanges instead of 32 butterfly reductions).
-FRANK_D void warp_transpose_sum(double (&p)[32]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k = 16; k >= 1; k >>= 1) {
-    const bool up = (lane & k) != 0;
-#pragma unroll
-    for (int i = 0; i < k; ++i) {
-      const double send = up ? p[i] : p[i + k];
-      const double keep = up ? p[i + k] : p[i];
-      p[i] = keep + __shfl_xor_sync(0xffffffffu, send, k);
-    }
-  }
-}
-
-// W (jn x r, ld QRB) = V^T X over rows [0, kr): V (jn <= 32 columns, ldv) in
-// shared memory, X (ldx) anywhere.  One warp per column of X, lanes down the
-// rows with jn partial sums each, then warp_transpose_sum.  Ends with a
-// block barrier.
-template <typename TX>
-FRANK_D void panel_vtx(int kr, int jn, const double* smV, int64_t ldv, const TX* X, int64_t ldx, int r, double* W) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // (column of X, half of V's columns) per warp: 16 partial sums per lane
-  const int halves = jn > 16 ? 2 : 1;
-  for (int t = wid; t < r * halves; t += nw) {
-    const int c = t / halves, j0 = (t % halves) * 16;
-    const int jm = min(16, jn - j0);
-    const TX* xc = X + (int64_t)c * ldx;
-    const double* vb = smV + (int64_t)j0 * ldv;
-    double p[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) p[j] = 0.0;
-    int row = lane;
-    for (; row + 96 < kr; row += 128) {
-      const double x0 = double(xc[row]), x1 = double(xc[row + 32]), x2 = double(xc[row + 64]),
-                   x3 = double(xc[row + 96]);
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (j < jm) {
-          const double* v = vb + (int64_t)j * ldv + row;
-          p[j] += v[0] * x0 + v[32] * x1 + v[64] * x2 + v[96] * x3;
-        }
-    }
-    for (; row < kr; row += 32) {
-      const double xv = double(xc[row]);
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (j < jm) p[j] += vb[row + (int64_t)j * ldv] * xv;
-    }
-    // recursive halving over 16 values, then one butterfly level: lane l
-    // (l < 16) ends with the sum of p[l]
-#pragma unroll
-    for (int k = 8; k >= 1; k >>= 1) {
-      const bool up = (lane & k) != 0;
-#pragma unroll
-      for (int i = 0; i < k; ++i) {
-        const double send = up ? p[i] : p[i + k];
-        const double keep = up ? p[i + k] : p[i];
-        p[i] = keep + __shfl_xor_sync(0xffffffffu, send, k);
-      }
-    }
-    const double tot = p[0] + __shfl_xor_sync(0xffffffffu, p[0], 16);
-    if (lane < jm) W[j0 + lane + (int64_t)c * QRB] = tot;
-  }
-  __syncthreads();
-}
-
-// X (rows [0, mr), r columns, ldx) -= V W with V (mr x jn, ldv) in shared
-// memory and W (jn x r, ld QRB): one thread per row, the row of V in
-// registers.  Ends with a block barrier.
-FRANK_D void panel_x_minus_vw(int mr, int jn, const double* smV, int64_t ldv, const double* W, int r, double* X,
-                              int64_t ldx) {
-  for (int row = threadIdx.x; row < mr; row += blockDim.x) {
-    double v[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = (j < jn) ? smV[row + (int64_t)j * ldv] : 0.0;
-    int c = 0;
-    for (; c + 1 < r; c += 2) {
-      const double* w0 = W + (int64_t)c * QRB;
-      const double* w1 = w0 + QRB;
-      double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < jn) { a0 += v[j] * w0[j]; a1 += v[j] * w1[j]; }
-      double* x0 = X + row + (int64_t)c * ldx;
-      double* x1 = x0 + ldx;
-      const double y0 = *x0, y1 = *x1;
-      *x0 = y0 - a0;
-      *x1 = y1 - a1;
-    }
-    if (c < r) {
-      const double* w0 = W + (int64_t)c * QRB;
-      double a0 = 0.0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < jn) a0 += v[j] * w0[j];
-      X[row + (int64_t)c * ldx] -= a0;
-    }
-  }
-  __syncthreads();
-}
-
-// Gram-based T factor of the panel V (mr x jn, unit lower trapezoid in smV).
-FRANK_D void cta_larft(int mr, int jn, const double* smV, const double* tau, double* smT) {
-  // G = V^T V (jn x jn, in smT), then T column by column (dlarft recurrence
-  // T(0:j, j) = -tau_j T(0:j, 0:j) G(0:j, j)): lane i keeps row i of T in
-  // registers, so the recurrence needs no barrier between columns.
-  panel_vtx(mr, jn, smV, mr, smV, mr, jn, smT);
-  if (threadIdx.x < 32) {
-    const int i = threadIdx.x;
-    double trow[32];
-#pragma unroll
-    for (int l = 0; l < 32; ++l) trow[l] = 0.0;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if (j < jn) {
-        double s = 0.0;
-#pragma unroll
-        for (int l = 0; l < 32; ++l)
-          if (l < j && l >= i) s += trow[l] * smT[l + j * QRB];
-        if (i < j) trow[j] = -tau[j] * s;
-        else if (i == j) trow[j] = tau[j];
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int l = 0; l < 32; ++l)
-      if (i < QRB && l < QRB) smT[i + l * QRB] = (i < jn && l < jn && l >= i) ? trow[l] : 0.0;
-  }
-  __syncthreads();
-}
-
-// Load the panel's reflectors from A (rows j0.., cols j0..j0+jn) into smV as a
-// clean unit-lower-trapezoidal matrix (mr x jn, ld mr).
-FRANK_D void cta_load_v(int mr, int jn, const double* Ap, int64_t lda, double* smV) {
-  for (int e = threadIdx.x; e < mr * jn; e += blockDim.x) {
-    const int r = e % mr, c = e / mr;
-    smV[e] = (r > c) ? Ap[r + (int64_t)c * lda] : (r == c ? 1.0 : 0.0);
-  }
-  __syncthreads();
-}
-
-
-template <int NT>
-FRANK_D void cta_qr_blocked(int m, int n, double* A, int64_t lda, double* tau, double* Tf, double* W,
-                            double* smP, double* smT, double* gsm, double* red, int max_panels = 1 << 20,
-                            int max_jn = QRB) {
-  const int kmin = m < n ? m : n;
-  for (int j0 = 0; j0 < kmin && j0 / QRB < max_panels; j0 += QRB) {
-    const int jn = min(min(QRB, max_jn), kmin - j0);
-    const int mr = m - j0;
-    double* Ap = A + j0 + (int64_t)j0 * lda;
-    for (int e = threadIdx.x; e < mr * jn; e += blockDim.x) {
-      const int r = e % mr, c = e / mr;
-      smP[e] = Ap[r + (int64_t)c * lda];
-    }
-    __syncthreads();
-    cta_householder_qr(mr, jn, smP, mr, tau + j0, red);
-    for (int e = threadIdx.x; e < mr * jn; e += blockDim.x) {
-      const int r = e % mr, c = e / mr;
-      Ap[r + (int64_t)c * lda] = smP[e];
-      smP[e] = (r > c) ? smP[e] : (r == c ? 1.0 : 0.0);
-    }
-    __syncthreads();
-    cta_larft(mr, jn, smP, tau + j0, smT);
-    double* Tp = Tf + (int64_t)(j0 / QRB) * QRB * QRB;
-    for (int e = threadIdx.x; e < QRB * QRB; e += blockDim.x) Tp[e] = smT[e];
-    const int nc = n - j0 - jn;
-    if (nc > 0) {
-      double* At = A + j0 + (int64_t)(j0 + jn) * lda;
-      // W = V^T At (jn x nc)
-      panel_vtx(mr, jn, smP, mr, At, lda, nc, W);
-      // W = T^T W (T upper triangular): column per thread
-      for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        // unrolled over the panel width so that w stays in registers
-        double w[QRB];
-#pragma unroll
-        for (int i = 0; i < QRB; ++i) w[i] = (i < jn) ? W[i + (int64_t)c * QRB] : 0.0;
-#pragma unroll
-        for (int i = QRB - 1; i >= 0; --i) {
-          if (i < jn) {
-            double s = 0.0;
-#pragma unroll
-            for (int l = 0; l <= i; ++l) s += smT[l + i * QRB] * w[l];
-            W[i + (int64_t)c * QRB] = s;
-          }
-        }
-      }
-      __syncthreads();
-      // At -= V W
-      panel_x_minus_vw(mr, jn, smP, mr, W, nc, At, lda);
-    }
-  }
-  __syncthreads();
-}
-
-// X (m x r, ldx, FP64) := Q X with Q from cta_qr_blocked (k = min(m, ncols)
-// reflectors).  Panels applied last to first: X -= V (T (V^T X)).  Rows of X
-// at or below nz are zero on entry (nz = m if unknown): the first panel
-// applied then only contracts rows j0 .. nz-1 in V^T X.
-template <int NT>
-FRANK_D void cta_apply_q_blocked(int m, int k, const double* A, int64_t lda, const double* Tf, int r,
-                                 double* X, int64_t ldx, double* W, double* smP, double* smT, double* gsm,
-                                 int nz = -1) {
-  if (k <= 0 || r <= 0) { __syncthreads(); return; }
-  if (nz < 0 || nz > m) nz = m;
-  const int np = (k + QRB - 1) / QRB;
-  for (int p = np - 1; p >= 0; --p) {
-    const int j0 = p * QRB;
-    const int jn = min(QRB, k - j0);
-    const int mr = m - j0;
-    const int kr = min(mr, max(0, nz - j0));   // rows of X that can be nonzero
-    nz = m;                                    // after this panel X is full
-    if (kr == 0) continue;                     // V^T X = 0: the panel is the identity on X
-    cta_load_v(mr, jn, A + j0 + (int64_t)j0 * lda, lda, smP);
-    for (int e = threadIdx.x; e < QRB * QRB; e += blockDim.x) smT[e] = Tf[(int64_t)p * QRB * QRB + e];
-    __syncthreads();
-    double* Xp = X + j0;
-    panel_vtx(kr, jn, smP, mr, Xp, ldx, r, W);
-    for (int c = threadIdx.x; c < r; c += blockDim.x) {
-      // unrolled over the panel width so that w stays in registers
-      double w[QRB];
-#pragma unroll
-      for (int i = 0; i < QRB; ++i) w[i] = (i < jn) ? W[i + (int64_t)c * QRB] : 0.0;
-#pragma unroll
-      for (int i = 0; i < QRB; ++i) {
-        if (i < jn) {
-          double s = 0.0;
-#pragma unroll
-          for (int l = i; l < QRB; ++l) s += smT[i + l * QRB] * w[l];
-          W[i + (int64_t)c * QRB] = s;
-        }
-      }
-    }
-    __syncthreads();
-    panel_x_minus_vw(mr, jn, smP, mr, W, r, Xp, ldx);
-  }
-}
-
-// T factors (dlarft, forward / columnwise) of the first k Householder
-// reflectors stored below the diagonal of A (m rows, lda; tau), panel by panel
-// of QRB columns into Tf + p * QRB * QRB -- the layout cta_apply_q_blocked
-// reads -- for reflectors produced by a column-by-column factorization.
-FRANK_D void cta_form_t(int m, int k, const double* A, int64_t lda, const double* tau, double* Tf, double* smP,
-                        double* smT) {
-  for (int j0 = 0; j0 < k; j0 += QRB) {
-    const int jn = min(QRB, k - j0);
-    const int mr = m - j0;
-    cta_load_v(mr, jn, A + j0 + (int64_t)j0 * lda, lda, smP);
-    cta_larft(mr, jn, smP, tau + j0, smT);
-    double* Tp = Tf + (int64_t)(j0 / QRB) * QRB * QRB;
-    for (int e = threadIdx.x; e < QRB * QRB; e += blockDim.x) Tp[e] = smT[e];
-    __syncthreads();
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Truncated column-pivoted Householder QR (restating
@@ -1099,162 +829,6 @@ FRANK_D int cta_truncated_geqp3_blocked(int m, int n, double* A, int64_t lda, do
       if (r >= n) maxc = 0.0;
     }
     if (k == 0) break;
-  }
-  __syncthreads();
-  return r;
-}
-
-
-// ---------------------------------------------------------------------------
-// Truncated column-pivoted QR with randomized block pivoting (Martinsson,
-// Quintana-Orti, Heavner, van de Geijn, "Householder QR factorization with
-// randomization for column pivoting (HQRRP)", SIAM J. Sci. Comput. 39, 2017):
-// per panel of QRB columns, a sketch Y = Omega A_trail (QRB + 8 rows, Omega
-// uniform in [-1, 1) from a counter-based hash) picks the panel's pivots by a
-// pivoted QR of Y, the chosen columns move to the panel, and an unpivoted
-// blocked Householder step factors the panel and updates the trailing matrix
-// with two CTA GEMMs -- instead of one pivot search and one pass over the
-// trailing matrix per column.  The stopping rule is the unblocked one,
-// evaluated exactly: after each panel the norms of every remaining column at
-// every step t of the panel follow from the updated rows (the later
-// reflectors act orthogonally below row t), and the rank is the first step
-// whose remaining columns are all at most thr.  Same outputs as
-// cta_truncated_geqp3 (R and reflectors in A, tau, jpvt); the pivots are a
-// randomized choice, so ranks can differ from the column-by-column search by
-// a few.  Scratch ws (global): 40 (m + n) + 40 + 33 n + 8 n + QRB^2 doubles
-// (rqrcp_scratch); smP / smT / gsm as cta_qr_blocked.  Returns the rank.
-// ---------------------------------------------------------------------------
-FRANK_HD int64_t rqrcp_scratch(int m, int n) {
-  return 40 * ((int64_t)m + n) + 40 + 33 * (int64_t)n + 8 * (int64_t)n + 32 * 32 + 64;
-}
-
-FRANK_D double rqrcp_omega(uint64_t k) {
-  k += 0x9E3779B97F4A7C15ull;
-  k = (k ^ (k >> 30)) * 0xBF58476D1CE4E5B9ull;
-  k = (k ^ (k >> 27)) * 0x94D049BB133111EBull;
-  k ^= k >> 31;
-  return (double)(k >> 11) * (2.0 / 9007199254740992.0) - 1.0;
-}
-
-template <int NT>
-FRANK_D int cta_rand_qrcp(int m, int n, double* A, int64_t lda, double thr, int maxr, double* tau, int* jpvt,
-                          double* ws, double* smP, double* smT, double* gsm, double* red, int* redi) {
-  constexpr int SBMAX = QRB + 8;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int mind = min(min(m, n), maxr);
-  double* Om = ws;                                   // SBMAX x m
-  double* Y = Om + (int64_t)SBMAX * m;               // SBMAX x n
-  double* tau_s = Y + (int64_t)SBMAX * n;            // SBMAX
-  double* cn_s = tau_s + SBMAX;                      // n
-  double* pn_s = cn_s + n;                           // n
-  double* nrm2 = pn_s + n;                           // n
-  double* Wt = nrm2 + n;                             // QRB x n
-  double* Tf = Wt + (int64_t)QRB * n;                // QRB x QRB
-  int* jp_s = reinterpret_cast<int*>(Tf + QRB * QRB);   // n
-  int* pos = jp_s + n;                               // n
-  int* inv = pos + n;                                // n
-  int* swp = inv + n;                                // QRB
-  for (int c = threadIdx.x; c < n; c += blockDim.x) jpvt[c] = c;
-  // the unblocked rule's first test: every column at most thr
-  double best = 0.0;
-  for (int c = wid; c < n; c += nw) {
-    double s2 = 0.0;
-    for (int e = lane; e < m; e += 32) s2 += A[e + (int64_t)c * lda] * A[e + (int64_t)c * lda];
-    s2 = warp_sum(s2);
-    best = fmax(best, s2);
-  }
-  if (lane == 0) red[wid] = best;
-  __syncthreads();
-  best = 0.0;
-  for (int w = 0; w < nw; ++w) best = fmax(best, red[w]);
-  __syncthreads();
-  if (mind == 0 || sqrt(best) <= thr) return 0;
-  int r = 0;
-  int panel = 0;
-  while (r < mind) {
-    const int b = min(QRB, mind - r);
-    const int mr = m - r, nr = n - r;
-    const int sb = min(b + 8, mr);
-    // 1. sketch of the trailing matrix
-    for (int64_t e = threadIdx.x; e < (int64_t)sb * mr; e += blockDim.x)
-      Om[e] = rqrcp_omega(((uint64_t)panel << 40) ^ (uint64_t)e);
-    __syncthreads();
-    cta_gemm<double, NT>(sb, nr, mr, 1.0, Om, sb, false, A + r + (int64_t)r * lda, lda, false, 0.0, Y, sb, gsm);
-    // 2. the panel's pivots: b steps of the pivoted QR of the sketch
-    cta_truncated_geqp3(sb, nr, Y, sb, -1.0, b, tau_s, cn_s, pn_s, jp_s, red, redi);
-    // 3. swaps that bring the chosen columns to r .. r+b-1, then applied row-parallel
-    if (threadIdx.x == 0) {
-      for (int c = 0; c < nr; ++c) { pos[c] = c; inv[c] = c; }
-      for (int t = 0; t < b; ++t) {
-        const int want = jp_s[t], cur = pos[want], o = inv[t];
-        swp[t] = cur;
-        inv[t] = want; inv[cur] = o; pos[want] = t; pos[o] = cur;
-        const int q = jpvt[r + t]; jpvt[r + t] = jpvt[r + cur]; jpvt[r + cur] = q;
-      }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < m; e += blockDim.x)
-      for (int t = 0; t < b; ++t) {
-        const int cur = swp[t];
-        if (cur != t) {
-          double* a0 = A + e + (int64_t)(r + t) * lda;
-          double* a1 = A + e + (int64_t)(r + cur) * lda;
-          const double v = *a0; *a0 = *a1; *a1 = v;
-        }
-      }
-    __syncthreads();
-    // 4. unpivoted Householder panel and its trailing update
-    cta_qr_blocked<NT>(mr, nr, A + r + (int64_t)r * lda, lda, tau + r, Tf, Wt, smP, smT, gsm, red, 1, b);
-    // 5. exact norms of the remaining columns at every step t of the panel:
-    //    panel column j (t <= j < b): sum_{i=t..j} R(r+i, r+j)^2; trailing
-    //    column c: ||A(r+b:, c)||^2 + sum_{i=t..b-1} A(r+i, c)^2
-    for (int c = r + b + wid; c < n; c += nw) {
-      double s2 = 0.0;
-      for (int e = r + b + lane; e < m; e += 32) s2 += A[e + (int64_t)c * lda] * A[e + (int64_t)c * lda];
-      s2 = warp_sum(s2);
-      if (lane == 0) nrm2[c] = s2;
-    }
-    __syncthreads();
-    // maxima over columns per step t, as the bits of non-negative doubles
-    // (ordered like unsigned integers) in gsm
-    unsigned long long* mx = reinterpret_cast<unsigned long long*>(gsm);
-    for (int t = threadIdx.x; t <= QRB; t += blockDim.x) mx[t] = 0ull;
-    __syncthreads();
-    for (int c0 = r + b; c0 < n; c0 += blockDim.x) {
-      const int c = c0 + threadIdx.x;
-      const bool on = c < n;
-      double s2 = on ? nrm2[c] : 0.0;
-      double v = s2;
-      for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (lane == 0) atomicMax(mx + b, (unsigned long long)__double_as_longlong(v));
-      for (int t = b - 1; t >= 0; --t) {
-        if (on) {
-          const double a = A[r + t + (int64_t)c * lda];
-          s2 += a * a;
-        }
-        v = s2;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0) atomicMax(mx + t, (unsigned long long)__double_as_longlong(v));
-      }
-    }
-    for (int j = threadIdx.x; j < b; j += blockDim.x) {
-      double s2 = 0.0;
-      for (int t = j; t >= 0; --t) {
-        const double a = A[r + t + (int64_t)(r + j) * lda];
-        s2 += a * a;
-        atomicMax(mx + t, (unsigned long long)__double_as_longlong(s2));
-      }
-    }
-    __syncthreads();
-    // every thread reads the same maxima: the first step whose remaining
-    // columns are all at most thr (b: none in this panel)
-    int stop = -1;
-    for (int t = 0; t <= b; ++t)
-      if (sqrt(__longlong_as_double((long long)mx[t])) <= thr) { stop = t; break; }
-    __syncthreads();
-    if (stop >= 0) return r + stop;
-    r += b;
-    ++panel;
   }
   __syncthreads();
   return r;
@@ -1592,27 +1166,6 @@ FRANK_D void cta_gemm_tall(int m, int n, int k, const TA* A, int64_t lda, const 
   __syncthreads();
 }
 
-// Project the columns of Y (m x p, ldy) out of the span of Q (m x k, ldq,
-// orthonormal columns), twice (classical Gram-Schmidt with one
-// re-orthogonalisation): Z (k x p, ldz) = Q^T Y_0, Y = (I - Q Q^T)^2 Y_0,
-// Y_0 = Q Z + Y.  Z2 (k x p, ld k) is scratch.  Skinny shapes use the warp /
-// row kernels, larger ones the tiled CTA GEMM.
-template <int NT>
-FRANK_D void cta_project_out(int m, int k, int p, const double* Q, int64_t ldq, double* Y, int64_t ldy, double* Z,
-                             int64_t ldz, double* Z2, double* gsm) {
-  for (int pass = 0; pass < 2; ++pass) {
-    double* Zp = pass ? Z2 : Z;
-    const int64_t ldp = pass ? k : ldz;
-    if ((int64_t)k * p <= 1024) cta_gemm_tn_dot(k, p, m, 1.0, Q, ldq, Y, ldy, Zp, ldp);
-    else cta_gemm<double, NT>(k, p, m, 1.0, Q, ldq, true, Y, ldy, false, 0.0, Zp, ldp, gsm);
-    if (p <= 16) cta_gemm_tall(m, p, k, Q, ldq, Zp, ldp, Y, ldy, true, -1.0);
-    else cta_gemm<double, NT>(m, p, k, -1.0, Q, ldq, false, Zp, ldp, false, 1.0, Y, ldy, gsm);
-  }
-  for (int64_t e = threadIdx.x; e < (int64_t)k * p; e += blockDim.x) {
-    const int r = e % k, c = e / k;
-    Z[r + (int64_t)c * ldz] += Z2[e];
-  }
-  __syncthreads();
-}
-
 }  // namespace frank
+
+#include "groups.cuh"
