@@ -831,7 +831,7 @@ FRANK_D void leaf_final_body(const BlrView<T>& A, const FactorWs<T>& ws, int i) 
     int nt = 0;
     for (int tile = wid; tile < TW * TW; tile += nw, ++nt) {
       double c1[1][1][2];
-      warp_dgemm_acc<1, 1>(rn, cn, 0, rn, D, 1, W, X + r0, lds, 1, (tile % TW) * 8, (tile / TW) * 8, c1);
+      warp_dgemm_acc<1, 1, false>(rn, cn, 0, rn, D, 1, W, X + r0, lds, 1, (tile % TW) * 8, (tile / TW) * 8, c1);
 #pragma unroll
       for (int z = 0; z < (TW * TW + 3) / 4; ++z)
         if (z == nt) { acc[z][0] = c1[0][0][0]; acc[z][1] = c1[0][0][1]; }
@@ -854,7 +854,7 @@ FRANK_D void leaf_final_body(const BlrView<T>& A, const FactorWs<T>& ws, int i) 
     for (int tile = wid; um > 0 && tile < tm * tn; tile += nw) {
       const int i0 = (tile % tm) * 32, j0 = (tile / tm) * 16;
       double ac[4][2][2];
-      warp_dgemm_acc<4, 2>(um, cn, 0, rn, L.Wm + (int64_t)r0 * b, 1, b, X + r0, lds, 1, i0, j0, ac, [&](int r) {
+      warp_dgemm_acc<4, 2, false>(um, cn, 0, rn, L.Wm + (int64_t)r0 * b, 1, b, X + r0, lds, 1, i0, j0, ac, [&](int r) {
         const int a = u0 + r;
         return lower && a >= jl && rb < np - 1 ? src[a] : a;
       });
@@ -1081,9 +1081,9 @@ FRANK_D UpdOps<T> update_operands(const BlrView<T>& A, const FactorWs<T>& ws, in
 
 // core T (p x q) = -WL^T WU, FP64, into Tm (ld p).
 template <typename T>
-FRANK_D void form_core(const Grp& g, const UpdOps<T>& o, int bi, int ld, double* Tm, GrpShared& s, GrpScratch x) {
+FRANK_D void form_core(const Grp& g, const UpdOps<T>& o, int bi, int ld, double* Tm, const GrpScratch& x) {
   if (!o.left_dense && !o.right_dense) {
-    g_gemm_tn(g, o.p, o.q, bi, -1.0, o.WL, ld, o.WU, ld, Tm, o.p, x.part, s.part);
+    g_mm(g, o.p, o.q, bi, -1.0, o.WL, ld, 1, o.WU, ld, 1, 0.0, Tm, o.p, x.part);
   } else if (!o.left_dense && o.right_dense) {
     // -WL^T (p x bi)
     for (int64_t e = threadIdx.x; e < (int64_t)o.p * o.q; e += blockDim.x) {
@@ -1213,7 +1213,7 @@ constexpr int RECOMP_THREADS = 512;
 constexpr int SPLIT_P = 32;       // split band-1 targets whose operand rank exceeds this (default)
 constexpr int SPLIT_MAX = 128;    // band-1 tasks eligible for the split (scratch slots)
 constexpr int RECOMP_BMAX = 810;  // largest block order (a panel of each side in shared memory)
-constexpr int RECOMP_SMEM_BYTES = 227 * 1024 - 512;     // dynamic shared memory (all but the static part)
+constexpr int RECOMP_SMEM_BYTES = 227 * 1024 - 1024;    // dynamic shared memory (all but the static part)
 
 struct RecompShared {
   GrpShared gs[2];               // one per half of the CTA
@@ -1225,11 +1225,10 @@ struct RecompShared {
 };
 constexpr int RECOMP_REGION = (RECOMP_SMEM_BYTES - (int)sizeof(RecompShared)) / 8;  // doubles for panels / core
 
-// Panel width of the bases' QR: both sides' panels fit side by side.
-FRANK_HD int recomp_panel(int bmax) {
-  const int w = RECOMP_REGION / 2 / panel_ld(bmax);
-  return w < GQ ? w : GQ;
-}
+// Panel width of the bases' QR; the panels of both sides fit side by side.
+FRANK_HD int recomp_panel(int bmax) { return panel_width(bmax); }
+static_assert(2 * ((RECOMP_BMAX + 15) / 16 * 16 + 4) * 8 <= RECOMP_REGION && 2 * (512 + 4) * GQ <= RECOMP_REGION,
+              "panels of both sides in shared memory");
 
 // Core of the recompression: RRQR (truncated pivoted QR + RQ of the core),
 // SVD (one-sided Jacobi, find_svd_truncation_rank or the fixed rank), FAST
@@ -1412,7 +1411,7 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
   L.tfr = take((mu / 8 + 2) * (int64_t)GQ * GQ);
   L.om = take((GQ + 8) * (int64_t)mu);
   L.w = take(4 * (int64_t)GQ * (smax > bmax ? smax : bmax));
-  L.part = take(2 * (int64_t)G_TN_PART);
+  L.part = take(2 * (int64_t)G_PART);
   L.tau_c = take(mu);
   L.sig = take(mu);
   L.cn = take(mu);
@@ -1423,8 +1422,30 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
   return L;
 }
 
+// One target's operands and scratch, in shared memory: the phases below are
+// long and inlined, and values kept in registers across all of them would
+// spill to local memory (beside 226 KB of shared memory there is no L1 left to
+// hold spills).
 template <typename T>
-FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
+struct RecompSide {
+  const T* X;                  // update basis (XL or YR)
+  T* C;                        // the target's basis
+  double *S, *G, *Tf, *Tn, *Z2;
+  GrpScratch x;
+  int bb, pp, mm, xt;          // rows, update rank, core dimension, X transposed
+};
+
+template <typename T>
+struct RecompTask {
+  RecompSide<T> s[2];
+  UpdOps<T> o;
+  double *base, *Tm, *Mtmp, *Mg, *Y1;
+  T* Sc;
+  int blk, kc, mu, mv, proj, side, tsk, ok;
+};
+
+template <typename T>
+FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i, int smax,
                                                                int core_method, double core_scale,
                                                                int only_dense_operands, int* counter, int nsplit,
                                                                double* split_base, int* split_done, int proj_tol,
@@ -1433,116 +1454,114 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
   RecompShared& sh = *reinterpret_cast<RecompShared*>(dsm);
   double* region = dsm + sizeof(RecompShared) / 8;
   __shared__ int s_rank, s_last, s_task;
-  const int m = A.nb - i - 1;
-  const int ld = A.bmax;
-  const int bi = A.bs(i);
-  const RecompLayout L = recomp_layout(A.bmax, smax);
-  const int wp = recomp_panel(A.bmax);
-  const Grp all = grp_all();
+  __shared__ RecompTask<T> tk;
   const int hf = threadIdx.x >= RECOMP_THREADS / 2;
-  const Grp half = grp_half(hf);
-  const int ntask = m * (m - 1);
-  // Split targets: band-1 targets (the first 2(m-1) tasks, largest ranks)
-  // whose operands have ranks above SPLIT_P get one task per side of the
-  // bases' QR, run on two CTAs into the target's own scratch slot;
-  // the CTA that finishes second does the rest (no waiting).  The test uses
-  // only operand ranks, which no CTA changes during the launch.
-  const int nspl = split_base ? min(nsplit, 2 * (m - 1)) : 0;
-  const int ntot = 2 * nspl + ntask;
-  for (int q = next_task(counter, &s_task); q < ntot; q = next_task(counter, &s_task)) {
-    const int side = q < 2 * nspl ? (q & 1) : -1;
-    const int tsk = q < 2 * nspl ? (q >> 1) : q - 2 * nspl;
-    int a_, c_;
-    band_task(m, tsk, a_, c_);
-    const int ic = i + 1 + a_, k = i + 1 + c_;
-    if (!A.is_lr(ic, k)) continue;
-    if (only_dense_operands && A.is_lr(ic, i) && A.is_lr(i, k)) continue;
-    const bool split_t = tsk < nspl && split_p > 0 && A.is_lr(ic, i) && A.is_lr(i, k) &&
-                         max(A.rank[ic * A.nb + i], A.rank[i * A.nb + k]) > split_p;
-    if ((side >= 0) != split_t) continue;
-    double* const base = side >= 0 ? split_base + (int64_t)tsk * ws.rscratch_stride
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    const int q = next_task(counter, &s_task);
+    // Split targets: band-1 targets (the first 2(m-1) tasks, largest ranks)
+    // whose operands have ranks above SPLIT_P get one task per side of the
+    // bases' QR, run on two CTAs into the target's own scratch slot;
+    // the CTA that finishes second does the rest (no waiting).  The test uses
+    // only operand ranks, which no CTA changes during the launch.
+    {
+      const int m = A.nb - i - 1;
+      const int nspl = split_base ? min(nsplit, 2 * (m - 1)) : 0;
+      if (q >= 2 * nspl + m * (m - 1)) break;
+      if (threadIdx.x == 0) {
+        const int side = q < 2 * nspl ? (q & 1) : -1;
+        const int tsk = q < 2 * nspl ? (q >> 1) : q - 2 * nspl;
+        int a_, c_;
+        band_task(m, tsk, a_, c_);
+        const int ic = i + 1 + a_, k = i + 1 + c_;
+        const bool ll = A.is_lr(ic, i), lr = A.is_lr(i, k);
+        const bool split_t = tsk < nspl && split_p > 0 && ll && lr &&
+                             max(A.rank[ic * A.nb + i], A.rank[i * A.nb + k]) > split_p;
+        tk.ok = A.is_lr(ic, k) && !(only_dense_operands && ll && lr) && (side >= 0) == split_t;
+        if (tk.ok) {
+          tk.o = update_operands(A, ws, i, ic, k);
+          tk.blk = ic * A.nb + k;
+          tk.kc = A.rank[tk.blk];
+          tk.side = side;
+          tk.tsk = tsk;
+          const int bc = A.bs(ic), bk = A.bs(k), kc = tk.kc, su = kc + tk.o.p, sv = kc + tk.o.q;
+          if (su > smax || sv > smax) {
+            atomicAdd(ws.err + ERR_BOUNDS, 1);
+            tk.ok = 0;
+          }
+          // Bases.  Stacked (rounded_addition, addition.cpp:93-127): Householder QR
+          // of [U_C | U_B] and of [V_C | V_B].  Projected (fast_rounded_addition,
+          // addition.cpp:133-189, the default of fixed-rank plans, and on request
+          // for tolerance plans): U_C and V_C have orthonormal columns (every
+          // target comes from construction, a core SVD / RRQR or the reset
+          // truncation), so U_B is projected out of span(U_C) twice, Zu = U_C^T U_B,
+          // and only the remainder Y_u = U_B - U_C Zu is QR-factored; the same on the
+          // V side.  Both give the same sum C + B = [U_C | Q] M [V_C | Q']^T.
+          tk.proj = (core_method == CORE_FAST ? ws.fixed_rank > 0 : proj_tol != 0) && kc > 0 && tk.o.p > 0 &&
+                    tk.o.q > 0 && !tk.o.left_dense && !tk.o.right_dense && su <= bc && sv <= bk;
+          tk.mu = tk.proj ? su : min(bc, su);
+          tk.mv = tk.proj ? sv : min(bk, sv);
+          const RecompLayout L = recomp_layout(A.bmax, smax);
+          double* base = side >= 0 ? split_base + (int64_t)tsk * ws.rscratch_stride
                                    : ws.rscratch + (int64_t)blockIdx.x * ws.rscratch_stride;
-    double *Ash = base + L.ash, *Bsh = base + L.bsh, *Tm = base + L.t, *Gu = base + L.gu, *Gv = base + L.gv,
-           *Mtmp = base + L.mtmp, *Mg = base + L.mglob, *Y1 = base + L.y1, *Tv = base + L.tv;
-    const int64_t wstep = (int64_t)GQ * max(smax, A.bmax);
-    auto scratch_of = [&](int sd) {
-      return GrpScratch{base + L.w + 2 * sd * wstep, base + L.w + (2 * sd + 1) * wstep, base + L.part + sd * (int64_t)G_TN_PART};
-    };
-    int* jpvt = reinterpret_cast<int*>(base + L.jp);
-    const int blk = ic * A.nb + k;
-    const int bc = A.bs(ic), bk = A.bs(k);
-    const int kc = A.rank[blk];
-    UpdOps<T> o = update_operands(A, ws, i, ic, k);
-    const int su = kc + o.p, sv = kc + o.q;
-    if (su > smax || sv > smax) {
-      if (threadIdx.x == 0) atomicAdd(ws.err + ERR_BOUNDS, 1);
-      continue;
-    }
-    T* Uc = A.u(ic, k);
-    T* Sc = A.s(ic, k);
-    T* Vc = A.vt(ic, k);
-    // Bases.  Stacked (rounded_addition, addition.cpp:93-127): Householder QR
-    // of [U_C | U_B] and of [V_C | V_B].  Projected (fast_rounded_addition,
-    // addition.cpp:133-189, the default of fixed-rank plans, and on request
-    // for tolerance plans): U_C and V_C have orthonormal columns (every
-    // target comes from construction, a core SVD / RRQR or the reset
-    // truncation), so U_B is projected out of span(U_C) twice, Zu = U_C^T U_B,
-    // and only the remainder Y_u = U_B - U_C Zu is QR-factored; the same on the
-    // V side.  Both give the same sum C + B = [U_C | Q] M [V_C | Q']^T.
-    const bool proj = (core_method == CORE_FAST ? ws.fixed_rank > 0 : proj_tol != 0) && kc > 0 && o.p > 0 &&
-                      o.q > 0 && !o.left_dense && !o.right_dense && su <= bc && sv <= bk;
-    const int mu = proj ? su : min(bc, su), mv = proj ? sv : min(bk, sv);
-    // one side's basis: projected, [Zu; Ru] (su x p) in Gu and the clean V of
-    // the remainder's QR in Ash; stacked, R (mu x su) in Gu and V in Ash
-    auto basis = [&](const Grp& g, int sd, double* smP) {
-      const int bb = sd ? bk : bc, pp = sd ? o.q : o.p, ss = kc + pp, mm = sd ? mv : mu;
-      const T* C = sd ? Vc : Uc;
-      const T* X = sd ? o.YR : o.XL;
-      const bool xt = sd && o.right_dense;     // A(i,k)^T
-      double* S = sd ? Bsh : Ash;
-      double* G = sd ? Gv : Gu;
-      double* Tf = base + (sd ? L.tfv : L.tfu);
-      const GrpScratch x = scratch_of(sd);
-      GrpShared& s = sh.gs[sd];
-      const int lane = threadIdx.x & 31;
-      if (proj) {
-        const bool one = pp <= wp;             // a single panel: kept in shared memory from the start
-        double* Y = one ? smP : S;
-        const int ldy = one ? panel_ld(bb) : bb;
-        for (int c = g.wid; c < pp; c += g.nw)
-#pragma unroll 4
-          for (int r = lane; r < bb; r += 32) Y[r + c * ldy] = double(X[r + (int64_t)c * ld]);
-        g.sync();
-        g_project_out(g, bb, kc, pp, C, ld, Y, ldy, G, ss, sd ? Mg : Mtmp, s, x);
-        if (one) {
-          g_panel_qr(g, bb, pp, Y, ldy, G + kc, ss, s);
-          for (int c = g.wid; c < pp; c += g.nw)
-#pragma unroll 4
-            for (int r = lane; r < bb; r += 32) S[r + (int64_t)c * bb] = Y[r + c * ldy];
-          for (int e = g.tid; e < GQ * GQ; e += g.nt) Tf[e] = s.T[e];
-          g.sync();
-        } else {
-          g_qr(g, bb, pp, S, bb, G + kc, ss, Tf, wp, smP, s, x);
+          tk.base = base;
+          tk.Tm = base + L.t; tk.Mtmp = base + L.mtmp; tk.Mg = base + L.mglob; tk.Y1 = base + L.y1;
+          tk.Sc = A.s(ic, k);
+          const int64_t wstep = (int64_t)GQ * max(smax, A.bmax);
+          for (int sd = 0; sd < 2; ++sd) {
+            RecompSide<T>& d = tk.s[sd];
+            d.X = sd ? tk.o.YR : tk.o.XL;
+            d.C = sd ? A.vt(ic, k) : A.u(ic, k);
+            d.S = base + (sd ? L.bsh : L.ash);
+            d.G = base + (sd ? L.gv : L.gu);
+            d.Tf = base + (sd ? L.tfv : L.tfu);
+            d.Tn = base + (sd ? L.tv : L.t);
+            d.Z2 = base + (sd ? L.mglob : L.mtmp);
+            d.x = GrpScratch{base + L.w + 2 * sd * wstep, base + L.w + (2 * sd + 1) * wstep,
+                             base + L.part + sd * (int64_t)G_PART};
+            d.bb = sd ? bk : bc;
+            d.pp = sd ? tk.o.q : tk.o.p;
+            d.mm = sd ? tk.mv : tk.mu;
+            d.xt = sd && tk.o.right_dense;     // A(i,k)^T
+          }
         }
-      } else {
-        for (int c = g.wid; c < ss; c += g.nw)
-#pragma unroll 4
-          for (int r = lane; r < bb; r += 32)
-            S[r + (int64_t)c * bb] = c < kc ? double(C[r + (int64_t)c * ld])
-                                            : double(xt ? X[(c - kc) + (int64_t)r * ld] : X[r + (int64_t)(c - kc) * ld]);
-        g.sync();
-        g_qr(g, bb, ss, S, bb, G, mm, Tf, wp, smP, s, x);
       }
-    };
-    if (side != 1) form_core(all, o, bi, ld, Tm, sh.gs[0], scratch_of(0));
-    if (side >= 0) basis(all, side, region);
-    else basis(half, hf, region + hf * (RECOMP_REGION / 2));
+      __syncthreads();
+      if (!tk.ok) continue;
+    }
+    const int ld = A.bmax, wp = recomp_panel(A.bmax);
+    if (tk.side != 1) form_core(grp_all(), tk.o, A.bs(i), ld, tk.Tm, tk.s[0].x);
+    {
+      // one side's basis per half (both halves on one side of a split target):
+      // projected, [Zu; Ru] (su x p) in G and the clean V of the remainder's
+      // QR in S; stacked, R (mu x su) in G and V in S
+      const int sd = tk.side >= 0 ? tk.side : hf;
+      const Grp g = tk.side >= 0 ? grp_all() : grp_half(hf);
+      const RecompSide<T>& d = tk.s[sd];
+      double* smP = region + (tk.side >= 0 ? 0 : hf * (RECOMP_REGION / 2));
+      const int kc = tk.kc, bb = d.bb, cols = tk.proj ? d.pp : kc + d.pp;
+      // the whole side in shared memory where it fits, else panel by panel
+      const bool sm = panel_ld(bb) * cols <= (tk.side >= 0 ? RECOMP_REGION : RECOMP_REGION / 2);
+      double* Y = sm ? smP : d.S;
+      const int ldy = sm ? panel_ld(bb) : bb;
+      for (int c = g.wid; c < cols; c += g.nw) {
+        const int cx = tk.proj ? c : c - kc;
+        const T* src = cx < 0 ? d.C + (int64_t)c * ld : d.X + (d.xt ? (int64_t)cx : (int64_t)cx * ld);
+        const int step = cx >= 0 && d.xt ? ld : 1;
+#pragma unroll 4
+        for (int r = lane; r < bb; r += 32) Y[r + (int64_t)c * ldy] = double(src[(int64_t)r * step]);
+      }
+      g.sync();
+      if (tk.proj) g_project_out(g, bb, kc, d.pp, (const T*)d.C, 1, ld, Y, ldy, d.G, kc + d.pp, d.Z2, d.x);
+      g_qr(g, bb, cols, Y, ldy, d.S, bb, d.G + (tk.proj ? kc : 0), tk.proj ? kc + d.pp : d.mm, d.Tf, wp,
+           sm ? nullptr : smP, sh.gs[sd], d.x);
+    }
     __syncthreads();
-    if (side >= 0) {
+    if (tk.side >= 0) {
       // publish this side; the second of the two CTAs goes on with the target
       __threadfence();
       __syncthreads();
-      if (threadIdx.x == 0) s_last = atomicAdd(split_done + tsk, 1);
+      if (threadIdx.x == 0) s_last = atomicAdd(split_done + tk.tsk, 1);
       __syncthreads();
       if (s_last == 0) continue;
       __threadfence();
@@ -1551,143 +1570,148 @@ FRANK_D void k_recompress_impl(BlrView<T> A, FactorWs<T> ws, int i, int smax,
     // (small cores always: the L2 path works on panels of its own).
     // Projected: M = [I Zu; 0 Ru] blockdiag(S_C, T) [I Zv; 0 Rv']^T = [Zu; Ru] T [Zv; Rv']^T + S_C;
     // stacked: M = [Ru(:, :kc) S_C | Ru(:, kc:) T] Rv^T.
-    const int ldm_s = rrqr_ld(mu);
-    const int64_t vecs = 3 * (int64_t)min(mu, mv) + 4 * (RECOMP_THREADS / 32) + (min(mu, mv) + mv + 2) / 2;
-    const int64_t core_need = (int64_t)ldm_s * mv + vecs;
-    const bool in_smem = core_need + 8 * (int64_t)panel_ld(mv) <= RECOMP_REGION && mu <= G_COLS_MAX &&
+    const int mu = tk.mu, mv = tk.mv, mn = min(mu, mv);
+    const int core_need = rrqr_ld(mu) * mv + 3 * mn + 4 * (RECOMP_THREADS / 32) + (mn + mv + 2) / 2;
+    const bool in_smem = core_need + 8 * panel_ld(mv) <= RECOMP_REGION && mu <= G_COLS_MAX &&
                          (mu < 64 || core_need <= core_smem);
-    double* Mm = in_smem ? region : Mg;
-    const int ldm = in_smem ? ldm_s : mu;
-    GrpShared& s0 = sh.gs[0];
-    const GrpScratch x0 = scratch_of(0);
-    if (proj) {
-      g_gemm(all, mu, o.q, o.p, 1.0, Gu, mu, false, Tm, o.p, false, 0.0, Mtmp, mu, s0.part);
-      g_gemm(all, mu, mv, o.q, 1.0, Mtmp, mu, false, Gv, mv, true, 0.0, Mm, ldm, s0.part);
-      for (int e = threadIdx.x; e < kc * kc; e += blockDim.x) {
-        const int r = e % kc, c = e / kc;
-        Mm[r + (int64_t)c * ldm] += double(Sc[r + (int64_t)c * A.kcap]);
+    double* const Mm = in_smem ? region : tk.Mg;
+    const int ldm = in_smem ? rrqr_ld(mu) : mu;
+    {
+      const Grp all = grp_all();
+      const int kc = tk.kc, p = tk.o.p, qq = tk.o.q;
+      const double *Gu = tk.s[0].G, *Gv = tk.s[1].G;
+      if (!tk.proj) {
+        // S_C in FP64 (Y1 is free)
+        for (int e = threadIdx.x; e < kc * kc; e += blockDim.x)
+          tk.Y1[e] = double(tk.Sc[e % kc + (int64_t)(e / kc) * A.kcap]);
+        __syncthreads();
       }
-      __syncthreads();
-    } else {
-      g_gemm(all, mu, kc, kc, 1.0, Gu, mu, false, Sc, A.kcap, false, 0.0, Mtmp, mu, s0.part);
-      g_gemm(all, mu, o.q, o.p, 1.0, Gu + (int64_t)kc * mu, mu, false, Tm, o.p, false, 0.0, Mtmp + (int64_t)kc * mu,
-             mu, s0.part);
-      g_gemm(all, mu, mv, sv, 1.0, Mtmp, mu, false, Gv, mv, true, 0.0, Mm, ldm, s0.part);
+      // projected: Mtmp = Gu T, M = Mtmp Gv^T; stacked: the two parts of Mtmp first
+      for (int op = tk.proj ? 1 : 0; op < 3; ++op) {
+        const double* a = op == 2 ? tk.Mtmp : Gu + (op == 1 && !tk.proj ? (int64_t)kc * mu : 0);
+        const double* b = op == 0 ? tk.Y1 : (op == 1 ? tk.Tm : Gv);
+        double* c = op == 2 ? Mm : tk.Mtmp + (op == 1 && !tk.proj ? (int64_t)kc * mu : 0);
+        const int kk = op == 0 ? kc : (op == 1 ? p : (tk.proj ? qq : kc + qq));
+        g_mm(all, mu, op == 0 ? kc : (op == 1 ? qq : mv), kk, 1.0, a, 1, mu, b, op == 2 ? 1 : kk, op == 2 ? mv : 1,
+             0.0, c, op == 2 ? ldm : mu, tk.s[0].x.part);
+      }
+      if (tk.proj) {
+        for (int e = threadIdx.x; e < kc * kc; e += blockDim.x)
+          Mm[e % kc + (e / kc) * ldm] += double(tk.Sc[e % kc + (int64_t)(e / kc) * A.kcap]);
+        __syncthreads();
+      }
     }
     int r = 0;
-    double* X1 = Gu;              // Q_core (mu x r); Gu is free once the core is formed
+    double* const X1 = tk.s[0].G;     // Q_core (mu x r); G is free once the core is formed
     if (core_method == CORE_RRQR && ws.fixed_rank == 0) {
-      double f = 0.0;
-      for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) {
-        const double v = Mm[e % mu + (int64_t)(e / mu) * ldm];
-        f += v * v;
-      }
-      f = block_sum(f, sh.red);
-      const double thr_c = core_scale * ws.eps * sqrt(f);
       // shared-memory vectors of the pivoted QR, behind the core
-      double* tau = region + (int64_t)ldm_s * mv;
-      double* cand = tau + 3 * min(mu, mv);
+      double* tau = region + rrqr_ld(mu) * mv;
+      double* cand = tau + 3 * mn;
       int* ord = reinterpret_cast<int*>(cand + 4 * (RECOMP_THREADS / 32));
-      int* at = ord + min(mu, mv);
-      double* Rm = Gv;            // rows of R of a core in L2 (Gv is free too)
-      double* Tfc = base + L.tfc;
+      int* at = ord + mn;
+      const RecompLayout L = recomp_layout(A.bmax, smax);
+      int* jpvt = reinterpret_cast<int*>(tk.base + L.jp);
       // panel width of the L2 path: its sketch and its panel fit shared memory
-      int wc = GQ;
+      int wc = panel_width(mu);
       while (wc > 8 && rand_qrcp_smem(mu, mv, wc) > RECOMP_REGION) wc -= 8;
-      if (in_smem)
-        r = g_rrqr(all, mu, mv, Mm, ldm, thr_c, A.kcap, tau, ord, at, tau + min(mu, mv), cand);
-      else
-        r = g_rand_qrcp(all, mu, mv, Mm, ldm, Rm, mu, thr_c, A.kcap, wc, jpvt, Tfc, base + L.om, base + L.cn, region,
-                        sh.iscr, sh.mx, s0, x0);
+      {
+        double f = 0.0;
+        for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) {
+          const double v = Mm[e % mu + (e / mu) * ldm];
+          f += v * v;
+        }
+        const double thr = core_scale * ws.eps * sqrt(block_sum(f, sh.red));
+        if (in_smem)
+          r = g_rrqr(grp_all(), mu, mv, Mm, ldm, thr, A.kcap, tau, ord, at, tau + mn, cand);
+        else
+          r = g_rand_qrcp(grp_all(), mu, mv, Mm, ldm, tk.s[1].G, mu, thr, A.kcap, wc, jpvt, tk.base + L.tfc,
+                          tk.base + L.om, tk.base + L.cn, region, sh.iscr, sh.mx, sh.gs[0], tk.s[0].x);
+      }
+      if (threadIdx.x == 0) {
+        if (r >= A.kcap && r < mn) atomicAdd(ws.err + ERR_RANK_OVERFLOW, 1);
+        atomicMax(ws.err + ERR_MAX_RANK, max(r, 1));
+        atomicAdd(ws.err + ERR_RECOMP, 1);
+      }
       if (r == 0) {
         // zero core: rank-1 zero block (geqp3.cpp:97-102)
-        if (threadIdx.x == 0) { atomicMax(ws.err + ERR_MAX_RANK, 1); atomicAdd(ws.err + ERR_RECOMP, 1); }
-        for (int64_t e = threadIdx.x; e < (int64_t)bc; e += blockDim.x) Uc[e] = T(e == 0 ? 1.0 : 0.0);
-        for (int64_t e = threadIdx.x; e < (int64_t)bk; e += blockDim.x) Vc[e] = T(e == 0 ? 1.0 : 0.0);
-        if (threadIdx.x == 0) { Sc[0] = T(0); A.rank[blk] = 1; }
+        for (int sd = 0; sd < 2; ++sd)
+          for (int e = threadIdx.x; e < tk.s[sd].bb; e += blockDim.x) tk.s[sd].C[e] = T(e == 0 ? 1.0 : 0.0);
+        if (threadIdx.x == 0) { tk.Sc[0] = T(0); A.rank[tk.blk] = 1; }
         __syncthreads();
         continue;
       }
-      if (threadIdx.x == 0) {
-        if (r >= A.kcap && r < min(mu, mv)) atomicAdd(ws.err + ERR_RANK_OVERFLOW, 1);
-        atomicMax(ws.err + ERR_MAX_RANK, r);
-        atomicAdd(ws.err + ERR_RECOMP, 1);
-      }
-      if (hf == 0) {
-        // X1 = Q_core(:, :r)
-        if (in_smem) {
-          g_apply_rrqr(half, mu, r, r, Mm, ldm, tau, ord, true, nullptr, 0, nullptr, X1, mu);
-        } else {
-          for (int e = half.tid; e < mu * r; e += half.nt) X1[e] = (e % mu) == (e / mu) ? 1.0 : 0.0;
-          half.sync();
-          g_apply_q(half, mu, r, Mm, ldm, Tfc, wc, r, X1, mu, r, s0, x0);
-        }
-      } else {
-        // RQ of the kept rows R P^T = S Q': QR of X2 (mv x r) = (R P^T)^T J, S = J Rt^T J
-        const GrpScratch x1 = scratch_of(1);
-        double* X2 = Mtmp;
+      // half 0: X1 = Q_core(:, :r).  Half 1: RQ of the kept rows R P^T = S Q', by the
+      // QR of X2 (mv x r) = (R P^T)^T J: S = J Rt^T J, and its explicit Q in Qt.
+      const Grp half = grp_half(hf);
+      double* const X2 = tk.Mtmp;
+      double* const Qt = tk.s[1].G;            // after the rows of R of an L2 core have been read
+      const int w2 = min(panel_width(mv), (RECOMP_REGION - (in_smem ? core_need : 0)) / panel_ld(mv));
+      if (hf == 1) {
         for (int e = half.tid; e < mv * r; e += half.nt) {
           const int c = e % mv, row = r - 1 - e / mv;
           if (in_smem) X2[e] = rrqr_r(Mm, ldm, at, row, c);
-          else X2[jpvt[c] + (int64_t)(e / mv) * mv] = row <= c ? Rm[row + (int64_t)c * mu] : 0.0;
+          else X2[jpvt[c] + (e / mv) * mv] = row <= c ? tk.s[1].G[row + (int64_t)c * mu] : 0.0;
         }
         half.sync();
-        double* smP = in_smem ? region + core_need : region;
-        const int w2 = min((int)GQ, (int)((RECOMP_REGION - (in_smem ? core_need : 0)) / panel_ld(mv)));
-        double* Tfr = base + L.tfr;
-        double* Rt = Y1;                       // r x r
-        g_qr(half, mv, r, X2, mv, Rt, r, Tfr, w2, smP, sh.gs[1], x1);
+        double* Rt = tk.Y1;                    // r x r
+        g_qr(half, mv, r, X2, mv, X2, mv, Rt, r, tk.base + L.tfr, w2, in_smem ? region + core_need : region,
+             sh.gs[1], tk.s[1].x);
         for (int e = half.tid; e < r * r; e += half.nt) {
           const int a = e % r, c = e / r;
           const int ra = r - 1 - c, ca = r - 1 - a;
-          Sc[a + (int64_t)c * A.kcap] = T(ra <= ca ? Rt[ra + (int64_t)ca * r] : 0.0);
+          tk.Sc[a + (int64_t)c * A.kcap] = T(ra <= ca ? Rt[ra + ca * r] : 0.0);
         }
-        double* Qt = Gv;                       // R has been read
-        for (int e = half.tid; e < mv * r; e += half.nt) Qt[e] = (e % mv) == (e / mv) ? 1.0 : 0.0;
+      } else if (in_smem) {
+        g_apply_rrqr(half, mu, r, r, Mm, ldm, tau, ord, true, nullptr, 0, nullptr, X1, mu);
+      }
+      // explicit factors by blocked application: Qt, and X1 of a core in L2
+      if (hf == 1 || !in_smem) {
+        double* X = hf ? Qt : X1;
+        const int mm = hf ? mv : mu;
+        for (int e = half.tid; e < mm * r; e += half.nt) X[e] = (e % mm) == (e / mm) ? 1.0 : 0.0;
         half.sync();
-        g_apply_q(half, mv, r, X2, mv, Tfr, w2, r, Qt, mv, r, sh.gs[1], x1);
-        for (int e = half.tid; e < mv * r; e += half.nt) Y1[e] = Qt[e % mv + (int64_t)(r - 1 - e / mv) * mv];
+        g_apply_q(half, mm, r, hf ? X2 : Mm, mm, tk.base + (hf ? L.tfr : L.tfc), hf ? w2 : wc, r, X, mm, r,
+                  tk.s[hf].x);
+        if (hf == 1)
+          for (int e = half.tid; e < mv * r; e += half.nt) tk.Y1[e] = Qt[e % mv + (r - 1 - e / mv) * mv];
       }
       __syncthreads();
     } else {
-      double* pn = base + L.pn;
-      r = svd_core<T, RECOMP_THREADS>(mu, mv, Mm, ldm, in_smem, ws, A.kcap, region, RECOMP_REGION, Tv,
-                                      base + L.tau_c, base + L.cn, pn, jpvt, base + L.sig,
-                                      reinterpret_cast<int*>(base + L.ji), X1, Y1, sh, &s_rank);
-      for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-        const int rr = e % r, c = e / r;
-        Sc[rr + (int64_t)c * A.kcap] = T(rr == c ? pn[c] : 0.0);
-      }
+      const RecompLayout L = recomp_layout(A.bmax, smax);
+      double* pn = tk.base + L.pn;
+      r = svd_core<T, RECOMP_THREADS>(mu, mv, Mm, ldm, in_smem, ws, A.kcap, region, RECOMP_REGION, tk.base + L.tv,
+                                      tk.base + L.tau_c, tk.base + L.cn, pn, reinterpret_cast<int*>(tk.base + L.jp),
+                                      tk.base + L.sig, reinterpret_cast<int*>(tk.base + L.ji), X1, tk.Y1, sh, &s_rank);
+      for (int e = threadIdx.x; e < r * r; e += blockDim.x)
+        tk.Sc[e % r + (int64_t)(e / r) * A.kcap] = T(e % r == e / r ? pn[e / r] : 0.0);
       __syncthreads();
     }
-    if (threadIdx.x == 0)
-      atomicAdd(ws.flops + FLOP_RECOMP,
-                (unsigned long long)(proj ? fast_rounded_addition_flops(bc, bk, bi, kc, o.p, o.q, r)
-                                          : rounded_addition_flops(bc, bk, bi, kc, o.p, o.q, r)));
     {
       // new bases, a side per half.  Stacked: U = Qu [X1; 0]; projected:
       // U = [U_C | Q_u] X1 = Q_u [X1(kc:); 0] + U_C X1(:kc), in FP64 scratch
       // (U_C is an operand, so the block itself is written last)
-      const int bb = hf ? bk : bc, pp = hf ? o.q : o.p, mm = hf ? mv : mu;
-      const double* X = hf ? Y1 : X1;
-      double* Tn = hf ? Tv : Tm;
-      T* out = hf ? Vc : Uc;
-      const GrpScratch x = scratch_of(hf);
-      const int skip = proj ? kc : 0, refl = proj ? pp : mm;
+      const Grp half = grp_half(hf);
+      const RecompSide<T>& d = tk.s[hf];
+      const double* X = hf ? tk.Y1 : X1;
+      const int bb = d.bb, mm = d.mm, skip = tk.proj ? tk.kc : 0, refl = tk.proj ? d.pp : mm;
       for (int c = half.wid; c < r; c += half.nw)
 #pragma unroll 4
-        for (int e = threadIdx.x & 31; e < bb; e += 32)
-          Tn[e + (int64_t)c * bb] = e < refl ? X[skip + e + (int64_t)c * mm] : 0.0;
+        for (int e = lane; e < bb; e += 32) d.Tn[e + c * bb] = e < refl ? X[skip + e + c * mm] : 0.0;
       half.sync();
-      g_apply_q(half, bb, refl, hf ? Bsh : Ash, bb, base + (hf ? L.tfv : L.tfu), wp, r, Tn, bb, refl, sh.gs[hf], x);
-      if (proj) g_gemm(half, bb, r, kc, 1.0, (const T*)out, ld, false, X, mm, false, 1.0, Tn, bb, sh.gs[hf].part);
+      g_apply_q(half, bb, refl, d.S, bb, d.Tf, wp, r, d.Tn, bb, refl, d.x);
+      if (tk.proj) g_mm(half, bb, r, skip, 1.0, (const T*)d.C, 1, ld, X, mm, 1, 1.0, d.Tn, bb, d.x.part);
       for (int c = half.wid; c < r; c += half.nw)
 #pragma unroll 4
-        for (int e = threadIdx.x & 31; e < bb; e += 32) out[e + (int64_t)c * ld] = T(Tn[e + (int64_t)c * bb]);
+        for (int e = lane; e < bb; e += 32) d.C[e + (int64_t)c * ld] = T(d.Tn[e + c * bb]);
     }
     __syncthreads();
-    if (threadIdx.x == 0) A.rank[blk] = r;
-    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int bc = tk.s[0].bb, bk = tk.s[1].bb, bi = A.bs(i);
+      atomicAdd(ws.flops + FLOP_RECOMP,
+                (unsigned long long)(tk.proj ? fast_rounded_addition_flops(bc, bk, bi, tk.kc, tk.o.p, tk.o.q, r)
+                                             : rounded_addition_flops(bc, bk, bi, tk.kc, tk.o.p, tk.o.q, r)));
+      A.rank[tk.blk] = r;
+    }
   }
 }
 
@@ -2977,7 +3001,12 @@ template <typename T>
 __global__ void __launch_bounds__(RECOMP_THREADS) k_recompress_b(const SysDev<T>* S, int i) {
   const SysDev<T>& s = S[blockIdx.z];
   if (i >= s.W.nb - 1 || !s.has_lr) return;
-  k_recompress_impl<T>(s.W, s.ws, i, s.smax, s.core_method, s.core_scale, 0, s.work + i, 0, nullptr, nullptr,
+  // the views in shared memory (as kernel parameters would be in constant memory)
+  __shared__ BlrView<T> A;
+  __shared__ FactorWs<T> ws;
+  if (threadIdx.x == 0) { A = s.W; ws = s.ws; }
+  __syncthreads();
+  k_recompress_impl<T>(A, ws, i, s.smax, s.core_method, s.core_scale, 0, s.work + i, 0, nullptr, nullptr,
                        s.proj_tol, s.split_p, s.core_smem);
 }
 

@@ -156,7 +156,11 @@ struct RowIdentity {
   FRANK_D int operator()(int r) const { return r; }
 };
 
-template <int MI, int NI, typename TA, typename TB, typename RowMap = RowIdentity>
+// INIT: acc holds starting values already.  The loads of U k-quads are in
+// flight together: an operand in L2 is some 700 cycles away, so what counts is
+// the number of dependent round trips, and a ragged end is one more batch (of
+// predicated loads), not a loop.
+template <int MI, int NI, bool INIT = false, typename TA, typename TB, typename RowMap = RowIdentity>
 FRANK_D void warp_dgemm_acc(int m, int n, int k0, int k1, const TA* A, int64_t sai, int64_t sak, const TB* B,
                             int64_t sbj, int64_t sbk, int i0, int j0, double (&acc)[MI][NI][2],
                             RowMap row = RowMap()) {
@@ -167,20 +171,32 @@ FRANK_D void warp_dgemm_acc(int m, int n, int k0, int k1, const TA* A, int64_t s
   for (int i = 0; i < MI; ++i) pa[i] = A + (int64_t)row(min(i0 + 8 * i + g, m - 1)) * sai + (int64_t)(k0 + t) * sak;
 #pragma unroll
   for (int j = 0; j < NI; ++j) pb[j] = B + (int64_t)min(j0 + 8 * j + g, n - 1) * sbj + (int64_t)(k0 + t) * sbk;
+  if (!INIT) {
 #pragma unroll
-  for (int i = 0; i < MI; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  constexpr int U = MI * NI >= 8 ? 2 : 4;   // k-quads whose loads are in flight together
-  int kk = k0;
-  for (; kk + 4 * U <= k1; kk += 4 * U) {
+      for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  }
+  constexpr int U = MI + NI <= 2 ? 8 : (MI + NI <= 4 ? 6 : 4);   // k-quads in flight
+  for (int kk = k0; kk < k1; kk += 4 * U) {
     double a[U][MI], b[U][NI];
+    if (kk + 4 * U <= k1) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < U; ++u) {
 #pragma unroll
-      for (int i = 0; i < MI; ++i) a[u][i] = double(pa[i][u * 4 * sak]);
+        for (int i = 0; i < MI; ++i) a[u][i] = double(pa[i][u * 4 * sak]);
 #pragma unroll
-      for (int j = 0; j < NI; ++j) b[u][j] = double(pb[j][u * 4 * sbk]);
+        for (int j = 0; j < NI; ++j) b[u][j] = double(pb[j][u * 4 * sbk]);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = kk + 4 * u + t < k1;
+#pragma unroll
+        for (int i = 0; i < MI; ++i) a[u][i] = in ? double(pa[i][u * 4 * sak]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < NI; ++j) b[u][j] = in ? double(pb[j][u * 4 * sbk]) : 0.0;
+      }
     }
 #pragma unroll
     for (int i = 0; i < MI; ++i) pa[i] += U * 4 * sak;
@@ -188,22 +204,11 @@ FRANK_D void warp_dgemm_acc(int m, int n, int k0, int k1, const TA* A, int64_t s
     for (int j = 0; j < NI; ++j) pb[j] += U * 4 * sbk;
 #pragma unroll
     for (int u = 0; u < U; ++u)
+      if (u == 0 || kk + 4 * u < k1)
 #pragma unroll
-      for (int i = 0; i < MI; ++i)
+        for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[u][i], b[u][j]);
-  }
-  for (; kk < k1; kk += 4) {
-    const bool in = kk + t < k1;
-    double a[MI], b[NI];
-#pragma unroll
-    for (int i = 0; i < MI; ++i) { a[i] = in ? double(*pa[i]) : 0.0; pa[i] += 4 * sak; }
-#pragma unroll
-    for (int j = 0; j < NI; ++j) { b[j] = in ? double(*pb[j]) : 0.0; pb[j] += 4 * sbk; }
-#pragma unroll
-    for (int i = 0; i < MI; ++i)
-#pragma unroll
-      for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[i], b[j]);
+          for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[u][i], b[u][j]);
   }
 }
 
@@ -214,16 +219,27 @@ FRANK_D void dgemm_store(TC* p, double v, double alpha, double beta) {
   *p = TC(v);
 }
 
-// One pass of the CTA's (or warp group's) warps over the 8 MI x 8 NI tiles.
+// One pass of the CTA's (or warp group's) warps over the 8 MI x 8 NI tiles.  C is
+// read (beta != 0) with the operands, ahead of the products.
 template <int MI, int NI, typename TA, typename TB, typename TC>
 FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, const TA* A, int64_t sai, int64_t sak,
                          const TB* B, int64_t sbj, int64_t sbk, double beta, TC* C, int64_t ldc) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tm = (m + 8 * MI - 1) / (8 * MI), tn = (n + 8 * NI - 1) / (8 * NI);
+  const double ba = beta / alpha;       // +-1 where C is updated
   for (int tile = wid; tile < tm * tn; tile += nw) {
     const int i0 = (tile % tm) * 8 * MI, j0 = (tile / tm) * 8 * NI;
     double acc[MI][NI][2];
-    warp_dgemm_acc<MI, NI>(m, n, 0, k, A, sai, sak, B, sbj, sbk, i0, j0, acc);
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NI; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = i0 + 8 * i + g, c = j0 + 8 * j + 2 * t + h;
+          acc[i][j][h] = (beta != 0.0 && r < m && c < n) ? ba * double(C[r + (int64_t)c * ldc]) : 0.0;
+        }
+    warp_dgemm_acc<MI, NI, true>(m, n, 0, k, A, sai, sak, B, sbj, sbk, i0, j0, acc);
 #pragma unroll
     for (int i = 0; i < MI; ++i) {
       const int r = i0 + 8 * i + g;
@@ -231,8 +247,8 @@ FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, con
 #pragma unroll
       for (int j = 0; j < NI; ++j) {
         const int c = j0 + 8 * j + 2 * t;
-        if (c < n) dgemm_store(C + r + (int64_t)c * ldc, acc[i][j][0], alpha, beta);
-        if (c + 1 < n) dgemm_store(C + r + (int64_t)(c + 1) * ldc, acc[i][j][1], alpha, beta);
+        if (c < n) C[r + (int64_t)c * ldc] = TC(alpha * acc[i][j][0]);
+        if (c + 1 < n) C[r + (int64_t)(c + 1) * ldc] = TC(alpha * acc[i][j][1]);
       }
     }
   }
@@ -259,7 +275,7 @@ static __device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha,
     if (tile < t8) {
       const int i0 = (tile % tm) * 8, j0 = (tile / tm) * 8;
       double acc[1][1][2];
-      warp_dgemm_acc<1, 1>(m, n, min(k, part * kc), min(k, (part + 1) * kc), A, sai, sak, B, sbj, sbk, i0, j0, acc);
+      warp_dgemm_acc<1, 1, false>(m, n, min(k, part * kc), min(k, (part + 1) * kc), A, sai, sak, B, sbj, sbk, i0, j0, acc);
       smem[wid * 64 + 2 * lane] = acc[0][0][0];
       smem[wid * 64 + 2 * lane + 1] = acc[0][0][1];
     }

@@ -33,111 +33,171 @@ FRANK_D Grp grp_half(int h) {
 }
 
 // Shared memory of a group's factorizations.
-constexpr int GQ = 32;   // widest panel
+constexpr int GQ = 16;   // widest panel
 struct GrpShared {
   double G[GQ * GQ];     // V^T V of a panel (strictly upper part)
   double T[GQ * GQ];     // its T factor
   double tau[GQ], beta[GQ], scal[GQ];
-  double part[8 * 64];   // partial tiles of short products
+  double part[9 * GQ];       // warps' partial sums of a column step, and its row
+  double coef[GQ + 2];       // its update coefficients
 };
 
-// C (m x n) = alpha op(A) op(B) + beta C as cta_gemm, on the group's warps.  An output
-// of at most four 8 x 8 tiles splits a long inner dimension over eight warps;
-// the split depends on the shape only, so a result does not depend on the
-// group's size.  part: 8 * 64 doubles.
-template <typename TA, typename TB, typename TC>
-static __device__ __noinline__ void g_gemm(Grp g, int m, int n, int k, double alpha, const TA* A, int64_t lda, bool ta,
-                                    const TB* B, int64_t ldb, bool tb, double beta, TC* C, int64_t ldc,
-                                    double* part) {
-  if (m <= 0 || n <= 0) { g.sync(); return; }
-  const int lane = threadIdx.x & 31;
-  const int64_t sai = ta ? lda : 1, sak = ta ? 1 : lda, sbj = tb ? 1 : ldb, sbk = tb ? ldb : 1;
-  const int tm = (m + 7) / 8, t8 = tm * ((n + 7) / 8);
-  if (t8 <= 4 && k >= 64 && g.nw >= 8) {
-    const int split = 8 / t8, kc = ((k + split - 1) / split + 3) & ~3;
-    const int tile = g.wid / split, q = g.wid % split;
-    if (tile < t8) {
-      double acc[1][1][2];
-      warp_dgemm_acc<1, 1>(m, n, min(k, q * kc), min(k, (q + 1) * kc), A, sai, sak, B, sbj, sbk, (tile % tm) * 8,
-                           (tile / tm) * 8, acc);
-      part[g.wid * 64 + 2 * lane] = acc[0][0][0];
-      part[g.wid * 64 + 2 * lane + 1] = acc[0][0][1];
-    }
-    g.sync();
-    for (int e = g.tid; e < t8 * 64; e += g.nt) {
-      const int tl = e >> 6, x = e & 63;
-      const int r = (tl % tm) * 8 + (x >> 3), c = (tl / tm) * 8 + (x & 7);
-      if (r < m && c < n) {
-        double v = 0.0;
-        for (int s = 0; s < split; ++s) v += part[(tl * split + s) * 64 + x];
-        dgemm_store(C + r + (int64_t)c * ldc, v, alpha, beta);
-      }
-    }
-    g.sync();
-    return;
-  }
-  auto cost = [&](int mi, int ni) {
-    const int tiles = ((m + 8 * mi - 1) / (8 * mi)) * ((n + 8 * ni - 1) / (8 * ni));
-    return ((tiles + g.nw - 1) / g.nw) * (2 * mi * ni + mi + ni);
-  };
-  const int c23 = cost(2, 3), c42 = cost(4, 2), c22 = cost(2, 2), c11 = cost(1, 1);
-  const int best = min(min(c23, c42), min(c22, c11));
-  if (best == c23)
-    warps_dgemm<2, 3>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
-  else if (best == c42)
-    warps_dgemm<4, 2>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
-  else if (best == c22)
-    warps_dgemm<2, 2>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
-  else
-    warps_dgemm<1, 1>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
-  g.sync();
+// C (m x n, ldc) = alpha A B + beta C over k, element (i, kk) of A at A[i sai +
+// kk sak], (kk, j) of B at B[j sbj + kk sbk].
+// Long inner dimension and a small output (bases against bases: k = b, m and n
+// ranks): every warp of a slice index q takes an eighth of k for all tiles, so
+// each operand row is read once per tile and the warps have equal work; the
+// eight partial products go to part (G_PART doubles, in L2) and are summed in
+// order.  Otherwise a tile per warp with the whole inner dimension.  Tile shapes
+// are the ones with the fewest tensor-pipe cycles; neither choice changes the
+// order in which an element is summed, and the slices do not depend on the
+// group's size, so results do not depend on it either.
+constexpr int G_SLICE_TILES = 81;            // 8 x 8 tiles of a sliced output
+constexpr int G_PART = 8 * 64 * G_SLICE_TILES;
+
+// Four consecutive values in FP64 by 16-byte loads.
+FRANK_D void load4(const double* p, double (&v)[4]) {
+  const double2 x = *reinterpret_cast<const double2*>(p), y = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+}
+FRANK_D void load4(const float* p, double (&v)[4]) {
+  const float4 x = *reinterpret_cast<const float4*>(p);
+  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
 }
 
-// C (m x n, ldc) = alpha A^T B over k rows, A (k x m, lda), B (k x n, ldb), k
-// long: every warp takes an eighth of the rows for 24 x 24 tiles of C, so that
-// each row of A and B is read once per tile and all warps have equal work; the
-// eight partial products go to part (in L2; G_TN_PART doubles) and are summed in
-// order.  Outputs above G_TN_TILES 8 x 8 tiles take g_gemm (they fill the
-// warps by themselves).
-constexpr int G_TN_TILES = 81;
-constexpr int G_TN_PART = 8 * 72 * 72;
-
-template <typename TA, typename TB>
-static __device__ __noinline__ void g_gemm_tn(Grp g, int m, int n, int k, double alpha, const TA* A, int64_t lda, const TB* B,
-                                       int64_t ldb, double* C, int64_t ldc, double* part, double* spart) {
-  const int m8 = (m + 7) / 8, n8 = (n + 7) / 8;
-  if (m8 * n8 > G_TN_TILES || m8 > 9 || n8 > 9 || k < 128 || g.nw < 8) {
-    g_gemm(g, m, n, k, alpha, A, lda, true, B, ldb, false, 0.0, C, ldc, spart);
-    return;
+// acc = A^T B over rows [k0, k1), both with contiguous rows and 16-byte aligned
+// columns: lane t of a quad takes rows 4 t .. 4 t + 3 of every 16 (the products
+// of a 16-row block may be summed in any order as long as A and B agree), so a
+// load covers 64 bytes of a column instead of 32 (FP32: 16); the L1 looks up
+// one line per column and load, and that was what bound these products.
+template <int MI, int NI, typename TA, typename TB>
+FRANK_D void warp_dgemm_tn(int m, int n, int k0, int k1, const TA* A, int64_t lda, const TB* B, int64_t ldb, int i0,
+                           int j0, double (&acc)[MI][NI][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const TA* pa[MI];
+  const TB* pb[NI];
+#pragma unroll
+  for (int i = 0; i < MI; ++i) pa[i] = A + (int64_t)min(i0 + 8 * i + g, m - 1) * lda + k0 + 4 * t;
+#pragma unroll
+  for (int j = 0; j < NI; ++j) pb[j] = B + (int64_t)min(j0 + 8 * j + g, n - 1) * ldb + k0 + 4 * t;
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  constexpr int U = MI + NI <= 2 ? 4 : (MI + NI <= 4 ? 2 : 1);   // 16-row blocks in flight
+  int kk = k0;
+  for (; kk + 16 * U <= k1; kk += 16 * U) {
+    double a[U][MI][4], b[U][NI][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int i = 0; i < MI; ++i) load4(pa[i] + 16 * u, a[u][i]);
+#pragma unroll
+      for (int j = 0; j < NI; ++j) load4(pb[j] + 16 * u, b[u][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i) pa[i] += 16 * U;
+#pragma unroll
+    for (int j = 0; j < NI; ++j) pb[j] += 16 * U;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+          for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[u][i][v], b[u][j][v]);
   }
+  for (; kk < k1; kk += 16) {
+    double a[MI][4], b[NI][4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const bool in = kk + 4 * t + v < k1;
+#pragma unroll
+      for (int i = 0; i < MI; ++i) a[i][v] = in ? double(pa[i][v]) : 0.0;
+#pragma unroll
+      for (int j = 0; j < NI; ++j) b[j][v] = in ? double(pb[j][v]) : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i) pa[i] += 16;
+#pragma unroll
+    for (int j = 0; j < NI; ++j) pb[j] += 16;
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) dmma884(acc[i][j], a[i][v], b[j][v]);
+  }
+}
+
+template <typename TA>
+FRANK_D bool aligned4(const TA* p, int64_t ld) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(ld * (int64_t)sizeof(TA))) & 15) == 0;
+}
+
+template <int MI, int NI, typename TA, typename TB>
+FRANK_D void g_slices(const Grp& g, int m, int n, int k, const TA* A, int64_t sai, int64_t sak, const TB* B,
+                      int64_t sbj, int64_t sbk, int tot, double* part) {
   const int lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
-  const int kc = ((k + 7) / 8 + 3) & ~3, q = g.wid & 7, sub = g.wid >> 3, nsub = g.nw >> 3;
+  const int kc = ((k + 7) / 8 + 15) & ~15, q = g.wid & 7, sub = g.wid >> 3, nsub = g.nw >> 3;
   const int k0 = min(k, q * kc), k1 = min(k, k0 + kc);
-  const int tm = (m8 + 2) / 3, tn = (n8 + 2) / 3, mp = tm * 24;
-  double* pq = part + (int64_t)q * mp * tn * 24;
+  const int tm = (m + 8 * MI - 1) / (8 * MI), tn = (n + 8 * NI - 1) / (8 * NI);
+  const bool vec = sak == 1 && sbk == 1 && aligned4(A, sai) && aligned4(B, sbj);
+  double* pq = part + q * tot;
   for (int tile = sub; tile < tm * tn; tile += nsub) {
-    const int i0 = (tile % tm) * 24, j0 = (tile / tm) * 24;
-    double acc[3][3][2];
-    warp_dgemm_acc<3, 3>(m, n, k0, k1, A, lda, 1, B, ldb, 1, i0, j0, acc);
+    const int i0 = (tile % tm) * 8 * MI, j0 = (tile / tm) * 8 * NI;
+    double acc[MI][NI][2];
+    if (vec) warp_dgemm_tn<MI, NI>(m, n, k0, k1, A, sai, B, sbj, i0, j0, acc);
+    else warp_dgemm_acc<MI, NI, false>(m, n, k0, k1, A, sai, sak, B, sbj, sbk, i0, j0, acc);
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        pq[(i0 + 8 * i + gr) + (int64_t)(j0 + 8 * j + 2 * t) * mp] = acc[i][j][0];
-        pq[(i0 + 8 * i + gr) + (int64_t)(j0 + 8 * j + 2 * t + 1) * mp] = acc[i][j][1];
+      for (int j = 0; j < NI; ++j) {
+        const int r = i0 + 8 * i + gr, c = j0 + 8 * j + 2 * t;
+        if (r < m && c < n) pq[r + c * m] = acc[i][j][0];
+        if (r < m && c + 1 < n) pq[r + (c + 1) * m] = acc[i][j][1];
       }
   }
-  g.sync();
-  for (int e = g.tid; e < m * n; e += g.nt) {
-    const int r = e % m, c = e / m;
-    const double* p = part + r + (int64_t)c * mp;
-    double v[8], s = 0.0;
+}
+
+template <typename TA, typename TB, typename TC>
+FRANK_D void g_mm(const Grp& g, int m, int n, int k, double alpha, const TA* A, int64_t sai, int64_t sak, const TB* B,
+                  int64_t sbj, int64_t sbk, double beta, TC* C, int64_t ldc, double* part) {
+  if (m <= 0 || n <= 0) { g.sync(); return; }
+  const int m8 = (m + 7) / 8, n8 = (n + 7) / 8;
+  auto cost = [&](int mi, int ni) {
+    return ((m8 + mi - 1) / mi) * ((n8 + ni - 1) / ni) * (4 * mi * ni + mi + ni);
+  };
+  if (m8 * n8 <= G_SLICE_TILES && k >= 128 && g.nw >= 8) {
+    const int c33 = cost(3, 3), c22 = cost(2, 2), c11 = cost(1, 1);
+    const int tot = m * n;
+    if (c33 <= c22 && c33 <= c11) g_slices<3, 3>(g, m, n, k, A, sai, sak, B, sbj, sbk, tot, part);
+    else if (c22 <= c11) g_slices<2, 2>(g, m, n, k, A, sai, sak, B, sbj, sbk, tot, part);
+    else g_slices<1, 1>(g, m, n, k, A, sai, sak, B, sbj, sbk, tot, part);
+    g.sync();
+    for (int e = g.tid; e < tot; e += g.nt) {
+      double v[8], s = 0.0;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) v[x] = p[(int64_t)x * mp * tn * 24];
+      for (int x = 0; x < 8; ++x) v[x] = part[e + x * tot];
 #pragma unroll
-    for (int x = 0; x < 8; ++x) s += v[x];
-    C[r + (int64_t)c * ldc] = alpha * s;
+      for (int x = 0; x < 8; ++x) s += v[x];
+      dgemm_store(C + e % m + (int64_t)(e / m) * ldc, s, alpha, beta);
+    }
+    g.sync();
+    return;
   }
+  auto rounds = [&](int mi, int ni) {
+    const int tiles = ((m8 + mi - 1) / mi) * ((n8 + ni - 1) / ni);
+    return ((tiles + g.nw - 1) / g.nw) * (4 * mi * ni + mi + ni);
+  };
+  const int c42 = rounds(4, 2), c23 = rounds(2, 3), c11 = rounds(1, 1);
+  if (c42 <= c23 && c42 <= c11)
+    warps_dgemm<4, 2>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  else if (c23 <= c11)
+    warps_dgemm<2, 3>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  else
+    warps_dgemm<1, 1>(g.wid, g.nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
   g.sync();
 }
 
@@ -150,140 +210,152 @@ FRANK_D void warp_sums(double (&v)[N]) {
     for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
 }
 
-// Householder quantities (dlarfg) of a column with leading entry alpha and
-// squared norm xn2 below it.
-FRANK_D void reflector(double alpha, double xn2, double& beta, double& tau, double& scal) {
-  if (xn2 > 0.0) {
-    const double nrm = sqrt(alpha * alpha + xn2);
-    beta = alpha >= 0.0 ? -nrm : nrm;
-    tau = (beta - alpha) / beta;
-    scal = 1.0 / (alpha - beta);
-  } else {
-    beta = alpha;
-    tau = 0.0;
-    scal = 0.0;
-  }
+// Householder reflector (dlarfg) of a column with leading entry alpha and
+// squared norm n2 = alpha^2 + (squared norm below it): v = [1; x scal],
+// H = I - tau v v^T, H x = beta e_1.  One reciprocal square root and one
+// reciprocal (every warp forms them, so the FP64 pipe pays for each): with
+// h = |alpha| + ||x||, tau = h / ||x|| and scal = sign / h.
+FRANK_D void reflector(double alpha, double n2, double& beta, double& tau, double& scal) {
+  const double rn = rsqrt(n2), nrm = n2 * rn, aa = fabs(alpha);
+  const double rh = __drcp_rn(aa + nrm);
+  beta = alpha >= 0.0 ? -nrm : nrm;
+  tau = fma(aa, rn, 1.0);
+  scal = alpha >= 0.0 ? rh : -rh;
 }
 
-// Householder QR (dgeqr2 conventions) of a panel P (m x n, ldp, n <= GQ, in
-// shared memory).  One barrier per column: every warp that updates columns
-// forms the reflector itself from the column it reads anyway, and reflectors
-// stay unscaled until the end.  The dot products of each reflector with the
-// earlier ones are formed in the same pass by the same warps, so the T factor
-// needs no product of its own.  On return P holds the clean V (unit lower
-// trapezoid), s.T the T factor (upper, zero below), s.tau; R (min(m, n) x n)
-// goes to R (ldr) with zeros below its diagonal.
-static __device__ __noinline__ void g_panel_qr(Grp g, int m, int n, double* P, int ldp, double* R, int64_t ldr,
-                                        GrpShared& s) {
-  const int lane = threadIdx.x & 31, km = min(m, n);
-  for (int j = 0; j < km; ++j) {
-    const double* x = P + (int64_t)j * ldp;
-    const double alpha = x[j];
-    // columns c != j of this warp: c = wid, wid + nw, ...; c > j updated, c < j dots only
-    double xn2 = 0.0, beta = 0.0, tau = 0.0, scal = 0.0;
-    bool have = false;
-    for (int c0 = g.wid; c0 < n; c0 += 4 * g.nw) {
-      double* p[4];
-      double d[5];
+// Householder QR (dgeqr2 conventions) of a panel P (m x n, ldp, n <= W, n <= m),
+// rows in registers: thread t of the first eight warps holds rows t, t + 256,
+// ... (RPT of them, m <= 256 RPT) of all W columns.  A column step is one
+// reduction of the column's dot products with every column -- later ones for
+// the update, itself for the norm, earlier ones for the T factor -- which a
+// warp does by recursive halving (W sums in W + 1 exchanges instead of 5 W);
+// the warps' sums meet in shared memory, where one warp forms the reflector.  Kept in shared memory instead, a
+// 512 x 16 panel of both sides was bound by its bandwidth (256 KB a step:
+// 51 us; 3.3 us a column).  On return V (clean, unit lower trapezoid, ldv)
+// holds the reflectors (V may be P), s.T the T factor (upper, zero below) and
+// R (n x n, ldr) the triangle with zeros below its diagonal.
+template <int W, int RPT>
+FRANK_D void panel_qr_rows(const Grp& g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
+                           int64_t ldr, GrpShared& s) {
+  const int lane = threadIdx.x & 31;
+  const bool on = g.wid < 8;
+  double a[RPT][W];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = c0 + i * g.nw;
-        p[i] = P + (int64_t)(c < n && c != j ? c : j) * ldp;
-        d[i] = 0.0;
-      }
-      d[4] = 0.0;
-      const int cnt = min(4, (n - c0 + g.nw - 1) / g.nw);
-      if (cnt > 2) {
-#pragma unroll 4
-        for (int e = j + 1 + lane; e < m; e += 32) {
-          const double v = x[e];
-          d[4] = fma(v, v, d[4]);
+  for (int k = 0; k < RPT; ++k)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) d[i] = fma(v, p[i][e], d[i]);
-        }
-        warp_sums<5>(d);
-      } else {
-#pragma unroll 4
-        for (int e = j + 1 + lane; e < m; e += 32) {
-          const double v = x[e];
-          d[4] = fma(v, v, d[4]);
-          d[0] = fma(v, p[0][e], d[0]);
-          d[1] = fma(v, p[1][e], d[1]);
-        }
-        double h[3] = {d[0], d[1], d[4]};
-        warp_sums<3>(h);
-        d[0] = h[0]; d[1] = h[1]; d[4] = h[2];
-      }
-      if (!have) {
-        xn2 = d[4];
-        reflector(alpha, xn2, beta, tau, scal);
-        have = true;
-      }
-      double f[4];
+    for (int c = 0; c < W; ++c) {
+      const int r = g.tid + 256 * k;
+      a[k][c] = (on && r < m && c < n) ? P[r + c * ldp] : 0.0;
+    }
+  for (int j = 0; j < n; ++j) {
+    double* part = s.part;                         // [8][GQ] warp sums, [GQ] row j
+    double x[RPT], f[W];
+    if (on) {
+      // column j of the rows below j (by selection: registers have no index)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = c0 + i * g.nw;
-        f[i] = 0.0;
-        if (c >= n) continue;
-        if (c > j) {
-          const double top = p[i][j], w = tau * fma(scal, d[i], top);
-          f[i] = w * scal;
-          __syncwarp();
-          if (lane == 0) p[i][j] = top - w;
-        } else if (c < j) {
-          // v_c . v_j: rows below j of both, and row j where v_j is 1
-          if (lane == 0) s.G[c + j * GQ] = s.scal[c] * fma(scal, d[i], p[i][j]);
-        } else if (lane == 0) {
-          s.tau[j] = tau; s.beta[j] = beta; s.scal[j] = scal;
+      for (int k = 0; k < RPT; ++k) {
+        double v = a[k][0];
+#pragma unroll
+        for (int c = 1; c < W; ++c) v = j == c ? a[k][c] : v;
+        x[k] = g.tid + 256 * k > j ? v : 0.0;
+      }
+      double d[W];
+#pragma unroll
+      for (int c = 0; c < W; ++c) {
+        d[c] = x[0] * a[0][c];
+#pragma unroll
+        for (int k = 1; k < RPT; ++k) d[c] = fma(x[k], a[k][c], d[c]);
+      }
+      if (g.tid == j) {
+#pragma unroll
+        for (int c = 0; c < W; ++c) part[8 * GQ + c] = a[0][c];
+      }
+      // recursive halving: lane l ends with the sum of column l % W
+#pragma unroll
+      for (int h = W / 2; h >= 1; h >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int c = 0; c < h; ++c) {
+          const double send = up ? d[c] : d[c + h], keep = up ? d[c + h] : d[c];
+          d[c] = keep + __shfl_xor_sync(0xffffffffu, send, h);
         }
       }
-      if (tau != 0.0) {
-        const bool two = c0 + 2 * g.nw < n && c0 + (cnt - 1) * g.nw > j;
-        if (two) {
-#pragma unroll 4
-          for (int e = j + 1 + lane; e < m; e += 32) {
-            const double v = x[e];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (f[i] != 0.0) p[i][e] = fma(-f[i], v, p[i][e]);
-          }
-        } else if (f[0] != 0.0 || f[1] != 0.0) {
-#pragma unroll 4
-          for (int e = j + 1 + lane; e < m; e += 32) {
-            const double v = x[e];
-            if (f[0] != 0.0) p[0][e] = fma(-f[0], v, p[0][e]);
-            if (f[1] != 0.0) p[1][e] = fma(-f[1], v, p[1][e]);
-          }
-        }
-      }
+      for (int h = W; h < 32; h <<= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], h);
+      if (lane < W) part[g.wid * GQ + lane] = d[0];
     }
     g.sync();
+    // one warp turns the sums into the reflector and the step's coefficients
+    // (eight of them doing it would cost the FP64 pipe more than a barrier)
+    if (g.wid == 0) {
+      const int c = lane & (W - 1);
+      double q[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) q[w] = part[w * GQ + c];
+      const double top = part[8 * GQ + c];
+      const double dot = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+      const double alpha = __shfl_sync(0xffffffffu, top, j), xn2 = __shfl_sync(0xffffffffu, dot, j);
+      double beta = alpha, tau = 0.0, scal = 0.0;
+      if (xn2 > 0.0) reflector(alpha, fma(alpha, alpha, xn2), beta, tau, scal);
+      const double w = fma(scal, dot, top);
+      if (lane < j) s.G[lane + j * GQ] = s.scal[lane] * w;
+      else if (lane == j) { s.tau[j] = tau; s.beta[j] = beta; s.scal[j] = scal; }
+      if (lane < W) s.coef[lane] = c > j && c < n ? tau * w : 0.0;
+      if (lane == 0) s.coef[GQ] = scal;
+    }
+    g.sync();
+    if (!on) continue;
+    // rows above j of R are final; row j: a_jc - tau w
+    const double scal = s.coef[GQ];
+#pragma unroll
+    for (int cc = 0; cc < W; ++cc) f[cc] = s.coef[cc];
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const double xs = g.tid + 256 * k == j ? 1.0 : x[k] * scal;
+#pragma unroll
+      for (int cc = 0; cc < W; ++cc) a[k][cc] = fma(-f[cc], xs, a[k][cc]);
+    }
   }
+  g.sync();
   // T = (triu(G, 1) + diag(1 / tau))^{-1}: lane = row, a column per warp and
   // pass, back substitution with the solved value by shuffle (tau_s multiplies
   // where the inverse would divide; tau = 0 gives a zero row and column)
   {
-    const double tr = lane < km ? s.tau[lane] : 0.0;
-    for (int c = g.wid; c < km; c += g.nw) {
+    const double tr = lane < n ? s.tau[lane] : 0.0;
+    for (int c = g.wid; c < n; c += g.nw) {
       double up = lane == c ? 1.0 : 0.0;
       for (int q = c; q >= 0; --q) {
         const double xq = __shfl_sync(0xffffffffu, up * tr, q);
         if (lane < q) up = fma(-s.G[lane + q * GQ], xq, up);
         else if (lane == q) up = xq;
       }
-      s.T[lane + c * GQ] = lane <= c ? up : 0.0;
+      if (lane < GQ) s.T[lane + c * GQ] = lane <= c ? up : 0.0;
     }
   }
-  // R out, clean V in place
-  for (int c = g.wid; c < n; c += g.nw) {
-    double* pc = P + (int64_t)c * ldp;
-    const double b = c < km ? s.beta[c] : 0.0, sc = c < km ? s.scal[c] : 0.0;
-    for (int e = lane; e < km; e += 32) R[e + (int64_t)c * ldr] = e < c ? pc[e] : (e == c ? b : 0.0);
-    __syncwarp();
-    if (c < km)
-      for (int e = lane; e < m; e += 32) pc[e] = e > c ? pc[e] * sc : (e == c ? 1.0 : 0.0);
+  if (on) {
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int r = g.tid + 256 * k;
+#pragma unroll
+      for (int c = 0; c < W; ++c)
+        if (r < m && c < n) {
+          if (r < n) R[r + c * ldr] = r < c ? a[k][c] : (r == c ? s.beta[c] : 0.0);
+          V[r + c * ldv] = r > c ? a[k][c] * s.scal[c] : (r == c ? 1.0 : 0.0);
+        }
+    }
   }
   g.sync();
+}
+
+// Widest panel of m rows: 16 columns of up to two rows a thread, 8 of up to four.
+constexpr int G_ROWS_MAX = 1024;
+FRANK_HD int panel_width(int m) { return m <= 512 ? 16 : 8; }
+
+FRANK_D void g_panel_qr(const Grp& g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
+                        int64_t ldr, GrpShared& s) {
+  if (m > 512) panel_qr_rows<8, 4>(g, m, n, P, ldp, V, ldv, R, ldr, s);
+  else if (m > 256) panel_qr_rows<16, 2>(g, m, n, P, ldp, V, ldv, R, ldr, s);
+  else panel_qr_rows<16, 1>(g, m, n, P, ldp, V, ldv, R, ldr, s);
 }
 
 FRANK_HD int panel_ld(int m) { return ((m + 15) & ~15) + 4; }   // 4 mod 16: conflict-free fragments
@@ -294,40 +366,49 @@ struct GrpScratch {
   double *W, *W2, *part;
 };
 
-// Blocked Householder QR of A (m x n, lda): panels of w <= GQ columns in smP
-// (panel_ld(m) x w doubles, shared), T factors in Tf (GQ x GQ per panel), the
-// clean V of each panel left in A (rows and columns j0 ..), R (min(m, n) x n,
-// ldr, zeros below the diagonal) apart.
-static __device__ __noinline__ void g_qr(Grp g, int m, int n, double* A, int64_t lda, double* R, int64_t ldr, double* Tf,
-                                  int w, double* smP, GrpShared& s, GrpScratch x) {
-  const int km = min(m, n), ldp = panel_ld(m);
+// Trailing products of a panel V (mr x jn, ldv, clean) with its T: X (mr x r,
+// ldx) -= V op(T) V^T X; rows of X at or below kr are zero on entry.
+FRANK_D void g_wy(const Grp& g, int mr, int kr, int jn, const double* V, int64_t ldv, const double* T, bool tt, int r,
+                  double* X, int64_t ldx, const GrpScratch& x) {
+  for (int op = 0; op < 3; ++op) {
+    // W = V^T X; W2 = op(T) W; X -= V W2
+    const double* A = op == 1 ? T : V;
+    const int64_t ld = op == 1 ? GQ : ldv;
+    const bool ta = op == 0 || (op == 1 && tt);
+    const double* B = op == 0 ? X : (op == 1 ? x.W : x.W2);
+    double* C = op == 0 ? x.W : (op == 1 ? x.W2 : X);
+    g_mm(g, op == 2 ? mr : jn, r, op == 0 ? kr : jn, op == 2 ? -1.0 : 1.0, A, ta ? ld : 1, ta ? 1 : ld, B,
+         op == 0 ? ldx : GQ, 1, op == 2 ? 1.0 : 0.0, C, op == 2 ? ldx : GQ, x.part);
+  }
+}
+
+// Blocked Householder QR of A (m x n, lda; overwritten): panels of w <= panel_width(m)
+// columns, T factors in Tf (GQ x GQ per panel), the clean V of panel p in rows
+// and columns j0 .. of V (ldv; may be A), R (min(m, n) x n, ldr, zeros below the
+// diagonal) apart.  The trailing products read the panel from smP (shared,
+// panel_ld(m) x w doubles), or from A where that is in shared memory (smP null).
+FRANK_D void g_qr(const Grp& g, int m, int n, double* A, int64_t lda, double* V, int64_t ldv, double* R, int64_t ldr,
+                  double* Tf, int w, double* smP, GrpShared& s, const GrpScratch& x) {
+  const int km = min(m, n), lane = threadIdx.x & 31;
   for (int j0 = 0, p = 0; j0 < km; j0 += w, ++p) {
-    const int jn = min(w, km - j0), mr = m - j0;
+    const int jn = min(w, km - j0), mr = m - j0, nc = n - j0 - jn;
     double* Ap = A + j0 + (int64_t)j0 * lda;
-    const int lane = threadIdx.x & 31;
-    for (int c = g.wid; c < jn; c += g.nw)
-#pragma unroll 4
-      for (int r = lane; r < mr; r += 32) smP[r + c * ldp] = Ap[r + (int64_t)c * lda];
-    // R rows below this panel's diagonal block are zero
+    double* At = Ap + (int64_t)jn * lda;
+    double* Vp = smP ? smP : Ap;
+    const int64_t ldp = smP ? panel_ld(m) : lda;
+    // R below this panel's diagonal block is zero
     for (int c = g.wid; c < jn; c += g.nw)
       for (int r = j0 + jn + lane; r < km; r += 32) R[r + (int64_t)(j0 + c) * ldr] = 0.0;
-    g.sync();
-    g_panel_qr(g, mr, jn, smP, ldp, R + j0 + (int64_t)j0 * ldr, ldr, s);
+    g_panel_qr(g, mr, jn, Ap, lda, Vp, ldp, R + j0 + (int64_t)j0 * ldr, ldr, s);
     for (int c = g.wid; c < jn; c += g.nw)
 #pragma unroll 4
-      for (int r = lane; r < mr; r += 32) Ap[r + (int64_t)c * lda] = smP[r + c * ldp];
-    for (int e = g.tid; e < GQ * GQ; e += g.nt) Tf[(int64_t)p * GQ * GQ + e] = s.T[e];
-    const int nc = n - j0 - jn;
+      for (int r = lane; r < mr; r += 32) V[(j0 + r) + (int64_t)(j0 + c) * ldv] = Vp[r + c * ldp];
+    for (int e = g.tid; e < GQ * GQ; e += g.nt) Tf[p * GQ * GQ + e] = s.T[e];
     if (nc > 0) {
-      double* At = A + j0 + (int64_t)(j0 + jn) * lda;
-      g_gemm_tn(g, jn, nc, mr, 1.0, smP, ldp, At, lda, x.W, GQ, x.part, s.part);
-      g_gemm(g, jn, nc, jn, 1.0, s.T, GQ, true, x.W, GQ, false, 0.0, x.W2, GQ, s.part);
-      g_gemm(g, mr, nc, jn, -1.0, smP, ldp, false, x.W2, GQ, false, 1.0, At, lda, s.part);
+      g_wy(g, mr, mr, jn, Vp, ldp, s.T, true, nc, At, lda, x);
       // the finished rows of R
-      for (int e = g.tid; e < jn * nc; e += g.nt) {
-        const int r = e % jn, c = e / jn;
-        R[(j0 + r) + (int64_t)(j0 + jn + c) * ldr] = At[r + (int64_t)c * lda];
-      }
+      for (int e = g.tid; e < jn * nc; e += g.nt)
+        R[(j0 + e % jn) + (int64_t)(j0 + jn + e / jn) * ldr] = At[e % jn + (int64_t)(e / jn) * lda];
     }
     g.sync();
   }
@@ -335,33 +416,29 @@ static __device__ __noinline__ void g_qr(Grp g, int m, int n, double* A, int64_t
 
 // X (m x r, ldx) := Q X with the k reflectors of g_qr (clean V in A, Tf, panels
 // of w).  Rows of X at or below nz are zero on entry.
-static __device__ __noinline__ void g_apply_q(Grp g, int m, int k, const double* A, int64_t lda, const double* Tf, int w,
-                                       int r, double* X, int64_t ldx, int nz, GrpShared& s, GrpScratch x) {
+FRANK_D void g_apply_q(const Grp& g, int m, int k, const double* A, int64_t lda, const double* Tf, int w, int r,
+                       double* X, int64_t ldx, int nz, const GrpScratch& x) {
   for (int p = (k + w - 1) / w - 1; p >= 0; --p) {
-    const int j0 = p * w, jn = min(w, k - j0), mr = m - j0;
-    const int kr = min(mr, max(0, nz - j0));
+    const int j0 = p * w, kr = min(m - j0, max(0, nz - j0));
     nz = m;
     if (kr == 0) continue;
-    const double* V = A + j0 + (int64_t)j0 * lda;
-    const double* T = Tf + (int64_t)p * GQ * GQ;
-    g_gemm_tn(g, jn, r, kr, 1.0, V, lda, X + j0, ldx, x.W, GQ, x.part, s.part);
-    g_gemm(g, jn, r, jn, 1.0, T, GQ, false, x.W, GQ, false, 0.0, x.W2, GQ, s.part);
-    g_gemm(g, mr, r, jn, -1.0, V, lda, false, x.W2, GQ, false, 1.0, X + j0, ldx, s.part);
+    g_wy(g, m - j0, kr, min(w, k - j0), A + j0 + (int64_t)j0 * lda, lda, Tf + p * GQ * GQ, false, r, X + j0, ldx, x);
   }
 }
 
-// Project the columns of Y (m x p, ldy) out of the span of Q (m x k, ldq,
-// orthonormal columns), twice (classical Gram-Schmidt with one
-// re-orthogonalisation): Z (k x p, ldz) = Q^T Y_0, Y = (I - Q Q^T)^2 Y_0,
+// Project the columns of Y (m x p, ldy) out of the span of Q (m x k, element (i,
+// j) at Q[i qi + j qj], orthonormal columns), twice (classical Gram-Schmidt
+// with one re-orthogonalisation): Z (k x p, ldz) = Q^T Y_0, Y = (I - Q Q^T)^2 Y_0,
 // Y_0 = Q Z + Y.  Z2 (k x p) is scratch.
 template <typename T>
-FRANK_D void g_project_out(Grp g, int m, int k, int p, const T* Q, int64_t ldq, double* Y, int64_t ldy, double* Z,
-                           int64_t ldz, double* Z2, GrpShared& s, GrpScratch x) {
-  for (int pass = 0; pass < 2; ++pass) {
-    double* Zp = pass ? Z2 : Z;
-    const int64_t ldp = pass ? k : ldz;
-    g_gemm_tn(g, k, p, m, 1.0, Q, ldq, Y, ldy, Zp, ldp, x.part, s.part);
-    g_gemm(g, m, p, k, -1.0, Q, ldq, false, Zp, ldp, false, 1.0, Y, ldy, s.part);
+FRANK_D void g_project_out(const Grp& g, int m, int k, int p, const T* Q, int64_t qi, int64_t qj, double* Y,
+                           int64_t ldy, double* Z, int64_t ldz, double* Z2, const GrpScratch& x) {
+  for (int op = 0; op < 4; ++op) {
+    const bool tn = !(op & 1);
+    double* Zp = op >= 2 ? Z2 : Z;
+    const int64_t ldp = op >= 2 ? k : ldz;
+    g_mm(g, tn ? k : m, p, tn ? m : k, tn ? 1.0 : -1.0, Q, tn ? qj : qi, tn ? qi : qj, tn ? Y : Zp, tn ? ldy : ldp, 1,
+         tn ? 0.0 : 1.0, tn ? Zp : Y, tn ? ldp : ldy, x.part);
   }
   for (int e = g.tid; e < k * p; e += g.nt) Z[(e % k) + (int64_t)(e / k) * ldz] += Z2[e];
   g.sync();
@@ -390,7 +467,7 @@ FRANK_D void warp_argmax_key(double& v, int& idx) {
 // row j and the scaled reflector below; every other column its rows of R.
 // cand: 4 * nw doubles (two rows of values and indices); vec: 2 min(m, n)
 // doubles.  All shared.
-static __device__ __noinline__ int g_rrqr(Grp g, int m, int n, double* A, int lda, double thr, int maxr, double* tau,
+FRANK_D int g_rrqr(const Grp& g, int m, int n, double* A, int lda, double thr, int maxr, double* tau,
                                    int* ord, int* at, double* vec, double* cand) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7;
   const int mind = min(min(m, n), maxr);
@@ -423,38 +500,22 @@ static __device__ __noinline__ int g_rrqr(Grp g, int m, int n, double* A, int ld
     int kp = lane < g.nw ? ci[lane] : -1;
     warp_argmax_key(mx, kp);
     if (r >= mind || kp < 0 || !(mx > thr2)) break;
-    const double* x = A + (int64_t)kp * lda;
+    // the pivot's remaining norm is the search's own maximum
+    const double* x = A + kp * lda;
     const double alpha = x[r];
-    double xn2 = 0.0, bt = 0.0, t = 0.0, sc = 0.0;
-    bool have = false;
+    double bt = 0.0, t = 0.0, sc = 0.0;
+    if (mx > 0.0) reflector(alpha, mx, bt, t, sc);
     bv = -1.0;
     bi = -1;
     for (int c0 = 0; c0 < n; c0 += ng) {
       const int c = c0 + gi;
       const bool live = c < n && c != kp && at[min(c, n - 1)] > r;
-      double* p = A + (int64_t)min(c, n - 1) * lda;
-      double d0 = 0.0, d1 = 0.0;
-      if (!have) {
+      double* p = A + min(c, n - 1) * lda;
+      double d0 = 0.0;
 #pragma unroll 4
-        for (int e = r + 1 + l8; e < m; e += 8) {
-          const double v = x[e];
-          d1 = fma(v, v, d1);
-          d0 = fma(v, p[e], d0);
-        }
+      for (int e = r + 1 + l8; e < m; e += 8) d0 = fma(x[e], p[e], d0);
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
-          d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-          d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-        }
-        xn2 = d1;
-        reflector(alpha, xn2, bt, t, sc);
-        have = true;
-      } else {
-#pragma unroll 4
-        for (int e = r + 1 + l8; e < m; e += 8) d0 = fma(x[e], p[e], d0);
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-      }
+      for (int o = 4; o > 0; o >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, o);
       const double top = p[r], w = live ? t * fma(sc, d0, top) : 0.0, f = w * sc;
       __syncwarp();
       double q = 0.0;
@@ -541,8 +602,8 @@ FRANK_D void g_apply_cols(const Grp& g, int m, int k, int r, const double* A, in
   }
 }
 
-constexpr int G_COLS_MAX = 256;   // rows the register columns of g_apply_cols hold
-static __device__ __noinline__ void g_apply_rrqr(Grp g, int m, int k, int r, const double* A, int lda, const double* tau,
+constexpr int G_COLS_MAX = 160;   // rows the register columns of g_apply_cols hold
+FRANK_D void g_apply_rrqr(const Grp& g, int m, int k, int r, const double* A, int lda, const double* tau,
                                           const int* ord, bool ident, const double* X0, int64_t ldx0,
                                           const int* perm, double* X, int64_t ldx) {
   if (m <= 48) g_apply_cols<6>(g, m, k, r, A, lda, tau, ord, ident, X0, ldx0, perm, X, ldx);
@@ -588,10 +649,10 @@ FRANK_HD int64_t rand_qrcp_smem(int m, int n, int w) {
   return sk > pn ? sk : pn;
 }
 
-static __device__ __noinline__ int g_rand_qrcp(Grp g, int m, int n, double* A, int64_t lda, double* R, int64_t ldr,
+FRANK_D int g_rand_qrcp(const Grp& g, int m, int n, double* A, int64_t lda, double* R, int64_t ldr,
                                         double thr, int maxr, int w, int* jpvt, double* Tf, double* om, double* nrm2,
                                         double* region, int* iscr, unsigned long long* mx, GrpShared& s,
-                                        GrpScratch x) {
+                                        const GrpScratch& x) {
   const int lane = threadIdx.x & 31;
   const int mind = min(min(m, n), maxr);
   for (int c = g.tid; c < n; c += g.nt) jpvt[c] = c;
@@ -622,7 +683,7 @@ static __device__ __noinline__ int g_rand_qrcp(Grp g, int m, int n, double* A, i
     int* ord = reinterpret_cast<int*>(cand + 4 * g.nw);
     int* at = ord + ((sb + 1) & ~1);
     g.sync();
-    g_gemm(g, sb, nr, mr, 1.0, om, sb, false, At, lda, false, 0.0, Y, ldy, s.part);
+    g_mm(g, sb, nr, mr, 1.0, om, 1, sb, At, lda, 1, 0.0, Y, ldy, x.part);
     const int got = g_rrqr(g, sb, nr, Y, ldy, -1.0, b, tau, ord, at, vec, cand);
     if (got < b) return r;   // not a number in the sketch: no pivots to take
     // the chosen columns go to positions 0 .. b-1 in order; the columns they
@@ -681,12 +742,8 @@ static __device__ __noinline__ int g_rand_qrcp(Grp g, int m, int n, double* A, i
       double* smP = region;
       double* Rp = R + r + (int64_t)r * ldr;
       for (int c = g.wid; c < b; c += g.nw)
-#pragma unroll 4
-        for (int e = lane; e < mr; e += 32) smP[e + c * ldp] = At[e + (int64_t)c * lda];
-      for (int c = g.wid; c < b; c += g.nw)
         for (int e = r + b + lane; e < min(m, n); e += 32) R[e + (int64_t)(r + c) * ldr] = 0.0;
-      g.sync();
-      g_panel_qr(g, mr, b, smP, ldp, Rp, ldr, s);
+      g_panel_qr(g, mr, b, At, lda, smP, ldp, Rp, ldr, s);
       for (int c = g.wid; c < b; c += g.nw)
 #pragma unroll 4
         for (int e = lane; e < mr; e += 32) At[e + (int64_t)c * lda] = smP[e + c * ldp];
@@ -694,9 +751,7 @@ static __device__ __noinline__ int g_rand_qrcp(Grp g, int m, int n, double* A, i
       const int nc = nr - b;
       if (nc > 0) {
         double* Ac = At + (int64_t)b * lda;
-        g_gemm_tn(g, b, nc, mr, 1.0, smP, ldp, Ac, lda, x.W, GQ, x.part, s.part);
-        g_gemm(g, b, nc, b, 1.0, s.T, GQ, true, x.W, GQ, false, 0.0, x.W2, GQ, s.part);
-        g_gemm(g, mr, nc, b, -1.0, smP, ldp, false, x.W2, GQ, false, 1.0, Ac, lda, s.part);
+        g_wy(g, mr, mr, b, smP, ldp, s.T, true, nc, Ac, lda, x);
       }
       if (g.tid <= GQ) mx[g.tid] = 0ull;
       // rows of R right of the panel, and the squared norms below it
@@ -751,7 +806,7 @@ static __device__ __noinline__ int g_rand_qrcp(Grp g, int m, int n, double* A, i
 // one barrier per round.  Rotation as Demmel and Veselic, "Jacobi's method is
 // more accurate than QR", SIAM J. Matrix Anal. Appl. 13, 1992.  flags: 2 ints
 // (shared).  Returns the number of sweeps, or -1 at the sweep limit.
-static __device__ __noinline__ int g_jacobi(Grp g, int m, int n, double* G, int64_t ldg, int max_sweeps, int* flags,
+FRANK_D int g_jacobi(const Grp& g, int m, int n, double* G, int64_t ldg, int max_sweeps, int* flags,
                                      int m_rot) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7;
   const int N2 = n + (n & 1);
@@ -788,10 +843,14 @@ static __device__ __noinline__ int g_jacobi(Grp g, int m, int n, double* G, int6
           b += __shfl_xor_sync(0xffffffffu, b, o);
           h += __shfl_xor_sync(0xffffffffu, h, o);
         }
-        if (!on || a == 0.0 || b == 0.0 || fabs(h) <= tol * sqrt(a) * sqrt(b)) continue;
+        // |h| <= tol ||g_p|| ||g_q||: nothing to rotate (squared while the squares are in range)
+        const double ab = a * b;
+        if (!on || a == 0.0 || b == 0.0) continue;
+        if (ab > 1e-280 && ab < 1e280 ? h * h <= tol * tol * ab : fabs(h) <= tol * sqrt(a) * sqrt(b)) continue;
         const double zeta = (b - a) / (2.0 * h);
-        const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = rsqrt(1.0 + t * t), s = c * t;
+        const double za = fabs(zeta), zc = fmin(za, 1e100), u = fma(zc, zc, 1.0);
+        const double t = copysign(__drcp_rn(za + u * rsqrt(u)), zeta);
+        const double c = rsqrt(fma(t, t, 1.0)), s = c * t;
 #pragma unroll 4
         for (int i = l8; i < m_rot; i += 8) {
           const double x = gp[i], y = gq[i];
