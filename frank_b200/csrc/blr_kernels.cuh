@@ -1213,7 +1213,7 @@ constexpr int RECOMP_THREADS = 512;
 constexpr int SPLIT_P = 32;       // split band-1 targets whose operand rank exceeds this (default)
 constexpr int SPLIT_MAX = 128;    // band-1 tasks eligible for the split (scratch slots)
 constexpr int RECOMP_BMAX = 810;  // largest block order (a panel of each side in shared memory)
-constexpr int RECOMP_SMEM_BYTES = 227 * 1024 - 1024;    // dynamic shared memory (all but the static part)
+constexpr int RECOMP_SMEM_BYTES = 194 * 1024;    // dynamic shared memory (all but the static part)
 
 struct RecompShared {
   GrpShared gs[2];               // one per half of the CTA

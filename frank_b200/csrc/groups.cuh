@@ -235,7 +235,7 @@ FRANK_D void reflector(double alpha, double n2, double& beta, double& tau, doubl
 // holds the reflectors (V may be P), s.T the T factor (upper, zero below) and
 // R (n x n, ldr) the triangle with zeros below its diagonal.
 template <int W, int RPT>
-FRANK_D void panel_qr_rows(const Grp& g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
+static __device__ __noinline__ void panel_qr_rows(Grp g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
                            int64_t ldr, GrpShared& s) {
   const int lane = threadIdx.x & 31;
   const bool on = g.wid < 8;
@@ -423,6 +423,100 @@ FRANK_D void g_apply_q(const Grp& g, int m, int k, const double* A, int64_t lda,
     nz = m;
     if (kr == 0) continue;
     g_wy(g, m - j0, kr, min(w, k - j0), A + j0 + (int64_t)j0 * lda, lda, Tf + p * GQ * GQ, false, r, X + j0, ldx, x);
+  }
+}
+
+// The same QR for any number of rows: a panel goes down the rows in chunks, the
+// first of GT_ROWS rows, each later one factored stacked under the panel's
+// triangle (flat-tree TSQR; Demmel, Grigori, Hoemmen, Langou,
+// "Communication-optimal parallel and sequential QR and LU factorizations",
+// SIAM J. Sci. Comput. 34, 2012).  The reflectors of a later chunk are [I; X]
+// over the panel's top rows and the chunk, so only X is stored, in the chunk's
+// place in A; T factors of panel p, chunk i at Tf + (p * gt_chunks(m) + i)
+// GQ^2.  smP: panel_ld(min(m, GT_ROWS)) x GQ doubles (shared).
+constexpr int GT_ROWS = 512;
+FRANK_HD int gt_chunks(int m) { return m <= GT_ROWS ? 1 : 1 + (m - GT_ROWS + GT_ROWS - GQ - 1) / (GT_ROWS - GQ); }
+
+// X (rows [0, jn) at Xt, chunk rows at Xc, ldx) <- (I - [I; V] op(T) [I; V]^T) X
+FRANK_D void g_wy_stacked(const Grp& g, int mr, int kr, int jn, const double* V, int64_t ldv, const double* T, bool tt,
+                          int r, double* Xt, double* Xc, int64_t ldx, const GrpScratch& x) {
+  for (int e = g.tid; e < jn * r; e += g.nt) x.W[e % jn + (e / jn) * GQ] = Xt[e % jn + (int64_t)(e / jn) * ldx];
+  g.sync();
+  for (int op = 0; op < 3; ++op) {
+    const double* A = op == 1 ? T : V;
+    const int64_t ld = op == 1 ? GQ : ldv;
+    const bool ta = op == 0 || (op == 1 && tt);
+    const double* B = op == 0 ? Xc : (op == 1 ? x.W : x.W2);
+    double* C = op == 0 ? x.W : (op == 1 ? x.W2 : Xc);
+    if (op == 0 && kr <= 0) continue;
+    g_mm(g, op == 2 ? mr : jn, r, op == 0 ? kr : jn, op == 2 ? -1.0 : 1.0, A, ta ? ld : 1, ta ? 1 : ld, B,
+         op == 0 ? ldx : GQ, 1, op == 1 ? 0.0 : 1.0, C, op == 2 ? ldx : GQ, x.part);
+  }
+  for (int e = g.tid; e < jn * r; e += g.nt) Xt[e % jn + (int64_t)(e / jn) * ldx] -= x.W2[e % jn + (e / jn) * GQ];
+  g.sync();
+}
+
+FRANK_D void g_qr_tall(const Grp& g, int m, int n, double* A, int64_t lda, double* R, int64_t ldr, double* Tf,
+                       double* smP, GrpShared& s, const GrpScratch& x) {
+  const int km = min(m, n), lane = threadIdx.x & 31, nch = gt_chunks(m), ldp = panel_ld(min(m, (int)GT_ROWS));
+  for (int j0 = 0, p = 0; j0 < km; j0 += GQ, ++p) {
+    const int jn = min((int)GQ, km - j0), nc = n - j0 - jn;
+    for (int c = g.wid; c < jn; c += g.nw)
+      for (int r = j0 + jn + lane; r < km; r += 32) R[r + (int64_t)(j0 + c) * ldr] = 0.0;
+    double* Rp = R + j0 + (int64_t)j0 * ldr;
+    double* Ct = A + j0 + (int64_t)(j0 + jn) * lda;      // the panel's rows of the later columns
+    int row = j0;
+    for (int i = 0; row < m; ++i) {
+      const int cr = min(m - row, i == 0 ? (int)GT_ROWS : GT_ROWS - GQ);
+      double* Ac = A + row + (int64_t)j0 * lda;
+      const int top = i == 0 ? 0 : jn;                   // stacked rows of the triangle
+      if (i > 0) {
+        for (int c = g.wid; c < jn; c += g.nw) {
+          if (lane < jn) smP[lane + c * ldp] = lane <= c ? Rp[lane + (int64_t)c * ldr] : 0.0;
+#pragma unroll 4
+          for (int r = lane; r < cr; r += 32) smP[jn + r + c * ldp] = Ac[r + (int64_t)c * lda];
+        }
+        g.sync();
+        g_panel_qr(g, jn + cr, jn, smP, ldp, smP, ldp, Rp, ldr, s);
+      } else {
+        g_panel_qr(g, cr, jn, Ac, lda, smP, ldp, Rp, ldr, s);
+      }
+      double* T = Tf + (int64_t)(p * nch + i) * GQ * GQ;
+      for (int c = g.wid; c < jn; c += g.nw)
+#pragma unroll 4
+        for (int r = lane; r < cr; r += 32) Ac[r + (int64_t)c * lda] = smP[top + r + c * ldp];
+      for (int e = g.tid; e < GQ * GQ; e += g.nt) T[e] = s.T[e];
+      if (nc > 0) {
+        if (i == 0) g_wy(g, cr, cr, jn, smP, ldp, s.T, true, nc, Ct, lda, x);
+        else g_wy_stacked(g, cr, cr, jn, smP + jn, ldp, s.T, true, nc, Ct, Ac + (int64_t)jn * lda, lda, x);
+      }
+      g.sync();
+      row += cr;
+    }
+    for (int e = g.tid; e < jn * nc; e += g.nt)
+      R[(j0 + e % jn) + (int64_t)(j0 + jn + e / jn) * ldr] = Ct[e % jn + (int64_t)(e / jn) * lda];
+    g.sync();
+  }
+}
+
+// X (m x r, ldx) := Q X with the k reflectors of g_qr_tall; rows of X at or below
+// nz are zero on entry.
+FRANK_D void g_apply_q_tall(const Grp& g, int m, int k, const double* A, int64_t lda, const double* Tf, int r,
+                            double* X, int64_t ldx, int nz, const GrpScratch& x) {
+  const int nch = gt_chunks(m);
+  for (int p = (k + GQ - 1) / GQ - 1; p >= 0; --p) {
+    const int j0 = p * GQ, jn = min((int)GQ, k - j0);
+    const int c0 = min(m - j0, (int)GT_ROWS);
+    const int later = m - j0 - c0, nl = (later + GT_ROWS - GQ - 1) / (GT_ROWS - GQ);
+    for (int i = nl; i >= 1; --i) {
+      const int row = j0 + c0 + (i - 1) * (GT_ROWS - GQ), cr = min(m - row, GT_ROWS - GQ);
+      g_wy_stacked(g, cr, min(cr, nz - row), jn, A + row + (int64_t)j0 * lda, lda,
+                   Tf + (int64_t)(p * nch + i) * GQ * GQ, false, r, X + j0, X + row, ldx, x);
+    }
+    // top rows: chunk 0 holds them all the same (they may be filled by the later chunks)
+    g_wy(g, c0, min(c0, max(nz - j0, jn)), jn, A + j0 + (int64_t)j0 * lda, lda, Tf + (int64_t)p * nch * GQ * GQ, false,
+         r, X + j0, ldx, x);
+    nz = m;
   }
 }
 
@@ -806,7 +900,7 @@ FRANK_D int g_rand_qrcp(const Grp& g, int m, int n, double* A, int64_t lda, doub
 // one barrier per round.  Rotation as Demmel and Veselic, "Jacobi's method is
 // more accurate than QR", SIAM J. Matrix Anal. Appl. 13, 1992.  flags: 2 ints
 // (shared).  Returns the number of sweeps, or -1 at the sweep limit.
-FRANK_D int g_jacobi(const Grp& g, int m, int n, double* G, int64_t ldg, int max_sweeps, int* flags,
+static __device__ __noinline__ int g_jacobi(Grp g, int m, int n, double* G, int64_t ldg, int max_sweeps, int* flags,
                                      int m_rot) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7;
   const int N2 = n + (n & 1);

@@ -74,10 +74,9 @@ void launch_qr(cudaStream_t s, int m, int n, int count, const double* a, int64_t
 void launch_svd(cudaStream_t s, int m, int n, int count, const double* a, int64_t lda, int64_t sa, double* u,
                 int64_t ldu, int64_t su, double* sv, int64_t ss, double* vt, int64_t ldvt, int64_t svt,
                 double* scratch, int64_t ws, int* err);
-int lr_add_shm_bytes(int ka, int kb);
-int lr_add_prepare(int bytes);
-void launch_lr_add_tasks(cudaStream_t s, int count, const LrAddTask* tasks, int kmax, int fast, double* scratch,
-                         int* err, int shm_bytes);
+int lr_add_prepare();
+void launch_lr_add_tasks(cudaStream_t s, int count, int mmax, const LrAddTask* tasks, int kmax, int fast,
+                         double* scratch, int* err);
 }  // namespace ops
 }  // namespace frank
 
@@ -726,7 +725,6 @@ struct frank_hodlr {
   ::frank::ops::LrAddTask* tasks_d = nullptr;   // every update's additions, in launch order
   std::vector<::frank::ops::LrAddTask> tasks_h;
   int64_t ntasks_cap = 0;
-  int lr_shm = 0;
   double* mv_part = nullptr;
   int64_t mv_part_cap = 0;
   double* work = nullptr;           // refinement: residual / correction (n x nrhs)
@@ -851,8 +849,8 @@ void enqueue_update(frank_hodlr* h, int lr, int cr, const double* Ux, const doub
     }
     cudaStream_t sj_stream = h->ls[j];
     cudaStreamWaitEvent(sj_stream, h->ev_core, 0);
-    ::frank::ops::launch_lr_add_tasks(sj_stream, idx, h->tasks_d + t0, k, h->fast, h->lr_scratch,
-                                      h->err + hk::HERR_JACOBI, h->lr_shm);
+    ::frank::ops::launch_lr_add_tasks(sj_stream, idx, (int)sj, h->tasks_d + t0, k, h->fast, h->lr_scratch,
+                                      h->err + hk::HERR_JACOBI);
     cudaEventRecord(h->lev[j], sj_stream);
     ++h->launches;
   }
@@ -1099,7 +1097,6 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaEventCreateWithFlags(&h->ev_ps, cudaEventDisableTiming));
   A(cudaStreamCreateWithFlags(&h->ps, cudaStreamNonBlocking));
   A(dalloc(&h->WZ, (size_t)nk));
-  h->lr_shm = ::frank::ops::lr_add_shm_bytes(rank, rank);
   A(cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking));
   A(cudaEventCreate(&h->e0));
   A(cudaEventCreate(&h->e1));
@@ -1120,7 +1117,7 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaFuncSetAttribute(blr::k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(blr::k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(hk::k_h_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::WALK_SMEM));
-  if (e == cudaSuccess && h->lr_shm > 0 && ::frank::ops::lr_add_prepare(h->lr_shm) != FRANK_OK) h->lr_shm = 0;
+  if (e == cudaSuccess && ::frank::ops::lr_add_prepare() != FRANK_OK) e = cudaErrorInvalidValue;
   if (e != cudaSuccess) {
     free_plan(h);
     return hfail(FRANK_ERR_CUDA, std::string("H-matrix set-up: ") + cudaGetErrorString(e));

@@ -86,15 +86,12 @@ FRANK_D void load_svd(int m, int n, const double* a, int64_t lda, bool trans, do
 // SVD of a (m x n, lda): U (m x k, ldu), s (k), Vt (k x n, ldvt), k = min(m, n),
 // singular values descending; columns with a zero singular value get a zero
 // left vector.  Scratch: (m + n) * k + 2 k doubles.  Returns false on a
-// Jacobi sweep limit.  When shm holds at least (max(m, n) + k) k doubles the
-// rotated matrix lives there instead of in the scratch (the sweeps are a
-// chain of dependent column loads, so shared memory's latency sets their
-// pace; the scratch layout is unchanged).
+// Jacobi sweep limit.
 FRANK_D bool cta_svd(int m, int n, const double* a, int64_t lda, double* U, int64_t ldu, double* s, double* Vt,
-                     int64_t ldvt, double* scratch, int* flag, double* shm = nullptr, int64_t shm_cap = 0) {
+                     int64_t ldvt, double* scratch, int* flag) {
   const bool trans = m < n;
   const int mm = trans ? n : m, k = trans ? m : n;
-  double* G = (shm && (int64_t)(mm + k) * k <= shm_cap) ? shm : scratch;
+  double* G = scratch;
   double* sig = scratch + (int64_t)(mm + k) * k;
   int* ord = reinterpret_cast<int*>(sig + k);
   load_svd(m, n, a, lda, trans, G);
@@ -115,47 +112,6 @@ FRANK_D bool cta_svd(int m, int n, const double* a, int64_t lda, double* U, int6
     else U[r + (int64_t)j * ldu] = v;
   }
   for (int j = threadIdx.x; j < k; j += blockDim.x) s[j] = sig[ord[j]];
-  __syncthreads();
-  return ok;
-}
-
-// SVD of a square a (n x n, lda) preconditioned by column-pivoted QR
-// (Drmac and Veselic, "New fast and accurate Jacobi SVD algorithm", 2008):
-// a P = Q R, one-sided Jacobi on the columns of R^T with the rotations V
-// accumulated, R^T V = Y; then a = (Q V) diag(sigma) (P Y diag(1/sigma))^T.
-// The pivoted R is graded, so the sweeps converge in a few passes.  All of it
-// in shared memory shm (3 n^2 doubles); sc: 4 n doubles + 2 n ints (global).
-// Outputs as cta_svd.
-FRANK_D bool cta_svd_pqr(int n, const double* a, int64_t lda, double* U, int64_t ldu, double* s, double* Vt,
-                         int64_t ldvt, double* sc, double* shm, int* flag, double* red, int* redi) {
-  double* W = shm;                                  // n x n: R above, reflectors below
-  double* G = shm + (int64_t)n * n;                 // 2n x n (ld 2n): [R^T; I], rotated
-  double* tau = sc;
-  double* cn = tau + n;
-  double* pn = cn + n;
-  double* sig = pn + n;
-  int* jpvt = reinterpret_cast<int*>(sig + n);
-  int* ord = jpvt + n;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) W[e] = a[e % n + (int64_t)(e / n) * lda];
-  __syncthreads();
-  cta_truncated_geqp3(n, n, W, n, -1.0, n, tau, cn, pn, jpvt, red, redi);
-  __syncthreads();
-  const int ldg = 2 * n;
-  for (int e = threadIdx.x; e < ldg * n; e += blockDim.x) {
-    const int r = e % ldg, c = e / ldg;
-    G[e] = r < n ? (c <= r ? W[c + r * n] : 0.0) : (r - n == c ? 1.0 : 0.0);
-  }
-  __syncthreads();
-  const bool ok = jacobi_svd(n, n, G, sig, ord, flag);
-  cta_apply_q(n, n, W, n, tau, n, G + n, ldg);     // rows n..2n-1 become Q V
-  __syncthreads();
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int r = e % n, j = e / n, c = ord[j];
-    U[r + (int64_t)j * ldu] = G[n + r + c * ldg];
-    const double sv = sig[c];
-    Vt[j + (int64_t)jpvt[r] * ldvt] = sv > 0.0 ? G[r + c * ldg] / sv : 0.0;
-  }
-  for (int j = threadIdx.x; j < n; j += blockDim.x) s[j] = sig[ord[j]];
   __syncthreads();
   return ok;
 }
@@ -398,32 +354,11 @@ __global__ void __launch_bounds__(OT) k_op_rid(int m, int n, int s, int k, Mat A
 // else ka.  fast (fixed rank, Ua and Va^T orthonormal): the projections
 // Zu = Ua^T Ub, Zv = Va Vb^T, QR of the remainders only, core
 // [I Zu; 0 Ru] blockdiag(Sa, Sb) [I Zv; 0 Rv]^T.
-// Optional phase counters of the LowRank addition (build with
-// -DFRANK_LRA_TIMING; off by default): [0] operands and projections,
-// [1] QR of the remainders, [2] core and its SVD, [3] new bases, [4] count.
-#ifdef FRANK_LRA_TIMING
-__device__ unsigned long long g_lra_cycles[8];
-#define LRA_MARK(k)                                                                          \
-  do {                                                                                       \
-    if (threadIdx.x == 0) {                                                                  \
-      const long long _t = clock64();                                                        \
-      atomicAdd(&g_lra_cycles[(k)], (unsigned long long)(_t - _lra_t0));                     \
-      _lra_t0 = _t;                                                                          \
-    }                                                                                        \
-  } while (0)
-#define LRA_BEGIN() long long _lra_t0 = clock64()
-#else
-#define LRA_MARK(k) do {} while (0)
-#define LRA_BEGIN() do {} while (0)
-#endif
-
-FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* ua_out, int64_t ldua, double* sa_out,
+FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, double* ua_out, int64_t ldua, double* sa_out,
                          int64_t ldsa, double* va_out, int64_t ldva, int* ka_io, const double* ub, int64_t ldub,
-                         const double* sb, int64_t ldsb, const double* vb, int64_t ldvb, int kb, double* X, int* err,
-                         double* shm, int64_t shm_cap) {
+                         const double* sb, int64_t ldsb, const double* vb, int64_t ldvb, int kb, double* X, int* err) {
   __shared__ double gsm[GSM];
   __shared__ double red[32];
-  __shared__ int redi[32];
   __shared__ int flag, s_rank;
   const int ka = *ka_io;
   const int kt = ka + kb;
@@ -440,7 +375,6 @@ FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* u
   double* sc = T + (int64_t)max(m, n) * kt;     // svd scratch (2 kt + 2) kt
   const double *ua = ua_out, *sa = sa_out, *va = va_out;
   struct LD { int64_t ld; } Ua{ldua}, Sa{ldsa}, Va{ldva}, Ub{ldub}, Sb{ldsb}, Vb{ldvb};
-  LRA_BEGIN();
   const bool use_fast = fast && eps == 0.0 && kt <= m && kt <= n;
   int mu, mv;
   if (!use_fast) {
@@ -489,10 +423,8 @@ FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* u
                          gsm);
     cta_gemm<double, OT>(n, kb, ka, -1.0, Y, n, false, Rv + (int64_t)ka * kt, kt, false, 1.0, Y + (int64_t)ka * n, n,
                          gsm);
-    LRA_MARK(0);
     cta_householder_qr(m, kb, X + (int64_t)ka * m, m, tu, red);
     cta_householder_qr(n, kb, Y + (int64_t)ka * n, n, tv, red);
-    LRA_MARK(1);
     for (int64_t e = threadIdx.x; e < (int64_t)kt * kt; e += blockDim.x) {
       const int r = e % kt, c = e / kt;
       if (c < ka) { Rc[e] = r == c ? 1.0 : 0.0; Rv[e] = r == c ? 1.0 : 0.0; }
@@ -508,11 +440,8 @@ FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* u
                          T + (int64_t)ka * kt, kt, gsm);
     cta_gemm<double, OT>(kt, kt, kt, 1.0, T, kt, false, Rv, kt, true, 0.0, M, kt, gsm);
   }
-  const bool svd_ok = (mu == mv && shm && 3 * (int64_t)mu * mu <= shm_cap)
-                          ? cta_svd_pqr(mu, M, mu, Um, mu, sv, Vmt, mu, sc, shm, &flag, red, redi)
-                          : cta_svd(mu, mv, M, mu, Um, mu, sv, Vmt, min(mu, mv), sc, &flag, shm, shm_cap);
+  const bool svd_ok = cta_svd(mu, mv, M, mu, Um, mu, sv, Vmt, min(mu, mv), sc, &flag);
   if (!svd_ok && threadIdx.x == 0) atomicAdd(err + OPS_ERR_JACOBI, 1);
-  LRA_MARK(2);
   const int nsv = min(mu, mv);
   if (threadIdx.x == 0) {
     int r;
@@ -576,10 +505,6 @@ FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* u
     }
     __syncthreads();
   }
-  LRA_MARK(3);
-#ifdef FRANK_LRA_TIMING
-  if (threadIdx.x == 0) atomicAdd(&g_lra_cycles[4], 1ull);
-#endif
   double* sp = sa_out;
   for (int64_t e = threadIdx.x; e < (int64_t)r * r; e += blockDim.x) {
     const int i = e % r, c = e / r;
@@ -588,23 +513,265 @@ FRANK_D void lr_add_body(int m, int n, int kmax, int fast, double eps, double* u
   if (threadIdx.x == 0) *ka_io = r;
 }
 
-__global__ void __launch_bounds__(OT) k_op_lr_add(int m, int n, int kmax, int fast, double eps, Mat Ua, Mat Sa, Mat Va,
-                                                  int* ka_io, Mat Ub, Mat Sb, Mat Vb, const int* kb_in,
-                                                  double* scratch, int64_t ws, int* err, int64_t shm_cap) {
+// Largest ka + kb of lr_add_body (its core, the Jacobi matrix and the panels
+// share 190 KB of shared memory); larger ranks take lr_add_large_body.
+constexpr int LR_T = 512;             // threads of an addition
+constexpr int LR_KT_MAX = 88;
+
+struct LrShared {
+  GrpShared gs[2];
+  double red[32];
+  int flags[4];
+  int rank;
+};
+
+// Scratch of one addition (doubles): per side the remainder's basis, the core
+// factors, T factors and the new basis.
+struct LrLayout {
+  int64_t y[2], g[2], tf[2], tn[2], w[2], part[2], mtmp, x1, y1, aj, sig, total;
+};
+FRANK_HD LrLayout lr_layout(int m, int n, int kt) {
+  LrLayout L;
+  int64_t o = 0;
+  auto take = [&](int64_t c) { const int64_t r = o; o += (c + 31) & ~int64_t(31); return r; };
+  for (int sd = 0; sd < 2; ++sd) {
+    const int rows = sd ? n : m;
+    L.y[sd] = take((int64_t)rows * kt);
+    L.tn[sd] = take((int64_t)rows * kt);
+    L.g[sd] = take((int64_t)kt * kt);
+    L.tf[sd] = take((int64_t)((kt + GQ - 1) / GQ) * gt_chunks(rows) * GQ * GQ);
+    L.w[sd] = take(2 * (int64_t)GQ * kt);
+    L.part[sd] = take(8 * (int64_t)kt * kt < G_PART ? 8 * (int64_t)kt * kt : G_PART);
+  }
+  L.mtmp = take((int64_t)kt * kt);
+  L.x1 = take((int64_t)kt * kt);
+  L.y1 = take((int64_t)kt * kt);
+  L.aj = take(2 * (int64_t)kt * kt);
+  L.sig = take(2 * (int64_t)kt);
+  L.total = o;
+  return L;
+}
+
+// Shared memory (doubles behind LrShared): a panel of each side, or the core
+// with its vectors and the Jacobi matrix.
+FRANK_HD int64_t lr_region(int m, int n, int kt) {
+  const int64_t pu = (int64_t)panel_ld(m < GT_ROWS ? m : GT_ROWS) * GQ, pv = (int64_t)panel_ld(n < GT_ROWS ? n : GT_ROWS) * GQ;
+  const int64_t core = (int64_t)rrqr_ld(kt) * kt + 3 * kt + 4 * (LR_T / 32) + kt + 1 + 2 * (int64_t)kt * kt;
+  return pu + pv > core ? pu + pv : core;
+}
+
+struct LrArgs {
+  int m, n, kmax, fast;
+  double eps;
+  double *ua, *sa, *va;
+  const double *ub, *sb, *vb;
+  int64_t ldua, ldsa, ldva, ldub, ldsb, ldvb;
+  int* ka;
+  int kb;
+};
+
+// The addition for ka + kb <= LR_KT_MAX: the two sides run beside each other
+// on the two halves of the CTA (projection of B's basis out of A's, QR of the
+// remainder down the rows in chunks, new bases by blocked reflectors), and
+// meet for the core, whose preconditioned Jacobi SVD (column-pivoted QR M P =
+// Q R, one-sided Jacobi on P R^T with the rotations accumulated) stays in
+// shared memory.  One CTA per addition, so its latency is what an H-LU level's
+// chain of additions is made of: unblocked reflectors through L2 and eight
+// warps took 4.9 ms for 256 x 256 blocks of rank 32.
+FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
   extern __shared__ double dyn[];
+  LrShared& sh = *reinterpret_cast<LrShared*>(dyn);
+  double* region = dyn + sizeof(LrShared) / 8;
+  const int hf = threadIdx.x >= LR_T / 2;
+  const Grp half = grp_half(hf), all = grp_all();
+  const int ka = *A.ka, kb = A.kb, kt = ka + kb, m = A.m, n = A.n;
+  const LrLayout L = lr_layout(m, n, kt);
+  const bool fast = A.fast && A.eps == 0.0 && kt <= m && kt <= n;
+  const int mu = fast ? kt : min(m, kt), mv = fast ? kt : min(n, kt), nsv = min(mu, mv);
+  const int lane = threadIdx.x & 31;
+  {
+    // U side: rows m, A's basis ua; V side: rows n, A's basis va^T
+    const int rows = hf ? n : m, cols = fast ? kb : kt, mm = hf ? mv : mu;
+    const GrpScratch x{scratch + L.w[hf], scratch + L.w[hf] + GQ * kt, scratch + L.part[hf]};
+    double* Y = scratch + L.y[hf];
+    double* G = scratch + L.g[hf];
+    if (fast) {
+      if (hf == 0) {
+        for (int c = half.wid; c < kb; c += half.nw)
+#pragma unroll 4
+          for (int r = lane; r < rows; r += 32) Y[r + (int64_t)c * rows] = A.ub[r + (int64_t)c * A.ldub];
+      } else {
+        for (int e = half.tid; e < rows * kb; e += half.nt) Y[e / kb + (int64_t)(e % kb) * rows] = A.vb[e % kb + (int64_t)(e / kb) * A.ldvb];
+      }
+      half.sync();
+      g_project_out(half, rows, ka, kb, (const double*)(hf ? A.va : A.ua), hf ? A.ldva : 1, hf ? 1 : A.ldua, Y, rows, G,
+                    kt, scratch + L.tn[hf], x);
+    } else if (hf == 0) {
+      // [Ua Sa | Ub Sb]
+      for (int q = 0; q < 2; ++q)
+        g_mm(half, rows, q ? kb : ka, q ? kb : ka, 1.0, q ? A.ub : (const double*)A.ua, 1, q ? A.ldub : A.ldua,
+             q ? A.sb : (const double*)A.sa, q ? A.ldsb : A.ldsa, 1, 0.0, Y + (q ? (int64_t)ka * rows : 0), rows, x.part);
+    } else {
+      for (int e = half.tid; e < rows * kt; e += half.nt) {
+        const int c = e % kt, r = e / kt;
+        Y[r + (int64_t)c * rows] = c < ka ? A.va[c + (int64_t)r * A.ldva] : A.vb[(c - ka) + (int64_t)r * A.ldvb];
+      }
+      half.sync();
+    }
+    // fast: [Zu; Ru] (kt x kb) in G; rounded: R (mm x kt)
+    const int64_t pu = (int64_t)panel_ld(min(m, (int)GT_ROWS)) * GQ;
+    g_qr_tall(half, rows, cols, Y, rows, G + (fast ? ka : 0), fast ? kt : mm, scratch + L.tf[hf],
+              region + (hf ? pu : 0), sh.gs[hf], x);
+  }
+  __syncthreads();
+  // core (mu x mv): fast M = [Zu; Ru] Sb [Zv; Rv]^T + Sa, rounded M = Ru Rv^T
+  const int ldm = rrqr_ld(mu);
+  double* M = region;
+  double* X1 = scratch + L.x1;
+  double* Y1 = scratch + L.y1;
+  int k;
+  double* Aj;
+  int ldj;
+  double* tau = region + ldm * mv;
+  double* cand = tau + 3 * nsv;
+  int* ord = reinterpret_cast<int*>(cand + 4 * (LR_T / 32));
+  int* at = ord + nsv;
+  double* sig = scratch + L.sig;
+  int* rank_of = reinterpret_cast<int*>(sig + kt);
+  {
+    const double *Gu = scratch + L.g[0], *Gv = scratch + L.g[1];
+    double* part = scratch + L.part[0];
+    double* Mt = scratch + L.mtmp;
+    if (fast) g_mm(all, mu, kb, kb, 1.0, Gu, 1, mu, A.sb, A.ldsb, 1, 0.0, Mt, mu, part);
+    g_mm(all, mu, mv, fast ? kb : kt, 1.0, fast ? Mt : Gu, 1, mu, Gv, 1, mv, 0.0, M, ldm, part);
+    if (fast) {
+      for (int e = threadIdx.x; e < ka * ka; e += blockDim.x)
+        M[e % ka + (e / ka) * ldm] += A.sa[e % ka + (int64_t)(e / ka) * A.ldsa];
+      __syncthreads();
+    }
+    k = g_rrqr(all, mu, mv, M, ldm, 0.0, nsv, tau, ord, at, tau + nsv, cand);
+    Aj = cand + 4 * (LR_T / 32) + (nsv + mv + 2) / 2;
+    ldj = mv + k;
+    for (int e = threadIdx.x; e < ldj * k; e += blockDim.x) {
+      const int c = e % ldj, j = e / ldj;
+      Aj[e] = c < mv ? rrqr_r(M, ldm, at, j, c) : (c - mv == j ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    const int sweeps = g_jacobi(all, mv, k, Aj, ldj, 60, sh.flags, ldj);
+    if (sweeps < 0 && threadIdx.x == 0) atomicAdd(err + OPS_ERR_JACOBI, 1);
+    for (int c = threadIdx.x >> 5; c < k; c += LR_T / 32) {
+      double q = 0.0;
+      for (int r = lane; r < mv; r += 32) q = fma(Aj[r + c * ldj], Aj[r + c * ldj], q);
+      q = warp_sum(q);
+      if (lane == 0) sig[c] = sqrt(q);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < k; c += blockDim.x) {
+      const double v = sig[c];
+      int pos = 0;
+      for (int d = 0; d < k; ++d) pos += (sig[d] > v) || (sig[d] == v && d < c);
+      rank_of[pos] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int r;
+      if (A.eps > 0.0) {
+        // find_svd_truncation_rank (misc.cpp:133-146, quirk included); values beyond k are zero
+        double fro = 0.0;
+        for (int j = 0; j < k; ++j) fro += sig[j] * sig[j];
+        const double thr = A.eps * sqrt(fro);
+        r = 0;
+        double e2;
+        do {
+          ++r;
+          const double v = r < k ? sig[rank_of[r]] : 0.0;
+          e2 = r < nsv ? (double)(nsv - r) * v * v : 0.0;
+        } while (r < nsv && sqrt(e2) > thr);
+      } else {
+        r = min(ka, nsv);
+      }
+      if (r > A.kmax) { atomicAdd(err + 1, 1); r = A.kmax; }
+      sh.rank = r;
+    }
+    __syncthreads();
+  }
+  const int r = sh.rank, rk = min(r, k);
+  for (int e = threadIdx.x; e < mv * r; e += blockDim.x) {
+    const int i = e % mv, c = e / mv, src = c < k ? rank_of[c] : -1;
+    const double v = src >= 0 ? sig[src] : 0.0;
+    Y1[e] = v > 0.0 ? Aj[i + src * ldj] / v : 0.0;
+  }
+  g_apply_rrqr(all, mu, k, rk, M, ldm, tau, ord, false, Aj + mv, ldj, rank_of, X1, mu);
+  for (int e = threadIdx.x; e < mu * (r - rk); e += blockDim.x) X1[mu * rk + e] = 0.0;
+  for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
+    const int i = e % r, c = e / r;
+    A.sa[i + (int64_t)c * A.ldsa] = i == c && c < k ? sig[rank_of[c]] : 0.0;
+  }
+  __syncthreads();
+  {
+    // new bases: fast [Ua | Qu] X1 = Qu [X1(ka:); 0] + Ua X1(:ka); rounded Qu [X1; 0]
+    const int rows = hf ? n : m, mm = hf ? mv : mu, skip = fast ? ka : 0, refl = fast ? kb : mm;
+    const GrpScratch x{scratch + L.w[hf], scratch + L.w[hf] + GQ * kt, scratch + L.part[hf]};
+    const double* X = hf ? Y1 : X1;
+    double* Tn = scratch + L.tn[hf];
+    for (int c = half.wid; c < r; c += half.nw)
+#pragma unroll 4
+      for (int e = lane; e < rows; e += 32) Tn[e + (int64_t)c * rows] = e < refl ? X[skip + e + c * mm] : 0.0;
+    half.sync();
+    g_apply_q_tall(half, rows, refl, scratch + L.y[hf], rows, scratch + L.tf[hf], r, Tn, rows, refl, x);
+    if (fast)
+      g_mm(half, rows, r, ka, 1.0, (const double*)(hf ? A.va : A.ua), hf ? A.ldva : 1, hf ? 1 : A.ldua, X, mm, 1, 1.0,
+           Tn, rows, x.part);
+    if (hf == 0) {
+      for (int c = half.wid; c < r; c += half.nw)
+#pragma unroll 4
+        for (int e = lane; e < rows; e += 32) A.ua[e + (int64_t)c * A.ldua] = Tn[e + (int64_t)c * rows];
+    } else {
+      for (int e = half.tid; e < rows * r; e += half.nt) A.va[e % r + (int64_t)(e / r) * A.ldva] = Tn[e / r + (int64_t)(e % r) * rows];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *A.ka = r;
+}
+
+__global__ void __launch_bounds__(LR_T) k_op_lr_add(int m, int n, int kmax, int fast, double eps, Mat Ua, Mat Sa, Mat Va,
+                                                  int* ka_io, Mat Ub, Mat Sb, Mat Vb, const int* kb_in,
+                                                  double* scratch, int64_t ws, int* err) {
+  __shared__ LrArgs a;
   const int b = blockIdx.x;
-  lr_add_body(m, n, kmax, fast, eps, Ua.at(b), Ua.ld, Sa.at(b), Sa.ld, Va.at(b), Va.ld, ka_io + b, Ub.at(b), Ub.ld,
-              Sb.at(b), Sb.ld, Vb.at(b), Vb.ld, kb_in[b], scratch + (int64_t)b * ws, err, dyn, shm_cap);
+  if (threadIdx.x == 0)
+    a = LrArgs{m, n, kmax, fast, eps, Ua.at(b), Sa.at(b), Va.at(b), Ub.at(b), Sb.at(b), Vb.at(b), Ua.ld, Sa.ld, Va.ld,
+               Ub.ld, Sb.ld, Vb.ld, ka_io + b, kb_in[b]};
+  __syncthreads();
+  lr_add_body(a, scratch + (int64_t)b * ws, err);
+}
+
+__global__ void __launch_bounds__(OT) k_op_lr_add_large(int m, int n, int kmax, int fast, double eps, Mat Ua, Mat Sa,
+                                                        Mat Va, int* ka_io, Mat Ub, Mat Sb, Mat Vb, const int* kb_in,
+                                                        double* scratch, int64_t ws, int* err) {
+  const int b = blockIdx.x;
+  lr_add_large_body(m, n, kmax, fast, eps, Ua.at(b), Ua.ld, Sa.at(b), Sa.ld, Va.at(b), Va.ld, ka_io + b, Ub.at(b),
+                    Ub.ld, Sb.at(b), Sb.ld, Vb.at(b), Vb.ld, kb_in[b], scratch + (int64_t)b * ws, err);
 }
 
 // One LowRank addition per CTA from a task table (blocks of different sizes
-// in one launch).
-__global__ void __launch_bounds__(OT) k_op_lr_add_tasks(const LrAddTask* tasks, int kmax, int fast, double* scratch,
-                                                        int* err, int64_t shm_cap) {
-  extern __shared__ double dyn[];
+// in one launch; ranks kmax, 2 kmax <= LR_KT_MAX).
+__global__ void __launch_bounds__(LR_T) k_op_lr_add_tasks(const LrAddTask* tasks, int kmax, int fast, double* scratch,
+                                                        int* err) {
+  __shared__ LrArgs a;
+  const LrAddTask& t = tasks[blockIdx.x];
+  if (threadIdx.x == 0)
+    a = LrArgs{t.m, t.n, kmax, fast, 0.0, t.ua, t.sa, t.va, t.ub, t.sb, t.vb, t.ldua, t.ldsa, t.ldva,
+               t.ldub, t.ldsb, t.ldvb, t.ka, *t.kb};
+  __syncthreads();
+  lr_add_body(a, scratch + t.scratch_off, err);
+}
+
+__global__ void __launch_bounds__(OT) k_op_lr_add_tasks_large(const LrAddTask* tasks, int kmax, int fast,
+                                                              double* scratch, int* err) {
   const LrAddTask t = tasks[blockIdx.x];
-  lr_add_body(t.m, t.n, kmax, fast, 0.0, t.ua, t.ldua, t.sa, t.ldsa, t.va, t.ldva, t.ka, t.ub, t.ldub, t.sb, t.ldsb,
-              t.vb, t.ldvb, *t.kb, scratch + t.scratch_off, err, dyn, shm_cap);
+  lr_add_large_body(t.m, t.n, kmax, fast, 0.0, t.ua, t.ldua, t.sa, t.ldsa, t.va, t.ldva, t.ka, t.ub, t.ldub, t.sb,
+                    t.ldsb, t.vb, t.ldvb, *t.kb, scratch + t.scratch_off, err);
 }
 
 // C = alpha op(A) op(B) + beta C (operations/BLAS/gemm.cpp:126-146,
@@ -728,9 +895,13 @@ int64_t svd_scratch(int m, int n) {
 
 int64_t qr_ws(int m, int n) { return (int64_t)m * n + std::min(m, n) + 2; }
 
-int64_t lr_add_ws(int m, int n, int ka, int kb) {
-  const int kt = ka + kb, mx = std::max(m, n);
+int64_t lr_add_large_ws(int m, int n, int kt) {
+  const int mx = std::max(m, n);
   return (int64_t)(m + n) * kt + 2 * kt + 5 * (int64_t)kt * kt + kt + (int64_t)mx * kt + svd_scratch(kt, kt) + 2;
+}
+
+int64_t lr_add_ws(int m, int n, int ka, int kb) {
+  return ka + kb <= LR_KT_MAX ? lr_layout(m, n, ka + kb).total : lr_add_large_ws(m, n, ka + kb);
 }
 
 void launch_gemm(cudaStream_t s, int m, int n, int k, int count, double alpha, const double* a, int64_t lda,
@@ -755,26 +926,24 @@ void launch_svd(cudaStream_t s, int m, int n, int count, const double* a, int64_
                                 Mat{vt, ldvt, svt}, scratch, ws, err);
 }
 
-// Shared memory (bytes) for the core SVD of an addition of ranks ka + kb
-// (the pivoted-QR-preconditioned Jacobi: 3 kt^2 doubles), or 0 when it does
-// not fit beside the kernel's static arrays.
-int lr_add_shm_bytes(int ka, int kb) {
-  const int64_t kt = ka + kb, b = (3 * kt) * kt * (int64_t)sizeof(double);
-  return b <= 160 * 1024 ? (int)b : 0;
-}
-
-// Opt the addition kernels in to the shared memory of lr_add_shm_bytes (once,
-// outside any stream capture).
-int lr_add_prepare(int bytes) {
+// Opt the addition kernels in to their shared memory (once, outside any stream
+// capture).
+int lr_add_prepare() {
+  const int bytes = (int)(sizeof(LrShared) + 8 * lr_region(GT_ROWS, GT_ROWS, LR_KT_MAX));
   if (cudaFuncSetAttribute(k_op_lr_add, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
       cudaFuncSetAttribute(k_op_lr_add_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
     return set_error(FRANK_ERR_CUDA, "LowRank addition: shared memory attribute");
   return FRANK_OK;
 }
 
-void launch_lr_add_tasks(cudaStream_t s, int count, const LrAddTask* tasks, int kmax, int fast, double* scratch,
-                         int* err, int shm_bytes) {
-  k_op_lr_add_tasks<<<count, OT, shm_bytes, s>>>(tasks, kmax, fast, scratch, err, shm_bytes / (int)sizeof(double));
+// The additions of `count` tasks, of order at most mmax and rank kmax each.
+void launch_lr_add_tasks(cudaStream_t s, int count, int mmax, const LrAddTask* tasks, int kmax, int fast,
+                         double* scratch, int* err) {
+  if (2 * kmax <= LR_KT_MAX)
+    k_op_lr_add_tasks<<<count, LR_T, sizeof(LrShared) + 8 * lr_region(mmax, mmax, 2 * kmax), s>>>(tasks, kmax, fast,
+                                                                                                  scratch, err);
+  else
+    k_op_lr_add_tasks_large<<<count, OT, 0, s>>>(tasks, kmax, fast, scratch, err);
 }
 
 }  // namespace ops
@@ -999,22 +1168,21 @@ int frank_lowrank_add_batched(int m, int n, int count, int kmax, const char* lra
   if (name == "rounded_addition") fast = 0;
   else if (name == "fast_rounded_addition") fast = 1;
   else return set_error(FRANK_ERR_UNSUPPORTED, "lowrank_add: unknown LowRank addition " + name);
-  const int kt = kmax + kb_max, mx = std::max(m, n);
-  const int64_t ws = (int64_t)(m + n) * kt + 2 * kt + 5 * (int64_t)kt * kt + kt + (int64_t)mx * kt +
-                     svd_scratch(kt, kt) + 2;
+  // ranks of a pair are at most kmax and kb_max: the bound picks the kernel
+  const int kt = kmax + kb_max;
+  const Mat ua{d_ua, ldua, sua}, sa{d_sa, ldsa, ssa}, va{d_va, ldva, sva};
+  const Mat ub{const_cast<double*>(d_ub), ldub, sub}, sb{const_cast<double*>(d_sb), ldsb, ssb},
+      vb{const_cast<double*>(d_vb), ldvb, svb};
+  const int64_t ws = lr_add_ws(m, n, kmax, kb_max);
+  if (kt <= LR_KT_MAX && (rc = lr_add_prepare())) return rc;
   return run(s, count, ws, [&](double* sc, int* err) {
-    k_op_lr_add<<<count, OT, 0, s>>>(m, n, kmax, fast, eps, Mat{d_ua, ldua, sua}, Mat{d_sa, ldsa, ssa},
-                                     Mat{d_va, ldva, sva}, d_ka, Mat{const_cast<double*>(d_ub), ldub, sub},
-                                     Mat{const_cast<double*>(d_sb), ldsb, ssb},
-                                     Mat{const_cast<double*>(d_vb), ldvb, svb}, d_kb, sc, ws, err, 0);
+    if (kt <= LR_KT_MAX)
+      k_op_lr_add<<<count, LR_T, sizeof(LrShared) + 8 * lr_region(m, n, kt), s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka,
+                                                                                  ub, sb, vb, d_kb, sc, ws, err);
+    else
+      k_op_lr_add_large<<<count, OT, 0, s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka, ub, sb, vb, d_kb, sc, ws, err);
   });
 }
 
-#ifdef FRANK_LRA_TIMING
-int frank_debug_lra_cycles(unsigned long long* out) {
-  OPS_TRY(cudaMemcpyFromSymbol(out, g_lra_cycles, sizeof(unsigned long long) * 8));
-  return FRANK_OK;
-}
-#endif
 
 }  // extern "C"
