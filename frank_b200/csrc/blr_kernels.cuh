@@ -494,13 +494,16 @@ __global__ void __launch_bounds__(GETRF_THREADS) k_getrf(BlrView<T> A, FactorWs<
 // apply the interchanges if there were any.  The tile lives in shared memory,
 // the panel in registers (RPT rows of W entries per thread), rows are never
 // moved: each thread keeps the position its row has been exchanged to.  A
-// column step is two block barriers (the pivot search on integer halves of
-// |a|, then the pivot row by broadcast), ties broken toward the smallest
-// position as in idamax.  A chain of b column steps bounds the whole thing,
-// so what counts is the latency of a step: the previous scheme (one CTA with
-// six barriers per step, a serial triangle inverse and exchanges through L2,
-// and a second launch for the trailing tiles) took 96 us + 19 us per panel at
-// b = 256 and 118 us + 21 us at b = 512.
+// column step is one block barrier: each warp's pivot candidate (found on the
+// integer halves of |a|, ties broken toward the smallest position as in
+// idamax) goes to shared memory together with its row, eight columns wide;
+// every eight columns the rest of the panel is updated at once.  A chain of b
+// column steps bounds the whole thing, so what counts is the latency of a
+// step (some 1100 cycles; an 8-panel leaf of b = 256 takes 270 us, its
+// inverses included).  The scheme before (one CTA with six barriers per step,
+// a serial triangle inverse and exchanges through L2, a second launch for the
+// trailing tiles) took 96 us + 19 us per panel at b = 256 and 118 us + 21 us
+// at b = 512.
 // After the last panel, k_leaf_final stores the packed LU (tile CTAs) and
 // forms Linv and Uinv: one CTA per column block of W of each, the block of
 // the inverse in shared memory, right-looking over the row blocks -- multiply
@@ -544,10 +547,14 @@ FRANK_D LeafScratch leaf_view(double* base, int bmax) {
   return s;
 }
 
+constexpr int LEAF_S = 8;             // columns between two updates of the rest of a panel
+
 struct LeafShared {
   double tri[LEAF_W * (LEAF_W + 1)];
-  double prow[LEAF_W];
-  uint4 cand[LEAF_THREADS / 32];
+  alignas(16) double u[LEAF_W][LEAF_W + 2];          // rows of U of the panel
+  double l11[LEAF_S][LEAF_S];                        // the sub-panel's triangle
+  double2 crow[2][LEAF_THREADS / 32][LEAF_S / 2];    // each warp's candidate row
+  uint4 cand[2][LEAF_THREADS / 32];
 };
 
 // Largest |a| among the lanes' candidates with ties toward the smallest
@@ -562,64 +569,119 @@ FRANK_D uint4 warp_pivot(unsigned hi, unsigned lo, unsigned pos) {
   return make_uint4(mh, ml, mp, 0u);
 }
 
-// Column steps j0 .. j1-1 of a panel whose current column is a[.][0] and whose
-// NV first entries are live (the entries shift down by one per step).
+// Columns j0 .. j0+7 of a panel whose current column is a[.][0] and whose NV
+// first entries are live (the entries of the sub-panel shift down by one per
+// step), then the update of its remaining NV - 8 columns at once.
 template <int W, int RPT, int NV>
-FRANK_D void leaf_columns(int m, int j0, int j1, int jn, double (&a)[RPT][W], unsigned (&pos)[RPT], unsigned& done,
-                          double* sm, int lds, int* piv, int jb, int& zero, LeafShared& sh) {
+FRANK_D void leaf_columns(int m, int j0, int jn, double (&a)[RPT][W], unsigned (&pos)[RPT], unsigned& done, double* sm,
+                          int lds, int* piv, int jb, int& zero, LeafShared& sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (j0 >= jn) return;
+  const int j1 = min(jn, j0 + LEAF_S);
   for (int jj = j0; jj < j1; ++jj) {
+    const int par = jj & 1;
     unsigned bh = 0u, bl = 0u, bp = ~0u;
+    int bk = 0;
 #pragma unroll
     for (int k = 0; k < RPT; ++k) {
       const int row = threadIdx.x + k * blockDim.x;
       if (row < m && !((done >> k) & 1u)) {
         const double v = fabs(a[k][0]);
         const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
-        if (bp == ~0u || h > bh || (h == bh && (l > bl || (l == bl && pos[k] < bp)))) { bh = h; bl = l; bp = pos[k]; }
+        if (bp == ~0u || h > bh || (h == bh && (l > bl || (l == bl && pos[k] < bp)))) { bh = h; bl = l; bp = pos[k]; bk = k; }
       }
     }
     const uint4 wc = warp_pivot(bh, bl, bp);
-    if (lane == 0) sh.cand[wid] = wc;
-    __syncthreads();
-    uint4 c = lane < nw ? sh.cand[lane] : make_uint4(0u, 0u, ~0u, 0u);
-    c = warp_pivot(c.x, c.y, c.z);
-    const unsigned p = c.z;
-    const bool nonzero = (c.x | c.y) != 0u;
+    // the warp's candidate with its row, so that the winner needs no second barrier
+    if (bp != ~0u ? bp == wc.z : (wc.z == ~0u && lane == 0)) {
+      sh.cand[par][wid] = wc;
 #pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int row = threadIdx.x + k * blockDim.x;
-      if (row >= m || ((done >> k) & 1u)) continue;
-      if (pos[k] == p) {
-        // the pivot row: broadcast, and final as row jj of U
+      for (int x = 0; x < LEAF_S / 2; ++x) {
+        double2 v = make_double2(a[0][2 * x], a[0][2 * x + 1]);
 #pragma unroll
-        for (int x = 0; x < NV; ++x) {
-          sh.prow[x] = a[k][x];
-          if (jj + x < jn) sm[row + (jj + x) * lds] = a[k][x];
-        }
-        pos[k] = jj;
-        done |= 1u << k;
-      } else if (pos[k] == (unsigned)jj) {
-        pos[k] = p;
+        for (int k = 1; k < RPT; ++k)
+          if (bk == k) v = make_double2(a[k][2 * x], a[k][2 * x + 1]);
+        sh.crow[par][wid][x] = v;
       }
     }
-    // 1 / |pivot| while the pivot row is on its way
-    const double ra = 1.0 / __hiloint2double((int)c.x, (int)c.y);
+    __syncthreads();
+    const uint4 q = lane < nw ? sh.cand[par][lane] : make_uint4(0u, 0u, ~0u, 0u);
+    const uint4 c = warp_pivot(q.x, q.y, q.z);
+    const int ww = __ffs(__ballot_sync(0xffffffffu, q.z == c.z)) - 1;
+    const unsigned p = c.z;
+    const bool nonzero = (c.x | c.y) != 0u;
+    const double ra = 1.0 / __hiloint2double((int)c.x, (int)c.y);   // 1 / |pivot|
+    double pr[LEAF_S];
+#pragma unroll
+    for (int x = 0; x < LEAF_S / 2; ++x) {
+      const double2 v = sh.crow[par][ww][x];
+      pr[2 * x] = v.x;
+      pr[2 * x + 1] = v.y;
+    }
+    const double rcp = pr[0] < 0.0 ? -ra : ra;
     if (threadIdx.x == 0) {
       piv[jj] = jb + (int)p;
       if (!nonzero && zero < 0) zero = jb + jj;
+#pragma unroll
+      for (int x = 0; x < LEAF_S; ++x)
+        if (jj + x < j0 + LEAF_S) sh.u[jj][jj + x] = pr[x];
     }
-    __syncthreads();
-    const double rcp = sh.prow[0] < 0.0 ? -ra : ra;
 #pragma unroll
     for (int k = 0; k < RPT; ++k) {
       const int row = threadIdx.x + k * blockDim.x;
+      if (row < m && !((done >> k) & 1u)) {
+        if (pos[k] == p) { pos[k] = jj; done |= 1u << k; }
+        else if (pos[k] == (unsigned)jj) pos[k] = p;
+      }
       const double l = nonzero ? a[k][0] * rcp : a[k][0];
       if (row < m && !((done >> k) & 1u)) sm[row + jj * lds] = l;
       const double lu = nonzero ? l : 0.0;
 #pragma unroll
-      for (int x = 1; x < NV; ++x) a[k][x - 1] = fma(-lu, sh.prow[x], a[k][x]);
-      a[k][NV - 1] = 0.0;
+      for (int x = 1; x < LEAF_S; ++x) a[k][x - 1] = fma(-lu, pr[x], a[k][x]);
+      a[k][LEAF_S - 1] = 0.0;
+    }
+  }
+  if (NV <= LEAF_S || j0 + LEAF_S >= jn) return;
+  // U12 = L11^{-1} A12 of the sub-panel's pivot rows, a column per lane
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int row = threadIdx.x + k * blockDim.x, i = (int)pos[k] - j0;
+    if (row < m && ((done >> k) & 1u) && i >= 0 && i < LEAF_S) {
+#pragma unroll
+      for (int x = LEAF_S; x < NV; ++x) sh.u[j0 + i][j0 + x] = a[k][x];
+      for (int t = 0; t < i; ++t) sh.l11[i][t] = sm[row + (j0 + t) * lds];
+    }
+  }
+  __syncthreads();
+  if (wid == 0 && lane < NV - LEAF_S) {
+    double v[LEAF_S];
+#pragma unroll
+    for (int i = 0; i < LEAF_S; ++i) v[i] = sh.u[j0 + i][j0 + LEAF_S + lane];
+#pragma unroll
+    for (int t = 0; t < LEAF_S; ++t)
+#pragma unroll
+      for (int i = t + 1; i < LEAF_S; ++i) v[i] = fma(-sh.l11[i][t], v[t], v[i]);
+#pragma unroll
+    for (int i = 1; i < LEAF_S; ++i) sh.u[j0 + i][j0 + LEAF_S + lane] = v[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int row = threadIdx.x + k * blockDim.x;
+    double l[LEAF_S];
+#pragma unroll
+    for (int t = 0; t < LEAF_S; ++t) l[t] = row < m && !((done >> k) & 1u) ? sm[row + (j0 + t) * lds] : 0.0;
+#pragma unroll
+    for (int x = LEAF_S; x < NV; x += 2) {
+      double v = a[k][x], w = a[k][x + 1];
+#pragma unroll
+      for (int t = 0; t < LEAF_S; ++t) {
+        const double2 u = *reinterpret_cast<const double2*>(&sh.u[j0 + t][j0 + x]);
+        v = fma(-l[t], u.x, v);
+        w = fma(-l[t], u.y, w);
+      }
+      a[k][x - LEAF_S] = v;
+      a[k][x + 1 - LEAF_S] = w;
     }
   }
 }
@@ -641,11 +703,13 @@ FRANK_D void leaf_panel(int b, int jb, double* sm, int lds, const LeafScratch& L
 #pragma unroll
     for (int c = 0; c < W; ++c) a[k][c] = (row < m && c < jn) ? sm[row + c * lds] : 0.0;
   }
-  constexpr int Q = W / 4;
-  leaf_columns<W, RPT, W>(m, 0, min(jn, Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
-  leaf_columns<W, RPT, 3 * Q>(m, Q, min(jn, 2 * Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
-  leaf_columns<W, RPT, 2 * Q>(m, 2 * Q, min(jn, 3 * Q), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
-  leaf_columns<W, RPT, Q>(m, 3 * Q, min(jn, W), jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  leaf_columns<W, RPT, W>(m, 0, jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  leaf_columns<W, RPT, W - 8>(m, 8, jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  if constexpr (W > 16) {
+    leaf_columns<W, RPT, 16>(m, 16, jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+    leaf_columns<W, RPT, 8>(m, 24, jn, a, pos, done, sm, lds, piv + jb, jb, zero, sh);
+  }
+  __syncthreads();
   if (threadIdx.x == 0 && zero >= 0) atomicCAS(err + ERR_SINGULAR_STEP, 0, step + 1);
   int mv = 0, pv[RPT];
 #pragma unroll
@@ -654,7 +718,8 @@ FRANK_D void leaf_panel(int b, int jb, double* sm, int lds, const LeafScratch& L
     pv[k] = 0;
     if (row >= m) continue;
     const int to = jb + (int)pos[k];
-    for (int c = 0; c < jn; ++c) L.Wm[to + (int64_t)(jb + c) * b] = sm[row + c * lds];
+    const int pr = (int)pos[k];
+    for (int c = 0; c < jn; ++c) L.Wm[to + (int64_t)(jb + c) * b] = pr < jn && c >= pr ? sh.u[pr][c] : sm[row + c * lds];
     L.src[par * b + to] = jb + row;
     pv[k] = jb == 0 ? row : perm[jb + row];
     mv |= (int)pos[k] != row;
@@ -669,7 +734,8 @@ FRANK_D void leaf_panel(int b, int jb, double* sm, int lds, const LeafScratch& L
 }
 
 // Inverses of the two W x W triangles of a factored panel (identity beyond
-// the block): a warp per column, lane = row, the solved value by shuffle.
+// the block): a warp per triangle, a column per lane in registers, the
+// triangle's entries broadcast from shared memory.
 template <int W>
 FRANK_D void leaf_dinv(int b, int jb, const double* Wm, double* out, LeafShared& sh) {
   const int jn = min(W, b - jb);
@@ -678,23 +744,28 @@ FRANK_D void leaf_dinv(int b, int jb, const double* Wm, double* out, LeafShared&
     sh.tri[r + c * (W + 1)] = (r < jn && c < jn) ? Wm[(jb + r) + (int64_t)(jb + c) * b] : (r == c ? 1.0 : 0.0);
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int r = min(lane, W - 1);
-  const double rd = 1.0 / sh.tri[r + r * (W + 1)];
-  for (int c = wid; c < W; c += nw) {
-    double lo = r == c ? 1.0 : 0.0, up = lo;
-    for (int t = 0; t < W; ++t) {
-      const double xl = __shfl_sync(0xffffffffu, lo, t);
-      if (r > t) lo = fma(-sh.tri[r + t * (W + 1)], xl, lo);
-      const int s = W - 1 - t;
-      const double xu = __shfl_sync(0xffffffffu, up * rd, s);
-      if (r < s) up = fma(-sh.tri[r + s * (W + 1)], xu, up);
-      else if (r == s) up = xu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (wid < 2) {
+    double v[W];
+#pragma unroll
+    for (int r = 0; r < W; ++r) v[r] = r == lane ? 1.0 : 0.0;
+    if (wid == 0) {
+#pragma unroll
+      for (int t = 0; t < W; ++t)
+#pragma unroll
+        for (int r = t + 1; r < W; ++r) v[r] = fma(-sh.tri[r + t * (W + 1)], v[t], v[r]);
+    } else {
+      const double rd = 1.0 / sh.tri[min(lane, W - 1) * (W + 2)];
+#pragma unroll
+      for (int t = W - 1; t >= 0; --t) {
+        v[t] *= __shfl_sync(0xffffffffu, rd, t);
+#pragma unroll
+        for (int r = 0; r < t; ++r) v[r] = fma(-sh.tri[r + t * (W + 1)], v[t], v[r]);
+      }
     }
-    if (lane < W) {
-      out[r + c * W] = lo;
-      out[W * W + r + c * W] = r <= c ? up : 0.0;
-    }
+    if (lane < W)
+#pragma unroll
+      for (int r = 0; r < W; ++r) out[(wid ? W * W : 0) + r + lane * W] = v[r];
   }
   __syncthreads();
 }
@@ -749,19 +820,21 @@ FRANK_D void leaf_step_body(const BlrView<T>& A, const FactorWs<T>& ws, int i, i
       sh.tri[e % W + (e / W) * (W + 1)] = L.Wm[(j0 + e % W) + (int64_t)(j0 + e / W) * b];
     __syncthreads();
     // U12 = L11^{-1} A12 (panel p - 1 has W columns: only the last one can have fewer)
-    for (int c = wid; c < cn; c += nw) {
-      const int r = min(lane, W - 1);
-      double v = lsm[r + c * lds];
-      for (int t = 0; t < W - 1; ++t) {
-        const double x = __shfl_sync(0xffffffffu, v, t);
-        if (r > t) v = fma(-sh.tri[r + t * (W + 1)], x, v);
-      }
-      if (lane < W) {
-        lsm[r + c * lds] = v;
-        L.Wm[(j0 + r) + (int64_t)(c0 + c) * b] = v;
-      }
+    // -- a column per lane, in registers
+    if (wid == 0 && lane < cn) {
+      double v[W];
+#pragma unroll
+      for (int r = 0; r < W; ++r) v[r] = lsm[r + lane * lds];
+#pragma unroll
+      for (int t = 0; t < W - 1; ++t)
+#pragma unroll
+        for (int r = t + 1; r < W; ++r) v[r] = fma(-sh.tri[r + t * (W + 1)], v[t], v[r]);
+#pragma unroll
+      for (int r = 0; r < W; ++r) lsm[r + lane * lds] = v[r];
     }
     __syncthreads();
+    for (int e = threadIdx.x; e < W * cn; e += blockDim.x)
+      L.Wm[(j0 + e % W) + (int64_t)(c0 + e / W) * b] = lsm[e % W + (e / W) * lds];
     // trailing rows: -= L21 U12
     warps_dgemm<4, 2>(wid, nw, m - W, cn, W, -1.0, L.Wm + (j0 + W) + (int64_t)j0 * b, 1, b, lsm, lds, 1, 1.0, lsm + W,
                       lds);
