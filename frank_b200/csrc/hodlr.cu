@@ -89,10 +89,6 @@ using blr::kernel_eval;
 constexpr int HMAX_RANK = 64;   // k <= 64: two rank rows per lane in the walks
 constexpr int HMAX_LEAF = 512;  // b <= 512
 constexpr int WT = 256;         // threads of the update / matvec kernels
-constexpr int WWT = 1024;       // threads of a substitution walk (many loads in flight per SM)
-constexpr int WCW = 4;          // right-hand-side columns per walking CTA
-// dynamic shared memory of a walk: r, per-warp partials, t1, t2
-constexpr int WALK_SMEM = (WCW * HMAX_LEAF + (WWT / 32) * WCW * HMAX_RANK + 2 * WCW * HMAX_RANK) * 8;
 constexpr int KG_P = 72;        // rsvd sample width the construction product holds (k + 5 <= 69)
 
 enum { HERR_JACOBI = 8, HERR_RANK = 9, HERR_SLOTS = 16 };
@@ -118,253 +114,252 @@ struct LeafFactors {
   const int* perm;      // [P][b] (P_p r)[i] = r[perm[i]]
 };
 
-// One substitution walk over the leaves of node (l0, c0) on ncols columns of
-// B (element (i, c) at B[i rs + c cs], i relative to the node's first row).
-//   mode 0: B <- L^{-1} P B  (forward; leaf p: x = Linv_p P_p r, then the
-//           lower block of every ancestor whose left child ends at p:
-//           B_right -= U (S (V B_left)))
-//   mode 1: B <- U^{-T} B    (forward on U^T; leaf: x = Uinv_p^T r, then the
-//           upper block: B_right -= V^T (S^T (U^T B_left)))
-//   mode 2: B <- U^{-1} B    (backward; leaf: x = Uinv_p r, then the upper
-//           block of every ancestor whose right child starts at p:
-//           B_left -= U (S (V B_right)))
-// Each CTA owns WCW columns and walks the leaves in order on its own; the
-// columns are independent, so no CTA waits for another.
-struct Walk {
-  int mode, l0, c0, ncols;
-  double* B;
-  int64_t rs, cs;
+// ---------------------------------------------------------------------------
+// Level-parallel substitution on a subtree (node (l0, c0) and everything below
+// it).  With W = M_right(U_low), Z = U_left^{-1} U_up and Zt = U_right^{-T}
+// V_up^T precomputed per node (M the pivoted forward substitution), the three
+// substitutions are: every leaf at once, then for each level from the bottom
+// up, every node at once:
+//   mode 0  X <- L^{-1} P X : x_right -= W  S_low  (V_low  x_left)
+//   mode 1  X <- U^{-T} X   : x_right -= Zt S_up^T (U_up^T x_left)
+//   mode 2  X <- U^{-1} X   : x_left  -= Z  S_up   (V_up   x_right)
+// (from L = [[L_l, 0], [U S V, L_r]] and U likewise), and the H-matvec has the
+// same two kernels per level:
+//   mode 3  Y = A X         : y(rows of c) += U_c S_c (V_c x(rows of c ^ 1)).
+// The walks over the leaves that did modes 0 to 2 before kept eight CTAs busy
+// with a chain of 2^h leaf steps (8.9 ms for the top of an n = 32768 tree).
+// The columns of X (right-hand sides, or the k columns of a basis) go through
+// the FP64 tensor pipe 32 at a time, so a block is read once for all of them.
+// ---------------------------------------------------------------------------
+struct HJob {
+  int mode;
+  const double* src;      // leaves read X here: element (i, c) at src[i srs + c scs]
+  int64_t srs, scs;
+  double* X;              // result, and X of the level steps: X[i xrs + c ldx] (xrs = 1 above the leaves)
+  int64_t xrs, ldx;
+  const double* xin;      // mode 3: the vector multiplied (X is the result)
+  int64_t ldin;
 };
 
-FRANK_D void walk_body(const HView& h, const LeafFactors& f, const Walk& J) {
-  extern __shared__ double wsm[];
-  double(*r)[HMAX_LEAF] = reinterpret_cast<double(*)[HMAX_LEAF]>(wsm);
-  double(*part)[WCW][HMAX_RANK] = reinterpret_cast<double(*)[WCW][HMAX_RANK]>(wsm + WCW * HMAX_LEAF);
-  double(*t1)[HMAX_RANK] =
-      reinterpret_cast<double(*)[HMAX_RANK]>(wsm + WCW * HMAX_LEAF + (WWT / 32) * WCW * HMAX_RANK);
-  double(*t2)[HMAX_RANK] = t1 + WCW;
-  const int col0 = blockIdx.x * WCW;
-  if (col0 >= J.ncols) return;
-  const int nc = min(WCW, J.ncols - col0);
-  const int b = h.b, k = h.k, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int hl = h.L - J.l0;
-  const int np = 1 << hl;
-  const int p0 = J.c0 << hl;
-  const int64_t row0 = (int64_t)p0 * b;
-  double* B = J.B + (int64_t)col0 * J.cs;
-  const int64_t rs = J.rs, cs = J.cs;
-  for (int step = 0; step < np; ++step) {
-    const int p = J.mode == 2 ? p0 + np - 1 - step : p0 + step;
-    const int64_t pr = (int64_t)p * b - row0;
-    // leaf solve
-    const int* perm = f.perm + (int64_t)p * b;
-    for (int e = tid; e < WCW * b; e += WWT) {
-      const int c = e / b, i = e % b;
-      const int src = J.mode == 0 ? perm[i] : i;
-      r[c][i] = c < nc ? B[(pr + src) * rs + c * cs] : 0.0;
-    }
-    __syncthreads();
-    const double* Op = (J.mode == 0 ? f.Linv : (J.mode == 1 ? f.UinvT : f.Uinv)) + (int64_t)p * b * b;
-    for (int i = tid; i < b; i += WWT) {
-      double acc[WCW];
+constexpr int HC = 32;            // columns of X per CTA
+constexpr int HLC = 8;            // columns per CTA of the leaf step
+constexpr int H_CHUNK = 512;      // least rows per partial product
+constexpr int H_NCH = 64;         // most partial products of one block
+constexpr int H_TSMEM = 8 * HC * HC * 8;   // dynamic shared memory of the partial products
+
+// Rows of a block of order s per partial product, and their number.
+inline __host__ __device__ int64_t h_chunk(int64_t s) {
+  const int64_t c = (s + H_NCH - 1) / H_NCH;
+  return c < H_CHUNK ? (int64_t)H_CHUNK : c;
+}
+inline __host__ __device__ int h_nch(int64_t s) { return (int)((s + h_chunk(s) - 1) / h_chunk(s)); }
+
+// X_p <- Op_p X_p for the leaves p0 .. of a subtree (Linv P, Uinv^T, Uinv or the
+// leaf of A_H itself); grid (leaves, groups of HLC columns, jobs).
+__global__ void __launch_bounds__(WT) k_h_leaf_mm(HView h, LeafFactors f, HJob j0, HJob j1, int p0, int ncols) {
+  __shared__ double R[HLC * (HMAX_LEAF + 4)];
+  const HJob& J = blockIdx.z ? j1 : j0;
+  const int p = p0 + blockIdx.x, b = h.b, c0 = blockIdx.y * HLC, nc = min(HLC, ncols - c0);
+  const int64_t r0 = (int64_t)blockIdx.x * b;
+  const int ldr = ((b + 15) & ~15) + 4;
+  const int* perm = f.perm + (int64_t)p * b;
+  for (int e = threadIdx.x; e < nc * b; e += WT) {
+    const int i = J.srs == 1 ? e % b : e / nc, c = J.srs == 1 ? e / b : e % nc;
+    R[i + c * ldr] = J.src[(r0 + (J.mode == 0 ? perm[i] : i)) * J.srs + (c0 + c) * J.scs];
+  }
+  __syncthreads();
+  const double* Op = (J.mode == 0 ? f.Linv : J.mode == 1 ? f.UinvT : J.mode == 2 ? f.Uinv : h.D) + (int64_t)p * b * b;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int i0 = (threadIdx.x >> 5) * 32; i0 < b; i0 += WT) {
+    double acc[4][1][2];
+    // the operators of modes 0 and 1 are lower triangular, that of mode 2 upper
+    const int k0 = J.mode == 2 ? i0 : 0, k1 = J.mode <= 1 ? min(b, i0 + 32) : b;
+    blr::warp_dgemm_acc<4, 1, false>(b, nc, k0, k1, Op, 1, b, R, ldr, 1, i0, 0, acc);
 #pragma unroll
-      for (int c = 0; c < WCW; ++c) acc[c] = 0.0;
-      if (J.mode == 2) {
-#pragma unroll 8
-        for (int j = i; j < b; ++j) {
-          const double a = Op[i + (int64_t)j * b];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[c] += a * r[c][j];
-        }
-      } else {
-        // Linv is unit lower (diagonal not read); Uinv^T is lower with its diagonal
-        const int jend = J.mode == 0 ? i : i + 1;
-#pragma unroll 8
-        for (int j = 0; j < jend; ++j) {
-          const double a = Op[i + (int64_t)j * b];
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[c] += a * r[c][j];
-        }
-        if (J.mode == 0) {
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[c] += r[c][i];
-        }
+      for (int q = 0; q < 2; ++q) {
+        const int r = i0 + 8 * i + g, c = 2 * t + q;
+        if (r < b && c < nc) J.X[(r0 + r) * J.xrs + (c0 + c) * J.ldx] = acc[i][0][q];
       }
-      for (int c = 0; c < nc; ++c) B[(pr + i) * rs + c * cs] = acc[c];
-    }
-    __syncthreads();
-    // updates of the ancestors' off-diagonal blocks that this leaf completes
-    for (int hh = 1; hh <= hl; ++hh) {
-      const int a = p >> hh, half = 1 << (hh - 1), first = a << hh;
-      const bool fire = J.mode == 2 ? (p == first + half) : (p == first + half - 1);
-      if (!fire) continue;
-      const int lv = h.L - hh + 1;
-      const int64_t sl = h.s(lv);
-      const int blk = J.mode == 0 ? 2 * a + 1 : 2 * a;
-      const double* Ub = h.u(lv, blk);
-      const double* Sb = h.sm(lv, blk);
-      const double* Vb = h.v(lv, blk);
-      const int64_t src = (int64_t)(J.mode == 2 ? first + half : first) * b - row0;
-      const int64_t dst = (int64_t)(J.mode == 2 ? first : first + half) * b - row0;
-      // t1 (k x nc) = V B_src (modes 0, 2) or U^T B_src (mode 1)
-      if (J.mode != 1) {
-        double acc[2][WCW];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[q][c] = 0.0;
-        for (int64_t i = wid; i < sl; i += WWT / 32) {
-          double xv[WCW];
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) xv[c] = c < nc ? B[(src + i) * rs + c * cs] : 0.0;
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int rr = lane + 32 * q;
-            if (rr < k) {
-              const double vv = Vb[rr + i * k];
-#pragma unroll
-              for (int c = 0; c < WCW; ++c) acc[q][c] += vv * xv[c];
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int rr = lane + 32 * q;
-          if (rr < k)
-#pragma unroll
-            for (int c = 0; c < WCW; ++c) part[wid][c][rr] = acc[q][c];
-        }
-      } else {
-        for (int rr = wid; rr < k; rr += WWT / 32) {
-          double acc[WCW];
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[c] = 0.0;
-          for (int64_t i = lane; i < sl; i += 32) {
-            const double uv = Ub[i + rr * sl];
-#pragma unroll
-            for (int c = 0; c < WCW; ++c) acc[c] += uv * (c < nc ? B[(src + i) * rs + c * cs] : 0.0);
-          }
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) {
-            const double v = blr::warp_sum(acc[c]);
-            if (lane == 0) {
-              part[0][c][rr] = v;
-              for (int w = 1; w < WWT / 32; ++w) part[w][c][rr] = 0.0;
-            }
-          }
-        }
-      }
-      __syncthreads();
-      for (int e = tid; e < WCW * k; e += WWT) {
-        const int c = e / k, rr = e % k;
-        double v = 0.0;
-        for (int w = 0; w < WWT / 32; ++w) v += part[w][c][rr];
-        t1[c][rr] = v;
-      }
-      __syncthreads();
-      // t2 = S t1 (modes 0, 2) or S^T t1 (mode 1)
-      for (int e = tid; e < WCW * k; e += WWT) {
-        const int c = e / k, rr = e % k;
-        double v = 0.0;
-        for (int q = 0; q < k; ++q) v += (J.mode == 1 ? Sb[q + (int64_t)rr * k] : Sb[rr + (int64_t)q * k]) * t1[c][q];
-        t2[c][rr] = v;
-      }
-      __syncthreads();
-      // B_dst -= U t2 (modes 0, 2) or V^T t2 (mode 1)
-      for (int64_t i = tid; i < sl; i += WWT) {
-        double acc[WCW];
-#pragma unroll
-        for (int c = 0; c < WCW; ++c) acc[c] = 0.0;
-        for (int q = 0; q < k; ++q) {
-          const double a = J.mode == 1 ? Vb[q + i * k] : Ub[i + (int64_t)q * sl];
-#pragma unroll
-          for (int c = 0; c < WCW; ++c) acc[c] += a * t2[c][q];
-        }
-        for (int c = 0; c < nc; ++c) B[(dst + i) * rs + c * cs] -= acc[c];
-      }
-      __syncthreads();
-    }
   }
 }
 
-__global__ void __launch_bounds__(WWT) k_h_walk(HView h, LeafFactors f, Walk j0, Walk j1) {
-  walk_body(h, f, blockIdx.y == 0 ? j0 : j1);
+// One CTA's share of T (m x n <= HC each) = A B over rows [k0, k1), element (i, kk)
+// of A at A[i sai + kk sak], B col-major: eight warps take an eighth of the rows
+// each and sum in shared memory (red, 8 HC HC doubles); T in red[0 .. m n).
+__device__ __forceinline__ void h_tprod(int m, int n, int64_t k0, int64_t k1, const double* A, int64_t sai, int64_t sak,
+                                        const double* B, int64_t ldb, double* red) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, wid = threadIdx.x >> 5;
+  const int64_t len = ((k1 - k0 + 7) / 8 + 3) & ~(int64_t)3;
+  const int64_t a0 = min(k1, k0 + wid * len), a1 = min(k1, a0 + len);
+  double acc[4][4][2];
+  blr::warp_dgemm_acc<4, 4, false>(m, n, 0, (int)(a1 - a0), A + a0 * sak, sai, sak, B + a0, ldb, 1, 0, 0, acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) red[wid * HC * HC + (8 * i + g) + (8 * j + 2 * t + q) * HC] = acc[i][j][q];
+  __syncthreads();
+  double v[HC * HC / WT];
+#pragma unroll
+  for (int x = 0; x < HC * HC / WT; ++x) {
+    v[x] = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v[x] += red[w * HC * HC + threadIdx.x + x * WT];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int x = 0; x < HC * HC / WT; ++x) red[threadIdx.x + x * WT] = v[x];
+  __syncthreads();
+}
+
+// T2 (k x ncols per node, ld k) = op(S) (inner product of the block with its side of
+// X) for the nodes of one level of a subtree: grid (chunks, nodes, jobs x column
+// groups).  The chunk that finishes last sums all of them in order and applies S.
+__global__ void __launch_bounds__(WT) k_h_t(HView h, HJob j0, HJob j1, int njobs, int l, int first, int ncols,
+                                            double* part, double* T2, int* counter) {
+  extern __shared__ double red[];
+  __shared__ double t1[HMAX_RANK * HC];
+  __shared__ int last;
+  const int job = blockIdx.z % njobs, grp = blockIdx.z / njobs;
+  const HJob& J = job ? j1 : j0;
+  const int k = h.k, nc = min(HC, ncols - grp * HC), nch = gridDim.x, node = blockIdx.y;
+  const int64_t sl = h.s(l), chunk = h_chunk(sl), i0 = blockIdx.x * chunk, i1 = min(sl, i0 + chunk);
+  // the block, and the cluster whose rows of X it reads
+  const int c = J.mode == 3 ? node : (J.mode == 0 ? first + 2 * node + 1 : first + 2 * node);
+  const int xc = J.mode == 0 || J.mode == 1 ? first + 2 * node : (J.mode == 2 ? first + 2 * node + 1 : c ^ 1);
+  const bool tr = J.mode == 1;
+  const double* A = tr ? h.u(l, c) : h.v(l, c);
+  const double* x = (J.mode == 3 ? J.xin : J.X) + (int64_t)(xc - (J.mode == 3 ? 0 : first)) * sl;
+  const int64_t ldx = J.mode == 3 ? J.ldin : J.ldx;
+  x += (int64_t)grp * HC * ldx;
+  const int64_t slot = ((int64_t)blockIdx.z * gridDim.y + node);
+  double* pt = part + slot * nch * k * HC;
+  for (int m0 = 0; m0 < k; m0 += HC) {
+    const int m = min(HC, k - m0);
+    h_tprod(m, nc, i0, i1, A + (tr ? (int64_t)m0 * sl : m0), tr ? sl : 1, tr ? 1 : k, x, ldx, red);
+    for (int e = threadIdx.x; e < m * nc; e += WT) {
+      const double v = red[e % m + (e / m) * HC];
+      if (nch == 1) t1[m0 + e % m + (e / m) * k] = v;
+      else pt[(int64_t)blockIdx.x * k * HC + m0 + e % m + (e / m) * k] = v;
+    }
+    __syncthreads();
+  }
+  if (nch > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      last = atomicAdd(counter + slot, 1) == nch - 1;
+      if (last) counter[slot] = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < k * nc; e += WT) {
+      double v = 0.0;
+#pragma unroll 8
+      for (int q = 0; q < nch; ++q) v += pt[(int64_t)q * k * HC + e];
+      t1[e] = v;
+    }
+    __syncthreads();
+  }
+  const double* S = h.sm(l, c);
+  double* out = T2 + ((int64_t)(job * gridDim.y + node) * ncols + grp * HC) * k;
+  for (int e = threadIdx.x; e < k * nc; e += WT) {
+    const int r = e % k, q = e / k;
+    double v = 0.0;
+#pragma unroll 4
+    for (int t = 0; t < k; ++t) v = fma(tr ? S[t + r * k] : S[r + t * k], t1[t + q * k], v);
+    out[e] = v;
+  }
+}
+
+// X(rows of the node's target) -= outer T2 (mode 3: +=); outer from the slabs W (modes
+// 0, 2), Zt (mode 1) or the block's own U; grid (row tiles of WT, nodes, jobs x
+// column groups).
+__global__ void __launch_bounds__(WT) k_h_u(HView h, const double* WZ, const double* WT_, HJob j0, HJob j1, int njobs,
+                                            int l, int first, int ncols, const double* T2) {
+  __shared__ double ts[HC * (HMAX_RANK + 4)];
+  const int job = blockIdx.z % njobs, grp = blockIdx.z / njobs, node = blockIdx.y;
+  const HJob& J = job ? j1 : j0;
+  const int k = h.k, nc = min(HC, ncols - grp * HC);
+  const int64_t sl = h.s(l), r0 = (int64_t)blockIdx.x * WT;
+  const int rows = (int)min((int64_t)WT, sl - r0);
+  const int c = J.mode == 3 ? node : (J.mode == 0 ? first + 2 * node + 1 : first + 2 * node);
+  const int target = J.mode == 1 ? c + 1 : c;       // cluster whose rows are updated
+  const int64_t off = (int64_t)(l - 1) * h.n * k + (int64_t)c * sl * k;
+  const double* O = (J.mode == 3 ? h.U : J.mode == 1 ? WT_ : WZ) + off + r0;
+  const int ldt = ((k + 15) & ~15) + 4;
+  const double* t2 = T2 + ((int64_t)(job * gridDim.y + node) * ncols + grp * HC) * k;
+  for (int e = threadIdx.x; e < k * nc; e += WT) ts[e % k + (e / k) * ldt] = t2[e];
+  __syncthreads();
+  double* X = J.X + (int64_t)(target - (J.mode == 3 ? 0 : first)) * sl + r0 + (int64_t)grp * HC * J.ldx;
+  blr::warps_dgemm<4, 2>(threadIdx.x >> 5, WT / 32, rows, nc, k, J.mode == 3 ? 1.0 : -1.0, O, 1, sl, ts, ldt, 1, 1.0, X,
+                         J.ldx);
+}
+
+// A (k x s, ld k) = X^T (s x k, ld s).
+__global__ void __launch_bounds__(WT) k_h_transpose(int64_t s, int k, const double* X, double* A) {
+  __shared__ double t[32][33];
+  const int64_t i0 = (int64_t)blockIdx.x * 32;
+  const int c0 = blockIdx.y * 32, lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
+  for (int c = ly; c < 32; c += WT / 32)
+    if (i0 + lx < s && c0 + c < k) t[c][lx] = X[i0 + lx + (int64_t)(c0 + c) * s];
+  __syncthreads();
+  for (int i = ly; i < 32; i += WT / 32)
+    if (i0 + i < s && c0 + lx < k) A[c0 + lx + (i0 + i) * k] = t[lx][i];
 }
 
 // S' = -(S_low (V_low U_up) S_up) (k x k) for the Schur update of a node:
-// V_low (k x s, ld k), U_up (s x k, ld s).  Each CTA reduces a range of s
-// into its partial; the last CTA to finish (counter) sums the partials in
-// CTA order and forms S'.  `counter` returns to 0.
+// V_low (k x s, ld k), U_up (s x k, ld s).  A CTA per chunk of s; the last one to
+// finish (counter, which returns to 0) sums the chunks in order and forms S'.
 __global__ void __launch_bounds__(WT) k_h_core(int64_t s, int k, const double* Vl, const double* Uu, const double* Sl,
-                                               const double* Su, double* partial, double* Sp, int* counter) {
-  // tiles of V_low and U_up during the reduction, X = V_low U_up after it
-  __shared__ double sm[2 * 32 * (HMAX_RANK + 1)];
+                                               const double* Su, double* part, double* Sp, int* counter) {
+  extern __shared__ double red[];                 // 8 HC HC; then X and Y (k x k each)
   __shared__ int last;
-  double(*tv)[HMAX_RANK + 1] = reinterpret_cast<double(*)[HMAX_RANK + 1]>(sm);
-  double(*tu)[HMAX_RANK + 1] = reinterpret_cast<double(*)[HMAX_RANK + 1]>(sm + 32 * (HMAX_RANK + 1));
-  double* X = sm;
-  const int tid = threadIdx.x;
-  const int64_t chunk = (s + gridDim.x - 1) / gridDim.x;
-  const int64_t i0 = (int64_t)blockIdx.x * chunk, i1 = min(s, i0 + chunk);
+  const int64_t chunk = h_chunk(s), i0 = blockIdx.x * chunk, i1 = min(s, i0 + chunk);
   const int kk = k * k;
-  double acc[HMAX_RANK * HMAX_RANK / WT];
-#pragma unroll
-  for (int q = 0; q < HMAX_RANK * HMAX_RANK / WT; ++q) acc[q] = 0.0;
-  for (int64_t t0 = i0; t0 < i1; t0 += 32) {
-    const int tn = (int)min((int64_t)32, i1 - t0);
-    for (int e = tid; e < 32 * k; e += WT) {
-      const int t = e / k, rr = e % k;
-      tv[t][rr] = t < tn ? Vl[rr + (t0 + t) * k] : 0.0;
+  double* mine = part + (int64_t)blockIdx.x * kk;
+  for (int m0 = 0; m0 < k; m0 += HC)
+    for (int n0 = 0; n0 < k; n0 += HC) {
+      const int m = min(HC, k - m0), n = min(HC, k - n0);
+      h_tprod(m, n, i0, i1, Vl + m0, 1, k, Uu + (int64_t)n0 * s, s, red);
+      for (int e = threadIdx.x; e < m * n; e += WT) mine[m0 + e % m + (n0 + e / m) * k] = red[e % m + (e / m) * HC];
+      __syncthreads();
     }
-    for (int e = tid; e < 32 * k; e += WT) {
-      const int rr = e / 32, t = e % 32;
-      tu[t][rr] = t < tn ? Uu[(t0 + t) + (int64_t)rr * s] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < HMAX_RANK * HMAX_RANK / WT; ++q) {
-      const int e = tid + q * WT;
-      if (e < kk) {
-        const int rr = e % k, cc = e / k;
-        double v = 0.0;
-        for (int t = 0; t < 32; ++t) v += tv[t][rr] * tu[t][cc];
-        acc[q] += v;
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < HMAX_RANK * HMAX_RANK / WT; ++q) {
-    const int e = tid + q * WT;
-    if (e < kk) partial[(int64_t)blockIdx.x * kk + e] = acc[q];
-  }
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+    if (last) *counter = 0;
+  }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int e = tid; e < kk; e += WT) {
+  double* X = red;
+  double* Y = red + kk;
+  for (int e = threadIdx.x; e < kk; e += WT) {
     double v = 0.0;
-    for (int g = 0; g < (int)gridDim.x; ++g) v += partial[(int64_t)g * kk + e];
-    X[e] = v;                                     // X = V_low U_up (col-major k x k)
+#pragma unroll 8
+    for (int q = 0; q < (int)gridDim.x; ++q) v += part[(int64_t)q * kk + e];
+    X[e] = v;
   }
   __syncthreads();
-  double* Y = partial;                            // Y = S_low X, over the partials (all read above)
-  for (int e = tid; e < kk; e += WT) {
-    const int rr = e % k, cc = e / k;
+  for (int e = threadIdx.x; e < kk; e += WT) {    // Y = S_low X
     double v = 0.0;
-    for (int q = 0; q < k; ++q) v += Sl[rr + q * k] * X[q + cc * k];
+#pragma unroll 4
+    for (int q = 0; q < k; ++q) v = fma(Sl[e % k + q * k], X[q + (e / k) * k], v);
     Y[e] = v;
   }
   __syncthreads();
-  for (int e = tid; e < kk; e += WT) {            // S' = -(Y S_up)
-    const int rr = e % k, cc = e / k;
+  for (int e = threadIdx.x; e < kk; e += WT) {    // S' = -(Y S_up)
     double v = 0.0;
-    for (int q = 0; q < k; ++q) v += Y[rr + q * k] * Su[q + cc * k];
+#pragma unroll 4
+    for (int q = 0; q < k; ++q) v = fma(Y[e % k + q * k], Su[q + (e / k) * k], v);
     Sp[e] = -v;
   }
-  if (tid == 0) *counter = 0;
 }
 
 // Dense leaves of A_H: D[p] = K(rows of p, cols of p).
@@ -455,200 +450,6 @@ __global__ void k_h_finish_v(int64_t s, int p, int k, int nblk, const double* U2
   }
 }
 
-constexpr int MV_CHUNK = 1024;
-
-// Level-parallel solve.  With W_X = M_right(U_low) and Z_X = U_left^{-1} U_up
-// precomputed per node X (M = the permuted forward substitution of a
-// subtree), L^{-1} P b and U^{-1} y are: every leaf at once, then for each
-// level from the bottom up, every node at once: x_right -= W_X S_low V_low
-// x_left (forward), x_left -= Z_X S_up V_up x_right (backward).
-//
-// Leaves: x_p <- Linv_p P_p x_p (mode 0) or Uinv_p x_p (mode 2); grid: leaves x
-// column groups of WCW.
-__global__ void __launch_bounds__(WT) k_h_leaf_apply(int b, int mode, LeafFactors f, double* x, int64_t ldx,
-                                                     int nrhs) {
-  __shared__ double r[WCW][HMAX_LEAF];
-  const int p = blockIdx.x, c0 = blockIdx.y * WCW;
-  const int nc = min(WCW, nrhs - c0);
-  const int* perm = f.perm + (int64_t)p * b;
-  double* xp = x + (int64_t)p * b + (int64_t)c0 * ldx;
-  for (int e = threadIdx.x; e < WCW * b; e += WT) {
-    const int c = e / b, i = e % b;
-    r[c][i] = c < nc ? xp[(mode == 0 ? perm[i] : i) + c * ldx] : 0.0;
-  }
-  __syncthreads();
-  const double* Op = (mode == 0 ? f.Linv : f.Uinv) + (int64_t)p * b * b;
-  for (int i = threadIdx.x; i < b; i += WT) {
-    double acc[WCW];
-#pragma unroll
-    for (int c = 0; c < WCW; ++c) acc[c] = mode == 0 ? r[c][i] : 0.0;
-    const int j0 = mode == 0 ? 0 : i, j1 = mode == 0 ? i : b;
-#pragma unroll 8
-    for (int j = j0; j < j1; ++j) {
-      const double a = Op[i + (int64_t)j * b];
-#pragma unroll
-      for (int c = 0; c < WCW; ++c) acc[c] += a * r[c][j];
-    }
-    for (int c = 0; c < nc; ++c) xp[i + c * ldx] = acc[c];
-  }
-}
-
-// Partials T[node][chunk] (k x nrhs) = V_c(:, chunk) x(cols of c, chunk) for
-// the blocks c = 2 node + parity of level l (grid: chunks x nodes).
-__global__ void __launch_bounds__(WT) k_h_sv_t(HView h, int l, int parity, const double* x, int64_t ldx, int nrhs,
-                                               double* part) {
-  __shared__ double red[WT / 32][HMAX_RANK];
-  const int node = blockIdx.y, c = 2 * node + parity, k = h.k;
-  const int64_t sl = h.s(l);
-  const int nch = (int)((sl + MV_CHUNK - 1) / MV_CHUNK);
-  const int64_t i0 = (int64_t)blockIdx.x * MV_CHUNK, i1 = min(sl, i0 + MV_CHUNK);
-  const double* Vb = h.v(l, c);
-  const int64_t col0 = (int64_t)(c ^ 1) * sl;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int q = 0; q < nrhs; ++q) {
-    double acc[2] = {0.0, 0.0};
-    for (int64_t i = i0 + wid; i < i1; i += WT / 32) {
-      const double xv = x[col0 + i + q * ldx];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int rr = lane + 32 * t;
-        if (rr < k) acc[t] += Vb[rr + i * k] * xv;
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-      if (lane + 32 * t < k) red[wid][lane + 32 * t] = acc[t];
-    __syncthreads();
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int w = 0; w < WT / 32; ++w) v += red[w][rr];
-      part[(((int64_t)node * nch + blockIdx.x) * nrhs + q) * k + rr] = v;
-    }
-    __syncthreads();
-  }
-}
-
-// x(rows of c) -= WZ_c S_c sum_chunks T[node][chunk], c = 2 node + parity
-// (grid: row tiles x nodes); hw.U addresses the W / Z slab, hw.S the factor's S.
-__global__ void __launch_bounds__(WT) k_h_sv_u(HView hw, int l, int parity, int nrhs, const double* part, double* x,
-                                               int64_t ldx) {
-  __shared__ double t1[HMAX_RANK];
-  __shared__ double t2[HMAX_RANK];
-  const int node = blockIdx.y, c = 2 * node + parity, k = hw.k;
-  const int64_t sl = hw.s(l);
-  const int nch = (int)((sl + MV_CHUNK - 1) / MV_CHUNK);
-  const double* Wb = hw.u(l, c);
-  const double* Sb = hw.sm(l, c);
-  const int64_t row0 = (int64_t)c * sl;
-  const int64_t i = (int64_t)blockIdx.x * WT + threadIdx.x;
-  for (int q = 0; q < nrhs; ++q) {
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int g = 0; g < nch; ++g) v += part[(((int64_t)node * nch + g) * nrhs + q) * k + rr];
-      t1[rr] = v;
-    }
-    __syncthreads();
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int t = 0; t < k; ++t) v += Sb[rr + t * k] * t1[t];
-      t2[rr] = v;
-    }
-    __syncthreads();
-    if (i < sl) {
-      double v = 0.0;
-      for (int t = 0; t < k; ++t) v += Wb[i + (int64_t)t * sl] * t2[t];
-      x[row0 + i + q * ldx] -= v;
-    }
-    __syncthreads();
-  }
-}
-
-// y_p = D_p x_p for every leaf (grid: leaves), nrhs columns.
-__global__ void __launch_bounds__(WT) k_h_mv_leaf(int b, const double* D, const double* x, int64_t ldx, double* y,
-                                                  int64_t ldy, int nrhs) {
-  __shared__ double xs[HMAX_LEAF];
-  const int p = blockIdx.x;
-  const double* Dp = D + (int64_t)p * b * b;
-  for (int c = 0; c < nrhs; ++c) {
-    for (int i = threadIdx.x; i < b; i += WT) xs[i] = x[(int64_t)p * b + i + c * ldx];
-    __syncthreads();
-    for (int i = threadIdx.x; i < b; i += WT) {
-      double v = 0.0;
-      for (int j = 0; j < b; ++j) v += Dp[i + (int64_t)j * b] * xs[j];
-      y[(int64_t)p * b + i + c * ldy] = v;
-    }
-    __syncthreads();
-  }
-}
-
-// Partials T[c][chunk] (k x nrhs) = V_c(:, chunk) x(cols of c, chunk) of one
-// level (grid: chunks x blocks).
-__global__ void __launch_bounds__(WT) k_h_mv_t(HView h, int l, const double* x, int64_t ldx, int nrhs,
-                                               double* part) {
-  __shared__ double red[WT / 32][HMAX_RANK];
-  const int c = blockIdx.y, k = h.k;
-  const int64_t sl = h.s(l);
-  const int nch = (int)((sl + MV_CHUNK - 1) / MV_CHUNK);
-  const int64_t i0 = (int64_t)blockIdx.x * MV_CHUNK, i1 = min(sl, i0 + MV_CHUNK);
-  const double* Vb = h.v(l, c);
-  const int64_t col0 = (int64_t)(c ^ 1) * sl;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int q = 0; q < nrhs; ++q) {
-    double acc[2] = {0.0, 0.0};
-    for (int64_t i = i0 + wid; i < i1; i += WT / 32) {
-      const double xv = x[col0 + i + q * ldx];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int rr = lane + 32 * t;
-        if (rr < k) acc[t] += Vb[rr + i * k] * xv;
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-      if (lane + 32 * t < k) red[wid][lane + 32 * t] = acc[t];
-    __syncthreads();
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int w = 0; w < WT / 32; ++w) v += red[w][rr];
-      part[(((int64_t)c * nch + blockIdx.x) * nrhs + q) * k + rr] = v;
-    }
-    __syncthreads();
-  }
-}
-
-// y(rows of c) += U_c S_c sum_chunks T[c][chunk] (grid: row tiles x blocks).
-__global__ void __launch_bounds__(WT) k_h_mv_u(HView h, int l, int nrhs, const double* part, double* y, int64_t ldy) {
-  __shared__ double t1[HMAX_RANK];
-  __shared__ double t2[HMAX_RANK];
-  const int c = blockIdx.y, k = h.k;
-  const int64_t sl = h.s(l);
-  const int nch = (int)((sl + MV_CHUNK - 1) / MV_CHUNK);
-  const double* Ub = h.u(l, c);
-  const double* Sb = h.sm(l, c);
-  const int64_t row0 = (int64_t)c * sl;
-  const int64_t i = (int64_t)blockIdx.x * WT + threadIdx.x;
-  for (int q = 0; q < nrhs; ++q) {
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int g = 0; g < nch; ++g) v += part[(((int64_t)c * nch + g) * nrhs + q) * k + rr];
-      t1[rr] = v;
-    }
-    __syncthreads();
-    for (int rr = threadIdx.x; rr < k; rr += WT) {
-      double v = 0.0;
-      for (int t = 0; t < k; ++t) v += Sb[rr + t * k] * t1[t];
-      t2[rr] = v;
-    }
-    __syncthreads();
-    if (i < sl) {
-      double v = 0.0;
-      for (int t = 0; t < k; ++t) v += Ub[i + (int64_t)t * sl] * t2[t];
-      y[row0 + i + q * ldy] += v;
-    }
-    __syncthreads();
-  }
-}
-
 // r = b - y (in y), column sums of squares of r and b into nrm[2 c], nrm[2 c + 1]
 // (one CTA per column, fixed reduction order).
 __global__ void __launch_bounds__(WT) k_h_residual(int64_t n, const double* bb, int64_t ldb, double* y, int64_t ldy,
@@ -709,9 +510,9 @@ struct frank_hodlr {
   unsigned long long* flops = nullptr;
   int* err = nullptr;
   int* kfill = nullptr;             // [L + 1][P] ranks, all k (one row per level's stream)
-  int* counter = nullptr;
+  int* counter = nullptr;           // chunk counters: [2][4 P] of the factorization's two streams, one of the core
   double* Sp = nullptr;             // S' of every internal node's update ([2^L - 1][k x k])
-  double* core_part = nullptr;      // [CORE_GRID][k*k]
+  double* core_part = nullptr;      // [H_NCH][k*k]
   double* Wu = nullptr;             // U_low S' (n/2 x k)
   double* lr_scratch = nullptr;     // addition scratch, one region per level
   int64_t lr_cap = 0;
@@ -720,6 +521,8 @@ struct frank_hodlr {
   std::vector<cudaEvent_t> lev;     // [L + 1] last addition enqueued on level j's stream
   cudaEvent_t ev_fork = nullptr, ev_core = nullptr;
   double* WZ = nullptr;             // per node: W (lower block's slot) and Z (upper block's slot), U-shaped
+  double* Zt = nullptr;             // per node: Zt (upper block's slot), U-shaped
+  double* sub[2] = {nullptr, nullptr};   // partial products and T2 of the subtree substitutions (main, side stream)
   cudaStream_t ps = nullptr;        // their walks, beside the factorization
   cudaEvent_t ev_pre = nullptr, ev_ps = nullptr;
   ::frank::ops::LrAddTask* tasks_d = nullptr;   // every update's additions, in launch order
@@ -727,6 +530,8 @@ struct frank_hodlr {
   int64_t ntasks_cap = 0;
   double* mv_part = nullptr;
   int64_t mv_part_cap = 0;
+  int* mv_counter = nullptr;
+  int64_t mv_groups = 0;
   double* work = nullptr;           // refinement: residual / correction (n x nrhs)
   int64_t work_cap = 0;
   double* nrm = nullptr;            // 2 x nrhs
@@ -739,7 +544,6 @@ struct frank_hodlr {
 
 namespace {
 
-constexpr int CORE_GRID = 64;
 
 #define H_TRY(expr)                                                                                         \
   do {                                                                                                      \
@@ -856,20 +660,39 @@ void enqueue_update(frank_hodlr* h, int lr, int cr, const double* Ux, const doub
   }
 }
 
-// WZ(l, c) <- the substitution (mode 0: L with pivots, 2: U) of cluster
-// (l, c)'s subtree applied to the U factor of block (l, c), on stream ps after
-// everything enqueued so far on s.
-void enqueue_precompute(frank_hodlr* h, int l, int c, int mode, cudaStream_t s) {
-  const int k = h->k;
-  const int64_t sl = s_of(h, l);
-  cudaEventRecord(h->ev_pre, s);
-  cudaStreamWaitEvent(h->ps, h->ev_pre, 0);
-  cudaMemcpyAsync(h->WZ + u_off(h, l, c), h->U + u_off(h, l, c), sizeof(double) * sl * k, cudaMemcpyDeviceToDevice,
-                  h->ps);
-  hk::Walk j0{mode, l, c, k, h->WZ + u_off(h, l, c), 1, sl}, none{0, 0, 0, 0, nullptr, 1, 1};
-  hk::k_h_walk<<<dim3((k + hk::WCW - 1) / hk::WCW, 1), hk::WWT, hk::WALK_SMEM, h->ps>>>(view(h, true),
-                                                                                       leaf_factors(h), j0, none);
+// Doubles of the partial products and of T2 for `jobs` substitutions of ncols columns.
+int64_t sub_part(const frank_hodlr* h, int jobs, int ncols) {
+  const int64_t groups = (ncols + hk::HC - 1) / hk::HC;
+  int64_t most = 0;
+  for (int l = 1; l <= h->L; ++l) most = std::max(most, ((int64_t)1 << l) * hk::h_nch(s_of(h, l)));
+  return most * jobs * groups * h->k * hk::HC;
+}
+int64_t sub_t2(const frank_hodlr* h, int jobs, int ncols) { return (int64_t)h->P * jobs * ncols * h->k; }
+
+// One or two substitutions (hk::HJob) on the subtree (l0, c0), or the H-matvec
+// (mode 3, the whole tree): the leaves, then the levels from the bottom up.
+void enqueue_sub(frank_hodlr* h, const hk::HView& v, int l0, int c0, int njobs, const hk::HJob& j0, const hk::HJob& j1,
+                 int ncols, double* buf, int* counter, cudaStream_t s) {
+  const int hl = h->L - l0, p0 = c0 << hl, groups = (ncols + hk::HC - 1) / hk::HC;
+  double* t2 = buf + sub_part(h, njobs, ncols);
+  hk::k_h_leaf_mm<<<dim3(1 << hl, (ncols + hk::HLC - 1) / hk::HLC, njobs), hk::WT, 0, s>>>(v, leaf_factors(h), j0, j1,
+                                                                                          p0, ncols);
   ++h->launches;
+  for (int l = h->L; l > l0; --l) {
+    const int64_t sl = s_of(h, l);
+    const int first = c0 << (l - l0);
+    const int nodes = j0.mode == 3 ? 1 << l : 1 << (l - l0 - 1);
+    hk::k_h_t<<<dim3(hk::h_nch(sl), nodes, njobs * groups), hk::WT, hk::H_TSMEM, s>>>(v, j0, j1, njobs, l, first, ncols,
+                                                                                     buf, t2, counter);
+    hk::k_h_u<<<dim3((unsigned)((sl + hk::WT - 1) / hk::WT), nodes, njobs * groups), hk::WT, 0, s>>>(
+        v, h->WZ, h->Zt, j0, j1, njobs, l, first, ncols, t2);
+    h->launches += 2;
+  }
+}
+
+// A substitution in place on X (col-major), read from src the first time.
+hk::HJob sub_job(int mode, const double* src, int64_t srs, int64_t scs, double* X, int64_t ldx) {
+  return hk::HJob{mode, src, srs, scs, X, 1, ldx, nullptr, 0};
 }
 
 void enqueue_node(frank_hodlr* h, int l, int c, cudaStream_t s) {
@@ -881,28 +704,44 @@ void enqueue_node(frank_hodlr* h, int l, int c, cudaStream_t s) {
   enqueue_node(h, l + 1, 2 * c, s);
   const int up = 2 * c, lo = 2 * c + 1;
   const int64_t sc = s_of(h, l + 1);
-  // the node's own off-diagonal blocks: every addition into them enqueued so far
+  const hk::HView v = view(h, true);
+  // the node's own off-diagonal blocks: every addition into them enqueued so
+  // far; and the left child's W, Z, Zt
   cudaStreamWaitEvent(s, h->lev[l + 1], 0);
+  cudaStreamWaitEvent(s, h->ev_ps, 0);
   // U_up <- L_left^{-1} P U_up (trsm.cpp:106-115 -> 117-125 -> leaves);
-  // V_low <- V_low U_left^{-1}
-  hk::Walk j0{0, l + 1, 2 * c, k, h->U + u_off(h, l + 1, up), 1, sc};
-  hk::Walk j1{1, l + 1, 2 * c, k, h->V + u_off(h, l + 1, lo), k, 1};
-  hk::k_h_walk<<<dim3((k + hk::WCW - 1) / hk::WCW, 2), hk::WWT, hk::WALK_SMEM, s>>>(view(h, true), leaf_factors(h),
-                                                                                   j0, j1);
-  // for the level-parallel solve, beside the factorization: Z = U_left^{-1} U_up
-  enqueue_precompute(h, l + 1, up, 2, s);
+  // V_low <- V_low U_left^{-1}, through its transpose in Wu (a leaf writes V_low itself)
+  double* Uu = h->U + u_off(h, l + 1, up);
+  double* Vl = h->V + u_off(h, l + 1, lo);
+  const bool leaf = l + 1 == h->L;
+  hk::HJob j0 = sub_job(0, Uu, 1, sc, Uu, sc), j1 = sub_job(1, Vl, k, 1, h->Wu, sc);
+  if (leaf) { j1.X = Vl; j1.xrs = k; j1.ldx = 1; }
+  enqueue_sub(h, v, l + 1, 2 * c, 2, j0, j1, k, h->sub[0], h->counter, s);
+  if (!leaf) {
+    hk::k_h_transpose<<<dim3((unsigned)((sc + 31) / 32), (k + 31) / 32), hk::WT, 0, s>>>(sc, k, h->Wu, Vl);
+    ++h->launches;
+  }
+  // for the later substitutions, beside the factorization: Z = U_left^{-1} U_up
+  cudaEventRecord(h->ev_pre, s);
+  cudaStreamWaitEvent(h->ps, h->ev_pre, 0);
+  hk::HJob jz = sub_job(2, Uu, 1, sc, h->WZ + u_off(h, l + 1, up), sc);
+  enqueue_sub(h, v, l + 1, 2 * c, 1, jz, jz, k, h->sub[1], h->counter + 4 * h->P, h->ps);
   // S' = -(S_low V_low)(U_up S_up), one k x k slot per internal node
   double* Sp = h->Sp + ((int64_t)(1 << l) - 1 + c) * k * k;
-  const int grid = (int)std::min<int64_t>(CORE_GRID, (sc + 511) / 512);
-  hk::k_h_core<<<grid, hk::WT, 0, s>>>(sc, k, h->V + u_off(h, l + 1, lo), h->U + u_off(h, l + 1, up),
-                                       h->S + s_off(h, l + 1, lo), h->S + s_off(h, l + 1, up), h->core_part, Sp,
-                                       h->counter);
+  hk::k_h_core<<<hk::h_nch(sc), hk::WT, hk::H_TSMEM, s>>>(sc, k, Vl, Uu, h->S + s_off(h, l + 1, lo),
+                                                          h->S + s_off(h, l + 1, up), h->core_part, Sp,
+                                                          h->counter + 8 * h->P);
   cudaEventRecord(h->ev_core, s);
-  h->launches += 2;
+  ++h->launches;
   enqueue_update(h, l + 1, lo, h->U + u_off(h, l + 1, lo), h->V + u_off(h, l + 1, up), Sp, s);
   enqueue_node(h, l + 1, 2 * c + 1, s);
-  // W = M_right(U_low), once the right child is factored
-  enqueue_precompute(h, l + 1, lo, 0, s);
+  // W = M_right(U_low) and Zt = U_right^{-T} V_up^T, once the right child is factored
+  cudaEventRecord(h->ev_pre, s);
+  cudaStreamWaitEvent(h->ps, h->ev_pre, 0);
+  hk::HJob jw = sub_job(0, h->U + u_off(h, l + 1, lo), 1, sc, h->WZ + u_off(h, l + 1, lo), sc);
+  hk::HJob jt = sub_job(1, h->V + u_off(h, l + 1, up), k, 1, h->Zt + u_off(h, l + 1, up), sc);
+  enqueue_sub(h, v, l + 1, 2 * c + 1, 2, jw, jt, k, h->sub[1], h->counter + 4 * h->P, h->ps);
+  cudaEventRecord(h->ev_ps, h->ps);
 }
 
 int enqueue_factor(frank_hodlr* h, cudaStream_t s) {
@@ -916,6 +755,7 @@ int enqueue_factor(frank_hodlr* h, cudaStream_t s) {
   h->tasks_h.clear();
   H_TRY(cudaEventRecord(h->ev_fork, s));
   H_TRY(cudaStreamWaitEvent(h->ps, h->ev_fork, 0));
+  H_TRY(cudaEventRecord(h->ev_ps, h->ps));
   for (int j = 1; j <= h->L; ++j) {
     H_TRY(cudaStreamWaitEvent(h->ls[j], h->ev_fork, 0));
     H_TRY(cudaEventRecord(h->lev[j], h->ls[j]));
@@ -947,7 +787,7 @@ void free_plan(frank_hodlr* h) {
                   (void*)h->V, (void*)h->Linv, (void*)h->Uinv, (void*)h->UinvT, (void*)h->perm, (void*)h->ipiv,
                   (void*)h->getrf_scratch, (void*)h->geom, (void*)h->flops, (void*)h->err, (void*)h->kfill,
                   (void*)h->counter, (void*)h->Sp, (void*)h->core_part, (void*)h->Wu, (void*)h->lr_scratch,
-                  (void*)h->mv_part, (void*)h->work, (void*)h->nrm, (void*)h->tasks_d})
+                  (void*)h->mv_part, (void*)h->mv_counter, (void*)h->work, (void*)h->nrm, (void*)h->tasks_d})
     if (p) cudaFree(p);
   if (h->e0) cudaEventDestroy(h->e0);
   if (h->e1) cudaEventDestroy(h->e1);
@@ -958,7 +798,7 @@ void free_plan(frank_hodlr* h) {
   if (h->ev_pre) cudaEventDestroy(h->ev_pre);
   if (h->ev_ps) cudaEventDestroy(h->ev_ps);
   if (h->ps) cudaStreamDestroy(h->ps);
-  if (h->WZ) cudaFree(h->WZ);
+  for (double* x : {h->WZ, h->Zt, h->sub[0], h->sub[1]}) if (x) cudaFree(x);
   if (h->s) cudaStreamDestroy(h->s);
   delete h;
 }
@@ -974,16 +814,26 @@ int check_block(const frank_hodlr* h, int l, int c) {
   return FRANK_OK;
 }
 
+// Buffers of the solves and matvecs: partial products and T2 of a level, and a
+// chunk counter per block and column group (zeroed here; every launch leaves
+// them zero).
 int ensure_mv(frank_hodlr* h, int nrhs) {
-  // the partials of one level at a time: 2^l blocks x chunks x nrhs x k
-  int64_t need = 0;
-  for (int l = 1; l <= h->L; ++l)
-    need = std::max(need, ((int64_t)1 << l) * ((s_of(h, l) + hk::MV_CHUNK - 1) / hk::MV_CHUNK) * nrhs * h->k);
+  const int64_t need = sub_part(h, 1, nrhs) + sub_t2(h, 1, nrhs);
+  const int64_t groups = (nrhs + hk::HC - 1) / hk::HC;
   if (need > h->mv_part_cap) {
     if (h->mv_part) cudaFree(h->mv_part);
     h->mv_part = nullptr;
+    h->mv_part_cap = 0;
     H_TRY(dalloc(&h->mv_part, (size_t)need));
     h->mv_part_cap = need;
+  }
+  if (groups > h->mv_groups) {
+    if (h->mv_counter) cudaFree(h->mv_counter);
+    h->mv_counter = nullptr;
+    h->mv_groups = 0;
+    H_TRY(dalloc(&h->mv_counter, (size_t)(groups * h->P)));
+    H_TRY(cudaMemset(h->mv_counter, 0, sizeof(int) * groups * h->P));
+    h->mv_groups = groups;
   }
   return FRANK_OK;
 }
@@ -992,15 +842,8 @@ int ensure_mv(frank_hodlr* h, int nrhs) {
 int enqueue_matvec(frank_hodlr* h, const double* x, int64_t ldx, double* y, int64_t ldy, int nrhs, cudaStream_t s) {
   int rc = ensure_mv(h, nrhs);
   if (rc) return rc;
-  const hk::HView v = view(h, false);
-  hk::k_h_mv_leaf<<<h->P, hk::WT, 0, s>>>(h->b, h->D0, x, ldx, y, ldy, nrhs);
-  for (int l = 1; l <= h->L; ++l) {
-    const int64_t sl = s_of(h, l);
-    const int nch = (int)((sl + hk::MV_CHUNK - 1) / hk::MV_CHUNK);
-    hk::k_h_mv_t<<<dim3(nch, 1 << l), hk::WT, 0, s>>>(v, l, x, ldx, nrhs, h->mv_part);
-    hk::k_h_mv_u<<<dim3((unsigned)((sl + hk::WT - 1) / hk::WT), 1 << l), hk::WT, 0, s>>>(v, l, nrhs, h->mv_part, y,
-                                                                                          ldy);
-  }
+  const hk::HJob j{3, x, 1, ldx, y, 1, ldy, x, ldx};
+  enqueue_sub(h, view(h, false), 0, 0, 1, j, j, nrhs, h->mv_part, h->mv_counter, s);
   H_TRY(cudaGetLastError());
   return FRANK_OK;
 }
@@ -1009,25 +852,10 @@ int enqueue_matvec(frank_hodlr* h, const double* x, int64_t ldx, double* y, int6
 int enqueue_solve(frank_hodlr* h, double* d_b, int64_t ldb, int nrhs, cudaStream_t s, int passes = 3) {
   int rc = ensure_mv(h, nrhs);
   if (rc) return rc;
-  const hk::HView v = view(h, true);
-  hk::HView vw = v;
-  vw.U = h->WZ;
-  const hk::LeafFactors f = leaf_factors(h);
-  const dim3 gleaf(h->P, (nrhs + hk::WCW - 1) / hk::WCW);
   for (int pass = 0; pass < 2; ++pass) {
     if (!(passes & (1 << pass))) continue;
-    // forward: leaves with L and pivots, then lower blocks (odd); backward:
-    // leaves with U, then upper blocks (even)
-    hk::k_h_leaf_apply<<<gleaf, hk::WT, 0, s>>>(h->b, pass == 0 ? 0 : 2, f, d_b, ldb, nrhs);
-    const int parity = pass == 0 ? 1 : 0;
-    for (int l = h->L; l >= 1; --l) {
-      const int64_t sl = s_of(h, l);
-      const int nch = (int)((sl + hk::MV_CHUNK - 1) / hk::MV_CHUNK);
-      const int nodes = 1 << (l - 1);
-      hk::k_h_sv_t<<<dim3(nch, nodes), hk::WT, 0, s>>>(v, l, parity, d_b, ldb, nrhs, h->mv_part);
-      hk::k_h_sv_u<<<dim3((unsigned)((sl + hk::WT - 1) / hk::WT), nodes), hk::WT, 0, s>>>(vw, l, parity, nrhs,
-                                                                                           h->mv_part, d_b, ldb);
-    }
+    const hk::HJob j = sub_job(pass == 0 ? 0 : 2, d_b, 1, ldb, d_b, ldb);
+    enqueue_sub(h, view(h, true), 0, 0, 1, j, j, nrhs, h->mv_part, h->mv_counter, s);
   }
   H_TRY(cudaGetLastError());
   return FRANK_OK;
@@ -1068,8 +896,8 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(dalloc(&h->perm, P * leaf)); A(dalloc(&h->ipiv, P * leaf));
   A(dalloc(&h->getrf_scratch, (size_t)blr::leaf_scratch(leaf)));
   A(dalloc(&h->geom, 4)); A(dalloc(&h->flops, blr::FLOP_SLOTS)); A(dalloc(&h->err, hk::HERR_SLOTS));
-  A(dalloc(&h->kfill, (size_t)(L + 1) * P)); A(dalloc(&h->counter, 1));
-  A(dalloc(&h->Sp, (size_t)P * rank * rank)); A(dalloc(&h->core_part, (size_t)CORE_GRID * rank * rank));
+  A(dalloc(&h->kfill, (size_t)(L + 1) * P)); A(dalloc(&h->counter, 8 * (size_t)P + 1));
+  A(dalloc(&h->Sp, (size_t)P * rank * rank)); A(dalloc(&h->core_part, (size_t)hk::H_NCH * rank * rank));
   A(dalloc(&h->Wu, (size_t)(n / 2) * rank));
   // LowRank additions: per level j a scratch region for its largest launch
   // (2^(j-1) blocks of order n >> j, the update of the root's right child),
@@ -1096,7 +924,8 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaEventCreateWithFlags(&h->ev_pre, cudaEventDisableTiming));
   A(cudaEventCreateWithFlags(&h->ev_ps, cudaEventDisableTiming));
   A(cudaStreamCreateWithFlags(&h->ps, cudaStreamNonBlocking));
-  A(dalloc(&h->WZ, (size_t)nk));
+  A(dalloc(&h->WZ, (size_t)nk)); A(dalloc(&h->Zt, (size_t)nk));
+  for (double*& x : h->sub) A(dalloc(&x, (size_t)(sub_part(h, 2, rank) + sub_t2(h, 2, rank))));
   A(cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking));
   A(cudaEventCreate(&h->e0));
   A(cudaEventCreate(&h->e1));
@@ -1108,7 +937,7 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   std::vector<int> kf((size_t)(L + 1) * P, rank);
   A(cudaMemcpy(h->geom, geom, sizeof(geom), cudaMemcpyHostToDevice));
   A(cudaMemcpy(h->kfill, kf.data(), sizeof(int) * kf.size(), cudaMemcpyHostToDevice));
-  A(cudaMemset(h->counter, 0, sizeof(int)));
+  A(cudaMemset(h->counter, 0, sizeof(int) * (8 * (size_t)P + 1)));
   A(cudaMemset(h->flops, 0, sizeof(unsigned long long) * blr::FLOP_SLOTS));
   A(cudaMemset(h->D0, 0, sizeof(double) * dd));
   A(cudaMemset(h->U0, 0, sizeof(double) * nk));
@@ -1116,7 +945,8 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaMemset(h->S0, 0, sizeof(double) * sk));
   A(cudaFuncSetAttribute(blr::k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(blr::k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
-  A(cudaFuncSetAttribute(hk::k_h_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::WALK_SMEM));
+  A(cudaFuncSetAttribute(hk::k_h_t, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::H_TSMEM));
+  A(cudaFuncSetAttribute(hk::k_h_core, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::H_TSMEM));
   if (e == cudaSuccess && ::frank::ops::lr_add_prepare() != FRANK_OK) e = cudaErrorInvalidValue;
   if (e != cudaSuccess) {
     free_plan(h);
