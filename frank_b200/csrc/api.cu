@@ -113,7 +113,7 @@ struct frank_blr {
   // solve / matvec temporaries (nrhs <= 8 per pass)
   void* z = nullptr;         // n x 8 (T)
   void* stmp = nullptr;      // bmax x 8 (T)
-  void* sctmp = nullptr;     // nb x bmax x 8 (T)
+  double* tbuf = nullptr;    // nb x kcap x 8: the solve's inner products, per target
   double* part = nullptr;    // nb*nb x bmax x 8
   double* vtmp = nullptr;    // n x 8 x 3 (residual, correction, rhs copy)
   double* nrm = nullptr;     // norm partials
@@ -148,7 +148,7 @@ struct frank_blr {
   };
   std::vector<SolveGraph> solve_graphs;
   cudaStream_t cap_stream = nullptr;   // private stream the solves are captured on
-  int solve_chunk = 8;                 // RHS per solve pass (bounded by the scatter's shared memory)
+  int solve_chunk = 8;                 // RHS per solve / matvec pass (bounded by the kernels' shared memory)
   // lookahead: second capture stream and its dependency events
   cudaStream_t aux = nullptr;
   cudaEvent_t fork = nullptr;
@@ -464,13 +464,22 @@ int enqueue_solve(frank_blr* p, T* z, int64_t ldz, int nrhs, bool transpose, cud
   FactorWs<T> ws = factor_ws<T>(p);
   T* ybuf = static_cast<T*>(p->stmp);
   const int nb = p->nb;
-  const int gd = (p->bmax + SOLVE_ROWS - 1) / SOLVE_ROWS;
-  const size_t shd = ((size_t)p->bmax * nrhs + (size_t)(SOLVE_THREADS / SOLVE_ROWS) * SOLVE_ROWS * 8) * sizeof(double);
-  const size_t shs = solve_scatter_cl_smem(p->bmax, p->kcap, nrhs);
+  const int ns = solve_ring<T>(p->bmax, p->kcap, nrhs);
+  const bool direct = solve_direct(p->bmax, p->fixed_rank > 0 ? p->fixed_rank : p->kcap);
+  const size_t shm = direct ? solve_direct_smem(p->bmax, p->kcap, nrhs) : solve_smem<T>(p->bmax, p->kcap, nrhs, ns);
   auto step = [&](int i, int dmode, int smode, int ntarget) {
-    k_solve_diag<T><<<gd, SOLVE_THREADS, shd, s>>>(W, ws, i, z, ldz, nrhs, dmode, ybuf);
-    k_solve_scatter_cl<T><<<std::max(ntarget, 1) * SC_CLUSTER, SOLVE_THREADS, shs, s>>>(W, i, z, ldz, nrhs, smode,
-                                                                                       ybuf, ntarget);
+    if (direct) {
+      k_solve_diag_direct<T><<<(p->bmax + SD_ROWS - 1) / SD_ROWS, SOLVE_THREADS, shm, s>>>(W, ws, i, z, ldz, nrhs,
+                                                                                           dmode, ybuf);
+      k_solve_scatter<T><<<std::max(ntarget, 1), SOLVE_THREADS, shm, s>>>(W, i, z, ldz, nrhs, smode, ybuf, ntarget);
+      return;
+    }
+    k_solve_diag<T><<<(p->bmax + SOLVE_ROWS - 1) / SOLVE_ROWS, SOLVE_THREADS, shm, s>>>(W, ws, i, z, ldz, nrhs, dmode,
+                                                                                        ybuf, ns);
+    if (ntarget > 0)
+      k_solve_inner<T><<<dim3((p->kcap + 15) / 16, ntarget), SOLVE_THREADS, shm, s>>>(W, i, nrhs, smode, ybuf, p->tbuf, ns);
+    k_solve_outer<T><<<dim3((p->bmax + 63) / 64, std::max(ntarget, 1)), SOLVE_THREADS, shm, s>>>(
+        W, i, z, ldz, nrhs, smode, ybuf, p->tbuf, ntarget, ns);
   };
   if (!transpose) {
     if (part != 2) for (int i = 0; i < nb; ++i) step(i, 0, 0, nb - i - 1);
@@ -550,12 +559,16 @@ int solve_device_impl(frank_blr* p, double* d_b, int64_t ldb, int nrhs, bool tra
 int matvec_device_impl(frank_blr* p, const double* x, int64_t ldx, double* y, int64_t ldy, int nrhs,
                        const double* bres, int64_t ldb, cudaStream_t s, bool transpose = false) {
   BlrView<double> H = h_view(p);
-  for (int c0 = 0; c0 < nrhs; c0 += 8) {
-    const int nr = std::min(8, nrhs - c0);
-    const size_t shm = matvec_smem(p->bmax, p->kcap, nr);
+  for (int c0 = 0; c0 < nrhs; c0 += p->solve_chunk) {
+    const int nr = std::min(p->solve_chunk, nrhs - c0);
+    const int ns = solve_ring<double>(p->bmax, p->kcap, nr);
+    const size_t shm = solve_smem<double>(p->bmax, p->kcap, nr, ns);
     p->solve_launches += 2;
-    k_matvec_blocks<<<dim3(p->nb, p->nb), MV_THREADS, shm, s>>>(H, x + c0 * ldx, ldx, nr, p->part, transpose ? 1 : 0);
-    k_matvec_reduce<<<p->nb, 256, 0, s>>>(H, p->part, nr, bres ? bres + c0 * ldb : nullptr, ldb, y + c0 * ldy, ldy);
+    k_matvec_blocks<<<dim3(p->nb, p->nb), SOLVE_THREADS, shm, s>>>(H, x + c0 * ldx, ldx, nr, p->part,
+                                                                   transpose ? 1 : 0, ns);
+    k_matvec_reduce<<<dim3(p->nb, (p->bmax + 255) / 256, nr), 256, 0, s>>>(H, p->part, nr,
+                                                                           bres ? bres + c0 * ldb : nullptr, ldb,
+                                                                           y + c0 * ldy, ldy);
   }
   CUDA_TRY(cudaGetLastError());
   return FRANK_OK;
@@ -635,7 +648,7 @@ void free_plan(frank_blr* p) {
   if (p->graph) cudaGraphDestroy(p->graph);
   void* ptrs[] = {p->d_off, p->d_dslot, p->d_lslot, p->d_rankH, p->d_rankW, p->Hd, p->Hu, p->Hs, p->Hv,
                   p->Wd, p->Wu, p->Ws, p->Wv, p->perm, p->ipiv, p->err, p->work, p->Linv, p->Uinv, p->WL, p->WU,
-                  p->getrf_scratch, p->dscratch, p->rscratch, p->z, p->stmp, p->sctmp, p->part, p->vtmp, p->nrm,
+                  p->getrf_scratch, p->dscratch, p->rscratch, p->z, p->stmp, p->tbuf, p->part, p->vtmp, p->nrm,
                   p->rsplit, p->split_done, p->host_io};
   for (void* q : ptrs) if (q) cudaFree(q);
   if (p->flops) cudaFree(p->flops);
@@ -821,7 +834,7 @@ int create_impl(const frank_blr_desc* d, const double* points, int dim, frank_bl
   // so frank_blr_set_grid can size them for batched use first.
   ALLOC(t, p->n * 8 * ts); p->z = t;
   ALLOC(t, bm * 8 * ts); p->stmp = t;
-  ALLOC(t, (int64_t)nb * bm * 8 * ts); p->sctmp = t;
+  ALLOC(p->tbuf, (int64_t)nb * kc * 8);
   ALLOC(p->part, (int64_t)nb * nb * bm * 8);
   ALLOC(p->vtmp, p->n * 8 * 3);
   ALLOC(p->nrm, p->nrm_blocks * 8);
@@ -858,19 +871,22 @@ int create_impl(const frank_blr_desc* d, const double* points, int dim, frank_bl
     free_plan(p);
     return fail(FRANK_ERR_CUDA, "plan upload");
   }
-  // dynamic shared memory of the solve / matvec kernels (8 RHS per pass)
-  const int shm = (int)matvec_smem((int)bm, (int)kc, 8);
-  const int shd = (int)((bm * 8 + (SOLVE_THREADS / SOLVE_ROWS) * SOLVE_ROWS * 8) * sizeof(double));
-  // RHS per solve pass: the most whose scatter shared memory fits a CTA
-  p->solve_chunk = 8;
-  while (p->solve_chunk > 1 && solve_scatter_cl_smem((int)bm, (int)kc, p->solve_chunk) > (size_t)SMEM_OPTIN_MAX)
+  // RHS per pass of the solve / matvec kernels: the most whose shared memory
+  // fits a CTA (with the smallest ring)
+  p->solve_chunk = SV_NR;
+  while (p->solve_chunk > 1 && solve_smem<double>((int)bm, (int)kc, p->solve_chunk, 2) > (size_t)SMEM_OPTIN_MAX)
     p->solve_chunk /= 2;
-  const int shs = (int)solve_scatter_cl_smem((int)bm, (int)kc, p->solve_chunk);
-  cudaFuncSetAttribute(k_matvec_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
-  cudaFuncSetAttribute(k_solve_scatter_cl<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, shs);
-  cudaFuncSetAttribute(k_solve_scatter_cl<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, shs);
-  cudaFuncSetAttribute(k_solve_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-  cudaFuncSetAttribute(k_solve_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+  cudaFuncSetAttribute(k_matvec_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_scatter<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_scatter<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_diag_direct<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_diag_direct<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_inner<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_outer<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_inner<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_solve_outer<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
   cudaFuncSetAttribute(k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
   cudaFuncSetAttribute(k_leaf_step<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);
   cudaFuncSetAttribute(k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, LEAF_SMEM_MAX);

@@ -11,8 +11,6 @@
 
 #include "common.cuh"
 
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
 namespace frank {
@@ -2131,457 +2129,564 @@ __global__ void __launch_bounds__(GRAM_THREADS) k_recompress_gram(BlrView<T> A, 
 //   x_i = Uinv_i z_i ; z_j -= U(j,i) x_i for j < i.
 // ---------------------------------------------------------------------------
 constexpr int SOLVE_THREADS = 256;
-constexpr int SOLVE_ROWS = 16;   // rows of the diagonal solve per CTA (16 inner-index slices each)
+constexpr int SOLVE_ROWS = 16;   // rows of the diagonal solve per CTA
+constexpr int SV_NR = 8;         // right-hand sides per pass: one column tile of the FP64 mma
+constexpr int SMEM_OPTIN_MAX = 226 * 1024;   // dynamic shared memory a CTA may opt into, beside 1 KB of static
 
-// y = M * P(z_i) (which 0: Linv, permuted input; 1: Uinv),
-// y = M^T z_i (2: Uinv^T), or y = P^T (Linv^T z_i) (3), into ybuf (ld bmax).
-// grid = ceil(b / SOLVE_ROWS) CTAs; each stages the whole input block in
-// shared memory (b x nrhs doubles) and produces SOLVE_ROWS rows.
+// The solves and the matvec read every factor entry once: memory bounds the
+// matvec, the latency of 2 nb dependent steps the solve.  Loads into registers
+// left too few bytes in flight (one warp instruction in 17 cycles a scheduler,
+// 1.0 TB/s; n = 16384, b = 512, 4 right-hand sides: matvec 452 us, 325 through
+// the ring; refinement 15.1 ms to 7.4), so a CTA streams its matrices as boxes through a ring in
+// shared memory (cp.async, two boxes ahead, also over the seams between
+// products) and multiplies them on the tensor pipe with the right-hand sides as
+// the columns.  MV_T: out = A^T X, boxes of 16 columns x 256 rows; MV_N*:
+// out = A X, boxes of 512 x 8, 64 x 56 and 16 x 128 (rows x columns).  The
+// column strides in shared memory make the fragment reads conflict-free.
+template <int N> struct IntC { static constexpr int value = N; };
+enum : int { MV_T, MV_N512, MV_N64, MV_N16 };
+constexpr int MV_BOX = 16 * 260;              // elements of a ring slot (the largest box)
+
 template <typename T>
-__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag(BlrView<T> A, FactorWs<T> ws, int i, const T* z,
-                                                              int64_t ldz, int nrhs, int which, T* ybuf) {
-  extern __shared__ double xs[];          // b x nrhs input, then the slices' partial sums
-  const int b = A.bs(i), ld = A.bmax;
-  const int64_t o = A.off[i];
-  const T* Mx = (which == 0 || which == 3) ? ws.Linv + (int64_t)i * ld * ld : ws.Uinv + (int64_t)i * ld * ld;
-  const int* perm = ws.perm + (int64_t)i * ld;
-  for (int e = threadIdx.x; e < b * nrhs; e += blockDim.x) {
-    const int r = e % b, c = e / b;
-    xs[e] = double(z[o + (which == 0 ? perm[r] : r) + (int64_t)c * ldz]);
+struct MvSeg {
+  const T* A;            // R x C, column stride ld
+  int64_t ld;
+  int R, C, kind, ldx, ldo, vec;
+  const double* X;       // k x nr (shared)
+  double* out;           // m x nr (shared); the last segment's results go to the sink
+  FRANK_D int m() const { return kind == MV_T ? C : R; }
+  FRANK_D int k() const { return kind == MV_T ? R : C; }
+  FRANK_D int tm() const { return kind == MV_N512 ? 512 : (kind == MV_N64 ? 64 : 16); }
+  FRANK_D int tk() const { return kind == MV_T ? 256 : (kind == MV_N512 ? 8 : (kind == MV_N64 ? 56 : 128)); }
+  FRANK_D void set(const T* A_, int64_t ld_, int R_, int C_, int kind_, const double* X_, int ldx_, double* out_, int ldo_) {
+    A = A_; ld = ld_; R = R_; C = C_; kind = kind_; X = X_; ldx = ldx_; out = out_; ldo = ldo_;
+    vec = (reinterpret_cast<uintptr_t>(A_) & 15) == 0 && ((ld_ * sizeof(T)) & 15) == 0;
   }
-  __syncthreads();
-  const int r0 = blockIdx.x * SOLVE_ROWS;
-  const int nr = min(SOLVE_ROWS, b - r0);
-  if (which <= 1) {
-    // rows r0.. of M x: thread (rl, sl) sums the inner slice sl of row rl
-    double* part = xs + (int64_t)b * nrhs;
-    const int rl = threadIdx.x % SOLVE_ROWS, sl = threadIdx.x / SOLVE_ROWS;  // SOLVE_THREADS / SOLVE_ROWS slices
-    const int nsl = SOLVE_THREADS / SOLVE_ROWS;
-    const int tlen = (b + nsl - 1) / nsl;
-    const int t0 = sl * tlen, t1 = min(b, t0 + tlen);
-    double acc[8];
+};
+
+// bytes < N: the rest of the N destination bytes is zero-filled
+template <int N>
+FRANK_D void cp_async(void* dst, const void* src, int bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(N), "r"(bytes) : "memory");
+}
+
+// Box (r0, c0) of a segment into a slot.  Entries beyond the inner dimension
+// are zero-filled (up to the next 16), those beyond the outer one left alone.
+template <int BR, int BC, int LDP, bool TR, typename T>
+FRANK_D void mv_issue_box(const MvSeg<T>& s, int r0, int c0, T* slot) {
+  const int vr = min(BR, s.R - r0), vc = min(BC, s.C - c0);
+  const int lr = TR ? min(BR, (vr + 15) & ~15) : vr, lc = TR ? vc : min(BC, (vc + 3) & ~3);
+  const T* A = s.A + r0 + (int64_t)c0 * s.ld;
+  if (s.vec && vr == BR && vc == BC) {     // a whole box: no predicates, constant strides
+    constexpr int E = 16 / (int)sizeof(T), UN = BR / E, CP = UN < SOLVE_THREADS ? SOLVE_THREADS / UN : 1;   // columns per pass
+    const int col = threadIdx.x / UN, u = (threadIdx.x % UN) * E;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(slot + col * LDP + u);
+    const T* src = A + u + (int64_t)col * s.ld;
+    const int64_t step = CP * s.ld;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-    if (rl < nr) {
-      const T* mrow = Mx + r0 + rl;
-#pragma unroll 4
-      for (int t = t0; t < t1; ++t) {
-        const double mv = double(mrow[(int64_t)t * ld]);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < nrhs) acc[c] += mv * xs[t + c * b];
+    for (int c = 0; c < BC; c += CP)
+      if (BC % CP == 0 || c + col < BC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + c * LDP * (int)sizeof(T)), "l"(src) : "memory");
+        src += step;
       }
+    return;
+  }
+  auto put = [&](auto e_, int n) {
+    constexpr int E = decltype(e_)::value, UN = BR / E;
+    for (int x = threadIdx.x; x < n * BC; x += SOLVE_THREADS) {
+      const int col = x / UN, u = (x % UN) * E;
+      if (u >= lr || col >= lc) continue;
+      const int ok = col < vc ? max(0, min(E, vr - u)) : 0;
+      cp_async<E * (int)sizeof(T)>(slot + col * LDP + u, ok ? A + u + (int64_t)col * s.ld : s.A, ok * (int)sizeof(T));
     }
-    #pragma unroll
-    for (int c = 0; c < 8; ++c) if (c < nrhs) part[(sl * SOLVE_ROWS + rl) * 8 + c] = acc[c];
-    __syncthreads();
-    for (int e = threadIdx.x; e < nr * nrhs; e += blockDim.x) {
-      const int r = e % nr, c = e / nr;
-      double s = 0.0;
-      for (int q = 0; q < nsl; ++q) s += part[(q * SOLVE_ROWS + r) * 8 + c];
-      ybuf[r0 + r + (int64_t)c * ld] = T(s);
-    }
-  } else {
-    // rows r0.. of M^T x: a warp per output row reads column r of M
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int rl = wid; rl < nr; rl += nw) {
-      const int r = r0 + rl;
-      const T* mcol = Mx + (int64_t)r * ld;
-      double acc[8];
+  };
+  if (s.vec) put(IntC<16 / (int)sizeof(T)>{}, BR * (int)sizeof(T) / 16);
+  else put(IntC<1>{}, BR);
+}
+
+// One warp's MI row tiles of a box: k quads q with 4 q < kv, at most KQ of
+// them; element (row tile i, quad q) of this lane at a0[i si + q sq].  Every 16
+// products start from zero and are added to the sum: 16 + k / 16 roundings
+// deep instead of k (the residual of a refinement rests on it).
+template <int MI, int KQ, bool FULL, typename T>
+FRANK_D void mv_box(const T* a0, int si, int sq, const double* x, int kv, double (&tot)[8][2]) {
+  const int t = threadIdx.x & 3;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-#pragma unroll 4
-      for (int t = lane; t < b; t += 32) {
-        const double mv = double(mcol[t]);
+  for (int q0 = 0; q0 < KQ; q0 += 4) {
+    if (!FULL && 4 * q0 >= kv) return;
+    double acc[MI][2];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < nrhs) acc[c] += mv * xs[t + c * b];
-      }
-      #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (c >= nrhs) break;
-        const double sum = warp_sum(acc[c]);
-        if (lane == 0) ybuf[(which == 3 ? perm[r] : r) + (int64_t)c * ld] = T(sum);
-      }
+    for (int i = 0; i < MI; ++i) acc[i][0] = acc[i][1] = 0.0;
+#pragma unroll
+    for (int q = q0; q < (q0 + 4 < KQ ? q0 + 4 : KQ); ++q) {
+      if (!FULL && 4 * q >= kv) break;
+      const double xv = FULL || 4 * q + t < kv ? x[4 * q + t] : 0.0;
+#pragma unroll
+      for (int i = 0; i < MI; ++i) dmma884(acc[i], double(a0[i * si + q * sq]), xv);
     }
+#pragma unroll
+    for (int i = 0; i < MI; ++i) { tot[i][0] += acc[i][0]; tot[i][1] += acc[i][1]; }
   }
 }
 
-// z_j -= Blk y_i for every target j of step i, with the solved block y_i in
-// ybuf, then z_i = y_i:
+template <int MI, int KQ, typename T>
+FRANK_D void mv_box(const T* a0, int si, int sq, const double* x, int kv, double (&tot)[8][2]) {
+  if (kv >= 4 * KQ) mv_box<MI, KQ, true>(a0, si, sq, x, kv, tot);
+  else mv_box<MI, KQ, false>(a0, si, sq, x, kv, tot);
+}
+
+// Runs the segments in order; prefetched() is called by all threads once the
+// first boxes are on their way (it stages X), sink(row, rhs, value) gets the
+// last segment's results, each from one thread.  red: 1024 doubles.
+template <typename T, typename Pre, typename Sink>
+FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double* red, Pre prefetched, Sink sink) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  int total = 0;
+  for (int p = 0; p < np; ++p)
+    total += ((seg[p].m() + seg[p].tm() - 1) / seg[p].tm()) * ((seg[p].k() + seg[p].tk() - 1) / seg[p].tk());
+  int ip = 0, im = 0, ik = 0, islot = 0, issued = 0;
+  auto issue = [&]() {
+    if (issued < total) {
+      const MvSeg<T>& s = seg[ip];
+      T* slot = ring + islot * MV_BOX;
+      if (s.kind == MV_T) mv_issue_box<256, 16, 260, true>(s, ik * 256, im * 16, slot);
+      else if (s.kind == MV_N512) mv_issue_box<512, 8, 520, false>(s, im * 512, ik * 8, slot);
+      else if (s.kind == MV_N64) mv_issue_box<64, 56, 72, false>(s, im * 64, ik * 56, slot);
+      else mv_issue_box<16, 128, 24, false>(s, im * 16, ik * 128, slot);
+      ++issued;
+      if (++islot == ns) islot = 0;
+      if (++ik * s.tk() >= s.k()) {
+        ik = 0;
+        if (++im * s.tm() >= s.m()) { im = 0; ++ip; }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < ns - 1; ++i) issue();
+  prefetched();
+  int p = 0, mb = 0, kb = 0, slot_i = 0;
+  int cur = -1, kind = 0, m = 0, k = 0, tk = 0, tm = 0;
+  const double* X0 = nullptr;
+  double tot[8][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) tot[i][0] = tot[i][1] = 0.0;
+  for (int b = 0; b < total; ++b) {
+    if (ns == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    issue();
+    if (p != cur) {
+      const MvSeg<T>& s = seg[p];
+      cur = p; kind = s.kind; m = s.m(); k = s.k(); tk = s.tk(); tm = s.tm();
+      X0 = s.X + (int64_t)min(g, nr - 1) * s.ldx;
+    }
+    const T* slot = ring + slot_i * MV_BOX;
+    const int m0 = mb * tm, kv = min(tk, k - kb * tk);
+    const double* X = X0 + kb * tk;
+    if (kind == MV_T) mv_box<2, 8>(slot + g * 260 + wid * 32 + t, 8 * 260, 4, X + wid * 32, kv - wid * 32, tot);
+    else if (kind == MV_N16) mv_box<2, 4>(slot + g + (wid * 16 + t) * 24, 8, 96, X + wid * 16, kv - wid * 16, tot);
+    else if (kind == MV_N64) {
+      if (m0 + wid * 8 < m) mv_box<1, 14>(slot + wid * 8 + g + t * 72, 8, 288, X, kv, tot);
+    } else if (m0 + wid * 64 < m) mv_box<8, 2>(slot + wid * 64 + g + t * 520, 8, 2080, X, kv, tot);
+    if (++slot_i == ns) slot_i = 0;
+    if (++kb * tk < k) continue;
+    auto deliver = [&](int row, int c, double v) {
+      if (row >= m || c >= nr) return;
+      if (p == np - 1) sink(row, c, v);
+      else seg[p].out[row + (int64_t)c * seg[p].ldo] = v;
+    };
+    if (kind == MV_T || kind == MV_N16) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) red[wid * 128 + 8 * i + g + (2 * t + h) * 16] = tot[i][h];
+      __syncthreads();
+      if (threadIdx.x < 128) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += red[w * 128 + threadIdx.x];
+        deliver(m0 + (threadIdx.x & 15), threadIdx.x >> 4, v);
+      }
+    } else {
+      const int per = kind == MV_N64 ? 1 : 8;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < per)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) deliver(m0 + (wid * per + i) * 8 + g, 2 * t + h, tot[i][h]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tot[i][0] = tot[i][1] = 0.0;
+    kb = 0;
+    if (++mb * tm >= m) { mb = 0; ++p; }
+  }
+}
+
+FRANK_HD int sv_ld(int m) { return ((m + 15) & ~15) + 4; }   // = 4 mod 16: conflict-free right-hand-side fragments
+
+// dynamic shared memory of the solve and matvec kernels: the partial tiles,
+// x or t2 (bmax x nrhs; kcap <= bmax), t1 (kcap x nrhs) and the ring
+template <typename T>
+FRANK_HD size_t solve_smem(int bmax, int kcap, int nrhs, int ns) {
+  return (1024 + ((size_t)sv_ld(bmax) + sv_ld(kcap)) * nrhs) * sizeof(double) + (size_t)ns * MV_BOX * sizeof(T);
+}
+
+// Boxes in the ring: three (two ahead), or two where that lets two CTAs share an SM or fits at all.
+template <typename T>
+inline int solve_ring(int bmax, int kcap, int nrhs) {
+  const size_t two = solve_smem<T>(bmax, kcap, nrhs, 2) + 1024, three = solve_smem<T>(bmax, kcap, nrhs, 3) + 1024;
+  const size_t sm = SMEM_OPTIN_MAX + 1024;
+  return three > sm || (2 * two <= sm && 2 * three > sm) ? 2 : 3;
+}
+
+template <typename T>
+struct MvShared {
+  double *red, *x, *t1;
+  T* ring;
+  FRANK_D MvShared(double* p, int bmax, int kcap, int nrhs) {
+    red = p;
+    x = red + 1024;
+    t1 = x + (size_t)sv_ld(bmax) * nrhs;
+    ring = reinterpret_cast<T*>(t1 + (size_t)sv_ld(kcap) * nrhs);
+  }
+};
+
+// y = M * P(z_i) (which 0: Linv, permuted input; 1: Uinv),
+// y = M^T z_i (2: Uinv^T), or y = P^T (Linv^T z_i) (3), into ybuf (ld bmax).
+// grid = ceil(b / SOLVE_ROWS) CTAs, SOLVE_ROWS rows each, from the part of M
+// that is not zero.
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag(BlrView<T> A, FactorWs<T> ws, int i, const T* z,
+                                                              int64_t ldz, int nrhs, int which, T* ybuf, int ns) {
+  extern __shared__ __align__(16) double ssm[];
+  __shared__ MvSeg<T> seg;
+  const int b = A.bs(i), ld = A.bmax, ldx = sv_ld(b);
+  const int64_t o = A.off[i];
+  const int r0 = blockIdx.x * SOLVE_ROWS, nr = min(SOLVE_ROWS, b - r0);
+  if (nr <= 0) return;
+  MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
+  const T* Mx = (which == 0 || which == 3) ? ws.Linv + (int64_t)i * ld * ld : ws.Uinv + (int64_t)i * ld * ld;
+  const int* perm = ws.perm + (int64_t)i * ld;
+  const bool lower = which == 0 || which == 2;      // the operator's triangle
+  const int k0 = lower ? 0 : r0, k1 = lower ? min(b, r0 + SOLVE_ROWS) : b;
+  if (threadIdx.x == 0) {
+    if (which <= 1) seg.set(Mx + r0 + (int64_t)k0 * ld, ld, nr, k1 - k0, MV_N16, sm.x, ldx, nullptr, 0);
+    else seg.set(Mx + k0 + (int64_t)r0 * ld, ld, k1 - k0, nr, MV_T, sm.x, ldx, nullptr, 0);
+  }
+  __syncthreads();
+  mv_run(
+      &seg, 1, nrhs, sm.ring, ns, sm.red,
+      [&]() {
+        for (int r = k0 + threadIdx.x; r < k1; r += SOLVE_THREADS) {
+          const T* src = z + o + (which == 0 ? perm[r] : r);
+#pragma unroll 8
+          for (int c = 0; c < nrhs; ++c) sm.x[r - k0 + c * ldx] = double(src[(int64_t)c * ldz]);
+        }
+      },
+      [&](int r, int c, double v) { ybuf[(which == 3 ? perm[r0 + r] : r0 + r) + (int64_t)c * ld] = T(v); });
+}
+
+// Step i's updates z_j -= Blk y_i of every target j, with the solved block y_i
+// in ybuf:
 // mode 0: targets j > i using blocks (j, i)        [forward, L]
 // mode 1: targets j < i using blocks (j, i)        [backward, U]
 // mode 2: targets j > i using blocks (i, j)^T      [transpose forward, U^T]
 // mode 3: targets j < i using blocks (i, j)^T      [transpose backward, L^T]
-// One thread-block cluster of SC_CLUSTER CTAs per target j (grid =
-// max(ntarget, 1) clusters; the first cluster also copies y_i into z_i).  For a low-rank block U S V^T the cluster's CTAs split the
-// work three ways and exchange the pieces through distributed shared memory:
-//   A: CTA q contracts columns [q cw, (q+1) cw) of the inner basis with y_i
-//      (t1 = inner^T y, one warp per column);
-//   B: after a cluster barrier every CTA gathers all of t1, then CTA q forms
-//      rows [q cw, (q+1) cw) of t2 = S t1 (S^T t1 when transposing);
-//   C: after a second barrier every CTA gathers all of t2 and updates its
-//      row tile z_j(tile) -= outer(tile, :) t2.
-// A third barrier keeps every CTA's shared memory alive until the gathers of
-// the others are done.  A dense block is applied tile by tile in phase C.
-// Every CTA reaches the three barriers.
-constexpr int SC_CLUSTER = 8;
-constexpr int SMEM_OPTIN_MAX = 227 * 1024;   // dynamic shared memory a CTA may opt into
-
-// Rows of t2 per CTA at most (the stride of the phase-B partial sums).
-FRANK_HD int solve_cl_rows(int kcap) { return (kcap + SC_CLUSTER - 1) / SC_CLUSTER; }
-
-// Doubles of the partial-sum area: phase B (SOLVE_THREADS / 32 warps x
-// solve_cl_rows x 8) and phase C (SOLVE_THREADS / 64 splits x 64 rows x 8).
-FRANK_HD int64_t solve_cl_part(int kcap) {
-  const int64_t b = (int64_t)(SOLVE_THREADS / 32) * solve_cl_rows(kcap) * 8, c = (int64_t)(SOLVE_THREADS / 64) * 64 * 8;
-  return b > c ? b : c;
-}
-
-// dynamic shared memory: ys (bmax x nrhs), t1, t2 (kcap x nrhs each) and the
-// partial sums
-FRANK_HD size_t solve_scatter_cl_smem(int bmax, int kcap, int nrhs) {
-  return ((size_t)bmax * nrhs + 2 * (size_t)kcap * nrhs + (size_t)solve_cl_part(kcap)) * sizeof(double);
-}
-
+// in two launches over all SMs: t1 = inner^T y by 16 columns of the inner
+// basis per CTA, then t2 = S t1 and 64 rows of the target per CTA (t2 formed by
+// each of them: it is a small part of the reads, and a third launch would cost
+// more).  One CTA per target, or a cluster of eight exchanging pieces through
+// distributed shared memory, took 41 and 36 us a step at n = 16384, b = 512.
 template <typename T>
-__global__ void __cluster_dims__(SC_CLUSTER, 1, 1) __launch_bounds__(SOLVE_THREADS)
-    k_solve_scatter_cl(BlrView<T> A, int i, T* z, int64_t ldz, int nrhs, int mode, const T* ybuf, int ntarget) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ double csm[];
-  const int ld = A.bmax;
-  const int bi = A.bs(i);
-  const int64_t oi = A.off[i];
-  const int q = (int)cl.block_rank();
-  const int t = blockIdx.x / SC_CLUSTER;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double* ys = csm;
-  double* t1 = ys + (int64_t)A.bmax * nrhs;
-  double* t2 = t1 + (int64_t)A.kcap * nrhs;
-  double* part = t2 + (int64_t)A.kcap * nrhs;   // partial sums (solve_cl_part doubles)
-  const int pstride = solve_cl_rows(A.kcap);
-  // y_i -> z_i, one row tile per CTA of the first cluster
-  if (t == 0) {
-    const int tl = (bi + SC_CLUSTER - 1) / SC_CLUSTER, r0 = q * tl, r1 = min(bi, r0 + tl);
-    for (int e = threadIdx.x; e < (r1 - r0) * nrhs; e += blockDim.x) {
-      const int r = r0 + e % (r1 - r0), c = e / (r1 - r0);
-      z[oi + r + (int64_t)c * ldz] = ybuf[r + (int64_t)c * ld];
-    }
-  }
-  const bool active = t < ntarget;
-  const bool tr = (mode >= 2);
-  int j = 0, bj = 0, r = 0, bi_ = 0, bj_ = 0;
-  bool lr = false;
-  if (active) {
+struct SvTarget {
+  int j, bj, gi, gj, r;     // target, its rows, stored block, rank (-1: dense)
+  FRANK_D SvTarget(const BlrView<T>& A, int i, int t, int mode) {
     j = (mode == 0 || mode == 2) ? i + 1 + t : t;
     bj = A.bs(j);
-    bi_ = tr ? i : j;
-    bj_ = tr ? j : i;
-    lr = A.is_lr(bi_, bj_);
-    r = lr ? A.rank[bi_ * A.nb + bj_] : 0;
+    gi = mode >= 2 ? i : j;
+    gj = mode >= 2 ? j : i;
+    r = A.is_lr(gi, gj) ? A.rank[gi * A.nb + gj] : -1;
   }
-  const int cw = (r + SC_CLUSTER - 1) / SC_CLUSTER;   // columns of t1 / rows of t2 per CTA
-  const int c0 = min(r, q * cw), c1 = min(r, c0 + cw);
-  if (active) {
-    for (int e = threadIdx.x; e < bi * nrhs; e += blockDim.x) {
-      const int rr = e % bi, c = e / bi;
-      ys[e] = double(ybuf[rr + (int64_t)c * ld]);
+};
+
+template <typename T>
+FRANK_D void sv_stage(double* x, int ldx, const T* src, int64_t ld, int n, int nrhs) {
+  for (int r = threadIdx.x; r < n; r += SOLVE_THREADS)
+#pragma unroll 8
+    for (int c = 0; c < nrhs; ++c) x[r + c * ldx] = double(src[r + (int64_t)c * ld]);
+}
+
+// grid (ceil(kcap / 16), targets); tbuf: kcap x 8 per target
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_inner(BlrView<T> A, int i, int nrhs, int mode, const T* ybuf,
+                                                               double* tbuf, int ns) {
+  extern __shared__ __align__(16) double ssm[];
+  __shared__ MvSeg<T> seg;
+  const SvTarget<T> tg(A, i, blockIdx.y, mode);
+  const int c0 = blockIdx.x * 16, ld = A.bmax, bi = A.bs(i), ldx = sv_ld(bi);
+  if (c0 >= tg.r) return;
+  MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
+  if (threadIdx.x == 0)
+    seg.set((mode >= 2 ? A.u(tg.gi, tg.gj) : A.vt(tg.gi, tg.gj)) + (int64_t)c0 * ld, ld, bi, min(16, tg.r - c0), MV_T,
+            sm.x, ldx, nullptr, 0);
+  __syncthreads();
+  double* t1 = tbuf + (int64_t)blockIdx.y * A.kcap * SV_NR + c0;
+  mv_run(&seg, 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldx, ybuf, ld, bi, nrhs); },
+         [&](int r, int c, double v) { t1[r + (int64_t)c * A.kcap] = v; });
+}
+
+// grid (ceil(bmax / 64), max(targets, 1)); the first target's CTAs also copy y_i into z_i
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_outer(BlrView<T> A, int i, T* z, int64_t ldz, int nrhs,
+                                                               int mode, const T* ybuf, const double* tbuf,
+                                                               int ntarget, int ns) {
+  extern __shared__ __align__(16) double ssm[];
+  __shared__ MvSeg<T> seg[2];
+  const int ld = A.bmax, bi = A.bs(i), r0 = blockIdx.x * 64;
+  if (blockIdx.y == 0)
+    for (int r = r0 + (threadIdx.x & 63); r < min(bi, r0 + 64); r += 64)
+      for (int c = threadIdx.x >> 6; c < nrhs; c += SOLVE_THREADS / 64)
+        z[A.off[i] + r + (int64_t)c * ldz] = ybuf[r + (int64_t)c * ld];
+  if ((int)blockIdx.y >= ntarget) return;
+  const SvTarget<T> tg(A, i, blockIdx.y, mode);
+  const bool lr = tg.r >= 0, tr = mode >= 2;
+  const int rows = min(64, tg.bj - r0);
+  if (rows <= 0 || tg.r == 0) return;
+  MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
+  const int k = lr ? tg.r : bi, ldk = sv_ld(k);
+  double* x = lr ? sm.t1 : sm.x;
+  if (threadIdx.x == 0) {
+    if (lr) {
+      seg[0].set(A.s(tg.gi, tg.gj), A.kcap, k, k, tr ? MV_T : MV_N64, x, ldk, sm.x, ldk);
+      seg[1].set((tr ? A.vt(tg.gi, tg.gj) : A.u(tg.gi, tg.gj)) + r0, ld, rows, k, MV_N64, sm.x, ldk, nullptr, 0);
+    } else if (tr) {
+      seg[0].set(A.dense(tg.gi, tg.gj) + (int64_t)r0 * ld, ld, k, rows, MV_T, x, ldk, nullptr, 0);
+    } else {
+      seg[0].set(A.dense(tg.gi, tg.gj) + r0, ld, rows, k, MV_N64, x, ldk, nullptr, 0);
     }
   }
   __syncthreads();
-  // A: t1(c0:c1, :) = inner(:, c0:c1)^T y
-  const T* U = lr ? A.u(bi_, bj_) : nullptr;
-  const T* S = lr ? A.s(bi_, bj_) : nullptr;
-  const T* V = lr ? A.vt(bi_, bj_) : nullptr;
-  const T* inner = tr ? U : V;
-  const T* outer = tr ? V : U;
-  if (lr) {
-    for (int cc = c0 + wid; cc < c1; cc += nw) {
-      const T* col = inner + (int64_t)cc * ld;
-      double acc[8];
+  T* zj = z + A.off[tg.j] + r0;
+  mv_run(
+      seg, lr ? 2 : 1, nrhs, sm.ring, ns, sm.red,
+      [&]() {
+        if (lr) sv_stage(x, ldk, tbuf + (int64_t)blockIdx.y * A.kcap * SV_NR, A.kcap, k, nrhs);
+        else sv_stage(x, ldk, ybuf, ld, k, nrhs);
+      },
+      [&](int r, int c, double v) {
+        T* q = zj + r + (int64_t)c * ldz;
+        *q = T(double(*q) - v);
+      });
+}
+
+// Small blocks (the inner product at most SV_DIRECT boxes): one CTA per target
+// does all of a step's update in one launch, reading the factors straight into
+// mma fragments.  The chain of a step is then too short for the ring's set-up
+// and a third launch to pay: n = 256 with b = 32 takes 0.93 ms for the
+// factorization and refinement, 1.08 through the ring; n = 2048 with b = 256
+// and rank 16 3.49 and 3.61.  At n = 16384, b = 512 this form takes 13.0 ms
+// for a refinement that takes 7.4 through the ring.
+constexpr int SV_DIRECT = 4;
+constexpr int SD_ROWS = 32;      // rows of the diagonal solve per CTA
+FRANK_HD bool solve_direct(int bmax, int rank) { return ((rank + 15) / 16) * ((bmax + 255) / 256) <= SV_DIRECT; }
+
+// One warp's 32 x 8 tile of A X over k0 <= kk < k1: element (i, kk) of A at
+// A[i sai + kk sak], X k x nr (shared, ldx); sums as in mv_box.
+template <typename T>
+FRANK_D void sd_tile(int m, int nr, int k0, int k1, const T* A, int64_t sai, int64_t sak, const double* X, int ldx,
+                     int i0, double (&tot)[4][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const T* pa[4];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-#pragma unroll 4
-      for (int x = lane; x < bi; x += 32) {
-        const double v = double(col[x]);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < nrhs) acc[c] += v * ys[x + c * bi];
-      }
-      #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (c >= nrhs) break;
-        const double sum = warp_sum(acc[c]);
-        if (lane == 0) t1[cc + c * r] = sum;
-      }
-    }
+  for (int i = 0; i < 4; ++i) {
+    pa[i] = A + (int64_t)min(i0 + 8 * i + g, m - 1) * sai + (int64_t)(k0 + t) * sak;
+    tot[i][0] = tot[i][1] = 0.0;
   }
-  cl.sync();
-  // B: gather t1, then t2(c0:c1, :) = S(c0:c1, :) t1 (warps split the inner index)
-  if (lr) {
-    for (int qq = 0; qq < SC_CLUSTER; ++qq) {
-      if (qq == q) continue;
-      const int a0 = min(r, qq * cw), a1 = min(r, a0 + cw);
-      const double* rt1 = cl.map_shared_rank(t1, qq);
-      for (int e = threadIdx.x; e < (a1 - a0) * nrhs; e += blockDim.x) {
-        const int c = a0 + e % (a1 - a0), h = e / (a1 - a0);
-        t1[c + h * r] = rt1[c + h * r];
-      }
+  const double* px = X + (int64_t)min(g, nr - 1) * ldx + k0 + t;
+  for (int kk = k0; kk < k1; kk += 16) {
+    double a[4][4], x[4], acc[4][2];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const bool in = kk + 4 * v + t < k1;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i][v] = in ? double(pa[i][4 * v * sak]) : 0.0;
+      x[v] = in ? px[4 * v] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { pa[i] += 16 * sak; acc[i][0] = acc[i][1] = 0.0; }
+    px += 16;
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dmma884(acc[i], a[i][v], x[v]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { tot[i][0] += acc[i][0]; tot[i][1] += acc[i][1]; }
+  }
+}
+
+// out (m x nr in shared memory, ldo) = A X, X k x nr.  Tiles of 32 rows; with
+// fewer tiles than warps the inner dimension is cut into slices, summed in
+// order.  red: 8 x 256 doubles.  Ends with a barrier.
+template <typename T>
+FRANK_D void sd_mv(int m, int nr, int k, const T* A, int64_t sai, int64_t sak, const double* X, int ldx, double* out,
+                   int ldo, double* red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int mt = (m + 31) / 32, sl = mt >= 5 ? 1 : (mt >= 3 ? 2 : (mt == 2 ? 4 : 8));
+  const int kc = ((k + sl - 1) / sl + 15) & ~15;
+  for (int m0 = 0; m0 < mt; m0 += 8 / sl) {
+    const int tile = m0 + wid / sl, q = wid % sl;
+    if (tile < mt) {
+      double acc[4][2];
+      const int k0 = min(k, q * kc), k1 = min(k, k0 + kc);
+      sd_tile(m, nr, k0, k1, A, sai, sak, X, ldx, tile * 32, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) red[wid * 256 + (8 * i + g) + (2 * t + h) * 32] = acc[i][h];
     }
     __syncthreads();
-    const int tw = (r + nw - 1) / nw, x0 = min(r, wid * tw), x1 = min(r, x0 + tw);
-    for (int cb = c0; cb < c1; cb += 32) {
-      const int c = cb + lane;
-      double acc[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-      if (c < c1) {
-#pragma unroll 4
-        for (int x = x0; x < x1; ++x) {
-          const double sv = tr ? double(S[x + (int64_t)c * A.kcap]) : double(S[c + (int64_t)x * A.kcap]);
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += sv * t1[x + h * r];
-        }
-      }
-      if (c < c1)
-        #pragma unroll
-        for (int h = 0; h < 8; ++h) if (h < nrhs) part[((int64_t)wid * pstride + (c - c0)) * 8 + h] = acc[h];
+    const int rows = min(m - m0 * 32, (8 / sl) * 32);
+    for (int e = threadIdx.x; e < rows * nr; e += SOLVE_THREADS) {
+      const int r = e % rows, c = e / rows;
+      double v = 0.0;
+      for (int s = 0; s < sl; ++s) v += red[((r >> 5) * sl + s) * 256 + (r & 31) + c * 32];
+      out[m0 * 32 + r + c * ldo] = v;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < (c1 - c0) * nrhs; e += blockDim.x) {
-      const int cl_ = e % (c1 - c0), h = e / (c1 - c0);
-      double sum = 0.0;
-      for (int w = 0; w < nw; ++w) sum += part[((int64_t)w * pstride + cl_) * 8 + h];
-      t2[c0 + cl_ + h * r] = sum;
-    }
   }
-  cl.sync();
-  // C: gather t2, then the row tile of the target
-  if (lr) {
-    for (int qq = 0; qq < SC_CLUSTER; ++qq) {
-      if (qq == q) continue;
-      const int a0 = min(r, qq * cw), a1 = min(r, a0 + cw);
-      const double* rt2 = cl.map_shared_rank(t2, qq);
-      for (int e = threadIdx.x; e < (a1 - a0) * nrhs; e += blockDim.x) {
-        const int c = a0 + e % (a1 - a0), h = e / (a1 - a0);
-        t2[c + h * r] = rt2[c + h * r];
-      }
-    }
+}
+
+// dynamic shared memory: partial tiles, x (bmax), t1 and t2 (kcap; the diagonal solve's SD_ROWS rows) x nrhs
+FRANK_HD size_t solve_direct_smem(int bmax, int kcap, int nrhs) {
+  return (8 * 256 + ((size_t)sv_ld(bmax) + 2 * (size_t)sv_ld(kcap) + SD_ROWS) * nrhs) * sizeof(double);
+}
+
+// k_solve_diag, SD_ROWS rows per CTA
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag_direct(BlrView<T> A, FactorWs<T> ws, int i, const T* z,
+                                                                     int64_t ldz, int nrhs, int which, T* ybuf) {
+  extern __shared__ __align__(16) double ssm[];
+  const int b = A.bs(i), ld = A.bmax, ldx = sv_ld(b);
+  const int64_t o = A.off[i];
+  const int r0 = blockIdx.x * SD_ROWS, nr = min(SD_ROWS, b - r0);
+  if (nr <= 0) return;
+  double* red = ssm;
+  double* out = red + 8 * 256;
+  double* x = out + SD_ROWS * nrhs;
+  const T* Mx = (which == 0 || which == 3) ? ws.Linv + (int64_t)i * ld * ld : ws.Uinv + (int64_t)i * ld * ld;
+  const int* perm = ws.perm + (int64_t)i * ld;
+  const bool lower = which == 0 || which == 2;      // the operator's triangle
+  const int k0 = lower ? 0 : r0, k1 = lower ? min(b, r0 + SD_ROWS) : b;
+  for (int c = threadIdx.x >> 5; c < nrhs; c += SOLVE_THREADS / 32)
+    for (int r = k0 + (threadIdx.x & 31); r < k1; r += 32)
+      x[r - k0 + c * ldx] = double(z[o + (which == 0 ? perm[r] : r) + (int64_t)c * ldz]);
+  __syncthreads();
+  if (which <= 1) sd_mv(nr, nrhs, k1 - k0, Mx + r0 + (int64_t)k0 * ld, 1, ld, x, ldx, out, SD_ROWS, red);
+  else sd_mv(nr, nrhs, k1 - k0, Mx + k0 + (int64_t)r0 * ld, ld, 1, x, ldx, out, SD_ROWS, red);
+  for (int e = threadIdx.x; e < nr * nrhs; e += SOLVE_THREADS) {
+    const int r = e % nr, c = e / nr;
+    ybuf[(which == 3 ? perm[r0 + r] : r0 + r) + (int64_t)c * ld] = T(out[r + c * SD_ROWS]);
   }
-  cl.sync();
-  if (!active) return;
-  const int64_t oj = A.off[j];
-  const int tl = (bj + SC_CLUSTER - 1) / SC_CLUSTER, row0 = q * tl, row1 = min(bj, row0 + tl);
+}
+
+// One CTA per target (grid = max(targets, 1)); the first also copies y_i into z_i
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_scatter(BlrView<T> A, int i, T* z, int64_t ldz, int nrhs,
+                                                                 int mode, const T* ybuf, int ntarget) {
+  extern __shared__ __align__(16) double ssm[];
+  const int ld = A.bmax, bi = A.bs(i), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double* red = ssm;
+  double* ys = red + 8 * 256;
+  double* t1 = ys + (size_t)sv_ld(A.bmax) * nrhs;
+  double* t2 = t1 + (size_t)sv_ld(A.kcap) * nrhs;
+  const int ldy = sv_ld(bi);
+  for (int c = wid; c < nrhs; c += SOLVE_THREADS / 32)
+    for (int r = lane; r < bi; r += 32) {
+      const T v = ybuf[r + (int64_t)c * ld];
+      ys[r + c * ldy] = double(v);
+      if (blockIdx.x == 0) z[A.off[i] + r + (int64_t)c * ldz] = v;
+    }
+  if ((int)blockIdx.x >= ntarget) return;
+  __syncthreads();
+  const SvTarget<T> tg(A, i, blockIdx.x, mode);
+  const bool tr = mode >= 2, lr = tg.r >= 0;
+  const int r = lr ? tg.r : bi, ldt = lr ? sv_ld(r) : ldy;
   if (lr) {
-    // 64 rows x (SOLVE_THREADS / 64) splits of the inner index per pass
-    const int ns = SOLVE_THREADS / 64, rl = threadIdx.x % 64, sl = threadIdx.x / 64;
-    const int xw = (r + ns - 1) / ns, x0 = min(r, sl * xw), x1 = min(r, x0 + xw);
-    for (int rb = row0; rb < row1; rb += 64) {
-      const int rr = rb + rl;
-      double acc[8];
+    const T* S = A.s(tg.gi, tg.gj);
+    sd_mv(r, nrhs, bi, tr ? A.u(tg.gi, tg.gj) : A.vt(tg.gi, tg.gj), ld, 1, ys, ldy, t1, ldt, red);
+    sd_mv(r, nrhs, r, S, tr ? A.kcap : 1, tr ? 1 : A.kcap, t1, ldt, t2, ldt, red);
+  }
+  const T* O = lr ? (tr ? A.vt(tg.gi, tg.gj) : A.u(tg.gi, tg.gj)) : A.dense(tg.gi, tg.gj);
+  const bool ot = !lr && tr;
+  T* zj = z + A.off[tg.j];
+  const int g = lane >> 2, q = lane & 3;
+  for (int i0 = wid * 32; i0 < tg.bj; i0 += SOLVE_THREADS) {
+    double acc[4][2];
+    sd_tile(tg.bj, nrhs, 0, r, O, ot ? ld : 1, ot ? 1 : ld, lr ? t2 : ys, ldt, i0, acc);
 #pragma unroll
-      for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-      if (rr < row1) {
-#pragma unroll 4
-        for (int x = x0; x < x1; ++x) {
-          const double ov = double(outer[rr + (int64_t)x * ld]);
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += ov * t2[x + h * r];
+      for (int h = 0; h < 2; ++h) {
+        const int row = i0 + 8 * a + g, c = 2 * q + h;
+        if (row < tg.bj && c < nrhs) {
+          T* p = zj + row + (int64_t)c * ldz;
+          *p = T(double(*p) - acc[a][h]);
         }
       }
-      __syncthreads();
-      #pragma unroll
-      for (int h = 0; h < 8; ++h) if (h < nrhs) part[((int64_t)sl * 64 + rl) * 8 + h] = acc[h];
-      __syncthreads();
-      for (int e = threadIdx.x; e < 64 * nrhs; e += blockDim.x) {
-        const int rl2 = e % 64, h = e / 64, row = rb + rl2;
-        if (row < row1) {
-          double sum = 0.0;
-          for (int w = 0; w < ns; ++w) sum += part[((int64_t)w * 64 + rl2) * 8 + h];
-          z[oj + row + (int64_t)h * ldz] = T(double(z[oj + row + (int64_t)h * ldz]) - sum);
-        }
-      }
-    }
-  } else {
-    const T* Dm = A.dense(bi_, bj_);
-    if (!tr) {
-      for (int rr = row0 + threadIdx.x; rr < row1; rr += blockDim.x) {
-        double acc[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-        for (int x = 0; x < bi; ++x) {
-          const double dv = double(Dm[rr + (int64_t)x * ld]);
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += dv * ys[x + h * bi];
-        }
-        #pragma unroll
-        for (int h = 0; h < 8; ++h) if (h < nrhs) z[oj + rr + (int64_t)h * ldz] = T(double(z[oj + rr + (int64_t)h * ldz]) - acc[h]);
-      }
-    } else {
-      for (int rr = row0 + wid; rr < row1; rr += nw) {
-        double acc[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-        for (int x = lane; x < bi; x += 32) {
-          const double dv = double(Dm[x + (int64_t)rr * ld]);
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += dv * ys[x + h * bi];
-        }
-        #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          if (h >= nrhs) break;
-          const double sum = warp_sum(acc[h]);
-          if (lane == 0) z[oj + rr + (int64_t)h * ldz] = T(double(z[oj + rr + (int64_t)h * ldz]) - sum);
-        }
-      }
-    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// K6: FP64 H-matvec partials: part[(i*nb + j)] = A(i,j) x_j  (bmax x nrhs each)
-// grid (nb, nb); then k_matvec_reduce sums over j in fixed order.
+// K6: FP64 H-matvec partials: part[(i*nb + j)] = A(i,j) x_j  (bmax x nrhs each),
+// or A(j,i)^T x_j when transposing.  One CTA per block, the diagonal's (dense,
+// the longest) first; k_matvec_reduce sums over j in fixed order.
 // ---------------------------------------------------------------------------
-constexpr int MV_THREADS = 256;
-
-// dynamic shared memory of k_matvec_blocks: x_j (bmax x nrhs), t1, t2 (kcap x nrhs)
-FRANK_HD size_t matvec_smem(int bmax, int kcap, int nrhs) {
-  return ((size_t)bmax * nrhs + 2 * (size_t)kcap * nrhs) * sizeof(double);
-}
-
-// Each element of the block (U, S, V or the dense block) is read once and
-// applied to all nrhs columns of x_j, which is staged in shared memory.
-static __global__ void __launch_bounds__(MV_THREADS) k_matvec_blocks(BlrView<double> H, const double* x, int64_t ldx,
-                                                              int nrhs, double* part, int transpose) {
-  // part(i, j) = A(i, j) x_j, or A(j, i)^T x_j when transposing
-  const int i = blockIdx.y, j = blockIdx.x;
-  const int nb = H.nb, ld = H.bmax;
-  const int bi = H.bs(i), bj = H.bs(j);
-  const int64_t oj = H.off[j];
+static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<double> H, const double* x, int64_t ldx,
+                                                              int nrhs, double* part, int transpose, int ns) {
+  extern __shared__ __align__(16) double ssm[];
+  __shared__ MvSeg<double> seg[3];
+  const int nb = H.nb, ld = H.bmax, i = blockIdx.x, j = (i + blockIdx.y) % nb;
+  const int bi = H.bs(i), bj = H.bs(j), ldb = sv_ld(bj);
   const int gi = transpose ? j : i, gj = transpose ? i : j;   // stored block (gi, gj)
   double* out = part + (int64_t)(i * nb + j) * ld * nrhs;
-  extern __shared__ double msm[];
-  double* xs = msm;                                  // bj x nrhs
-  double* t1 = xs + (int64_t)H.bmax * nrhs;          // r x nrhs
-  double* t2 = t1 + (int64_t)H.kcap * nrhs;          // r x nrhs
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int e = threadIdx.x; e < bj * nrhs; e += blockDim.x) {
-    const int t = e % bj, h = e / bj;
-    xs[e] = x[oj + t + (int64_t)h * ldx];
+  const bool lr = H.is_lr(gi, gj), tr = transpose != 0;
+  const int r = lr ? H.rank[gi * nb + gj] : 0, ldr = sv_ld(r);
+  const int nk = bi > 256 ? MV_N512 : MV_N64;
+  if (lr && r == 0) {
+    for (int e = threadIdx.x; e < bi * nrhs; e += SOLVE_THREADS) out[e % bi + (int64_t)(e / bi) * ld] = 0.0;
+    return;
+  }
+  MvShared<double> sm(ssm, H.bmax, H.kcap, nrhs);
+  if (threadIdx.x == 0) {
+    if (lr) {
+      seg[0].set(tr ? H.u(gi, gj) : H.vt(gi, gj), ld, bj, r, MV_T, sm.x, ldb, sm.t1, ldr);
+      seg[1].set(H.s(gi, gj), H.kcap, r, r, tr ? MV_T : MV_N64, sm.t1, ldr, sm.x, ldr);
+      seg[2].set(tr ? H.vt(gi, gj) : H.u(gi, gj), ld, bi, r, nk, sm.x, ldr, nullptr, 0);
+    } else if (tr) {
+      seg[0].set(H.dense(gi, gj), ld, bj, bi, MV_T, sm.x, ldb, nullptr, 0);
+    } else {
+      seg[0].set(H.dense(gi, gj), ld, bi, bj, nk, sm.x, ldb, nullptr, 0);
+    }
   }
   __syncthreads();
-  if (H.is_lr(gi, gj)) {
-    const int r = H.rank[gi * nb + gj];
-    const double* U = H.u(gi, gj);
-    const double* S = H.s(gi, gj);
-    const double* V = H.vt(gi, gj);
-    const double* inner = transpose ? U : V;   // length bj (rows of x_j)
-    const double* outer = transpose ? V : U;   // length bi
-    for (int c = wid; c < r; c += nw) {
-      const double* col = inner + (int64_t)c * ld;
-      double acc[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-      for (int t = lane; t < bj; t += 32) {
-        const double v = col[t];
-#pragma unroll
-        for (int h = 0; h < 8; ++h)
-          if (h < nrhs) acc[h] += v * xs[t + h * bj];
-      }
-      #pragma unroll
-      for (int h = 0; h < 8; ++h) {
-        if (h >= nrhs) break;
-        const double sum = warp_sum(acc[h]);
-        if (lane == 0) t1[c + h * r] = sum;
-      }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < r; c += blockDim.x) {
-      double acc[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-      for (int t = 0; t < r; ++t) {
-        const double sv = transpose ? S[t + (int64_t)c * H.kcap] : S[c + (int64_t)t * H.kcap];
-#pragma unroll
-        for (int h = 0; h < 8; ++h)
-          if (h < nrhs) acc[h] += sv * t1[t + h * r];
-      }
-      #pragma unroll
-      for (int h = 0; h < 8; ++h) if (h < nrhs) t2[c + h * r] = acc[h];
-    }
-    __syncthreads();
-    for (int rr = threadIdx.x; rr < bi; rr += blockDim.x) {
-      double acc[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-      for (int t = 0; t < r; ++t) {
-        const double ov = outer[rr + (int64_t)t * ld];
-#pragma unroll
-        for (int h = 0; h < 8; ++h)
-          if (h < nrhs) acc[h] += ov * t2[t + h * r];
-      }
-      #pragma unroll
-      for (int h = 0; h < 8; ++h) if (h < nrhs) out[rr + (int64_t)h * ld] = acc[h];
-    }
-  } else {
-    const double* Dm = H.dense(gi, gj);
-    if (!transpose) {
-      for (int rr = threadIdx.x; rr < bi; rr += blockDim.x) {
-        double acc[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-        for (int t = 0; t < bj; ++t) {
-          const double dv = Dm[rr + (int64_t)t * ld];
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += dv * xs[t + h * bj];
-        }
-        #pragma unroll
-        for (int h = 0; h < 8; ++h) if (h < nrhs) out[rr + (int64_t)h * ld] = acc[h];
-      }
-    } else {
-      for (int rr = wid; rr < bi; rr += nw) {
-        double acc[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) acc[h] = 0.0;
-#pragma unroll 4
-        for (int t = lane; t < bj; t += 32) {
-          const double dv = Dm[t + (int64_t)rr * ld];
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nrhs) acc[h] += dv * xs[t + h * bj];
-        }
-        #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          if (h >= nrhs) break;
-          const double sum = warp_sum(acc[h]);
-          if (lane == 0) out[rr + (int64_t)h * ld] = sum;
-        }
-      }
-    }
-  }
+  mv_run(seg, lr ? 3 : 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldb, x + H.off[j], ldx, bj, nrhs); },
+         [&](int row, int c, double v) { out[row + (int64_t)c * ld] = v; });
 }
 
 // y_i = sum_j part(i,j) (fixed order).  If b != null: y = b - A x (residual).
 static __global__ void k_matvec_reduce(BlrView<double> H, const double* part, int nrhs, const double* bvec, int64_t ldb,
                                 double* y, int64_t ldy) {
-  const int i = blockIdx.x;
+  // grid (nb, row tiles of blockDim.x, nrhs)
+  const int i = blockIdx.x, h = blockIdx.z;
   const int nb = H.nb, ld = H.bmax;
   const int bi = H.bs(i);
   const int64_t oi = H.off[i];
-  for (int e = threadIdx.x; e < bi * nrhs; e += blockDim.x) {
-    const int rr = e % bi, h = e / bi;
+  const int rr = blockIdx.y * blockDim.x + threadIdx.x;
+  if (rr >= bi) return;
+  {
     double s = 0.0;
+#pragma unroll 8
     for (int j = 0; j < nb; ++j) s += part[(int64_t)(i * nb + j) * ld * nrhs + rr + (int64_t)h * ld];
     if (bvec) s = bvec[oi + rr + (int64_t)h * ldb] - s;
     y[oi + rr + (int64_t)h * ldy] = s;
