@@ -78,7 +78,7 @@ def test_solve_and_matvec(gpu_lib, n, nb, kmax, rank, nrhs, admis, precision):
 
 
 def test_the_largest_blocks(gpu_lib):
-    n, nrhs = 2047, 9                       # blocks of 1024 and 1023, the largest accepted
+    n, nrhs = 1619, 9                       # blocks of 810 and 809, the largest accepted
     M = _matrix(n, 2, 20, 0.0, 5, eps=1e-13, max_rank=0)
     A = M.to_dense()
     X = np.random.default_rng(1).standard_normal((n, nrhs))
