@@ -347,7 +347,9 @@ int enqueue_factor(frank_blr* p, cudaStream_t s, bool timing = true) {
       const int nbands = (p->bmax + band - 1) / band;
       if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, i, EV_DENSE_NEXT, 0), sd, cudaEventRecordExternal));
       // one task per band; its CTA index picks a scratch slot (grid_dense of them)
-      k_update_dense<T><<<std::min(nbands, p->grid_dense), DUPD_THREADS, 0, sd>>>(W, ws, i, p->dupd_band, DUPD_NEXT);
+      const int next = std::min(band, dupd_next_rows<T>());
+      k_update_dense<T><<<std::min((p->bmax + next - 1) / next, p->grid_dense), DUPD_THREADS, 0, sd>>>(
+          W, ws, i, p->dupd_band, DUPD_NEXT);
       if (timing) CUDA_TRY(cudaEventRecordWithFlags(ev_at(p, i, EV_DENSE_NEXT, 1), sd, cudaEventRecordExternal));
       ++launches;
       if (sd == s) {
@@ -1807,6 +1809,7 @@ int enqueue_factor_stepwise(frank_batch* B, cudaStream_t s) {
   const int rt = (b + PANEL_TILE - 1) / PANEL_TILE;
   const int band = std::min(q->dupd_band, b);
   const int nbands = (b + band - 1) / band;
+  const int next = std::min(band, dupd_next_rows<T>()), nnext = (b + next - 1) / next;
   k_reset_b<T><<<dim3(max_nb * max_nb, 1, K), 256, 0, s>>>(S);
   for (frank_blr* p : B->plans) {
     CUDA_TRY(cudaMemsetAsync(p->err, 0, ERR_SLOTS * sizeof(int), s));
@@ -1837,7 +1840,7 @@ int enqueue_factor_stepwise(frank_batch* B, cudaStream_t s) {
     k_panel_fin_b<T><<<dim3(2 * m, rt, Kz), PANEL_THREADS, 0, s>>>(S, i);
     CUDA_TRY(cudaEventRecord(B->ev_panel[i], s));
     CUDA_TRY(cudaStreamWaitEvent(s2, B->ev_panel[i], 0));
-    k_update_dense_b<T><<<dim3(std::min(nbands, q->grid_dense), 1, Kz), DUPD_THREADS, 0, s2>>>(S, i, DUPD_NEXT);
+    k_update_dense_b<T><<<dim3(std::min(nnext, q->grid_dense), 1, Kz), DUPD_THREADS, 0, s2>>>(S, i, DUPD_NEXT);
     if ((rc = getrf_step(i + 1))) return rc;
     if (m > 1)
       k_update_dense_b<T><<<dim3((int)std::min<int64_t>((int64_t)m * m * nbands, q->grid_dense), 1, Kz), DUPD_THREADS,

@@ -1180,8 +1180,7 @@ FRANK_D void form_core(const Grp& g, const UpdOps<T>& o, int bi, int ld, double*
 template <typename T, int NT>
 FRANK_D void form_core_cta(const UpdOps<T>& o, int bi, int ld, double* Tm, double* gsm) {
   if (!o.left_dense && !o.right_dense) {
-    if (o.p * o.q <= 1024) cta_gemm_tn_dot(o.p, o.q, bi, -1.0, o.WL, ld, o.WU, ld, Tm, o.p);
-    else cta_gemm<double, NT>(o.p, o.q, bi, -1.0, o.WL, ld, true, o.WU, ld, false, 0.0, Tm, o.p, gsm);
+    cta_gemm<double, NT>(o.p, o.q, bi, -1.0, o.WL, ld, true, o.WU, ld, false, 0.0, Tm, o.p, gsm);
     return;
   }
   for (int64_t e = threadIdx.x; e < (int64_t)o.p * o.q; e += blockDim.x) {
@@ -1201,8 +1200,15 @@ FRANK_D void form_core_cta(const UpdOps<T>& o, int bi, int ld, double* Tm, doubl
 // ceil(b / band_rows) times per target and C is streamed in full rows.
 // Modes: every dense target of the step, only the next diagonal block
 // (i+1, i+1) (which the next leaf getrf waits for), or all but that block.
+// The next diagonal block is on the critical path and alone on the device, so
+// its bands are no higher than one tile of the product (dupd_next_rows): at
+// b = 256, rank 16 its launch takes 19 us, 58 in bands of 128.  Targets
+// are numbered by diagonals: in row order the diagonal blocks, usually the only
+// dense ones, met in the same few CTAs (m + 1 and the grid share factors).
 // ---------------------------------------------------------------------------
 constexpr int DUPD_THREADS = 256;
+template <typename T>
+FRANK_HD constexpr int dupd_next_rows() { return sizeof(T) == 8 ? 32 : 64; }
 constexpr int DUPD_BAND = 128;    // rows of a dense update task (default; the autotuner may change it)
 enum DenseUpdateMode { DUPD_ALL = 0, DUPD_NEXT = 1, DUPD_REST = 2 };
 
@@ -1217,7 +1223,7 @@ FRANK_D void k_update_dense_impl(BlrView<T> A, FactorWs<T> ws, int i, int band_r
   double* Tm = ws.dscratch + (int64_t)blockIdx.x * ws.dscratch_stride;
   // X (rn x q, ld ldx) in the second ld x ld half of the slot: ldx * q <= ld * ld
   T* X = reinterpret_cast<T*>(Tm + (int64_t)ld * ld);
-  const int bandr = min(band_rows, ld);
+  const int bandr = min(mode == DUPD_NEXT ? min(band_rows, dupd_next_rows<T>()) : band_rows, ld);
   const int ldx = bandr;
   const int nbands = (ld + bandr - 1) / bandr;
   // pair 0 is the next diagonal block (i+1, i+1)
@@ -1225,7 +1231,7 @@ FRANK_D void k_update_dense_impl(BlrView<T> A, FactorWs<T> ws, int i, int band_r
   for (int tsk = blockIdx.x; tsk < ntask; tsk += gridDim.x) {
     const int pair = tsk / nbands, band = tsk % nbands;
     if (mode == DUPD_REST && pair == 0) continue;
-    const int ic = i + 1 + pair / m, k = i + 1 + pair % m;
+    const int ic = i + 1 + pair % m, k = i + 1 + (pair % m + pair / m) % m;
     if (A.is_lr(ic, k)) continue;
     const int bc = A.bs(ic), bk = A.bs(k);
     const int r0 = band * bandr;
