@@ -409,7 +409,7 @@ def kernel_roofline(arm, peaks, hbm):
         ms, fl = kt[cls]["ms"], kt[cls]["flops"]
         ach = fl / (ms / 1e3) / 1e12 if ms > 0 else 0.0
         out[cls] = {"ms": ms, "achieved": ach, "unit": "TFLOP/s", "peak": peaks[pipe], "frac": ach / peaks[pipe],
-                    "bound": "compute (%s, SIMT)" % pipe}
+                    "bound": "compute (%s)" % pipe}
     for cls, key in (("solve", "solve"), ("matvec", "matvec")):
         ms, by = arm[key + "_ms"], arm[key + "_bytes"]
         ach = by / (ms / 1e3) / 1e9 if ms > 0 else 0.0
@@ -785,7 +785,7 @@ def main():
                       "source": "cuBLAS DGEMM / SGEMM (TF32 off) 8192^3 measured in this run; HBM " + hbm_src},
             "e2e": {"value": statistics.median(mx["e2e"]), "unit": "s", "fp64_value": statistics.median(fp["e2e"]),
                     "h2d_bytes_per_step": n * nrhs * 8, "d2h_bytes_per_step": n * nrhs * 8},
-            "roofline": {"kernel": "k_recompress (mixed factor)", "bound": "compute (fp64, SIMT)",
+            "roofline": {"kernel": "k_recompress (mixed factor)", "bound": "compute (fp64)",
                          "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                          "frac": achieved / peak64 if peak64 else None,
                          "peak_source": "cuBLAS FP64 GEMM 8192^3 measured in this run (FP64 is not in "

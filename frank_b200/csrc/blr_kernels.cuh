@@ -282,13 +282,14 @@ __global__ void __launch_bounds__(TRUNC_THREADS) k_truncate_lr(BlrView<double> H
 }
 
 // ---------------------------------------------------------------------------
-// K1: leaf getrf of diagonal block i with partial pivoting, FP64, one CTA
-// (512 threads).  Blocked right-looking LU (panel width 32): the panel is
+// Dense getrf with partial pivoting, FP64, one CTA (512 threads), for the entry
+// point that may not allocate (plans factor their leaves by column tiles on
+// several CTAs, k_leaf_step).  Blocked right-looking LU (panel width 32): the panel is
 // factored column by column (idamax pivot, row swap across the whole block,
 // reciprocal scaling and rank-1 update as in LAPACK dgetf2), then the row
 // block is solved with the unit-lower 32x32 triangle and the trailing matrix
 // updated by a CTA GEMM.  Writes the packed LU back into the block and the
-// pivots/permutation; the explicit inverses Linv, Uinv are formed by k_trinv.
+// pivots/permutation.
 // ---------------------------------------------------------------------------
 constexpr int GETRF_THREADS = 512;
 

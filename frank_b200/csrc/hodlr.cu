@@ -17,7 +17,8 @@
 //   per leaf    Linv, Uinv, Uinv^T (b x b), pivots.
 //
 // getrf(node) = getrf(left); U_up <- L_left^{-1} P U_up and V_low <- V_low
-// U_left^{-1} (two substitution walks in one launch); the Schur update
+// U_left^{-1} (level-parallel substitutions on the left subtree, see
+// enqueue_sub); the Schur update
 // -L_low U_up = LowRank(U_low, S', V_up), S' = -(S_low V_low)(U_up S_up)
 // (gemm.cpp:374-393), added into the right child by splitting it over the
 // child's blocks (addition.cpp:62-66): dense leaves += (U S') V, LowRank
@@ -29,8 +30,8 @@
 //
 // Pivoting: the leaves take dgetrf's partial pivoting with the interchanges
 // applied (P A = L U with P = blockdiag(P_p)); the L blocks keep their rows
-// in natural order and each substitution applies P_p to its running
-// right-hand side when it reaches leaf p, which is the same thing.  The
+// in natural order and each substitution applies P_p with leaf p's inverse,
+// which is the same thing.  The
 // reference discards the pivots (getrf.cpp:67-84); the two agree whenever
 // dgetrf does not swap rows.
 #include <cuda_runtime.h>
@@ -86,7 +87,7 @@ namespace hk {
 using blr::KernelDesc;
 using blr::kernel_eval;
 
-constexpr int HMAX_RANK = 64;   // k <= 64: two rank rows per lane in the walks
+constexpr int HMAX_RANK = 64;   // largest accepted rank
 constexpr int HMAX_LEAF = 512;  // b <= 512
 constexpr int WT = 256;         // threads of the update / matvec kernels
 constexpr int KG_P = 72;        // rsvd sample width the construction product holds (k + 5 <= 69)
@@ -523,7 +524,7 @@ struct frank_hodlr {
   double* WZ = nullptr;             // per node: W (lower block's slot) and Z (upper block's slot), U-shaped
   double* Zt = nullptr;             // per node: Zt (upper block's slot), U-shaped
   double* sub[2] = {nullptr, nullptr};   // partial products and T2 of the subtree substitutions (main, side stream)
-  cudaStream_t ps = nullptr;        // their walks, beside the factorization
+  cudaStream_t ps = nullptr;        // their substitutions, beside the factorization
   cudaEvent_t ev_pre = nullptr, ev_ps = nullptr;
   ::frank::ops::LrAddTask* tasks_d = nullptr;   // every update's additions, in launch order
   std::vector<::frank::ops::LrAddTask> tasks_h;
