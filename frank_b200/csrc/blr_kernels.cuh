@@ -1392,7 +1392,10 @@ FRANK_D int svd_core(int mu, int mv, double* Mm, int ldm, bool in_smem, const Fa
   __syncthreads();
   const int ldj = mv + k;
   double* Aj = off + (int64_t)ldj * k <= cap ? region + off : Atmp;
-  const int sweeps = g_jacobi(g, mv, k, Aj, ldj, 60, sh.flags, ldj);
+  // in shared memory eight lanes a pair (more pairs at once, fewer shuffles); in
+  // L2 a warp a pair, whose loads are whole lines
+  const int sweeps = off + (int64_t)ldj * k <= cap ? g_jacobi(g, mv, k, Aj, ldj, 60, sh.flags, ldj)
+                                                   : cta_jacobi_columns(mv, k, Aj, ldj, 60, sh.flags, ldj);
   if (sweeps < 0 && threadIdx.x == 0) atomicAdd(ws.err + ERR_JACOBI, 1);
   for (int c = threadIdx.x >> 5; c < k; c += blockDim.x >> 5) {
     double sacc = 0.0;
