@@ -803,7 +803,9 @@ def main():
                 line["hlu"] = run_hlu(131072, args.steps, max(args.warmup, 3))
             except Exception as exc:  # reported, never silently dropped
                 line["hlu"] = {"error": str(exc)}
-        if not args.no_cpu_baseline:
+        if not args.no_cpu_baseline and not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "frank_ref")):
+            line["cpu_baseline"] = {"unavailable": "oracle/_ref/frank_ref is not built (python oracle/build_ref.py)"}
+        elif not args.no_cpu_baseline:
             cores = os.cpu_count()
             t, info = run_reference_sample(3, 1, cores)
             line["cpu_baseline"] = {
