@@ -219,14 +219,16 @@ FRANK_D void dgemm_store(TC* p, double v, double alpha, double beta) {
   *p = TC(v);
 }
 
-// One pass of the CTA's (or warp group's) warps over the 8 MI x 8 NI tiles.  C is
-// read (beta != 0) with the operands, ahead of the products.
-template <int MI, int NI, typename TA, typename TB, typename TC>
+// One pass of the CTA's (or warp group's) warps over the 8 MI x 8 NI tiles.  UNIT:
+// alpha is 1 or -1 wherever beta != 0, so alpha beta C is exact as the
+// accumulators' start and C is read with the operands, ahead of the products;
+// any other alpha (0 among them) goes without, and C is added at the end.
+template <int MI, int NI, bool UNIT = true, typename TA, typename TB, typename TC>
 FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, const TA* A, int64_t sai, int64_t sak,
                          const TB* B, int64_t sbj, int64_t sbk, double beta, TC* C, int64_t ldc) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tm = (m + 8 * MI - 1) / (8 * MI), tn = (n + 8 * NI - 1) / (8 * NI);
-  const double ba = beta / alpha;       // +-1 where C is updated
+  const double ba = alpha < 0.0 ? -beta : beta;
   for (int tile = wid; tile < tm * tn; tile += nw) {
     const int i0 = (tile % tm) * 8 * MI, j0 = (tile / tm) * 8 * NI;
     double acc[MI][NI][2];
@@ -237,7 +239,7 @@ FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, con
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int r = i0 + 8 * i + g, c = j0 + 8 * j + 2 * t + h;
-          acc[i][j][h] = (beta != 0.0 && r < m && c < n) ? ba * double(C[r + (int64_t)c * ldc]) : 0.0;
+          acc[i][j][h] = (UNIT && beta != 0.0 && r < m && c < n) ? ba * double(C[r + (int64_t)c * ldc]) : 0.0;
         }
     warp_dgemm_acc<MI, NI, true>(m, n, 0, k, A, sai, sak, B, sbj, sbk, i0, j0, acc);
 #pragma unroll
@@ -247,8 +249,9 @@ FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, con
 #pragma unroll
       for (int j = 0; j < NI; ++j) {
         const int c = j0 + 8 * j + 2 * t;
-        if (c < n) C[r + (int64_t)c * ldc] = TC(alpha * acc[i][j][0]);
-        if (c + 1 < n) C[r + (int64_t)(c + 1) * ldc] = TC(alpha * acc[i][j][1]);
+        TC* p = C + r + (int64_t)c * ldc;
+        if (c < n) dgemm_store(p, acc[i][j][0], alpha, UNIT ? 0.0 : beta);
+        if (c + 1 < n) dgemm_store(p + ldc, acc[i][j][1], alpha, UNIT ? 0.0 : beta);
       }
     }
   }
@@ -298,7 +301,9 @@ static __device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha,
   };
   const int c42 = cost(4, 2), c22 = cost(2, 2), c11 = cost(1, 1);
   const int best = min(c42, min(c22, c11));
-  if (best == c42)
+  if (beta != 0.0 && fabs(alpha) != 1.0)
+    warps_dgemm<4, 2, false>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
+  else if (best == c42)
     warps_dgemm<4, 2>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
   else if (best == c22)
     warps_dgemm<2, 2>(wid, nw, m, n, k, alpha, A, sai, sak, B, sbj, sbk, beta, C, ldc);
