@@ -816,9 +816,9 @@ int check_block(const frank_hodlr* h, int l, int c) {
 }
 
 // Buffers of the solves and matvecs: partial products and T2 of a level, and a
-// chunk counter per block and column group (zeroed here; every launch leaves
-// them zero).
-int ensure_mv(frank_hodlr* h, int nrhs) {
+// chunk counter per block and column group (zeroed here, on the stream that the
+// launches go to; every launch leaves them zero).
+int ensure_mv(frank_hodlr* h, int nrhs, cudaStream_t s) {
   const int64_t need = sub_part(h, 1, nrhs) + sub_t2(h, 1, nrhs);
   const int64_t groups = (nrhs + hk::HC - 1) / hk::HC;
   if (need > h->mv_part_cap) {
@@ -833,7 +833,7 @@ int ensure_mv(frank_hodlr* h, int nrhs) {
     h->mv_counter = nullptr;
     h->mv_groups = 0;
     H_TRY(dalloc(&h->mv_counter, (size_t)(groups * h->P)));
-    H_TRY(cudaMemset(h->mv_counter, 0, sizeof(int) * groups * h->P));
+    H_TRY(cudaMemsetAsync(h->mv_counter, 0, sizeof(int) * groups * h->P, s));
     h->mv_groups = groups;
   }
   return FRANK_OK;
@@ -841,7 +841,7 @@ int ensure_mv(frank_hodlr* h, int nrhs) {
 
 // y = A_H x (FP64), stream-ordered.
 int enqueue_matvec(frank_hodlr* h, const double* x, int64_t ldx, double* y, int64_t ldy, int nrhs, cudaStream_t s) {
-  int rc = ensure_mv(h, nrhs);
+  int rc = ensure_mv(h, nrhs, s);
   if (rc) return rc;
   const hk::HJob j{3, x, 1, ldx, y, 1, ldy, x, ldx};
   enqueue_sub(h, view(h, false), 0, 0, 1, j, j, nrhs, h->mv_part, h->mv_counter, s);
@@ -851,7 +851,7 @@ int enqueue_matvec(frank_hodlr* h, const double* x, int64_t ldx, double* y, int6
 
 // passes: 1 = forward (L with the pivots), 2 = backward (U), 3 = both.
 int enqueue_solve(frank_hodlr* h, double* d_b, int64_t ldb, int nrhs, cudaStream_t s, int passes = 3) {
-  int rc = ensure_mv(h, nrhs);
+  int rc = ensure_mv(h, nrhs, s);
   if (rc) return rc;
   for (int pass = 0; pass < 2; ++pass) {
     if (!(passes & (1 << pass))) continue;
@@ -944,6 +944,7 @@ int frank_hodlr_create(int64_t n, int leaf, int rank, frank_hodlr** out) {
   A(cudaMemset(h->U0, 0, sizeof(double) * nk));
   A(cudaMemset(h->V0, 0, sizeof(double) * nk));
   A(cudaMemset(h->S0, 0, sizeof(double) * sk));
+  A(cudaStreamSynchronize(cudaStreamLegacy));   // calls may come on non-blocking streams
   A(cudaFuncSetAttribute(blr::k_leaf_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(blr::k_leaf_final<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, blr::LEAF_SMEM_MAX));
   A(cudaFuncSetAttribute(hk::k_h_t, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::H_TSMEM));
