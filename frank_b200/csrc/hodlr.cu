@@ -672,13 +672,13 @@ int64_t sub_t2(const frank_hodlr* h, int jobs, int ncols) { return (int64_t)h->P
 
 // One or two substitutions (hk::HJob) on the subtree (l0, c0), or the H-matvec
 // (mode 3, the whole tree): the leaves, then the levels from the bottom up.
-void enqueue_sub(frank_hodlr* h, const hk::HView& v, int l0, int c0, int njobs, const hk::HJob& j0, const hk::HJob& j1,
+// Returns the number of launches.
+int enqueue_sub(frank_hodlr* h, const hk::HView& v, int l0, int c0, int njobs, const hk::HJob& j0, const hk::HJob& j1,
                  int ncols, double* buf, int* counter, cudaStream_t s) {
   const int hl = h->L - l0, p0 = c0 << hl, groups = (ncols + hk::HC - 1) / hk::HC;
   double* t2 = buf + sub_part(h, njobs, ncols);
   hk::k_h_leaf_mm<<<dim3(1 << hl, (ncols + hk::HLC - 1) / hk::HLC, njobs), hk::WT, 0, s>>>(v, leaf_factors(h), j0, j1,
                                                                                           p0, ncols);
-  ++h->launches;
   for (int l = h->L; l > l0; --l) {
     const int64_t sl = s_of(h, l);
     const int first = c0 << (l - l0);
@@ -687,8 +687,8 @@ void enqueue_sub(frank_hodlr* h, const hk::HView& v, int l0, int c0, int njobs, 
                                                                                      buf, t2, counter);
     hk::k_h_u<<<dim3((unsigned)((sl + hk::WT - 1) / hk::WT), nodes, njobs * groups), hk::WT, 0, s>>>(
         v, h->WZ, h->Zt, j0, j1, njobs, l, first, ncols, t2);
-    h->launches += 2;
   }
+  return 1 + 2 * (h->L - l0);
 }
 
 // A substitution in place on X (col-major), read from src the first time.
@@ -717,7 +717,7 @@ void enqueue_node(frank_hodlr* h, int l, int c, cudaStream_t s) {
   const bool leaf = l + 1 == h->L;
   hk::HJob j0 = sub_job(0, Uu, 1, sc, Uu, sc), j1 = sub_job(1, Vl, k, 1, h->Wu, sc);
   if (leaf) { j1.X = Vl; j1.xrs = k; j1.ldx = 1; }
-  enqueue_sub(h, v, l + 1, 2 * c, 2, j0, j1, k, h->sub[0], h->counter, s);
+  h->launches += enqueue_sub(h, v, l + 1, 2 * c, 2, j0, j1, k, h->sub[0], h->counter, s);
   if (!leaf) {
     hk::k_h_transpose<<<dim3((unsigned)((sc + 31) / 32), (k + 31) / 32), hk::WT, 0, s>>>(sc, k, h->Wu, Vl);
     ++h->launches;
@@ -726,7 +726,7 @@ void enqueue_node(frank_hodlr* h, int l, int c, cudaStream_t s) {
   cudaEventRecord(h->ev_pre, s);
   cudaStreamWaitEvent(h->ps, h->ev_pre, 0);
   hk::HJob jz = sub_job(2, Uu, 1, sc, h->WZ + u_off(h, l + 1, up), sc);
-  enqueue_sub(h, v, l + 1, 2 * c, 1, jz, jz, k, h->sub[1], h->counter + 4 * h->P, h->ps);
+  h->launches += enqueue_sub(h, v, l + 1, 2 * c, 1, jz, jz, k, h->sub[1], h->counter + 4 * h->P, h->ps);
   // S' = -(S_low V_low)(U_up S_up), one k x k slot per internal node
   double* Sp = h->Sp + ((int64_t)(1 << l) - 1 + c) * k * k;
   hk::k_h_core<<<hk::h_nch(sc), hk::WT, hk::H_TSMEM, s>>>(sc, k, Vl, Uu, h->S + s_off(h, l + 1, lo),
@@ -741,7 +741,7 @@ void enqueue_node(frank_hodlr* h, int l, int c, cudaStream_t s) {
   cudaStreamWaitEvent(h->ps, h->ev_pre, 0);
   hk::HJob jw = sub_job(0, h->U + u_off(h, l + 1, lo), 1, sc, h->WZ + u_off(h, l + 1, lo), sc);
   hk::HJob jt = sub_job(1, h->V + u_off(h, l + 1, up), k, 1, h->Zt + u_off(h, l + 1, up), sc);
-  enqueue_sub(h, v, l + 1, 2 * c + 1, 2, jw, jt, k, h->sub[1], h->counter + 4 * h->P, h->ps);
+  h->launches += enqueue_sub(h, v, l + 1, 2 * c + 1, 2, jw, jt, k, h->sub[1], h->counter + 4 * h->P, h->ps);
   cudaEventRecord(h->ev_ps, h->ps);
 }
 
