@@ -1407,10 +1407,7 @@ FRANK_D int svd_core(int mu, int mv, double* Mm, int ldm, bool in_smem, const Fa
   for (int c = threadIdx.x; c < k; c += blockDim.x) {
     const double v = sig[c];
     int pos = 0;
-    for (int d = 0; d < k; ++d) {
-      const double w = sig[d];
-      pos += (w > v) || (w == v && d < c);
-    }
+    for (int d = 0; d < k; ++d) pos += sorts_before(sig[d], d, v, c);
     ord[pos] = c;
   }
   __syncthreads();
@@ -3078,7 +3075,7 @@ static __global__ void __launch_bounds__(BUILD_THREADS) k_build_lowrank_rsvd(Blr
     for (int c = threadIdx.x; c < p; c += blockDim.x) {
       const double v = sig[c];
       int pos = 0;
-      for (int d = 0; d < p; ++d) pos += (sig[d] > v) || (sig[d] == v && d < c);
+      for (int d = 0; d < p; ++d) pos += sorts_before(sig[d], d, v, c);
       ord[pos] = c;
     }
     __syncthreads();

@@ -132,6 +132,14 @@ FRANK_D int block_argmax_abs1(double v, int idx, double* redv, int* redi, double
   return idx;
 }
 
+// Whether value w of index d stands before value v of index c in descending
+// order: ties by index and NaN first, so that the positions are a permutation
+// whatever the values (they index the columns afterwards).
+FRANK_D bool sorts_before(double w, int d, double v, int c) {
+  const bool nw = w != w, nv = v != v;
+  return nw || nv ? nw && (!nv || d < c) : w > v || (w == v && d < c);
+}
+
 // ---------------------------------------------------------------------------
 // FP64 products on the tensor pipe: mma.sync m8n8k4 (the FP64 matrix shape of
 // this chip; FP64 has no tcgen05 kind).  Its peak equals the FP64 FMA peak

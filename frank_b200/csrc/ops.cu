@@ -62,7 +62,7 @@ FRANK_D bool jacobi_svd(int m, int n, double* G, double* sig, int* ord, int* fla
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
     const double v = sig[c];
     int pos = 0;
-    for (int d = 0; d < n; ++d) pos += (sig[d] > v) || (sig[d] == v && d < c);
+    for (int d = 0; d < n; ++d) pos += sorts_before(sig[d], d, v, c);
     ord[pos] = c;
   }
   __syncthreads();
@@ -629,7 +629,7 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
   double* M = region;
   double* X1 = scratch + L.x1;
   double* Y1 = scratch + L.y1;
-  int k;
+  int k, bad = 0;
   double* Aj;
   int ldj;
   double* tau = region + ldm * mv;
@@ -649,6 +649,10 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
         M[e % ka + (e / ka) * ldm] += A.sa[e % ka + (int64_t)(e / ka) * A.ldsa];
       __syncthreads();
     }
+    // a core that is not finite has no SVD: reported like Jacobi's sweep limit, and
+    // the result is NaN (the pivoted QR passes over columns that are not numbers)
+    for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) bad |= !isfinite(M[e % mu + (e / mu) * ldm]);
+    bad = __syncthreads_or(bad);
     k = g_rrqr(all, mu, mv, M, ldm, 0.0, nsv, tau, ord, at, tau + nsv, cand);
     Aj = cand + 4 * (LR_T / 32) + (nsv + mv + 2) / 2;
     ldj = mv + k;
@@ -657,7 +661,7 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
       Aj[e] = c < mv ? rrqr_r(M, ldm, at, j, c) : (c - mv == j ? 1.0 : 0.0);
     }
     __syncthreads();
-    const int sweeps = g_jacobi(all, mv, k, Aj, ldj, 60, sh.flags, ldj);
+    const int sweeps = bad ? -1 : g_jacobi(all, mv, k, Aj, ldj, 60, sh.flags, ldj);
     if (sweeps < 0 && threadIdx.x == 0) atomicAdd(err + OPS_ERR_JACOBI, 1);
     for (int c = threadIdx.x >> 5; c < k; c += LR_T / 32) {
       double q = 0.0;
@@ -669,7 +673,7 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
     for (int c = threadIdx.x; c < k; c += blockDim.x) {
       const double v = sig[c];
       int pos = 0;
-      for (int d = 0; d < k; ++d) pos += (sig[d] > v) || (sig[d] == v && d < c);
+      for (int d = 0; d < k; ++d) pos += sorts_before(sig[d], d, v, c);
       rank_of[pos] = c;
     }
     __syncthreads();
@@ -705,7 +709,7 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
   for (int e = threadIdx.x; e < mu * (r - rk); e += blockDim.x) X1[mu * rk + e] = 0.0;
   for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
     const int i = e % r, c = e / r;
-    A.sa[i + (int64_t)c * A.ldsa] = i == c && c < k ? sig[rank_of[c]] : 0.0;
+    A.sa[i + (int64_t)c * A.ldsa] = i != c ? 0.0 : (bad ? nan("") : (c < k ? sig[rank_of[c]] : 0.0));
   }
   __syncthreads();
   {
