@@ -1071,7 +1071,7 @@ int frank_hodlr_build_kernel(frank_hodlr* h, int kernel, const double* points, i
   double *W = nullptr, *Y = nullptr, *Q = nullptr, *R = nullptr, *Z = nullptr, *U2 = nullptr, *sv = nullptr,
          *Vt2 = nullptr, *Ur = nullptr, *om = nullptr, *sc = nullptr;
   int* errd = h->err;
-  const int64_t pmax = std::min<int64_t>(k + 5, h->b);
+  const int64_t pmax = std::min<int64_t>(k + 5, n / 2);   // the widest sample: that of the largest blocks
   const size_t slab = (size_t)n * pmax;   // one level: 2^l blocks of s_l x p
   cudaError_t e = cudaSuccess;
   auto A = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
