@@ -144,6 +144,7 @@ struct HJob {
 
 constexpr int HC = 32;            // columns of X per CTA
 constexpr int HLC = 8;            // columns per CTA of the leaf step
+constexpr int HPASS = 128;        // columns of a solve or product per pass: bounds its buffers
 constexpr int H_CHUNK = 512;      // least rows per partial product
 constexpr int H_NCH = 64;         // most partial products of one block
 constexpr int H_TSMEM = 8 * HC * HC * 8;   // dynamic shared memory of the partial products
@@ -815,7 +816,7 @@ int check_block(const frank_hodlr* h, int l, int c) {
   return FRANK_OK;
 }
 
-// Buffers of the solves and matvecs: partial products and T2 of a level, and a
+// Buffers of the solves and matvecs (nrhs <= HPASS): partial products and T2 of a level, and a
 // chunk counter per block and column group (zeroed here, on the stream that the
 // launches go to; every launch leaves them zero).
 int ensure_mv(frank_hodlr* h, int nrhs, cudaStream_t s) {
@@ -841,23 +842,28 @@ int ensure_mv(frank_hodlr* h, int nrhs, cudaStream_t s) {
 
 // y = A_H x (FP64), stream-ordered.
 int enqueue_matvec(frank_hodlr* h, const double* x, int64_t ldx, double* y, int64_t ldy, int nrhs, cudaStream_t s) {
-  int rc = ensure_mv(h, nrhs, s);
+  int rc = ensure_mv(h, std::min(nrhs, hk::HPASS), s);
   if (rc) return rc;
-  const hk::HJob j{3, x, 1, ldx, y, 1, ldy, x, ldx};
-  enqueue_sub(h, view(h, false), 0, 0, 1, j, j, nrhs, h->mv_part, h->mv_counter, s);
+  for (int c = 0; c < nrhs; c += hk::HPASS) {
+    const double* xc = x + c * ldx;
+    const hk::HJob j{3, xc, 1, ldx, y + c * ldy, 1, ldy, xc, ldx};
+    enqueue_sub(h, view(h, false), 0, 0, 1, j, j, std::min(nrhs - c, hk::HPASS), h->mv_part, h->mv_counter, s);
+  }
   H_TRY(cudaGetLastError());
   return FRANK_OK;
 }
 
 // passes: 1 = forward (L with the pivots), 2 = backward (U), 3 = both.
 int enqueue_solve(frank_hodlr* h, double* d_b, int64_t ldb, int nrhs, cudaStream_t s, int passes = 3) {
-  int rc = ensure_mv(h, nrhs, s);
+  int rc = ensure_mv(h, std::min(nrhs, hk::HPASS), s);
   if (rc) return rc;
-  for (int pass = 0; pass < 2; ++pass) {
-    if (!(passes & (1 << pass))) continue;
-    const hk::HJob j = sub_job(pass == 0 ? 0 : 2, d_b, 1, ldb, d_b, ldb);
-    enqueue_sub(h, view(h, true), 0, 0, 1, j, j, nrhs, h->mv_part, h->mv_counter, s);
-  }
+  for (int c = 0; c < nrhs; c += hk::HPASS)
+    for (int pass = 0; pass < 2; ++pass) {
+      if (!(passes & (1 << pass))) continue;
+      double* bc = d_b + c * ldb;
+      const hk::HJob j = sub_job(pass == 0 ? 0 : 2, bc, 1, ldb, bc, ldb);
+      enqueue_sub(h, view(h, true), 0, 0, 1, j, j, std::min(nrhs - c, hk::HPASS), h->mv_part, h->mv_counter, s);
+    }
   H_TRY(cudaGetLastError());
   return FRANK_OK;
 }
