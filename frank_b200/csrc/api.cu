@@ -563,11 +563,20 @@ int matvec_device_impl(frank_blr* p, const double* x, int64_t ldx, double* y, in
   BlrView<double> H = h_view(p);
   for (int c0 = 0; c0 < nrhs; c0 += p->solve_chunk) {
     const int nr = std::min(p->solve_chunk, nrhs - c0);
-    const int ns = solve_ring<double>(p->bmax, p->kcap, nr);
-    const size_t shm = solve_smem<double>(p->bmax, p->kcap, nr, ns);
+    const int nt = matvec_threads(p->bmax, p->nb, nr, p->fixed_rank == 0), tr = transpose ? 1 : 0;
+    const dim3 grid(p->nb, p->nb);
     p->solve_launches += 2;
-    k_matvec_blocks<<<dim3(p->nb, p->nb), SOLVE_THREADS, shm, s>>>(H, x + c0 * ldx, ldx, nr, p->part,
-                                                                   transpose ? 1 : 0, ns);
+    if (nt == 128) {
+      k_matvec_direct<128><<<grid, 128, matvec_direct_smem(p->bmax, p->kcap, nr, 128), s>>>(H, x + c0 * ldx, ldx, nr,
+                                                                                           p->part, tr);
+    } else if (nt == 256) {
+      k_matvec_direct<256><<<grid, 256, matvec_direct_smem(p->bmax, p->kcap, nr, 256), s>>>(H, x + c0 * ldx, ldx, nr,
+                                                                                           p->part, tr);
+    } else {
+      const int ns = solve_ring<double>(p->bmax, p->kcap, nr);
+      k_matvec_blocks<<<grid, SOLVE_THREADS, solve_smem<double>(p->bmax, p->kcap, nr, ns), s>>>(
+          H, x + c0 * ldx, ldx, nr, p->part, tr, ns);
+    }
     k_matvec_reduce<<<dim3(p->nb, (p->bmax + 255) / 256, nr), 256, 0, s>>>(H, p->part, nr,
                                                                            bres ? bres + c0 * ldb : nullptr, ldb,
                                                                            y + c0 * ldy, ldy);
@@ -878,6 +887,8 @@ int create_impl(const frank_blr_desc* d, const double* points, int dim, frank_bl
   p->solve_chunk = SV_NR;
   while (p->solve_chunk > 1 && solve_smem<double>((int)bm, (int)kc, p->solve_chunk, 2) > (size_t)SMEM_OPTIN_MAX)
     p->solve_chunk /= 2;
+  cudaFuncSetAttribute(k_matvec_direct<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
+  cudaFuncSetAttribute(k_matvec_direct<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
   cudaFuncSetAttribute(k_matvec_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
   cudaFuncSetAttribute(k_solve_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
   cudaFuncSetAttribute(k_solve_scatter<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);

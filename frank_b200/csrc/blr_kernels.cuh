@@ -2417,9 +2417,9 @@ struct SvTarget {
   }
 };
 
-template <typename T>
+template <int NT = SOLVE_THREADS, typename T>
 FRANK_D void sv_stage(double* x, int ldx, const T* src, int64_t ld, int n, int nrhs) {
-  for (int r = threadIdx.x; r < n; r += SOLVE_THREADS)
+  for (int r = threadIdx.x; r < n; r += NT)
 #pragma unroll 8
     for (int c = 0; c < nrhs; ++c) x[r + c * ldx] = double(src[r + (int64_t)c * ld]);
 }
@@ -2532,16 +2532,17 @@ FRANK_D void sd_tile(int m, int nr, int k0, int k1, const T* A, int64_t sai, int
   }
 }
 
-// out (m x nr in shared memory, ldo) = A X, X k x nr.  Tiles of 32 rows; with
-// fewer tiles than warps the inner dimension is cut into slices, summed in
-// order.  red: 8 x 256 doubles.  Ends with a barrier.
-template <typename T>
+// out (m x nr in shared memory, ldo) = A X, X k x nr, by NT threads.  Tiles of 32
+// rows; with fewer tiles than warps the inner dimension is cut into slices,
+// summed in order.  red: 8 NT doubles.  Ends with a barrier.
+template <int NT, typename T>
 FRANK_D void sd_mv(int m, int nr, int k, const T* A, int64_t sai, int64_t sak, const double* X, int ldx, double* out,
                    int ldo, double* red) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int mt = (m + 31) / 32, sl = mt >= 5 ? 1 : (mt >= 3 ? 2 : (mt == 2 ? 4 : 8));
+  constexpr int NW = NT / 32;
+  const int mt = (m + 31) / 32, sl = max(1, mt >= 5 ? NW / 8 : (mt >= 3 ? NW / 4 : (mt == 2 ? NW / 2 : NW)));
   const int kc = ((k + sl - 1) / sl + 15) & ~15;
-  for (int m0 = 0; m0 < mt; m0 += 8 / sl) {
+  for (int m0 = 0; m0 < mt; m0 += NW / sl) {
     const int tile = m0 + wid / sl, q = wid % sl;
     if (tile < mt) {
       double acc[4][2];
@@ -2553,8 +2554,8 @@ FRANK_D void sd_mv(int m, int nr, int k, const T* A, int64_t sai, int64_t sak, c
         for (int h = 0; h < 2; ++h) red[wid * 256 + (8 * i + g) + (2 * t + h) * 32] = acc[i][h];
     }
     __syncthreads();
-    const int rows = min(m - m0 * 32, (8 / sl) * 32);
-    for (int e = threadIdx.x; e < rows * nr; e += SOLVE_THREADS) {
+    const int rows = min(m - m0 * 32, (NW / sl) * 32);
+    for (int e = threadIdx.x; e < rows * nr; e += NT) {
       const int r = e % rows, c = e / rows;
       double v = 0.0;
       for (int s = 0; s < sl; ++s) v += red[((r >> 5) * sl + s) * 256 + (r & 31) + c * 32];
@@ -2589,8 +2590,8 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag_direct(BlrView<T> 
     for (int r = k0 + (threadIdx.x & 31); r < k1; r += 32)
       x[r - k0 + c * ldx] = double(z[o + (which == 0 ? perm[r] : r) + (int64_t)c * ldz]);
   __syncthreads();
-  if (which <= 1) sd_mv(nr, nrhs, k1 - k0, Mx + r0 + (int64_t)k0 * ld, 1, ld, x, ldx, out, SD_ROWS, red);
-  else sd_mv(nr, nrhs, k1 - k0, Mx + k0 + (int64_t)r0 * ld, ld, 1, x, ldx, out, SD_ROWS, red);
+  if (which <= 1) sd_mv<SOLVE_THREADS>(nr, nrhs, k1 - k0, Mx + r0 + (int64_t)k0 * ld, 1, ld, x, ldx, out, SD_ROWS, red);
+  else sd_mv<SOLVE_THREADS>(nr, nrhs, k1 - k0, Mx + k0 + (int64_t)r0 * ld, ld, 1, x, ldx, out, SD_ROWS, red);
   for (int e = threadIdx.x; e < nr * nrhs; e += SOLVE_THREADS) {
     const int r = e % nr, c = e / nr;
     ybuf[(which == 3 ? perm[r0 + r] : r0 + r) + (int64_t)c * ld] = T(out[r + c * SD_ROWS]);
@@ -2621,8 +2622,8 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_scatter(BlrView<T> A, i
   const int r = lr ? tg.r : bi, ldt = lr ? sv_ld(r) : ldy;
   if (lr) {
     const T* S = A.s(tg.gi, tg.gj);
-    sd_mv(r, nrhs, bi, tr ? A.u(tg.gi, tg.gj) : A.vt(tg.gi, tg.gj), ld, 1, ys, ldy, t1, ldt, red);
-    sd_mv(r, nrhs, r, S, tr ? A.kcap : 1, tr ? 1 : A.kcap, t1, ldt, t2, ldt, red);
+    sd_mv<SOLVE_THREADS>(r, nrhs, bi, tr ? A.u(tg.gi, tg.gj) : A.vt(tg.gi, tg.gj), ld, 1, ys, ldy, t1, ldt, red);
+    sd_mv<SOLVE_THREADS>(r, nrhs, r, S, tr ? A.kcap : 1, tr ? 1 : A.kcap, t1, ldt, t2, ldt, red);
   }
   const T* O = lr ? (tr ? A.vt(tg.gi, tg.gj) : A.u(tg.gi, tg.gj)) : A.dense(tg.gi, tg.gj);
   const bool ot = !lr && tr;
@@ -2679,6 +2680,69 @@ static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<
   __syncthreads();
   mv_run(seg, lr ? 3 : 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldb, x + H.off[j], ldx, bj, nrhs); },
          [&](int row, int c, double v) { out[row + (int64_t)c * ld] = v; });
+}
+
+// The same without the ring: the CTA reads its block straight into mma fragments
+// (sd_mv, sd_tile), and shared memory holds just the vectors (t2 takes x's place),
+// so that it does not limit how many CTAs share an SM.  A ring slot is as large
+// whatever the block, and its boxes are whole only for blocks of 256 rows and
+// more: through the ring alone a product with many small blocks was several waves
+// of CTAs waiting at barriers (b = 32, 48 x 48 blocks, one right-hand side 72 us,
+// 34 here; b = 128, 32 x 32 55 and 34; b = 512, 8 x 8 100 and 64; one warp per
+// column and thread per row, before the ring, 40, 38 and 86).
+template <int NT>
+static __global__ void __launch_bounds__(NT) k_matvec_direct(BlrView<double> H, const double* x, int64_t ldx, int nrhs,
+                                                             double* part, int transpose) {
+  extern __shared__ __align__(16) double ssm[];
+  const int nb = H.nb, ld = H.bmax, i = blockIdx.x, j = (i + blockIdx.y) % nb;
+  const int bi = H.bs(i), bj = H.bs(j), ldb = sv_ld(bj), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int gi = transpose ? j : i, gj = transpose ? i : j;   // stored block (gi, gj)
+  double* out = part + (int64_t)(i * nb + j) * ld * nrhs;
+  const bool lr = H.is_lr(gi, gj), tr = transpose != 0;
+  const int k = lr ? H.rank[gi * nb + gj] : bj, ldk = sv_ld(k);
+  if (k == 0) {
+    for (int e = threadIdx.x; e < bi * nrhs; e += NT) out[e % bi + (int64_t)(e / bi) * ld] = 0.0;
+    return;
+  }
+  double* red = ssm;
+  double* xs = red + 8 * NT;
+  double* t1 = xs + (size_t)sv_ld(ld) * nrhs;
+  sv_stage<NT>(xs, ldb, x + H.off[j], ldx, bj, nrhs);
+  __syncthreads();
+  if (lr) {
+    const double* S = H.s(gi, gj);
+    sd_mv<NT>(k, nrhs, bj, tr ? H.u(gi, gj) : H.vt(gi, gj), ld, 1, xs, ldb, t1, ldk, red);
+    sd_mv<NT>(k, nrhs, k, S, tr ? H.kcap : 1, tr ? 1 : H.kcap, t1, ldk, xs, ldk, red);
+  }
+  const double* O = lr ? (tr ? H.vt(gi, gj) : H.u(gi, gj)) : H.dense(gi, gj);
+  const bool ot = !lr && tr;
+  const int g = lane >> 2, q = lane & 3;
+  for (int i0 = wid * 32; i0 < bi; i0 += NT) {
+    double acc[4][2];
+    sd_tile(bi, nrhs, 0, k, O, ot ? ld : 1, ot ? 1 : ld, xs, ldk, i0, acc);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = i0 + 8 * a + g, c = 2 * q + h;
+        if (row < bi && c < nrhs) out[row + (int64_t)c * ld] = acc[a][h];
+      }
+  }
+}
+
+// Threads of k_matvec_direct, or 0 for the ring: tolerance plans with blocks of
+// whole boxes, enough of them to be bound by memory and few right-hand sides (n =
+// 16384, b = 512, 3-D at 1e-8: 315 us through the ring and 347 direct for four,
+// 380 and 350 for eight; n = 4096 at 1e-6 100 and 64).  128 threads where a block
+// has at most four tiles of 32 rows, or five and the grid several waves (b = 128, 48
+// x 48 blocks 50 us, 66 with 256 threads; b = 160 74 and 87; b = 256, 24 x 24 at
+// 1e-7 131 and 104).
+inline int matvec_threads(int bmax, int nb, int nrhs, bool tolerance) {
+  if (tolerance && bmax % 512 == 0 && nb >= 16 && nrhs <= 4) return 0;
+  return bmax <= 128 || (bmax <= 160 && nb >= 32) ? 128 : 256;
+}
+FRANK_HD size_t matvec_direct_smem(int bmax, int kcap, int nrhs, int threads) {
+  return (8 * (size_t)threads + ((size_t)sv_ld(bmax) + sv_ld(kcap)) * nrhs) * sizeof(double);
 }
 
 // y_i = sum_j part(i,j) (fixed order).  If b != null: y = b - A x (residual).
