@@ -459,6 +459,23 @@ int run_factor(frank_blr* p, cudaStream_t s) {
 
 // ---- solve --------------------------------------------------------------
 
+// Launch that may begin before the end of the one before it on the stream: for
+// kernels that call pdl_wait().
+template <typename... P, typename... A>
+void launch_pdl(cudaStream_t s, dim3 grid, size_t shm, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(SOLVE_THREADS);
+  c.dynamicSmemBytes = shm;
+  c.stream = s;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // part: 0 both sweeps, 1 the forward sweep only (L), 2 the backward sweep only (U).
 template <typename T>
 int enqueue_solve(frank_blr* p, T* z, int64_t ldz, int nrhs, bool transpose, cudaStream_t s, int part = 0) {
@@ -467,21 +484,21 @@ int enqueue_solve(frank_blr* p, T* z, int64_t ldz, int nrhs, bool transpose, cud
   T* ybuf = static_cast<T*>(p->stmp);
   const int nb = p->nb;
   const int ns = solve_ring<T>(p->bmax, p->kcap, nrhs);
-  const bool direct = solve_direct(p->bmax, p->fixed_rank > 0 ? p->fixed_rank : p->kcap);
+  const bool direct = solve_direct(p->bmax);
   const size_t shm = direct ? solve_direct_smem(p->bmax, p->kcap, nrhs) : solve_smem<T>(p->bmax, p->kcap, nrhs, ns);
   auto step = [&](int i, int dmode, int smode, int ntarget) {
     if (direct) {
-      k_solve_diag_direct<T><<<(p->bmax + SD_ROWS - 1) / SD_ROWS, SOLVE_THREADS, shm, s>>>(W, ws, i, z, ldz, nrhs,
-                                                                                           dmode, ybuf);
-      k_solve_scatter<T><<<std::max(ntarget, 1), SOLVE_THREADS, shm, s>>>(W, i, z, ldz, nrhs, smode, ybuf, ntarget);
+      launch_pdl(s, dim3((p->bmax + SD_ROWS - 1) / SD_ROWS), shm, k_solve_diag_direct<T>, W, ws, i, z, ldz, nrhs, dmode,
+                 ybuf);
+      launch_pdl(s, dim3(std::max(ntarget, 1)), shm, k_solve_scatter<T>, W, i, z, ldz, nrhs, smode, ybuf, ntarget);
       return;
     }
-    k_solve_diag<T><<<(p->bmax + SOLVE_ROWS - 1) / SOLVE_ROWS, SOLVE_THREADS, shm, s>>>(W, ws, i, z, ldz, nrhs, dmode,
-                                                                                        ybuf, ns);
+    launch_pdl(s, dim3((p->bmax + SOLVE_ROWS - 1) / SOLVE_ROWS), shm, k_solve_diag<T>, W, ws, i, z, ldz, nrhs, dmode,
+               ybuf, ns);
     if (ntarget > 0)
-      k_solve_inner<T><<<dim3((p->kcap + 15) / 16, ntarget), SOLVE_THREADS, shm, s>>>(W, i, nrhs, smode, ybuf, p->tbuf, ns);
-    k_solve_outer<T><<<dim3((p->bmax + 63) / 64, std::max(ntarget, 1)), SOLVE_THREADS, shm, s>>>(
-        W, i, z, ldz, nrhs, smode, ybuf, p->tbuf, ntarget, ns);
+      launch_pdl(s, dim3((p->kcap + 15) / 16, ntarget), shm, k_solve_inner<T>, W, i, nrhs, smode, ybuf, p->tbuf, ns);
+    launch_pdl(s, dim3((p->bmax + 63) / 64, std::max(ntarget, 1)), shm, k_solve_outer<T>, W, i, z, ldz, nrhs, smode,
+               ybuf, p->tbuf, ntarget, ns);
   };
   if (!transpose) {
     if (part != 2) for (int i = 0; i < nb; ++i) step(i, 0, 0, nb - i - 1);
@@ -525,8 +542,8 @@ void drop_solve_graphs(frank_blr* p) {
   p->solve_graphs.clear();
 }
 
-// d_b (double, n x nrhs) -> solve in T -> back into d_b.  The 2 nb launches
-// per pass are captured once per (buffer, ld, nrhs, direction) on the plan's
+// d_b (double, n x nrhs) -> solve in T -> back into d_b.  The launches of a pass
+// (two or three a step, 2 nb steps) are captured once per (buffer, ld, nrhs, direction) on the plan's
 // private capture stream and replayed as one graph launch on `s`.
 int solve_device_impl(frank_blr* p, double* d_b, int64_t ldb, int nrhs, bool transpose, cudaStream_t s,
                       int part = 0) {

@@ -2147,11 +2147,12 @@ constexpr int SMEM_OPTIN_MAX = 226 * 1024;   // dynamic shared memory a CTA may 
 // the ring; refinement 15.1 ms to 7.4), so a CTA streams its matrices as boxes through a ring in
 // shared memory (cp.async, two boxes ahead, also over the seams between
 // products) and multiplies them on the tensor pipe with the right-hand sides as
-// the columns.  MV_T: out = A^T X, boxes of 16 columns x 256 rows; MV_N*:
-// out = A X, boxes of 512 x 8, 64 x 56 and 16 x 128 (rows x columns).  The
+// the columns.  MV_T, MV_T64: out = A^T X, boxes of 256 x 16 and 56 x 64 (rows x
+// columns; the second for matrices of few rows: eight outputs a warp and no sum
+// over the warps); MV_N*: out = A X, boxes of 512 x 8, 64 x 56 and 16 x 128.  The
 // column strides in shared memory make the fragment reads conflict-free.
 template <int N> struct IntC { static constexpr int value = N; };
-enum : int { MV_T, MV_N512, MV_N64, MV_N16 };
+enum : int { MV_T, MV_T64, MV_N512, MV_N64, MV_N16 };
 constexpr int MV_BOX = 16 * 260;              // elements of a ring slot (the largest box)
 
 template <typename T>
@@ -2161,10 +2162,10 @@ struct MvSeg {
   int R, C, kind, ldx, ldo, vec;
   const double* X;       // k x nr (shared)
   double* out;           // m x nr (shared); the last segment's results go to the sink
-  FRANK_D int m() const { return kind == MV_T ? C : R; }
-  FRANK_D int k() const { return kind == MV_T ? R : C; }
-  FRANK_D int tm() const { return kind == MV_N512 ? 512 : (kind == MV_N64 ? 64 : 16); }
-  FRANK_D int tk() const { return kind == MV_T ? 256 : (kind == MV_N512 ? 8 : (kind == MV_N64 ? 56 : 128)); }
+  FRANK_D int m() const { return kind <= MV_T64 ? C : R; }
+  FRANK_D int k() const { return kind <= MV_T64 ? R : C; }
+  FRANK_D int tm() const { return kind == MV_N512 ? 512 : (kind == MV_N64 || kind == MV_T64 ? 64 : 16); }
+  FRANK_D int tk() const { return kind == MV_T ? 256 : (kind == MV_N512 ? 8 : (kind == MV_N16 ? 128 : 56)); }
   FRANK_D void set(const T* A_, int64_t ld_, int R_, int C_, int kind_, const double* X_, int ldx_, double* out_, int ldo_) {
     A = A_; ld = ld_; R = R_; C = C_; kind = kind_; X = X_; ldx = ldx_; out = out_; ldo = ldo_;
     vec = (reinterpret_cast<uintptr_t>(A_) & 15) == 0 && ((ld_ * sizeof(T)) & 15) == 0;
@@ -2199,17 +2200,17 @@ FRANK_D void mv_issue_box(const MvSeg<T>& s, int r0, int c0, T* slot) {
       }
     return;
   }
-  auto put = [&](auto e_, int n) {
-    constexpr int E = decltype(e_)::value, UN = BR / E;
-    for (int x = threadIdx.x; x < n * BC; x += SOLVE_THREADS) {
-      const int col = x / UN, u = (x % UN) * E;
-      if (u >= lr || col >= lc) continue;
+  auto put = [&](auto e_) {                 // a partial box: the units in use only
+    constexpr int E = decltype(e_)::value;
+    const int un = (lr + E - 1) / E;
+    for (int x = threadIdx.x; x < un * lc; x += SOLVE_THREADS) {
+      const int col = x / un, u = (x % un) * E;
       const int ok = col < vc ? max(0, min(E, vr - u)) : 0;
       cp_async<E * (int)sizeof(T)>(slot + col * LDP + u, ok ? A + u + (int64_t)col * s.ld : s.A, ok * (int)sizeof(T));
     }
   };
-  if (s.vec) put(IntC<16 / (int)sizeof(T)>{}, BR * (int)sizeof(T) / 16);
-  else put(IntC<1>{}, BR);
+  if (s.vec) put(IntC<16 / (int)sizeof(T)>{});
+  else put(IntC<1>{});
 }
 
 // One warp's MI row tiles of a box: k quads q with 4 q < kv, at most KQ of
@@ -2245,10 +2246,13 @@ FRANK_D void mv_box(const T* a0, int si, int sq, const double* x, int kv, double
 
 // Runs the segments in order; prefetched() is called by all threads once the
 // first boxes are on their way (it stages X), sink(row, rhs, value) gets the
-// last segment's results, each from one thread.  red: 1024 doubles.
-template <typename T, typename Pre, typename Sink>
+// last segment's results, each from one thread.  KINDS: the kinds that occur, a
+// bit each (the code of the others costs the short kernels registers and time).
+// red: 1024 doubles.
+template <int KINDS, typename T, typename Pre, typename Sink>
 FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double* red, Pre prefetched, Sink sink) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  auto is = [](int kind, int want) { return ((KINDS >> want) & 1) != 0 && (KINDS == 1 << want || kind == want); };
   int total = 0;
   for (int p = 0; p < np; ++p)
     total += ((seg[p].m() + seg[p].tm() - 1) / seg[p].tm()) * ((seg[p].k() + seg[p].tk() - 1) / seg[p].tk());
@@ -2257,10 +2261,11 @@ FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double
     if (issued < total) {
       const MvSeg<T>& s = seg[ip];
       T* slot = ring + islot * MV_BOX;
-      if (s.kind == MV_T) mv_issue_box<256, 16, 260, true>(s, ik * 256, im * 16, slot);
-      else if (s.kind == MV_N512) mv_issue_box<512, 8, 520, false>(s, im * 512, ik * 8, slot);
-      else if (s.kind == MV_N64) mv_issue_box<64, 56, 72, false>(s, im * 64, ik * 56, slot);
-      else mv_issue_box<16, 128, 24, false>(s, im * 16, ik * 128, slot);
+      if (is(s.kind, MV_T)) mv_issue_box<256, 16, 260, true>(s, ik * 256, im * 16, slot);
+      else if (is(s.kind, MV_T64)) mv_issue_box<56, 64, 60, true>(s, ik * 56, im * 64, slot);
+      else if (is(s.kind, MV_N512)) mv_issue_box<512, 8, 520, false>(s, im * 512, ik * 8, slot);
+      else if (is(s.kind, MV_N64)) mv_issue_box<64, 56, 72, false>(s, im * 64, ik * 56, slot);
+      else if (is(s.kind, MV_N16)) mv_issue_box<16, 128, 24, false>(s, im * 16, ik * 128, slot);
       ++issued;
       if (++islot == ns) islot = 0;
       if (++ik * s.tk() >= s.k()) {
@@ -2291,11 +2296,13 @@ FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double
     const T* slot = ring + slot_i * MV_BOX;
     const int m0 = mb * tm, kv = min(tk, k - kb * tk);
     const double* X = X0 + kb * tk;
-    if (kind == MV_T) mv_box<2, 8>(slot + g * 260 + wid * 32 + t, 8 * 260, 4, X + wid * 32, kv - wid * 32, tot);
-    else if (kind == MV_N16) mv_box<2, 4>(slot + g + (wid * 16 + t) * 24, 8, 96, X + wid * 16, kv - wid * 16, tot);
-    else if (kind == MV_N64) {
+    if (is(kind, MV_T)) mv_box<2, 8>(slot + g * 260 + wid * 32 + t, 8 * 260, 4, X + wid * 32, kv - wid * 32, tot);
+    else if (is(kind, MV_N16)) mv_box<2, 4>(slot + g + (wid * 16 + t) * 24, 8, 96, X + wid * 16, kv - wid * 16, tot);
+    else if (is(kind, MV_T64)) {
+      if (m0 + wid * 8 < m) mv_box<1, 14>(slot + (wid * 8 + g) * 60 + t, 0, 4, X, kv, tot);
+    } else if (is(kind, MV_N64)) {
       if (m0 + wid * 8 < m) mv_box<1, 14>(slot + wid * 8 + g + t * 72, 8, 288, X, kv, tot);
-    } else if (m0 + wid * 64 < m) mv_box<8, 2>(slot + wid * 64 + g + t * 520, 8, 2080, X, kv, tot);
+    } else if (is(kind, MV_N512) && m0 + wid * 64 < m) mv_box<8, 2>(slot + wid * 64 + g + t * 520, 8, 2080, X, kv, tot);
     if (++slot_i == ns) slot_i = 0;
     if (++kb * tk < k) continue;
     auto deliver = [&](int row, int c, double v) {
@@ -2303,7 +2310,7 @@ FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double
       if (p == np - 1) sink(row, c, v);
       else seg[p].out[row + (int64_t)c * seg[p].ldo] = v;
     };
-    if (kind == MV_T || kind == MV_N16) {
+    if (is(kind, MV_T) || is(kind, MV_N16)) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -2316,7 +2323,7 @@ FRANK_D void mv_run(const MvSeg<T>* seg, int np, int nr, T* ring, int ns, double
         deliver(m0 + (threadIdx.x & 15), threadIdx.x >> 4, v);
       }
     } else {
-      const int per = kind == MV_N64 ? 1 : 8;
+      const int per = is(kind, MV_N512) ? 8 : 1;
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         if (i < per)
@@ -2359,6 +2366,18 @@ struct MvShared {
   }
 };
 
+// A solve is a chain of 4 nb to 6 nb launches of a few microseconds, each launched
+// with programmatic stream serialization: its CTAs start, and its ring fetches
+// the first boxes (factors, which no launch of the chain writes), while the launch
+// before it ends.  Every CTA calls pdl_wait() before it touches vectors, also one
+// without work: the end of a grid has to stand for the end of all grids before it.
+// (One right-hand side, us a step: b = 512, nb = 32 12.7, with plain launches and
+// padded boxes 18.0, 24.9 before the ring; b = 256, nb = 16 9.0, 13.5 and 13.6.)
+FRANK_D void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // y = M * P(z_i) (which 0: Linv, permuted input; 1: Uinv),
 // y = M^T z_i (2: Uinv^T), or y = P^T (Linv^T z_i) (3), into ybuf (ld bmax).
 // grid = ceil(b / SOLVE_ROWS) CTAs, SOLVE_ROWS rows each, from the part of M
@@ -2371,7 +2390,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag(BlrView<T> A, Fact
   const int b = A.bs(i), ld = A.bmax, ldx = sv_ld(b);
   const int64_t o = A.off[i];
   const int r0 = blockIdx.x * SOLVE_ROWS, nr = min(SOLVE_ROWS, b - r0);
-  if (nr <= 0) return;
+  if (nr <= 0) { pdl_wait(); return; }
   MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
   const T* Mx = (which == 0 || which == 3) ? ws.Linv + (int64_t)i * ld * ld : ws.Uinv + (int64_t)i * ld * ld;
   const int* perm = ws.perm + (int64_t)i * ld;
@@ -2382,9 +2401,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag(BlrView<T> A, Fact
     else seg.set(Mx + k0 + (int64_t)r0 * ld, ld, k1 - k0, nr, MV_T, sm.x, ldx, nullptr, 0);
   }
   __syncthreads();
-  mv_run(
+  mv_run<1 << MV_N16 | 1 << MV_T>(
       &seg, 1, nrhs, sm.ring, ns, sm.red,
       [&]() {
+        pdl_wait();
         for (int r = k0 + threadIdx.x; r < k1; r += SOLVE_THREADS) {
           const T* src = z + o + (which == 0 ? perm[r] : r);
 #pragma unroll 8
@@ -2432,15 +2452,20 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_inner(BlrView<T> A, int
   __shared__ MvSeg<T> seg;
   const SvTarget<T> tg(A, i, blockIdx.y, mode);
   const int c0 = blockIdx.x * 16, ld = A.bmax, bi = A.bs(i), ldx = sv_ld(bi);
-  if (c0 >= tg.r) return;
+  if (c0 >= tg.r) { pdl_wait(); return; }
   MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
   if (threadIdx.x == 0)
     seg.set((mode >= 2 ? A.u(tg.gi, tg.gj) : A.vt(tg.gi, tg.gj)) + (int64_t)c0 * ld, ld, bi, min(16, tg.r - c0), MV_T,
             sm.x, ldx, nullptr, 0);
   __syncthreads();
   double* t1 = tbuf + (int64_t)blockIdx.y * A.kcap * SV_NR + c0;
-  mv_run(&seg, 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldx, ybuf, ld, bi, nrhs); },
-         [&](int r, int c, double v) { t1[r + (int64_t)c * A.kcap] = v; });
+  mv_run<1 << MV_T>(
+      &seg, 1, nrhs, sm.ring, ns, sm.red,
+      [&]() {
+        pdl_wait();
+        sv_stage(sm.x, ldx, ybuf, ld, bi, nrhs);
+      },
+      [&](int r, int c, double v) { t1[r + (int64_t)c * A.kcap] = v; });
 }
 
 // grid (ceil(bmax / 64), max(targets, 1)); the first target's CTAs also copy y_i into z_i
@@ -2451,21 +2476,24 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_outer(BlrView<T> A, int
   extern __shared__ __align__(16) double ssm[];
   __shared__ MvSeg<T> seg[2];
   const int ld = A.bmax, bi = A.bs(i), r0 = blockIdx.x * 64;
-  if (blockIdx.y == 0)
-    for (int r = r0 + (threadIdx.x & 63); r < min(bi, r0 + 64); r += 64)
-      for (int c = threadIdx.x >> 6; c < nrhs; c += SOLVE_THREADS / 64)
-        z[A.off[i] + r + (int64_t)c * ldz] = ybuf[r + (int64_t)c * ld];
-  if ((int)blockIdx.y >= ntarget) return;
+  auto wait_and_copy = [&]() {
+    pdl_wait();
+    if (blockIdx.y == 0)
+      for (int r = r0 + (threadIdx.x & 63); r < min(bi, r0 + 64); r += 64)
+        for (int c = threadIdx.x >> 6; c < nrhs; c += SOLVE_THREADS / 64)
+          z[A.off[i] + r + (int64_t)c * ldz] = ybuf[r + (int64_t)c * ld];
+  };
+  if ((int)blockIdx.y >= ntarget) { wait_and_copy(); return; }
   const SvTarget<T> tg(A, i, blockIdx.y, mode);
   const bool lr = tg.r >= 0, tr = mode >= 2;
   const int rows = min(64, tg.bj - r0);
-  if (rows <= 0 || tg.r == 0) return;
+  if (rows <= 0 || tg.r == 0) { wait_and_copy(); return; }
   MvShared<T> sm(ssm, A.bmax, A.kcap, nrhs);
   const int k = lr ? tg.r : bi, ldk = sv_ld(k);
   double* x = lr ? sm.t1 : sm.x;
   if (threadIdx.x == 0) {
     if (lr) {
-      seg[0].set(A.s(tg.gi, tg.gj), A.kcap, k, k, tr ? MV_T : MV_N64, x, ldk, sm.x, ldk);
+      seg[0].set(A.s(tg.gi, tg.gj), A.kcap, k, k, tr ? MV_T64 : MV_N64, x, ldk, sm.x, ldk);
       seg[1].set((tr ? A.vt(tg.gi, tg.gj) : A.u(tg.gi, tg.gj)) + r0, ld, rows, k, MV_N64, sm.x, ldk, nullptr, 0);
     } else if (tr) {
       seg[0].set(A.dense(tg.gi, tg.gj) + (int64_t)r0 * ld, ld, k, rows, MV_T, x, ldk, nullptr, 0);
@@ -2475,9 +2503,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_outer(BlrView<T> A, int
   }
   __syncthreads();
   T* zj = z + A.off[tg.j] + r0;
-  mv_run(
+  mv_run<1 << MV_N64 | 1 << MV_T64 | 1 << MV_T>(
       seg, lr ? 2 : 1, nrhs, sm.ring, ns, sm.red,
       [&]() {
+        wait_and_copy();
         if (lr) sv_stage(x, ldk, tbuf + (int64_t)blockIdx.y * A.kcap * SV_NR, A.kcap, k, nrhs);
         else sv_stage(x, ldk, ybuf, ld, k, nrhs);
       },
@@ -2487,16 +2516,14 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_outer(BlrView<T> A, int
       });
 }
 
-// Small blocks (the inner product at most SV_DIRECT boxes): one CTA per target
-// does all of a step's update in one launch, reading the factors straight into
-// mma fragments.  The chain of a step is then too short for the ring's set-up
-// and a third launch to pay: n = 256 with b = 32 takes 0.93 ms for the
-// factorization and refinement, 1.08 through the ring; n = 2048 with b = 256
-// and rank 16 3.49 and 3.61.  At n = 16384, b = 512 this form takes 13.0 ms
-// for a refinement that takes 7.4 through the ring.
-constexpr int SV_DIRECT = 4;
+// Small blocks: one CTA per target does all of a step's update in one launch,
+// reading the factors straight into mma fragments.  The chain of a step is then
+// too short for a third launch to pay: n = 256 with b = 32, fixed rank 16, four
+// right-hand sides 134 us, 147 through the ring; with b = 64 the two are within 10 %
+// either way for one to eight right-hand sides; n = 1600 with b = 100 at 1e-3 takes
+// 329 us so and 260 through the ring.
 constexpr int SD_ROWS = 32;      // rows of the diagonal solve per CTA
-FRANK_HD bool solve_direct(int bmax, int rank) { return ((rank + 15) / 16) * ((bmax + 255) / 256) <= SV_DIRECT; }
+FRANK_HD bool solve_direct(int bmax) { return bmax <= 64; }
 
 // One warp's 32 x 8 tile of A X over k0 <= kk < k1: element (i, kk) of A at
 // A[i sai + kk sak], X k x nr (shared, ldx); sums as in mv_box.
@@ -2578,6 +2605,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_diag_direct(BlrView<T> 
   const int b = A.bs(i), ld = A.bmax, ldx = sv_ld(b);
   const int64_t o = A.off[i];
   const int r0 = blockIdx.x * SD_ROWS, nr = min(SD_ROWS, b - r0);
+  pdl_wait();
   if (nr <= 0) return;
   double* red = ssm;
   double* out = red + 8 * 256;
@@ -2609,6 +2637,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_solve_scatter(BlrView<T> A, i
   double* t1 = ys + (size_t)sv_ld(A.bmax) * nrhs;
   double* t2 = t1 + (size_t)sv_ld(A.kcap) * nrhs;
   const int ldy = sv_ld(bi);
+  pdl_wait();
   for (int c = wid; c < nrhs; c += SOLVE_THREADS / 32)
     for (int r = lane; r < bi; r += 32) {
       const T v = ybuf[r + (int64_t)c * ld];
@@ -2669,7 +2698,7 @@ static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<
   if (threadIdx.x == 0) {
     if (lr) {
       seg[0].set(tr ? H.u(gi, gj) : H.vt(gi, gj), ld, bj, r, MV_T, sm.x, ldb, sm.t1, ldr);
-      seg[1].set(H.s(gi, gj), H.kcap, r, r, tr ? MV_T : MV_N64, sm.t1, ldr, sm.x, ldr);
+      seg[1].set(H.s(gi, gj), H.kcap, r, r, tr ? MV_T64 : MV_N64, sm.t1, ldr, sm.x, ldr);
       seg[2].set(tr ? H.vt(gi, gj) : H.u(gi, gj), ld, bi, r, nk, sm.x, ldr, nullptr, 0);
     } else if (tr) {
       seg[0].set(H.dense(gi, gj), ld, bj, bi, MV_T, sm.x, ldb, nullptr, 0);
@@ -2678,8 +2707,9 @@ static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<
     }
   }
   __syncthreads();
-  mv_run(seg, lr ? 3 : 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldb, x + H.off[j], ldx, bj, nrhs); },
-         [&](int row, int c, double v) { out[row + (int64_t)c * ld] = v; });
+  mv_run<1 << MV_T | 1 << MV_T64 | 1 << MV_N64 | 1 << MV_N512>(
+      seg, lr ? 3 : 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldb, x + H.off[j], ldx, bj, nrhs); },
+      [&](int row, int c, double v) { out[row + (int64_t)c * ld] = v; });
 }
 
 // The same without the ring: the CTA reads its block straight into mma fragments
