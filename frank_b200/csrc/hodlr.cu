@@ -187,33 +187,35 @@ __global__ void __launch_bounds__(WT) k_h_leaf_mm(HView h, LeafFactors f, HJob j
   }
 }
 
-// One CTA's share of T (m x n <= HC each) = A B over rows [k0, k1), element (i, kk)
-// of A at A[i sai + kk sak], B col-major: eight warps take an eighth of the rows
-// each and sum in shared memory (red, 8 HC HC doubles); T in red[0 .. m n).
+// One CTA's share of T (m <= HC, n <= 8 NJ <= HC) = A B over rows [k0, k1), element (i,
+// kk) of A at A[i sai + kk sak], B col-major: eight warps take an eighth of the rows
+// each and sum in shared memory (red, 8 HC HC doubles); sink(i, j, value) gets the
+// results, each from one thread.  NJ = 1 for up to eight columns: n = 512 in leaves of
+// 32, one right-hand side, takes 93 us a solve so and 108 with the products and sums
+// of 32 columns (106 by the walks before).
+template <int NJ, typename Sink>
 __device__ __forceinline__ void h_tprod(int m, int n, int64_t k0, int64_t k1, const double* A, int64_t sai, int64_t sak,
-                                        const double* B, int64_t ldb, double* red) {
+                                        const double* B, int64_t ldb, double* red, Sink sink) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, wid = threadIdx.x >> 5;
   const int64_t len = ((k1 - k0 + 7) / 8 + 3) & ~(int64_t)3;
   const int64_t a0 = min(k1, k0 + wid * len), a1 = min(k1, a0 + len);
-  double acc[4][4][2];
-  blr::warp_dgemm_acc<4, 4, false>(m, n, 0, (int)(a1 - a0), A + a0 * sak, sai, sak, B + a0, ldb, 1, 0, 0, acc);
+  double acc[4][NJ][2];
+  blr::warp_dgemm_acc<4, NJ, false>(m, n, 0, (int)(a1 - a0), A + a0 * sak, sai, sak, B + a0, ldb, 1, 0, 0, acc);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) red[wid * HC * HC + (8 * i + g) + (8 * j + 2 * t + q) * HC] = acc[i][j][q];
+      for (int q = 0; q < 2; ++q) red[wid * HC * 8 * NJ + (8 * i + g) + (8 * j + 2 * t + q) * HC] = acc[i][j][q];
   __syncthreads();
-  double v[HC * HC / WT];
 #pragma unroll
-  for (int x = 0; x < HC * HC / WT; ++x) {
-    v[x] = 0.0;
+  for (int x = 0; x < HC * 8 * NJ / WT; ++x) {
+    const int e = threadIdx.x + x * WT;
+    double v = 0.0;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) v[x] += red[w * HC * HC + threadIdx.x + x * WT];
+    for (int w = 0; w < 8; ++w) v += red[w * HC * 8 * NJ + e];
+    if (e % HC < m && e / HC < n) sink(e % HC, e / HC, v);
   }
-  __syncthreads();
-#pragma unroll
-  for (int x = 0; x < HC * HC / WT; ++x) red[threadIdx.x + x * WT] = v[x];
   __syncthreads();
 }
 
@@ -241,13 +243,13 @@ __global__ void __launch_bounds__(WT) k_h_t(HView h, HJob j0, HJob j1, int njobs
   double* pt = part + slot * nch * k * HC;
   for (int m0 = 0; m0 < k; m0 += HC) {
     const int m = min(HC, k - m0);
-    h_tprod(m, nc, i0, i1, A + (tr ? (int64_t)m0 * sl : m0), tr ? sl : 1, tr ? 1 : k, x, ldx, red);
-    for (int e = threadIdx.x; e < m * nc; e += WT) {
-      const double v = red[e % m + (e / m) * HC];
-      if (nch == 1) t1[m0 + e % m + (e / m) * k] = v;
-      else pt[(int64_t)blockIdx.x * k * HC + m0 + e % m + (e / m) * k] = v;
-    }
-    __syncthreads();
+    auto keep = [&](int r, int q, double v) {
+      if (nch == 1) t1[m0 + r + q * k] = v;
+      else pt[(int64_t)blockIdx.x * k * HC + m0 + r + q * k] = v;
+    };
+    const double* Am = A + (tr ? (int64_t)m0 * sl : m0);
+    if (nc <= 8) h_tprod<1>(m, nc, i0, i1, Am, tr ? sl : 1, tr ? 1 : k, x, ldx, red, keep);
+    else h_tprod<4>(m, nc, i0, i1, Am, tr ? sl : 1, tr ? 1 : k, x, ldx, red, keep);
   }
   if (nch > 1) {
     __threadfence();
@@ -327,9 +329,8 @@ __global__ void __launch_bounds__(WT) k_h_core(int64_t s, int k, const double* V
   for (int m0 = 0; m0 < k; m0 += HC)
     for (int n0 = 0; n0 < k; n0 += HC) {
       const int m = min(HC, k - m0), n = min(HC, k - n0);
-      h_tprod(m, n, i0, i1, Vl + m0, 1, k, Uu + (int64_t)n0 * s, s, red);
-      for (int e = threadIdx.x; e < m * n; e += WT) mine[m0 + e % m + (n0 + e / m) * k] = red[e % m + (e / m) * HC];
-      __syncthreads();
+      h_tprod<4>(m, n, i0, i1, Vl + m0, 1, k, Uu + (int64_t)n0 * s, s, red,
+                 [&](int r, int q, double v) { mine[m0 + r + (n0 + q) * k] = v; });
     }
   __threadfence();
   __syncthreads();
