@@ -325,18 +325,14 @@ static __device__ __noinline__ void cta_dgemm(int m, int n, int k, double alpha,
 // op(A) is m x k: A is (m x k, lda) when !ta, (k x m, lda) when ta.
 // op(B) is k x n: B is (k x n, ldb) when !tb, (n x k, ldb) when tb.
 // beta == 0 never reads C.  FP64 accumulation takes the tensor pipe
-// (cta_dgemm); FP32 accumulation 64x64 output tiles, k in steps of 16,
-// operands staged through shared memory.  `smem` must hold 2 * 16 * 64 TACC
+// (cta_dgemm); FP32 accumulation cta_gemm_tiled: 64x64 output tiles, k in steps of
+// 16, operands staged through shared memory.  `smem` must hold 2 * 16 * 64 TACC
 // values.  Requires blockDim.x == NT (256 or 512).
 // ---------------------------------------------------------------------------
 template <typename TACC, int NT, typename TA, typename TB, typename TC>
-FRANK_D void cta_gemm(int m, int n, int k, TACC alpha, const TA* A, int64_t lda, bool ta,
-                      const TB* B, int64_t ldb, bool tb, TACC beta, TC* C, int64_t ldc,
-                      TACC* smem) {
-  if constexpr (sizeof(TACC) == 8) {
-    cta_dgemm<NT>(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, smem);
-    return;
-  }
+FRANK_D void cta_gemm_tiled(int m, int n, int k, TACC alpha, const TA* A, int64_t lda, bool ta,
+                            const TB* B, int64_t ldb, bool tb, TACC beta, TC* C, int64_t ldc,
+                            TACC* smem) {
   constexpr int BM = 64, BN = 64, BK = 16;
   constexpr int TM = 4, TN = (NT == 256) ? 4 : 2;
   static_assert((BM / TM) * (BN / TN) == NT, "tile/threads mismatch");
@@ -402,6 +398,16 @@ FRANK_D void cta_gemm(int m, int n, int k, TACC alpha, const TA* A, int64_t lda,
     }
   }
   __syncthreads();
+}
+
+template <typename TACC, int NT, typename TA, typename TB, typename TC>
+FRANK_D void cta_gemm(int m, int n, int k, TACC alpha, const TA* A, int64_t lda, bool ta,
+                      const TB* B, int64_t ldb, bool tb, TACC beta, TC* C, int64_t ldc,
+                      TACC* smem) {
+  if constexpr (sizeof(TACC) == 8)
+    cta_dgemm<NT>(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, smem);
+  else
+    cta_gemm_tiled<TACC, NT>(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, smem);
 }
 
 // ---------------------------------------------------------------------------

@@ -34,6 +34,17 @@ enum { OPS_ERR_JACOBI = 0, OPS_ERR_SLOTS = 2 };
 // Device building blocks (all threads of the CTA; each ends with a barrier)
 // ---------------------------------------------------------------------------
 
+// FP64 product of a one-CTA operation.  MANY: the variants for batches of more
+// small blocks than SMs, where several CTAs have to share an SM: the tensor-pipe
+// product needs 128 registers itself and 190 to 240 with its caller, one CTA of
+// 256 threads an SM; the tiled one leaves room for two (additions) or three.
+template <bool MANY>
+FRANK_D void op_gemm(int m, int n, int k, double alpha, const double* a, int64_t lda, bool ta, const double* b,
+                     int64_t ldb, bool tb, double beta, double* c, int64_t ldc, double* gsm) {
+  if constexpr (MANY) cta_gemm_tiled<double, OT>(m, n, k, alpha, a, lda, ta, b, ldb, tb, beta, c, ldc, gsm);
+  else cta_gemm<double, OT>(m, n, k, alpha, a, lda, ta, b, ldb, tb, beta, c, ldc, gsm);
+}
+
 // Explicit Q (m x k, ldq) = H_0 ... H_{k-1} [I; 0] from reflectors V (ldv).
 FRANK_D void form_q(int m, int k, const double* V, int64_t ldv, const double* tau, double* Q, int64_t ldq) {
   for (int64_t e = threadIdx.x; e < (int64_t)m * k; e += blockDim.x) {
@@ -232,32 +243,34 @@ __global__ void __launch_bounds__(OT) k_op_svd(int m, int n, Mat A, Mat U, Mat S
 // Randomized range finder shared by rsvd / rid: Q (m x s, ld m) orthonormal
 // basis of A Omega (plus `power` subspace iterations), B = Q^T A (s x n, ld s).
 // Omega: n x s row-major (the reference's random_uniform fill order).
+template <bool MANY>
 FRANK_D void range_finder(int m, int n, int s, int power, const double* a, int64_t lda, const double* omega,
                           double* Q, double* B, double* Z, double* tau, double* gsm, double* red) {
   // Y = A Omega into Q
-  cta_gemm<double, OT>(m, s, n, 1.0, a, lda, false, omega, s, true, 0.0, Q, m, gsm);
+  op_gemm<MANY>(m, s, n, 1.0, a, lda, false, omega, s, true, 0.0, Q, m, gsm);
   cta_householder_qr(m, s, Q, m, tau, red);
   form_q(m, s, Q, m, tau, B, m);               // B as scratch for the explicit Q (m x s)
   for (int64_t e = threadIdx.x; e < (int64_t)m * s; e += blockDim.x) Q[e] = B[e];
   __syncthreads();
   for (int it = 0; it < power; ++it) {
     // Z = A^T Q (n x s), orthonormalise, Y = A Z, orthonormalise
-    cta_gemm<double, OT>(n, s, m, 1.0, a, lda, true, Q, m, false, 0.0, Z, n, gsm);
+    op_gemm<MANY>(n, s, m, 1.0, a, lda, true, Q, m, false, 0.0, Z, n, gsm);
     cta_householder_qr(n, s, Z, n, tau, red);
     form_q(n, s, Z, n, tau, B, n);
-    cta_gemm<double, OT>(m, s, n, 1.0, a, lda, false, B, n, false, 0.0, Q, m, gsm);
+    op_gemm<MANY>(m, s, n, 1.0, a, lda, false, B, n, false, 0.0, Q, m, gsm);
     cta_householder_qr(m, s, Q, m, tau, red);
     form_q(m, s, Q, m, tau, B, m);
     for (int64_t e = threadIdx.x; e < (int64_t)m * s; e += blockDim.x) Q[e] = B[e];
     __syncthreads();
   }
   // B = Q^T A (s x n)
-  cta_gemm<double, OT>(s, n, m, 1.0, Q, m, true, a, lda, false, 0.0, B, s, gsm);
+  op_gemm<MANY>(s, n, m, 1.0, Q, m, true, a, lda, false, 0.0, B, s, gsm);
 }
 
 // rsvd (operations/randomized/rsvd.cpp:17-29, via LowRank(Dense, rank),
 // low_rank.cpp:40-48): U (m x rank), S (rank x rank, diagonal), V (rank x n).
-__global__ void __launch_bounds__(OT) k_op_rsvd(int m, int n, int s, int rank, int power, Mat A, const double* omega,
+template <bool MANY>
+__global__ void __launch_bounds__(OT, MANY ? 3 : 1) k_op_rsvd(int m, int n, int s, int rank, int power, Mat A, const double* omega,
                                                 Mat U, Mat S, Mat V, double* scratch, int64_t ws, int* err) {
   __shared__ double gsm[GSM];
   __shared__ double red[32];
@@ -271,10 +284,10 @@ __global__ void __launch_bounds__(OT) k_op_rsvd(int m, int n, int s, int rank, i
   double* sv = Ub + (int64_t)s * s;             // s
   double* Vbt = sv + s;                         // s x n
   double* sc = Vbt + (int64_t)s * n;            // svd scratch
-  range_finder(m, n, s, power, A.at(b), A.ld, omega, Q, B, Z, tau, gsm, red);
+  range_finder<MANY>(m, n, s, power, A.at(b), A.ld, omega, Q, B, Z, tau, gsm, red);
   if (!cta_svd(s, n, B, s, Ub, s, sv, Vbt, s, sc, &flag) && threadIdx.x == 0) atomicAdd(err + OPS_ERR_JACOBI, 1);
   // U = Q Ub(:, :rank), S = diag(sv), V = Vbt(:rank, :)
-  cta_gemm<double, OT>(m, rank, s, 1.0, Q, m, false, Ub, s, false, 0.0, U.at(b), U.ld, gsm);
+  op_gemm<MANY>(m, rank, s, 1.0, Q, m, false, Ub, s, false, 0.0, U.at(b), U.ld, gsm);
   double* sp = S.at(b);
   for (int64_t e = threadIdx.x; e < (int64_t)rank * rank; e += blockDim.x) {
     const int i = e % rank, c = e / rank;
@@ -325,7 +338,8 @@ __global__ void __launch_bounds__(OT) k_op_id(int m, int n, int k, Mat A, Mat U,
          cols + (int64_t)b * k, AC, Ut, sc, red, redi);
 }
 
-__global__ void __launch_bounds__(OT) k_op_rid(int m, int n, int s, int k, Mat A, const double* omega, Mat U, Mat S,
+template <bool MANY>
+__global__ void __launch_bounds__(OT, MANY ? 3 : 1) k_op_rid(int m, int n, int s, int k, Mat A, const double* omega, Mat U, Mat S,
                                                Mat V, double* scratch, int64_t ws) {
   __shared__ double gsm[GSM];
   __shared__ double red[32];
@@ -341,9 +355,9 @@ __global__ void __launch_bounds__(OT) k_op_rid(int m, int n, int s, int k, Mat A
   int* rw = reinterpret_cast<int*>(Ut + (int64_t)k * s);
   int* cl = rw + k;
   double* sc = reinterpret_cast<double*>(cl + k + (k & 1));
-  range_finder(m, n, s, 0, A.at(b), A.ld, omega, Q, B, Z, tau, gsm, red);
+  range_finder<MANY>(m, n, s, 0, A.at(b), A.ld, omega, Q, B, Z, tau, gsm, red);
   cta_id(s, n, k, B, s, Ub, s, S.at(b), S.ld, V.at(b), V.ld, rw, cl, AC, Ut, sc, red, redi);
-  cta_gemm<double, OT>(m, k, s, 1.0, Q, m, false, Ub, s, false, 0.0, U.at(b), U.ld, gsm);
+  op_gemm<MANY>(m, k, s, 1.0, Q, m, false, Ub, s, false, 0.0, U.at(b), U.ld, gsm);
 }
 
 // LowRank += LowRank (operations/arithmetic/addition.cpp:93-127 rounded,
@@ -354,6 +368,7 @@ __global__ void __launch_bounds__(OT) k_op_rid(int m, int n, int s, int k, Mat A
 // else ka.  fast (fixed rank, Ua and Va^T orthonormal): the projections
 // Zu = Ua^T Ub, Zv = Va Vb^T, QR of the remainders only, core
 // [I Zu; 0 Ru] blockdiag(Sa, Sb) [I Zv; 0 Rv]^T.
+template <bool MANY>
 FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, double* ua_out, int64_t ldua, double* sa_out,
                          int64_t ldsa, double* va_out, int64_t ldva, int* ka_io, const double* ub, int64_t ldub,
                          const double* sb, int64_t ldsb, const double* vb, int64_t ldvb, int kb, double* X, int* err) {
@@ -379,8 +394,8 @@ FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, dou
   int mu, mv;
   if (!use_fast) {
     // X = [Ua Sa | Ub Sb], Y = [Va^T | Vb^T]
-    cta_gemm<double, OT>(m, ka, ka, 1.0, ua, Ua.ld, false, sa, Sa.ld, false, 0.0, X, m, gsm);
-    cta_gemm<double, OT>(m, kb, kb, 1.0, ub, Ub.ld, false, sb, Sb.ld, false, 0.0, X + (int64_t)ka * m, m, gsm);
+    op_gemm<MANY>(m, ka, ka, 1.0, ua, Ua.ld, false, sa, Sa.ld, false, 0.0, X, m, gsm);
+    op_gemm<MANY>(m, kb, kb, 1.0, ub, Ub.ld, false, sb, Sb.ld, false, 0.0, X + (int64_t)ka * m, m, gsm);
     for (int64_t e = threadIdx.x; e < (int64_t)n * kt; e += blockDim.x) {
       const int r = e % n, c = e / n;
       Y[e] = c < ka ? va[c + (int64_t)r * Va.ld] : vb[(c - ka) + (int64_t)r * Vb.ld];
@@ -400,7 +415,7 @@ FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, dou
     }
     __syncthreads();
     // M (mu x mv) = Rc Rv^T
-    cta_gemm<double, OT>(mu, mv, kt, 1.0, Rc, mu, false, Rv, mv, true, 0.0, M, mu, gsm);
+    op_gemm<MANY>(mu, mv, kt, 1.0, Rc, mu, false, Rv, mv, true, 0.0, M, mu, gsm);
   } else {
     mu = kt;
     mv = kt;
@@ -415,13 +430,13 @@ FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, dou
     }
     __syncthreads();
     // Zu into Rc(0:ka, ka:kt), Yu = Ub - Ua Zu; same for V
-    cta_gemm<double, OT>(ka, kb, m, 1.0, X, m, true, X + (int64_t)ka * m, m, false, 0.0, Rc + (int64_t)ka * kt, kt,
+    op_gemm<MANY>(ka, kb, m, 1.0, X, m, true, X + (int64_t)ka * m, m, false, 0.0, Rc + (int64_t)ka * kt, kt,
                          gsm);
-    cta_gemm<double, OT>(m, kb, ka, -1.0, X, m, false, Rc + (int64_t)ka * kt, kt, false, 1.0, X + (int64_t)ka * m, m,
+    op_gemm<MANY>(m, kb, ka, -1.0, X, m, false, Rc + (int64_t)ka * kt, kt, false, 1.0, X + (int64_t)ka * m, m,
                          gsm);
-    cta_gemm<double, OT>(ka, kb, n, 1.0, Y, n, true, Y + (int64_t)ka * n, n, false, 0.0, Rv + (int64_t)ka * kt, kt,
+    op_gemm<MANY>(ka, kb, n, 1.0, Y, n, true, Y + (int64_t)ka * n, n, false, 0.0, Rv + (int64_t)ka * kt, kt,
                          gsm);
-    cta_gemm<double, OT>(n, kb, ka, -1.0, Y, n, false, Rv + (int64_t)ka * kt, kt, false, 1.0, Y + (int64_t)ka * n, n,
+    op_gemm<MANY>(n, kb, ka, -1.0, Y, n, false, Rv + (int64_t)ka * kt, kt, false, 1.0, Y + (int64_t)ka * n, n,
                          gsm);
     cta_householder_qr(m, kb, X + (int64_t)ka * m, m, tu, red);
     cta_householder_qr(n, kb, Y + (int64_t)ka * n, n, tv, red);
@@ -435,10 +450,10 @@ FRANK_D void lr_add_large_body(int m, int n, int kmax, int fast, double eps, dou
     }
     __syncthreads();
     // M = Rc blockdiag(Sa, Sb) Rv^T, through T = Rc blockdiag(Sa, Sb) (kt x kt)
-    cta_gemm<double, OT>(kt, ka, ka, 1.0, Rc, kt, false, sa, Sa.ld, false, 0.0, T, kt, gsm);
-    cta_gemm<double, OT>(kt, kb, kb, 1.0, Rc + (int64_t)ka * kt, kt, false, sb, Sb.ld, false, 0.0,
+    op_gemm<MANY>(kt, ka, ka, 1.0, Rc, kt, false, sa, Sa.ld, false, 0.0, T, kt, gsm);
+    op_gemm<MANY>(kt, kb, kb, 1.0, Rc + (int64_t)ka * kt, kt, false, sb, Sb.ld, false, 0.0,
                          T + (int64_t)ka * kt, kt, gsm);
-    cta_gemm<double, OT>(kt, kt, kt, 1.0, T, kt, false, Rv, kt, true, 0.0, M, kt, gsm);
+    op_gemm<MANY>(kt, kt, kt, 1.0, T, kt, false, Rv, kt, true, 0.0, M, kt, gsm);
   }
   const bool svd_ok = cta_svd(mu, mv, M, mu, Um, mu, sv, Vmt, min(mu, mv), sc, &flag);
   if (!svd_ok && threadIdx.x == 0) atomicAdd(err + OPS_ERR_JACOBI, 1);
@@ -525,28 +540,29 @@ struct LrShared {
   int rank;
 };
 
-// Scratch of one addition (doubles): per side the remainder's basis, the core
-// factors, T factors and the new basis.
+// Scratch of one addition (doubles) of joint rank kt: per side the factored basis (cols
+// columns: B's with the projected bases, the stacked ones otherwise), the core
+// factors, T factors and the new basis (at most kmax columns).
 struct LrLayout {
-  int64_t y[2], g[2], tf[2], tn[2], w[2], part[2], mtmp, x1, y1, aj, sig, total;
+  int64_t y[2], g[2], tf[2], tn[2], w[2], part[2], mtmp, x1, y1, sig, total;
 };
-FRANK_HD LrLayout lr_layout(int m, int n, int kt) {
+FRANK_HD LrLayout lr_layout(int m, int n, int kt, int cols, int kmax) {
   LrLayout L;
   int64_t o = 0;
   auto take = [&](int64_t c) { const int64_t r = o; o += (c + 31) & ~int64_t(31); return r; };
   for (int sd = 0; sd < 2; ++sd) {
     const int rows = sd ? n : m;
-    L.y[sd] = take((int64_t)rows * kt);
-    L.tn[sd] = take((int64_t)rows * kt);
+    L.y[sd] = take((int64_t)rows * cols);
+    L.tn[sd] = take((int64_t)rows * (kmax < kt ? kmax : kt));
     L.g[sd] = take((int64_t)kt * kt);
     L.tf[sd] = take((int64_t)((kt + GQ - 1) / GQ) * gt_chunks(rows) * GQ * GQ);
     L.w[sd] = take(2 * (int64_t)GQ * kt);
-    L.part[sd] = take(8 * (int64_t)kt * kt < G_PART ? 8 * (int64_t)kt * kt : G_PART);
+    // g_mm slices inner dimensions of 128 and more: the rows only (kt <= LR_KT_MAX)
+    L.part[sd] = take(rows < 128 ? 0 : (8 * (int64_t)kt * kt < G_PART ? 8 * (int64_t)kt * kt : G_PART));
   }
   L.mtmp = take((int64_t)kt * kt);
   L.x1 = take((int64_t)kt * kt);
   L.y1 = take((int64_t)kt * kt);
-  L.aj = take(2 * (int64_t)kt * kt);
   L.sig = take(2 * (int64_t)kt);
   L.total = o;
   return L;
@@ -585,8 +601,8 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
   const int hf = threadIdx.x >= LR_T / 2;
   const Grp half = grp_half(hf), all = grp_all();
   const int ka = *A.ka, kb = A.kb, kt = ka + kb, m = A.m, n = A.n;
-  const LrLayout L = lr_layout(m, n, kt);
   const bool fast = A.fast && A.eps == 0.0 && kt <= m && kt <= n;
+  const LrLayout L = lr_layout(m, n, kt, fast ? kb : kt, A.kmax);
   const int mu = fast ? kt : min(m, kt), mv = fast ? kt : min(n, kt), nsv = min(mu, mv);
   const int lane = threadIdx.x & 31;
   {
@@ -750,11 +766,12 @@ __global__ void __launch_bounds__(LR_T) k_op_lr_add(int m, int n, int kmax, int 
   lr_add_body(a, scratch + (int64_t)b * ws, err);
 }
 
-__global__ void __launch_bounds__(OT) k_op_lr_add_large(int m, int n, int kmax, int fast, double eps, Mat Ua, Mat Sa,
+template <bool MANY>
+__global__ void __launch_bounds__(OT, MANY ? 2 : 1) k_op_lr_add_large(int m, int n, int kmax, int fast, double eps, Mat Ua, Mat Sa,
                                                         Mat Va, int* ka_io, Mat Ub, Mat Sb, Mat Vb, const int* kb_in,
                                                         double* scratch, int64_t ws, int* err) {
   const int b = blockIdx.x;
-  lr_add_large_body(m, n, kmax, fast, eps, Ua.at(b), Ua.ld, Sa.at(b), Sa.ld, Va.at(b), Va.ld, ka_io + b, Ub.at(b),
+  lr_add_large_body<MANY>(m, n, kmax, fast, eps, Ua.at(b), Ua.ld, Sa.at(b), Sa.ld, Va.at(b), Va.ld, ka_io + b, Ub.at(b),
                     Ub.ld, Sb.at(b), Sb.ld, Vb.at(b), Vb.ld, kb_in[b], scratch + (int64_t)b * ws, err);
 }
 
@@ -774,7 +791,7 @@ __global__ void __launch_bounds__(LR_T) k_op_lr_add_tasks(const LrAddTask* tasks
 __global__ void __launch_bounds__(OT) k_op_lr_add_tasks_large(const LrAddTask* tasks, int kmax, int fast,
                                                               double* scratch, int* err) {
   const LrAddTask t = tasks[blockIdx.x];
-  lr_add_large_body(t.m, t.n, kmax, fast, 0.0, t.ua, t.ldua, t.sa, t.ldsa, t.va, t.ldva, t.ka, t.ub, t.ldub, t.sb,
+  lr_add_large_body<false>(t.m, t.n, kmax, fast, 0.0, t.ua, t.ldua, t.sa, t.ldsa, t.va, t.ldva, t.ka, t.ub, t.ldub, t.sb,
                     t.ldsb, t.vb, t.ldvb, *t.kb, scratch + t.scratch_off, err);
 }
 
@@ -904,8 +921,35 @@ int64_t lr_add_large_ws(int m, int n, int kt) {
   return (int64_t)(m + n) * kt + 2 * kt + 5 * (int64_t)kt * kt + kt + (int64_t)mx * kt + svd_scratch(kt, kt) + 2;
 }
 
-int64_t lr_add_ws(int m, int n, int ka, int kb) {
-  return ka + kb <= LR_KT_MAX ? lr_layout(m, n, ka + kb).total : lr_add_large_ws(m, n, ka + kb);
+int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Whether `count` additions of joint rank kt take one addition per SM at a time
+// (lr_add_body, 512 threads) or several of 256 threads (lr_add_large_body), which
+// take longer each: ranks above LR_KT_MAX, and more additions than SMs of blocks and
+// ranks that leave most of 512 threads idle (the stacked bases of rounded additions
+// do a little more work per thread in the second).  B200, 1024 additions, us, one and
+// several per SM: projected, 64 x 64, joint rank 8 718 and 691, 16 1704 and 1770; 256 x
+// 256, joint rank 16 2593 and 3130; rounded, 64 x 64, joint rank 8 949 and 629; 256 x
+// 256, joint rank 16 3380 and 3001; 1024 x 1024 7548 and 8446; 148 additions of 64 x 64,
+// joint rank 16: 301 and 473.
+bool lr_add_one_per_sm(int m, int n, int kt, int count, bool projected) {
+  const bool small = kt <= 16 && std::max(m, n) <= (projected ? 128 : 256);
+  return kt <= LR_KT_MAX && !(small && count > sm_count());
+}
+
+// Batches of rsvd / rid that take the variants for many small blocks: 512 blocks of
+// 64 x 64 at rank 8 1020 us and 1260 without, 256 x 256 4100 and 2710.
+bool many_small(int m, int n, int count) { return (int64_t)m * n <= 128 * 128 && count > sm_count(); }
+
+// Scratch of an addition of ranks up to kmax and kb by either algorithm.
+int64_t lr_add_ws(int m, int n, int kmax, int kb) {
+  const int kt = kmax + kb;
+  return kt <= LR_KT_MAX ? lr_layout(m, n, kt, kt, kmax).total : lr_add_large_ws(m, n, kt);
 }
 
 void launch_gemm(cudaStream_t s, int m, int n, int k, int count, double alpha, const double* a, int64_t lda,
@@ -1052,8 +1096,9 @@ int frank_rsvd_batched(int m, int n, int count, int rank, int oversample, int po
   const int64_t ws = (int64_t)m * smp + (int64_t)std::max(m, n) * smp + (int64_t)n * smp + smp + (int64_t)smp * smp +
                      smp + (int64_t)smp * n + svd_scratch(smp, n) + 2;
   rc = run(s, count, ws, [&](double* sc, int* err) {
-    k_op_rsvd<<<count, OT, 0, s>>>(m, n, smp, rank, power_its, Mat{const_cast<double*>(d_a), lda, sa}, d_om,
-                                   Mat{d_u, ldu, su}, Mat{d_s, lds, ss}, Mat{d_v, ldv, sv}, sc, ws, err);
+    (many_small(m, n, count) ? k_op_rsvd<true> : k_op_rsvd<false>)<<<count, OT, 0, s>>>(
+        m, n, smp, rank, power_its, Mat{const_cast<double*>(d_a), lda, sa}, d_om, Mat{d_u, ldu, su}, Mat{d_s, lds, ss},
+        Mat{d_v, ldv, sv}, sc, ws, err);
   });
   cudaFreeAsync(d_om, s);
   cudaStreamSynchronize(s);
@@ -1095,8 +1140,9 @@ int frank_rid_batched(int m, int n, int count, int sample, int k, const double* 
                      3 * (int64_t)sample * k + 2 * (int64_t)k + 2 + (int64_t)mx * mx + 4 * (int64_t)mx +
                      (int64_t)k * mx + mx + 4;
   rc = run(s, count, ws, [&](double* sc, int*) {
-    k_op_rid<<<count, OT, 0, s>>>(m, n, sample, k, Mat{const_cast<double*>(d_a), lda, sa}, d_om, Mat{d_u, ldu, su},
-                                  Mat{d_s, lds, ss}, Mat{d_v, ldv, sv}, sc, ws);
+    (many_small(m, n, count) ? k_op_rid<true> : k_op_rid<false>)<<<count, OT, 0, s>>>(
+        m, n, sample, k, Mat{const_cast<double*>(d_a), lda, sa}, d_om, Mat{d_u, ldu, su}, Mat{d_s, lds, ss},
+        Mat{d_v, ldv, sv}, sc, ws);
   });
   cudaFreeAsync(d_om, s);
   cudaStreamSynchronize(s);
@@ -1141,7 +1187,7 @@ static int lowrank_add_naive(int m, int n, int count, int kmax, double* d_ua, in
     const int64_t ws = (int64_t)m * smp + (int64_t)std::max(m, n) * smp + (int64_t)n * smp + smp +
                        (int64_t)smp * smp + smp + (int64_t)smp * n + svd_scratch(smp, n) + 2;
     int rc = run(s, 1, ws, [&](double* sc, int* err) {
-      k_op_rsvd<<<1, OT, 0, s>>>(m, n, smp, rank, 0, Mat{d_dense, m, 0}, d_om, Mat{d_ua + b * sua, ldua, 0},
+      k_op_rsvd<false><<<1, OT, 0, s>>>(m, n, smp, rank, 0, Mat{d_dense, m, 0}, d_om, Mat{d_ua + b * sua, ldua, 0},
                                  Mat{d_sa + b * ssa, ldsa, 0}, Mat{d_va + b * sva, ldva, 0}, sc, ws, err);
     });
     cudaFreeAsync(d_om, s);
@@ -1174,17 +1220,21 @@ int frank_lowrank_add_batched(int m, int n, int count, int kmax, const char* lra
   else return set_error(FRANK_ERR_UNSUPPORTED, "lowrank_add: unknown LowRank addition " + name);
   // ranks of a pair are at most kmax and kb_max: the bound picks the kernel
   const int kt = kmax + kb_max;
+  const bool projected = fast && eps == 0.0 && kt <= m && kt <= n;   // then so for the ranks themselves
+  const bool one = lr_add_one_per_sm(m, n, kt, count, projected);
   const Mat ua{d_ua, ldua, sua}, sa{d_sa, ldsa, ssa}, va{d_va, ldva, sva};
   const Mat ub{const_cast<double*>(d_ub), ldub, sub}, sb{const_cast<double*>(d_sb), ldsb, ssb},
       vb{const_cast<double*>(d_vb), ldvb, svb};
-  const int64_t ws = lr_add_ws(m, n, kmax, kb_max);
-  if (kt <= LR_KT_MAX && (rc = lr_add_prepare())) return rc;
+  const int64_t ws = one ? lr_layout(m, n, kt, projected ? kb_max : kt, kmax).total : lr_add_large_ws(m, n, kt);
+  if (one && (rc = lr_add_prepare())) return rc;
   return run(s, count, ws, [&](double* sc, int* err) {
-    if (kt <= LR_KT_MAX)
+    if (one)
       k_op_lr_add<<<count, LR_T, sizeof(LrShared) + 8 * lr_region(m, n, kt), s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka,
                                                                                   ub, sb, vb, d_kb, sc, ws, err);
+    else if (kt <= LR_KT_MAX)
+      k_op_lr_add_large<true><<<count, OT, 0, s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka, ub, sb, vb, d_kb, sc, ws, err);
     else
-      k_op_lr_add_large<<<count, OT, 0, s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka, ub, sb, vb, d_kb, sc, ws, err);
+      k_op_lr_add_large<false><<<count, OT, 0, s>>>(m, n, kmax, fast, eps, ua, sa, va, d_ka, ub, sb, vb, d_kb, sc, ws, err);
   });
 }
 
