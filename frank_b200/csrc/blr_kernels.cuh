@@ -1473,8 +1473,8 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
   auto take = [&](int64_t n) { int64_t r = o; o += (n + 31) & ~int64_t(31); return r; };
   const int mu = smax < bmax ? smax : bmax;
   const int64_t np = bmax / recomp_panel(bmax) + 1;
-  L.ash = take((int64_t)bmax * smax);
-  L.bsh = take((int64_t)bmax * smax);
+  L.ash = take((int64_t)panel_ld(bmax) * smax);
+  L.bsh = take((int64_t)panel_ld(bmax) * smax);
   L.t = take((int64_t)bmax * bmax);
   L.gu = take((int64_t)mu * smax);
   L.gv = take((int64_t)mu * smax);
@@ -1618,10 +1618,12 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
       const RecompSide<T>& d = tk.s[sd];
       double* smP = region + (tk.side >= 0 ? 0 : hf * (RECOMP_REGION / 2));
       const int kc = tk.kc, bb = d.bb, cols = tk.proj ? d.pp : kc + d.pp;
-      // the whole side in shared memory where it fits, else panel by panel
+      // the whole side in shared memory where it fits, else panel by panel; the leading
+      // dimension is the same, so that the products take the same loads and sums (a
+      // split target has twice the shared memory for a side)
       const bool sm = panel_ld(bb) * cols <= (tk.side >= 0 ? RECOMP_REGION : RECOMP_REGION / 2);
       double* Y = sm ? smP : d.S;
-      const int ldy = sm ? panel_ld(bb) : bb;
+      const int ldy = panel_ld(bb);
       for (int c = g.wid; c < cols; c += g.nw) {
         const int cx = tk.proj ? c : c - kc;
         const T* src = cx < 0 ? d.C + (int64_t)c * ld : d.X + (d.xt ? (int64_t)cx : (int64_t)cx * ld);
@@ -1631,7 +1633,7 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
       }
       g.sync();
       if (tk.proj) g_project_out(g, bb, kc, d.pp, (const T*)d.C, 1, ld, Y, ldy, d.G, kc + d.pp, d.Z2, d.x);
-      g_qr(g, bb, cols, Y, ldy, d.S, bb, d.G + (tk.proj ? kc : 0), tk.proj ? kc + d.pp : d.mm, d.Tf, wp,
+      g_qr(g, bb, cols, Y, ldy, d.S, ldy, d.G + (tk.proj ? kc : 0), tk.proj ? kc + d.pp : d.mm, d.Tf, wp,
            sm ? nullptr : smP, sh.gs[sd], d.x);
     }
     __syncthreads();
@@ -1776,7 +1778,7 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
 #pragma unroll 4
         for (int e = lane; e < bb; e += 32) d.Tn[e + c * bb] = e < refl ? X[skip + e + c * mm] : 0.0;
       half.sync();
-      g_apply_q(half, bb, refl, d.S, bb, d.Tf, wp, r, d.Tn, bb, refl, d.x);
+      g_apply_q(half, bb, refl, d.S, panel_ld(bb), d.Tf, wp, r, d.Tn, bb, refl, d.x);
       if (tk.proj) g_mm(half, bb, r, skip, 1.0, (const T*)d.C, 1, ld, X, mm, 1, 1.0, d.Tn, bb, d.x.part);
       for (int c = half.wid; c < r; c += half.nw)
 #pragma unroll 4

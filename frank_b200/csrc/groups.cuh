@@ -49,9 +49,11 @@ struct GrpShared {
 // each operand row is read once per tile and the warps have equal work; the
 // eight partial products go to part (G_PART doubles, in L2) and are summed in
 // order.  Otherwise a tile per warp with the whole inner dimension.  Tile shapes
-// are the ones with the fewest tensor-pipe cycles; neither choice changes the
-// order in which an element is summed, and the slices do not depend on the
-// group's size, so results do not depend on it either.
+// are the ones with the fewest tensor-pipe cycles and do not change the order in
+// which an element is summed.  That order depends on the sizes, and in a slice on
+// whether both operands are 16-byte aligned, not on the group's size (from eight
+// warps) or on where the operands lie; callers give a matrix the same leading
+// dimension wherever they put it.
 constexpr int G_SLICE_TILES = 81;            // 8 x 8 tiles of a sliced output
 constexpr int G_PART = 8 * 64 * G_SLICE_TILES;
 
