@@ -433,15 +433,17 @@ def sample_inputs():
     return x, b
 
 
+REFERENCE = os.path.join(ROOT, "oracle", "_ref", "frank_ref")
+REFERENCE_MISSING = "oracle/_ref/frank_ref is not built (python oracle/build_ref.py, from the reference's sources)"
+
+
 def run_reference_sample(steps, warmup, threads):
     """The reference itself (FRANK's C++ compiled into oracle/_ref, on scipy's
     OpenBLAS with `threads` threads) on the sample: A_H built once, then
     warmup + steps factorizations of fresh copies of it, each followed by
     the two block substitutions; returns the per-step getrf + solve times
     (its own std::chrono timings, examples/h_lu.cpp:40-48) and its output."""
-    exe = os.path.join(ROOT, "oracle", "_ref", "frank_ref")
-    if not os.path.exists(exe):
-        raise SystemExit("oracle/_ref/frank_ref is missing: build it with python oracle/build_ref.py")
+    exe = REFERENCE
     x, b = sample_inputs()
     with tempfile.TemporaryDirectory() as wd:
         px, pb = os.path.join(wd, "pts.bin"), os.path.join(wd, "rhs.bin")
@@ -459,8 +461,12 @@ def run_reference_sample(steps, warmup, threads):
 def bench_reference(args, rank, world):
     """--impl reference: rank 0 runs the reference's own factor + solve on the
     bounded sample (unscaled; the full N=32768 workload takes tens of minutes
-    of host time), other ranks exit without work."""
+    of host time), other ranks exit without work.  Where the reference is not
+    built, the line says so."""
     if rank != 0:
+        return
+    if not os.path.exists(REFERENCE):
+        print(json.dumps({"impl": "reference", "unavailable": REFERENCE_MISSING}), flush=True)
         return
     cores = os.cpu_count()
     t, info = run_reference_sample(max(1, args.steps), args.warmup, cores)
@@ -803,8 +809,8 @@ def main():
                 line["hlu"] = run_hlu(131072, args.steps, max(args.warmup, 3))
             except Exception as exc:  # reported, never silently dropped
                 line["hlu"] = {"error": str(exc)}
-        if not args.no_cpu_baseline and not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "frank_ref")):
-            line["cpu_baseline"] = {"unavailable": "oracle/_ref/frank_ref is not built (python oracle/build_ref.py)"}
+        if not args.no_cpu_baseline and not os.path.exists(REFERENCE):
+            line["cpu_baseline"] = {"unavailable": REFERENCE_MISSING}
         elif not args.no_cpu_baseline:
             cores = os.cpu_count()
             t, info = run_reference_sample(3, 1, cores)
