@@ -218,7 +218,10 @@ FRANK_D void warp_sums(double (&v)[N]) {
 // reciprocal (every warp forms them, so the FP64 pipe pays for each): with
 // h = |alpha| + ||x||, tau = h / ||x|| and scal = sign / h.
 FRANK_D void reflector(double alpha, double n2, double& beta, double& tau, double& scal) {
-  const double rn = rsqrt(n2), nrm = n2 * rn, aa = fabs(alpha);
+  double rn = rsqrt(n2), nrm = n2 * rn;
+  const double aa = fabs(alpha);
+  nrm = fma(0.5 * rn, fma(-nrm, nrm, n2), nrm);   // a Newton step each: both to half a unit in the last
+  rn = fma(rn, fma(-nrm, rn, 1.0), rn);           // place, on which H's orthogonality rests
   const double rh = __drcp_rn(aa + nrm);
   beta = alpha >= 0.0 ? -nrm : nrm;
   tau = fma(aa, rn, 1.0);
@@ -946,7 +949,10 @@ static __device__ __noinline__ int g_jacobi(Grp g, int m, int n, double* G, int6
         const double zeta = (b - a) / (2.0 * h);
         const double za = fabs(zeta), zc = fmin(za, 1e100), u = fma(zc, zc, 1.0);
         const double t = copysign(__drcp_rn(za + u * rsqrt(u)), zeta);
-        const double c = rsqrt(fma(t, t, 1.0)), s = c * t;
+        const double f = fma(t, t, 1.0);
+        double c = rsqrt(f);
+        c = fma(0.5 * c, fma(-f * c, c, 1.0), c);
+        const double s = c * t;
 #pragma unroll 4
         for (int i = l8; i < m_rot; i += 8) {
           const double x = gp[i], y = gq[i];
