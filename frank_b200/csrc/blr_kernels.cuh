@@ -1291,7 +1291,13 @@ constexpr int RECOMP_THREADS = 512;
 constexpr int SPLIT_P = 32;       // split band-1 targets whose operand rank exceeds this (default)
 constexpr int SPLIT_MAX = 128;    // band-1 tasks eligible for the split (scratch slots)
 constexpr int RECOMP_BMAX = 810;  // largest block order (a panel of each side in shared memory)
-constexpr int RECOMP_SMEM_BYTES = 194 * 1024;    // dynamic shared memory (all but the static part)
+// Dynamic shared memory.  What it leaves of an SM's 256 KB is the L1 that the
+// products' operands and the spills live on: with 226 KB the factorization of n = 8192
+// at 1e-8 takes 322 ms, with 194 KB 282.  Cores up to about 141 x 141 fit with the panel
+// of their RQ and take column-by-column pivoting (up to about 160 did in 226 KB, before
+// that panel had to fit too); larger ones take randomized block pivoting, whose ranks
+// can differ by a few at the same stopping rule.
+constexpr int RECOMP_SMEM_BYTES = 194 * 1024;
 
 struct RecompShared {
   GrpShared gs[2];               // one per half of the CTA
@@ -1502,8 +1508,7 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
 
 // One target's operands and scratch, in shared memory: the phases below are
 // long and inlined, and values kept in registers across all of them would
-// spill to local memory (beside 226 KB of shared memory there is no L1 left to
-// hold spills).
+// spill to local memory, which beside RECOMP_SMEM_BYTES has some 30 KB of L1.
 template <typename T>
 struct RecompSide {
   const T* X;                  // update basis (XL or YR)

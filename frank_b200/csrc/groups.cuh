@@ -203,15 +203,6 @@ FRANK_D void g_mm(const Grp& g, int m, int n, int k, double alpha, const TA* A, 
   g.sync();
 }
 
-// Sums of v[0..N) over the warp (every lane gets them).
-template <int N>
-FRANK_D void warp_sums(double (&v)[N]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-}
-
 // Householder reflector (dlarfg) of a column with leading entry alpha and
 // squared norm n2 = alpha^2 + (squared norm below it): v = [1; x scal],
 // H = I - tau v v^T, H x = beta e_1.  One reciprocal square root and one
@@ -353,7 +344,6 @@ static __device__ __noinline__ void panel_qr_rows(Grp g, int m, int n, const dou
 }
 
 // Widest panel of m rows: 16 columns of up to two rows a thread, 8 of up to four.
-constexpr int G_ROWS_MAX = 1024;
 FRANK_HD int panel_width(int m) { return m <= 512 ? 16 : 8; }
 
 FRANK_D void g_panel_qr(const Grp& g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,

@@ -37,7 +37,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
-#include <cooperative_groups.h>
 
 #include <algorithm>
 
@@ -54,7 +53,6 @@ namespace blr = frank_blr_private;
 #include "../../include/frank_b200.h"
 #include "ops_tasks.h"
 
-#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <random>
