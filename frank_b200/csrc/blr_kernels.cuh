@@ -1469,6 +1469,11 @@ FRANK_D int svd_core(int mu, int mv, double* Mm, int ldm, bool in_smem, const Fa
   return r;
 }
 
+// Leading dimension of a side's scratch: 16-byte aligned columns, as in shared
+// memory, so that the products take the same loads and sums in both (a split
+// target has twice the shared memory for a side).
+FRANK_HD int side_ld(int rows) { return (rows + 1) & ~1; }
+
 struct RecompLayout {
   int64_t ash, bsh, t, gu, gv, mtmp, mglob, y1, tv, tfu, tfv, tfc, tfr, om, w, part, tau_c, sig, cn, pn, jp, ji, total;
 };
@@ -1479,8 +1484,8 @@ FRANK_HD RecompLayout recomp_layout(int bmax, int smax) {
   auto take = [&](int64_t n) { int64_t r = o; o += (n + 31) & ~int64_t(31); return r; };
   const int mu = smax < bmax ? smax : bmax;
   const int64_t np = bmax / recomp_panel(bmax) + 1;
-  L.ash = take((int64_t)panel_ld(bmax) * smax);
-  L.bsh = take((int64_t)panel_ld(bmax) * smax);
+  L.ash = take((int64_t)side_ld(bmax) * smax);
+  L.bsh = take((int64_t)side_ld(bmax) * smax);
   L.t = take((int64_t)bmax * bmax);
   L.gu = take((int64_t)mu * smax);
   L.gv = take((int64_t)mu * smax);
@@ -1623,12 +1628,10 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
       const RecompSide<T>& d = tk.s[sd];
       double* smP = region + (tk.side >= 0 ? 0 : hf * (RECOMP_REGION / 2));
       const int kc = tk.kc, bb = d.bb, cols = tk.proj ? d.pp : kc + d.pp;
-      // the whole side in shared memory where it fits, else panel by panel; the leading
-      // dimension is the same, so that the products take the same loads and sums (a
-      // split target has twice the shared memory for a side)
+      // the whole side in shared memory where it fits, else panel by panel
       const bool sm = panel_ld(bb) * cols <= (tk.side >= 0 ? RECOMP_REGION : RECOMP_REGION / 2);
       double* Y = sm ? smP : d.S;
-      const int ldy = panel_ld(bb);
+      const int ldy = sm ? panel_ld(bb) : side_ld(bb);
       for (int c = g.wid; c < cols; c += g.nw) {
         const int cx = tk.proj ? c : c - kc;
         const T* src = cx < 0 ? d.C + (int64_t)c * ld : d.X + (d.xt ? (int64_t)cx : (int64_t)cx * ld);
@@ -1638,7 +1641,7 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
       }
       g.sync();
       if (tk.proj) g_project_out(g, bb, kc, d.pp, (const T*)d.C, 1, ld, Y, ldy, d.G, kc + d.pp, d.Z2, d.x);
-      g_qr(g, bb, cols, Y, ldy, d.S, ldy, d.G + (tk.proj ? kc : 0), tk.proj ? kc + d.pp : d.mm, d.Tf, wp,
+      g_qr(g, bb, cols, Y, ldy, d.S, side_ld(bb), d.G + (tk.proj ? kc : 0), tk.proj ? kc + d.pp : d.mm, d.Tf, wp,
            sm ? nullptr : smP, sh.gs[sd], d.x);
     }
     __syncthreads();
@@ -1783,7 +1786,7 @@ FRANK_D void k_recompress_impl(const BlrView<T>& A, const FactorWs<T>& ws, int i
 #pragma unroll 4
         for (int e = lane; e < bb; e += 32) d.Tn[e + c * bb] = e < refl ? X[skip + e + c * mm] : 0.0;
       half.sync();
-      g_apply_q(half, bb, refl, d.S, panel_ld(bb), d.Tf, wp, r, d.Tn, bb, refl, d.x);
+      g_apply_q(half, bb, refl, d.S, side_ld(bb), d.Tf, wp, r, d.Tn, bb, refl, d.x);
       if (tk.proj) g_mm(half, bb, r, skip, 1.0, (const T*)d.C, 1, ld, X, mm, 1, 1.0, d.Tn, bb, d.x.part);
       for (int c = half.wid; c < r; c += half.nw)
 #pragma unroll 4
@@ -2705,7 +2708,7 @@ static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<
   if (threadIdx.x == 0) {
     if (lr) {
       seg[0].set(tr ? H.u(gi, gj) : H.vt(gi, gj), ld, bj, r, MV_T, sm.x, ldb, sm.t1, ldr);
-      seg[1].set(H.s(gi, gj), H.kcap, r, r, tr ? MV_T64 : MV_N64, sm.t1, ldr, sm.x, ldr);
+      seg[1].set(H.s(gi, gj), H.kcap, r, r, tr ? MV_T : MV_N64, sm.t1, ldr, sm.x, ldr);
       seg[2].set(tr ? H.vt(gi, gj) : H.u(gi, gj), ld, bi, r, nk, sm.x, ldr, nullptr, 0);
     } else if (tr) {
       seg[0].set(H.dense(gi, gj), ld, bj, bi, MV_T, sm.x, ldb, nullptr, 0);
@@ -2714,7 +2717,7 @@ static __global__ void __launch_bounds__(SOLVE_THREADS) k_matvec_blocks(BlrView<
     }
   }
   __syncthreads();
-  mv_run<1 << MV_T | 1 << MV_T64 | 1 << MV_N64 | 1 << MV_N512>(
+  mv_run<1 << MV_T | 1 << MV_N64 | 1 << MV_N512>(
       seg, lr ? 3 : 1, nrhs, sm.ring, ns, sm.red, [&]() { sv_stage(sm.x, ldb, x + H.off[j], ldx, bj, nrhs); },
       [&](int row, int c, double v) { out[row + (int64_t)c * ld] = v; });
 }

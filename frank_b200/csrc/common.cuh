@@ -257,9 +257,12 @@ FRANK_D void warps_dgemm(int wid, int nw, int m, int n, int k, double alpha, con
 #pragma unroll
       for (int j = 0; j < NI; ++j) {
         const int c = j0 + 8 * j + 2 * t;
-        TC* p = C + r + (int64_t)c * ldc;
-        if (c < n) dgemm_store(p, acc[i][j][0], alpha, UNIT ? 0.0 : beta);
-        if (c + 1 < n) dgemm_store(p + ldc, acc[i][j][1], alpha, UNIT ? 0.0 : beta);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (c + h >= n) continue;
+          if (UNIT) C[r + (int64_t)(c + h) * ldc] = TC(alpha * acc[i][j][h]);
+          else dgemm_store(C + r + (int64_t)(c + h) * ldc, acc[i][j][h], alpha, beta);
+        }
       }
     }
   }

@@ -52,8 +52,8 @@ struct GrpShared {
 // are the ones with the fewest tensor-pipe cycles and do not change the order in
 // which an element is summed.  That order depends on the sizes, and in a slice on
 // whether both operands are 16-byte aligned, not on the group's size (from eight
-// warps) or on where the operands lie; callers give a matrix the same leading
-// dimension wherever they put it.
+// warps) or on where the operands lie; callers align a matrix the same way wherever
+// they put it.
 constexpr int G_SLICE_TILES = 81;            // 8 x 8 tiles of a sliced output
 constexpr int G_PART = 8 * 64 * G_SLICE_TILES;
 
@@ -208,11 +208,18 @@ FRANK_D void g_mm(const Grp& g, int m, int n, int k, double alpha, const TA* A, 
 // H = I - tau v v^T, H x = beta e_1.  One reciprocal square root and one
 // reciprocal (every warp forms them, so the FP64 pipe pays for each): with
 // h = |alpha| + ||x||, tau = h / ||x|| and scal = sign / h.
+// FINE: a Newton step each on the norm and its reciprocal, to half a unit in the last
+// place, on which H's orthogonality rests.  The additions of single blocks, whose
+// results are the factors themselves, take it (2 to 5 % closer to 64 bits); a
+// factorization does not show it and would take 3 % longer (n = 8192 at 1e-8).
+template <bool FINE>
 FRANK_D void reflector(double alpha, double n2, double& beta, double& tau, double& scal) {
   double rn = rsqrt(n2), nrm = n2 * rn;
   const double aa = fabs(alpha);
-  nrm = fma(0.5 * rn, fma(-nrm, nrm, n2), nrm);   // a Newton step each: both to half a unit in the last
-  rn = fma(rn, fma(-nrm, rn, 1.0), rn);           // place, on which H's orthogonality rests
+  if (FINE) {
+    nrm = fma(0.5 * rn, fma(-nrm, nrm, n2), nrm);
+    rn = fma(rn, fma(-nrm, rn, 1.0), rn);
+  }
   const double rh = __drcp_rn(aa + nrm);
   beta = alpha >= 0.0 ? -nrm : nrm;
   tau = fma(aa, rn, 1.0);
@@ -230,7 +237,7 @@ FRANK_D void reflector(double alpha, double n2, double& beta, double& tau, doubl
 // 51 us; 3.3 us a column).  On return V (clean, unit lower trapezoid, ldv)
 // holds the reflectors (V may be P), s.T the T factor (upper, zero below) and
 // R (n x n, ldr) the triangle with zeros below its diagonal.
-template <int W, int RPT>
+template <int W, int RPT, bool FINE>
 static __device__ __noinline__ void panel_qr_rows(Grp g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
                            int64_t ldr, GrpShared& s) {
   const int lane = threadIdx.x & 31;
@@ -292,7 +299,7 @@ static __device__ __noinline__ void panel_qr_rows(Grp g, int m, int n, const dou
       const double dot = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
       const double alpha = __shfl_sync(0xffffffffu, top, j), xn2 = __shfl_sync(0xffffffffu, dot, j);
       double beta = alpha, tau = 0.0, scal = 0.0;
-      if (xn2 > 0.0) reflector(alpha, fma(alpha, alpha, xn2), beta, tau, scal);
+      if (xn2 > 0.0) reflector<FINE>(alpha, fma(alpha, alpha, xn2), beta, tau, scal);
       const double w = fma(scal, dot, top);
       if (lane < j) s.G[lane + j * GQ] = s.scal[lane] * w;
       else if (lane == j) { s.tau[j] = tau; s.beta[j] = beta; s.scal[j] = scal; }
@@ -346,11 +353,12 @@ static __device__ __noinline__ void panel_qr_rows(Grp g, int m, int n, const dou
 // Widest panel of m rows: 16 columns of up to two rows a thread, 8 of up to four.
 FRANK_HD int panel_width(int m) { return m <= 512 ? 16 : 8; }
 
+template <bool FINE = false>
 FRANK_D void g_panel_qr(const Grp& g, int m, int n, const double* P, int64_t ldp, double* V, int64_t ldv, double* R,
                         int64_t ldr, GrpShared& s) {
-  if (m > 512) panel_qr_rows<8, 4>(g, m, n, P, ldp, V, ldv, R, ldr, s);
-  else if (m > 256) panel_qr_rows<16, 2>(g, m, n, P, ldp, V, ldv, R, ldr, s);
-  else panel_qr_rows<16, 1>(g, m, n, P, ldp, V, ldv, R, ldr, s);
+  if (m > 512) panel_qr_rows<8, 4, FINE>(g, m, n, P, ldp, V, ldv, R, ldr, s);
+  else if (m > 256) panel_qr_rows<16, 2, FINE>(g, m, n, P, ldp, V, ldv, R, ldr, s);
+  else panel_qr_rows<16, 1, FINE>(g, m, n, P, ldp, V, ldv, R, ldr, s);
 }
 
 FRANK_HD int panel_ld(int m) { return ((m + 15) & ~15) + 4; }   // 4 mod 16: conflict-free fragments
@@ -472,9 +480,9 @@ FRANK_D void g_qr_tall(const Grp& g, int m, int n, double* A, int64_t lda, doubl
           for (int r = lane; r < cr; r += 32) smP[jn + r + c * ldp] = Ac[r + (int64_t)c * lda];
         }
         g.sync();
-        g_panel_qr(g, jn + cr, jn, smP, ldp, smP, ldp, Rp, ldr, s);
+        g_panel_qr<true>(g, jn + cr, jn, smP, ldp, smP, ldp, Rp, ldr, s);
       } else {
-        g_panel_qr(g, cr, jn, Ac, lda, smP, ldp, Rp, ldr, s);
+        g_panel_qr<true>(g, cr, jn, Ac, lda, smP, ldp, Rp, ldr, s);
       }
       double* T = Tf + (int64_t)(p * nch + i) * GQ * GQ;
       for (int c = g.wid; c < jn; c += g.nw)
@@ -556,6 +564,7 @@ FRANK_D void warp_argmax_key(double& v, int& idx) {
 // row j and the scaled reflector below; every other column its rows of R.
 // cand: 4 * nw doubles (two rows of values and indices); vec: 2 min(m, n)
 // doubles.  All shared.
+template <bool FINE = false>
 FRANK_D int g_rrqr(const Grp& g, int m, int n, double* A, int lda, double thr, int maxr, double* tau,
                                    int* ord, int* at, double* vec, double* cand) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7;
@@ -593,7 +602,7 @@ FRANK_D int g_rrqr(const Grp& g, int m, int n, double* A, int lda, double thr, i
     const double* x = A + kp * lda;
     const double alpha = x[r];
     double bt = 0.0, t = 0.0, sc = 0.0;
-    if (mx > 0.0) reflector(alpha, mx, bt, t, sc);
+    if (mx > 0.0) reflector<FINE>(alpha, mx, bt, t, sc);
     bv = -1.0;
     bi = -1;
     for (int c0 = 0; c0 < n; c0 += ng) {

@@ -669,7 +669,7 @@ FRANK_D void lr_add_body(const LrArgs& A, double* scratch, int* err) {
     // the result is NaN (the pivoted QR passes over columns that are not numbers)
     for (int e = threadIdx.x; e < mu * mv; e += blockDim.x) bad |= !isfinite(M[e % mu + (e / mu) * ldm]);
     bad = __syncthreads_or(bad);
-    k = g_rrqr(all, mu, mv, M, ldm, 0.0, nsv, tau, ord, at, tau + nsv, cand);
+    k = g_rrqr<true>(all, mu, mv, M, ldm, 0.0, nsv, tau, ord, at, tau + nsv, cand);
     Aj = cand + 4 * (LR_T / 32) + (nsv + mv + 2) / 2;
     ldj = mv + k;
     for (int e = threadIdx.x; e < ldj * k; e += blockDim.x) {
