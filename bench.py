@@ -530,7 +530,7 @@ def run_ours_sample(stream, steps):
 # capture whole).  The roofline's `traffic` scales it to the mean headline
 # launch by the FLOPs that launch performs
 # (profiles/k_recompress_blr_laplace3d_n8192.md).
-RECOMP_BYTES_PER_FLOP = 1.071e9 / 4.695e10
+RECOMP_BYTES_PER_FLOP = 1.095e9 / 4.695e10
 
 
 def profile_case(name):

@@ -2154,8 +2154,9 @@ constexpr int SMEM_OPTIN_MAX = 226 * 1024;   // dynamic shared memory a CTA may 
 // matvec, the latency of 2 nb dependent steps the solve.  Loads into registers
 // left too few bytes in flight (one warp instruction in 17 cycles a scheduler,
 // 1.0 TB/s; n = 16384, b = 512, 4 right-hand sides: matvec 452 us, 325 through
-// the ring; refinement 15.1 ms to 7.4), so a CTA streams its matrices as boxes through a ring in
-// shared memory (cp.async, two boxes ahead, also over the seams between
+// the ring; 8 right-hand sides: refinement 15.1 ms, 7.4 through the ring and 6.3
+// with launches that overlap), so a CTA streams its matrices as boxes through a
+// ring in shared memory (cp.async, two boxes ahead, also over the seams between
 // products) and multiplies them on the tensor pipe with the right-hand sides as
 // the columns.  MV_T, MV_T64: out = A^T X, boxes of 256 x 16 and 56 x 64 (rows x
 // columns; the second for matrices of few rows: eight outputs a warp and no sum
